@@ -42,9 +42,10 @@ _SIGNATURES = {
     },
     "gemm_simple": {
         "oe_gemm_simple": [_P, _P, _P, _I, _I, _I, _L, _L, _I, _P],
+        "oe_gemm_simple_kind_f32": [_P, _P, _P, _I, _I, _I, _L, _L, _I, _I, _P],
     },
     "attention": {
-        "oe_attn_paged": [_P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
+        "oe_attn_paged": [_P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P],
     },
     "rowwise": {
         "oe_cast_rows_bf16": [_P, _P, _L, _P],
@@ -291,11 +292,13 @@ def gather_rows_f32(out: torch.Tensor, x: torch.Tensor, rows: torch.Tensor) -> N
                                                     _stream()), "gather_rows_f32")
 
 
-def gemm_simple(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool = False) -> None:
-    """out (+)= a @ w.T on the CUDA cores with float32 accumulation in k order.
+def gemm_simple(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool = False, kind: int = 0) -> None:
+    """out (+)= a @ w.T on the CUDA cores with float32 accumulation, every element summed in the same order whatever
+    the shapes (csrc/gemm_simple.cu).
 
     a [M, K] and w [N, K] of one dtype (float32 or bfloat16); out [M, N] of that dtype or
-    float32; accumulate needs a float32 out."""
+    float32; accumulate needs a float32 out.  kind (float32 only): 0 the kernel is chosen by size, 1 weight streaming,
+    2 tiles of 64, 3 tiles of 128, 4 the general one; the same bits."""
     _dev(out, a, w)
     M, K = a.shape
     N = w.shape[0]
@@ -306,25 +309,30 @@ def gemm_simple(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate:
     if accumulate:
         if out.dtype != torch.float32:
             raise KernelError("gemm: accumulate needs a float32 output")
-        kind = 2
+        out_kind = 2
     elif out.dtype == a.dtype:
-        kind = 0
+        out_kind = 0
     elif out.dtype == torch.float32:
-        kind = 1
+        out_kind = 1
     else:
         raise KernelError("gemm: output must have the inputs' dtype or float32")
+    if a.dtype == torch.float32 and kind:
+        _check(_fn("gemm_simple", "oe_gemm_simple_kind_f32")(
+            _ptr(out), _ptr(a), _ptr(w), M, N, K, a.stride(0), out.stride(0), int(bool(accumulate)), int(kind), _stream()), "gemm_simple")
+        return
     _check(_fn("gemm_simple", "oe_gemm_simple", a.dtype)(
-        _ptr(out), _ptr(a), _ptr(w), M, N, K, a.stride(0), out.stride(0), kind, _stream()), "gemm_simple")
+        _ptr(out), _ptr(a), _ptr(w), M, N, K, a.stride(0), out.stride(0), out_kind, _stream()), "gemm_simple")
 
 
 def attn_paged(out: torch.Tensor, q: torch.Tensor, cache: torch.Tensor, tables: torch.Tensor,
                tok_seq: torch.Tensor, tok_pos: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int,
-               window: int, scale: float, sink: bool = False) -> None:
+               window: int, scale: float, sink: bool = False, kind: int = 0) -> None:
     """out[t] = attention of token t's query heads over keys (pos-window, pos] of its sequence (window 0:
     all keys up to pos; -n: the keys of the chunk of n positions that pos lies in).
 
     q [T, >= H hd] (row stride free, e.g. a view of the qkv buffer), out [T, H hd].
-    sink: the softmax's denominator gets one added (a key of score 0 without a value)."""
+    sink: the softmax's denominator gets one added (a key of score 0 without a value).  kind: 0 the kernel is chosen by the
+    numbers of tokens and sequences, 1 a CTA per token, 2 a CTA per 64 rows of tokens and heads; the same bits."""
     _dev(out, q, cache, tables, tok_seq, tok_pos)
     for t, n in ((tables, "tables"), (tok_seq, "tok_seq"), (tok_pos, "tok_pos")):
         _i32(t, n)
@@ -336,7 +344,7 @@ def attn_paged(out: torch.Tensor, q: torch.Tensor, cache: torch.Tensor, tables: 
         raise KernelError("attn_paged: cache entry must be [pages, 2, KVH, PAGE, head_dim]")
     _check(_fn("attention", "oe_attn_paged", out.dtype)(
         _ptr(out), _ptr(q), q.stride(0), _ptr(cache), _ptr(tables), tables.shape[1], _ptr(tok_seq), _ptr(tok_pos),
-        T, n_heads, n_kv_heads, head_dim, int(window), float(scale), int(bool(sink)), _stream()), "attn_paged")
+        T, tables.shape[0], n_heads, n_kv_heads, head_dim, int(window), float(scale), int(bool(sink)), int(kind), _stream()), "attn_paged")
 
 
 # ---------------------------------------------------------------------------------------- rowwise.cu

@@ -1,0 +1,109 @@
+"""The kernels of the 32-bit path: products and attention whose results do not depend on the kernel that a shape goes to."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rand(*shape, seed=0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
+
+
+@pytest.mark.parametrize("N,K", [(1, 4), (17, 60), (16, 64), (33, 68), (130, 512), (65, 516), (200, 1100), (4750, 576), (9500, 100)])
+def test_products_give_the_same_bits_by_every_kernel(N, K):
+    """Edges of segments (64), of rounds of eight segments (512), of row tiles (16, 32, 64), of the tiles of rows of A
+    (1, 2, 4, 8) and of the tiles of 64 and 128; rows of A inside wider ones; accumulation."""
+    from oracle_engine_b200.csrc import ops
+    w = _rand(N, K, seed=2)
+    wide = _rand(140, K + 8, seed=1)
+    base = _rand(140, N, seed=3)
+    for M in (1, 2, 3, 5, 8, 9, 17, 33, 64, 65, 140):
+        a = wide[:M, :K]
+        want = a.double() @ w.double().T
+        plain = torch.full((M, N), 7.0, device=DEV)
+        ops.gemm_simple(plain, a, w, kind=4)
+        # eight chains of K / 8 additions: an error of each sum of at most (K / 8 + 8) 2^-24 of the products' absolute sum
+        bound = (K / 8 + 9) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+        assert ((plain.double() - want).abs() <= bound).all()
+        for kind in (0, 1, 2, 3):
+            out = torch.full((M + 1, N), 7.0, device=DEV)
+            ops.gemm_simple(out[:M], a, w, kind=kind)
+            assert torch.equal(out[:M], plain), (M, N, K, kind)
+            assert (out[M] == 7.0).all()
+            acc = base[:M].clone()
+            ops.gemm_simple(acc, a, w, accumulate=True, kind=kind)
+            assert torch.equal(acc, base[:M] + plain), (M, N, K, kind)
+
+
+def test_a_product_of_unaligned_rows_takes_the_general_kernel():
+    from oracle_engine_b200.csrc import ops
+    buf = _rand(5 * 64 + 1, seed=4)
+    a, w = buf[1:].view(5, 64), _rand(40, 64, seed=5)
+    out, same = torch.empty(5, 40, device=DEV), torch.empty(5, 40, device=DEV)
+    ops.gemm_simple(out, a, w)
+    ops.gemm_simple(same, a.clone(), w)
+    assert torch.equal(out, same)
+    with pytest.raises(ops.KernelError):
+        ops.gemm_simple(out, a, w, kind=1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,KVH,hd,window,sink", [(4, 2, 64, 0, False), (9, 1, 18, 0, True), (20, 2, 128, 40, False), (3, 3, 256, -50, True),
+                                                  (2, 1, 34, 1, False), (33, 1, 16, 0, False)])
+def test_attention_gives_the_same_bits_by_both_kernels(dtype, H, KVH, hd, window, sink):
+    """Chunks of 32 keys at their edges, more heads a group than a warp takes at a time, windows and chunks of positions,
+    padding rows; the values that a query does not see are infinite, and what the last page holds behind a sequence is NaN."""
+    from oracle_engine_b200.csrc import ops
+    lens = [1, 32, 33, 300, 65]
+    G, pages = H // KVH, [(n + 63) // 64 for n in lens]
+    cache = torch.full((sum(pages) + 1, 2, KVH, 64, hd), float("nan"))
+    tables = torch.full((len(lens) + 1, max(pages) + 1), -1, dtype=torch.int32)
+    g = torch.Generator().manual_seed(H * 100 + hd)
+    order, at = torch.randperm(sum(pages), generator=g).tolist(), 0
+    ks, vs = [torch.randn(n, KVH, hd, generator=g) for n in lens], [torch.randn(n, KVH, hd, generator=g) for n in lens]
+    for b, n in enumerate(lens):
+        if b == 3:
+            vs[b][290:] = float("inf")                       # seen by the last ten queries only
+        for p in range(pages[b]):
+            tables[b, p] = page = order[at]
+            at += 1
+            m = min(64, n - 64 * p)
+            cache[page, 0, :, :m] = ks[b][64 * p:64 * p + m].transpose(0, 1)
+            cache[page, 1, :, :m] = vs[b][64 * p:64 * p + m].transpose(0, 1)
+    cache, tables = cache.to(dtype).to(DEV), tables.to(DEV)
+    rd = lambda t: t.to(dtype).double()                      # noqa: E731
+    for mode in ("prompt", "last"):
+        seq, pos, rows = [], [], []
+        for b, n in enumerate(lens):
+            for p in range(n if mode == "prompt" else 1):
+                seq.append(b)
+                pos.append(p if mode == "prompt" else n - 1 - (15 if b == 3 else 0))
+            seq.append(-1)                                   # a padding row between sequences
+            pos.append(0)
+        T = len(seq)
+        q = torch.randn(T, H * hd + 6, generator=g).to(dtype)
+        outs = []
+        for kind in (0, 1, 2):
+            out = torch.full((T, H * hd), 7.0, dtype=dtype, device=DEV)
+            ops.attn_paged(out, q.to(DEV), cache, tables, torch.tensor(seq, dtype=torch.int32, device=DEV),
+                           torch.tensor(pos, dtype=torch.int32, device=DEV), H, KVH, hd, window, hd ** -0.5, sink, kind)
+            outs.append(out.cpu())
+        assert torch.equal(outs[0].nan_to_num(9.0, 8.0, -8.0), outs[1].nan_to_num(9.0, 8.0, -8.0))
+        assert torch.equal(outs[0].nan_to_num(9.0, 8.0, -8.0), outs[2].nan_to_num(9.0, 8.0, -8.0))
+        for t in range(T):
+            got = outs[0][t].double().view(H, hd)
+            if seq[t] < 0:
+                assert (got == 0).all()
+                continue
+            b, p = seq[t], pos[t]
+            if b == 3 and p >= 290:
+                continue                                     # infinite values
+            lo = max(0, p - window + 1) if window > 0 else p // -window * -window if window < 0 else 0
+            for h in (0, H - 1):
+                s = (rd(ks[b][lo:p + 1, h // G]) @ rd(q[t, h * hd:(h + 1) * hd])) * hd ** -0.5
+                e = torch.exp(s - s.max())
+                o = (e @ rd(vs[b][lo:p + 1, h // G])) / (e.sum() + (math.exp(-s.max()) if sink else 0.0))
+                assert (got[h] - o).abs().max() <= (2e-5 if dtype == torch.float32 else 2.0 ** -8 * o.abs().max() + 2e-5)
