@@ -1,6 +1,6 @@
 // Token selection on the device: first-maximum argmax, and the reference's sampling
 // chain  repeat penalty -> temperature -> softmax -> top-k -> top-p -> draw
-// (core/sampler.cpp:15-27, 35-39, 48-86, 91-97), one block per row of float32 logits.
+// (core/sampler.cpp:15-27, 35-39, 48-86, 91-97), one block or one cluster of blocks per row of float32 logits.
 //
 // Differences from the reference, on purpose:
 //  * the draw is one uniform per (sequence, draw number) from a counter-based generator
@@ -134,6 +134,32 @@ struct SampleState {
     int hist_cap;
 };
 
+constexpr int PENALTY_CAP = 256;                    // the longest history whose tokens fit the shared array of penalise()
+
+// The repeat penalty over the last `repeat_last` recorded tokens, for those in [lo, hi), by the whole block: the first of
+// equal tokens is penalised once for each of them.  (One thread going through the history took 1.2 us a token.)
+__device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, int repeat_last, const SampleState& st, int* s_ids) {
+    const int count = st.hist_count[slot];
+    int n = count < repeat_last ? count : repeat_last;
+    if (n > st.hist_cap) n = st.hist_cap;
+    const int* ring = st.hist + (size_t)slot * st.hist_cap;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) s_ids[j] = ring[(count - n + j) % st.hist_cap];
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const int id = s_ids[j];
+        if (id < lo || id >= hi) continue;
+        bool first = true;
+        int times = 1;
+        for (int i = 0; i < j; i++) first &= s_ids[i] != id;
+        if (!first) continue;
+        for (int i = j + 1; i < n; i++) times += s_ids[i] == id;
+        float v = x[id];
+        for (int i = 0; i < times; i++) v = v > 0.f ? v / repeat_pen : v * repeat_pen;
+        x[id] = v;
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int* __restrict__ row_slot,
                    int V, float temperature, int top_k, float top_p, float repeat_pen, int repeat_last,
@@ -142,7 +168,7 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
     __shared__ float s_val[32];
     __shared__ int s_idx[32];
     __shared__ float s_scan[SAMPLE_THREADS];
-    __shared__ int s_pick;
+    __shared__ int s_pick, s_ids[PENALTY_CAP];
     pdl_launch_dependents();
     pdl_wait();
     const int slot = row_slot[blockIdx.x];
@@ -151,7 +177,9 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
     const int tid = threadIdx.x;
 
     // 1. repeat penalty over the last `repeat_last` recorded tokens, in order
-    if (repeat_pen > 1.f && st.hist != nullptr) {
+    if (repeat_pen > 1.f && st.hist != nullptr && st.hist_cap <= PENALTY_CAP) {
+        penalise(x, 0, V, slot, repeat_pen, repeat_last, st, s_ids);
+    } else if (repeat_pen > 1.f && st.hist != nullptr) {
         if (tid == 0) {
             const int count = st.hist_count[slot];
             int n = count < repeat_last ? count : repeat_last;
@@ -262,6 +290,265 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
     }
 }
 
+// ------------------------------------------------------------------------------------------------------------------
+// The same chain for wide rows (a temperature above zero): a cluster of eight CTAs per row, the row's values in registers
+// (up to 32 a thread) from the first pass to the draw.  With one block per row the row came from the L2 again for each of
+// the 62 passes of the two threshold searches: 1.35 ms for 128,256 tokens whatever the number of rows.  Here a pass is a
+// few compares in registers, one exchange of every warp's sums through the cluster's shared memory and one cluster
+// barrier; it settles two bits of a threshold (three candidates), and a search ends as soon as the tokens it keeps are
+// known: top-k when a candidate keeps exactly k, top-p when one token is left between the bounds.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int CL = 8, CT = 512, CW = CT / 32;        // CTAs of a cluster, threads and warps of a CTA
+
+struct __align__(16) Sums { float a[4]; unsigned n[4]; };
+
+__device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void store_remote(void* local, unsigned rank, float4 v) {
+    const unsigned here = (unsigned)__cvta_generic_to_shared(local);
+    unsigned there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(rank));
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(there), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// Every thread of the cluster gets the sums (or, MAX, the largest first value) over all threads, added in one order.
+template <bool MAX>
+__device__ __forceinline__ Sums cluster_sums(Sums v, Sums (*box)[CL * CW], int& turn) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (MAX) v.a[0] = fmaxf(v.a[0], __shfl_xor_sync(0xffffffffu, v.a[0], o));
+        else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) v.a[c] += __shfl_xor_sync(0xffffffffu, v.a[c], o);
+        }
+    }
+    if (!MAX) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) v.n[c] = __reduce_add_sync(0xffffffffu, v.n[c]);
+    }
+    Sums* b = box[turn];
+    turn ^= 1;                                        // the other box may still be read by a slower CTA
+    if (lane < CL) {
+        Sums* at = b + cluster_rank() * CW + warp;
+        store_remote(&at->a[0], lane, make_float4(v.a[0], v.a[1], v.a[2], 0.f));
+        store_remote(&at->n[0], lane, make_float4(__uint_as_float(v.n[0]), __uint_as_float(v.n[1]), __uint_as_float(v.n[2]), 0.f));
+    }
+    cluster_barrier();
+    Sums t = b[lane];
+#pragma unroll
+    for (int i = 1; i < CL * CW / 32; i++) {
+        const Sums u = b[lane + 32 * i];
+        if (MAX) t.a[0] = fmaxf(t.a[0], u.a[0]);
+        else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) { t.a[c] += u.a[c]; t.n[c] += u.n[c]; }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (MAX) t.a[0] = fmaxf(t.a[0], __shfl_xor_sync(0xffffffffu, t.a[0], o));
+        else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) t.a[c] += __shfl_xor_sync(0xffffffffu, t.a[c], o);
+        }
+    }
+    if (!MAX) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) t.n[c] = __reduce_add_sync(0xffffffffu, t.n[c]);
+    }
+    return t;
+}
+
+template <int EPT>
+__global__ void __launch_bounds__(CT)
+sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float temperature, int top_k, float top_p, float repeat_pen,
+                      int repeat_last, SampleState st, int record) {
+    __shared__ Sums box[2][CL * CW];
+    __shared__ int s_ids[PENALTY_CAP];
+    __shared__ float s_part[EPT * CW], s_excl[EPT * CW], s_total[CL];
+    __shared__ int s_entry, s_last[CL], s_warp_last[CW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = (int)cluster_rank(), row = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int slot = row_slot[row];
+    if (slot < 0) { if (rank == 0 && tid == 0) out[row] = -1; return; }      // the whole cluster
+    float* x = logits + (size_t)row * V;
+    const int slice = EPT * CT, base = rank * slice;  // this CTA's values are base + 512 j + tid
+    int turn = 0;
+
+    cluster_barrier();                                // every CTA of the cluster is there before its memory is written
+
+    // repeat penalty, of the tokens in this CTA's slice
+    if (repeat_pen > 1.f && st.hist != nullptr) penalise(x, base, min(base + slice, V), slot, repeat_pen, repeat_last, st, s_ids);
+
+    // temperature, softmax
+    const float inv_t = temperature == 1.f ? 1.f : 1.f / temperature;
+    float v[EPT];
+    Sums sums = {};
+    float mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < EPT; j++) {
+        const int i = base + j * CT + tid;
+        v[j] = i < V ? x[i] : -INFINITY;
+    }
+#pragma unroll
+    for (int j = 0; j < EPT; j++) { v[j] *= inv_t; mx = fmaxf(mx, v[j]); }
+    sums.a[0] = mx;
+    mx = cluster_sums<true>(sums, box, turn).a[0];
+    sums = {};
+#pragma unroll
+    for (int j = 0; j < EPT; j++) { v[j] = base + j * CT + tid < V ? expf(v[j] - mx) : 0.f; sums.a[0] += v[j]; }
+    const float inv = 1.f / cluster_sums<false>(sums, box, turn).a[0];
+#pragma unroll
+    for (int j = 0; j < EPT; j++) v[j] *= inv;
+
+    // top-k: the largest threshold with at least k probabilities at or above it; positions behind V hold 0 and are below
+    // any candidate.  No probability reaches 2, so that bit 30 is never set.
+    unsigned thr = 0u;
+    if (top_k > 0 && top_k < V) {
+        for (int bit = 28; bit >= 0; bit -= 2) {
+            sums = {};
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const unsigned cand = thr | ((unsigned)(c + 1) << bit);
+#pragma unroll
+                for (int j = 0; j < EPT; j++) sums.n[c] += __float_as_uint(v[j]) >= cand ? 1u : 0u;
+            }
+            const Sums t = cluster_sums<false>(sums, box, turn);
+            unsigned add = 0;
+            bool exact = false;
+#pragma unroll
+            for (int c = 0; c < 3; c++) if (t.n[c] >= (unsigned)top_k) { add = c + 1; exact = t.n[c] == (unsigned)top_k; }
+            thr |= add << bit;
+            if (exact) break;
+        }
+    }
+    // top-p within those: the largest threshold whose kept mass reaches top_p
+    if (top_p < 1.f) {
+        unsigned thp = 0u, above = 0u, kept = 0xffffffffu;    // tokens kept at the upper bound and at thp
+        for (int bit = 28; bit >= 0; bit -= 2) {
+            sums = {};
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const unsigned cand = thp | ((unsigned)(c + 1) << bit), eff = cand > thr ? cand : thr;
+#pragma unroll
+                for (int j = 0; j < EPT; j++) {
+                    const bool in = __float_as_uint(v[j]) >= eff;
+                    sums.a[c] += in ? v[j] : 0.f;
+                    sums.n[c] += in ? 1u : 0u;
+                }
+            }
+            const Sums t = cluster_sums<false>(sums, box, turn);
+            if (t.a[0] < top_p && (thp | (1u << bit)) <= thr) break;      // all that top-k left does not reach top_p
+            unsigned add = 0;
+            bool open = true;                         // the first candidate that is not reached is the upper bound
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                if (t.a[c] >= top_p) { add = c + 1; kept = t.n[c]; }
+                else if (open) { above = t.n[c]; open = false; }
+            }
+            thp |= add << bit;
+            if (kept != 0xffffffffu && kept - above <= 1u) break;     // nothing but the last kept token lies between the bounds
+        }
+        if (thp > thr) thr = thp;
+    }
+
+    // the draw: kept tokens in order of their index; first the sums of runs of 32 of them
+    int last = -1;
+#pragma unroll
+    for (int j = 0; j < EPT; j++) {
+        const bool in = __float_as_uint(v[j]) >= thr && base + j * CT + tid < V;
+        v[j] = in ? v[j] : 0.f;
+        if (in && v[j] > 0.f) last = base + j * CT + tid;
+        const float s = warp_sum(v[j]);
+        if (lane == 0) s_part[j * CW + warp] = s;
+    }
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) s_warp_last[warp] = last;
+    __syncthreads();
+    constexpr int PER = EPT * CW / 32;                // runs a lane of warp 0 adds up
+    float mine = 0.f;
+    if (warp == 0) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) mine += s_part[lane * PER + i];
+        float scan = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, scan, o); if (lane >= o) scan += u; }
+        const float before = __shfl_up_sync(0xffffffffu, scan, 1);
+        float run = lane == 0 ? 0.f : before;
+#pragma unroll
+        for (int i = 0; i < PER; i++) { s_excl[lane * PER + i] = run; run += s_part[lane * PER + i]; }
+        last = __reduce_max_sync(0xffffffffu, lane < CW ? s_warp_last[lane] : -1);
+        const float total = __shfl_sync(0xffffffffu, scan, 31);
+        if (lane < CL) store_remote(&box[turn][rank], lane, make_float4(total, __int_as_float(last), 0.f, 0.f));
+        if (lane == 0) s_entry = -1;
+    }
+    cluster_barrier();
+    if (tid < CL) { s_total[tid] = box[turn][tid].a[0]; s_last[tid] = __float_as_int(box[turn][tid].a[1]); }
+    turn ^= 1;
+    __syncthreads();
+    float from = 0.f, total = 0.f;
+#pragma unroll
+    for (int c = 0; c < CL; c++) { if (c == rank) from = total; total += s_total[c]; }
+    float to = from + s_total[rank];
+    const float u = uniform_from_counter((unsigned long long)st.rng_seed[slot], (unsigned long long)st.rng_counter[slot]);
+    const float r = u * total;
+    int pick = -1;
+    if (from <= r && r < to) {                        // one CTA at most
+        for (int e = tid; e < EPT * CW; e += CT) {
+            // the last run that begins at or below r among those that hold something
+            if (s_part[e] > 0.f && from + s_excl[e] <= r) atomicMax(&s_entry, e);
+        }
+        __syncthreads();
+        const int e = s_entry;
+        if (e >= 0 && e % CW == warp) {
+            float mass = 0.f;
+#pragma unroll
+            for (int j = 0; j < EPT; j++) if (j == e / CW) mass = v[j];
+            float run = from + s_excl[e];
+            int at = -1, some = -1;
+            for (int l = 0; l < 32; l++) {
+                const float m = __shfl_sync(0xffffffffu, mass, l);
+                if (m <= 0.f) continue;
+                run += m;
+                some = l;
+                if (at < 0 && run > r) at = l;
+            }
+            pick = base + e / CW * CT + warp * 32 + (at >= 0 ? at : some);
+            if (lane == 0) store_remote(&box[turn][0], 0, make_float4(__int_as_float(pick), 0.f, 0.f, 0.f));
+        }
+    } else if (tid == 0 && rank == 0 && !(r < total)) {
+        // r fell at or beyond the total through rounding (or nothing is kept): the last kept token
+        int l = -1;
+        for (int c = 0; c < CL; c++) l = max(l, s_last[c]);
+        box[turn][0].a[0] = __int_as_float(l);
+    }
+    cluster_barrier();
+    if (rank == 0 && tid == 0) {
+        const int token = __float_as_int(box[turn][0].a[0]);
+        out[row] = token;
+        if (record) {
+            st.rng_counter[slot] += 1;
+            if (st.hist != nullptr) {
+                const int c = st.hist_count[slot];
+                st.hist[(size_t)slot * st.hist_cap + (c % st.hist_cap)] = token;
+                st.hist_count[slot] = c + 1;
+            }
+        }
+    }
+}
+
+template <int EPT>
+int launch_cluster(float* logits, int* out, const int* row_slot, int rows, int V, float temperature, int top_k, float top_p,
+                   float repeat_pen, int repeat_last, const SampleState& state, int record, cudaStream_t st) {
+    return oe_launch_cluster(sample_cluster_kernel<EPT>, CL, dim3(CL, rows), dim3(CT), 0, st, logits, out, row_slot, V, temperature, top_k, top_p,
+                             repeat_pen, repeat_last, state, record);
+}
+
 }  // namespace
 
 extern "C" {
@@ -289,6 +576,13 @@ int oe_sample_rows(float* logits, int* out, const int* row_slot, int rows, int V
     if (rows <= 0) return 0;
     if (V <= 0 || (hist != nullptr && hist_cap <= 0)) return OE_ERR_UNSUPPORTED;
     SampleState st{rng_seed, rng_counter, hist, hist_count, hist_cap};
+    // A row per cluster from 8,192 tokens on (below that the row fits a block's first-level cache) up to what the registers of a
+    // cluster hold, 131,072; the history's bound is that of the ring in shared memory.
+    if (temperature > 0.f && V >= 8192 && V <= CL * CT * 32 && rows <= 65535 && (hist == nullptr || hist_cap <= PENALTY_CAP)) {
+        if (V <= CL * CT * 8)
+            return launch_cluster<8>(logits, out, row_slot, rows, V, temperature, top_k, top_p, repeat_pen, repeat_last, st, record, stream);
+        return launch_cluster<32>(logits, out, row_slot, rows, V, temperature, top_k, top_p, repeat_pen, repeat_last, st, record, stream);
+    }
     const int launch_rc = oe_launch(sample_rows_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, stream, logits, out, row_slot, V, temperature, top_k, top_p,
                                                             repeat_pen, repeat_last, st, record);
     return launch_rc;
