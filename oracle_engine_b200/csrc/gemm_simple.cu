@@ -2,10 +2,10 @@
 //
 // This is the matrix product of the true 32-bit path (no tensor cores, no reduced-
 // precision mode) and the product for shapes the tensor-core kernels refuse.  Every
-// output element is summed in ONE order, whatever kernel computes it: k is cut into
-// segments of 64, segment s belongs to class s mod 8, a class is one chain of fused
-// multiply-adds over its segments in order of k, and the (up to) eight classes are added
-// in order.  An element's value therefore does not depend on M, on the tile it falls in, or
+// output element is summed in ONE order, whatever kernel computes it: up to K = 512 one chain
+// of fused multiply-adds over k; beyond, k is cut into segments of 64, segment s belongs to
+// class s mod 8, a class is one chain over its segments in order of k, and the eight classes are
+// added in order.  An element's value therefore does not depend on M, on the tile it falls in, or
 // on what else is in the batch: the 32-bit logits are identical under every way of cutting
 // the work.  Eight chains instead of one are what lets a handful of rows stream a weight
 // matrix at the speed of the memory: eight threads share an output element.
@@ -18,11 +18,12 @@
 
 namespace {
 
-constexpr int SEG = 64, CLASSES = 8;
+constexpr int CLASSES = 8, ONE_CHAIN = 512;
 
-// The classes that have a segment, and how many rounds of segments the first class has.
-__host__ __device__ __forceinline__ int class_count(int K) { const int n = (K + SEG - 1) / SEG; return n < CLASSES ? n : CLASSES; }
-__host__ __device__ __forceinline__ int class_rounds(int K) { return (K + SEG * CLASSES - 1) / (SEG * CLASSES); }
+// A segment's length (a multiple of 64), the classes that have a segment, and how many rounds of segments there are.
+__host__ __device__ __forceinline__ int segment(int K) { return K > ONE_CHAIN ? 64 : (K + 63) / 64 * 64; }
+__host__ __device__ __forceinline__ int class_count(int K) { return K > ONE_CHAIN ? CLASSES : 1; }
+__host__ __device__ __forceinline__ int class_rounds(int K) { return (K + segment(K) * CLASSES - 1) / (segment(K) * CLASSES); }
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src, bool on) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -37,12 +38,13 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // CTA of four warps has 16 R rows, and CTAs walk over the tiles of rows.  Every warp has a ring of its own: a stage is KS
 // values of k of its rows and classes (4 KS consecutive bytes a row and class) and the same k of MT rows of A; the ring
 // runs on from tile to tile, so that loads stay in flight while a tile's classes are added up.  A lane reads its weights
-// and A's values from the stage; rows and classes are spaced so that no eight lanes meet in a bank.
+// and A's values from the stage (rows four words apart from a multiple of 32: no eight lanes meet in a bank).  The next
+// stage is asked for behind the products: before them it cost 5 to 15 %.
 // ------------------------------------------------------------------------------------------------------------------
 template <int R, int MT>
 struct StreamShape {
     static constexpr int KS = R == 1 && MT <= 4 ? 32 : 16;                                 // k per stage and class
-    static constexpr int CLS = KS + 4;                                           // words between two classes of a row
+    static constexpr int CLS = KS;                                           // words between two classes of a row
     static constexpr int WROW = 4 * CLS + 4;                                     // words of a weight row in a stage
     static constexpr int STAGE = 8 * R * WROW + MT * 4 * CLS;                    // floats
     static constexpr int PER_SM = R == 4 ? 1 : 2;                                // CTAs an SM
@@ -56,14 +58,15 @@ __global__ void __launch_bounds__(128)
 gemm_stream_kernel(float* C, const float* A, const float* __restrict__ W, int M, int N, int K, long long lda, long long ldc,
                    int tiles_m, int tiles) {
     using S = StreamShape<R, MT>;
-    constexpr int KS = S::KS, WROW = S::WROW, CLS = S::CLS, STEPS = SEG / KS;
+    constexpr int KS = S::KS, WROW = S::WROW, CLS = S::CLS;
+    const int seg = segment(K), steps = seg / KS;
     extern __shared__ __align__(16) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int half = warp & 1, group = warp >> 1;    // classes 4 half .. 4 half + 3; rows 8 R group .. of the tile
     const int rl = lane & 7, sub = lane >> 3;
     float* ring = smem + warp * S::STAGES * S::STAGE;
     float* part = smem + 4 * S::STAGES * S::STAGE;   // [class][row of the tile][MT]
-    const int per_tile = class_rounds(K) * STEPS;
+    const int per_tile = class_rounds(K) * steps;
     const int mine = tiles > (int)blockIdx.x ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int total = mine * per_tile;
 
@@ -77,7 +80,7 @@ gemm_stream_kernel(float* C, const float* A, const float* __restrict__ W, int M,
         if (++p.it == per_tile) { p.it = 0; p.tile += gridDim.x; }
         if (++p.stage == S::STAGES) p.stage = 0;
     };
-    auto k_of = [&](const Place& p) { return (p.it / STEPS * CLASSES + 4 * half + ls) * SEG + p.it % STEPS * KS + 4 * lq; };
+    auto k_of = [&](const Place& p) { return (p.it / steps * CLASSES + 4 * half + ls) * seg + p.it % steps * KS + 4 * lq; };
     auto load_w = [&](const Place& p) {
         const int n0 = p.tile / tiles_m * (16 * R) + group * 8 * R, k = k_of(p);
         float* st = ring + p.stage * S::STAGE + ls * CLS + 4 * lq;
@@ -123,39 +126,28 @@ gemm_stream_kernel(float* C, const float* A, const float* __restrict__ W, int M,
         __syncwarp();                                 // the stage is there, and the one before it is free
         const float* st = ring + stage * S::STAGE;
         if (++stage == S::STAGES) stage = 0;
-        if (i + S::STAGES - 1 < total) { load_w(pa); load_a(pa); next(pa); }
-        cp_commit();
         const float* wr = st + rl * WROW + sub * CLS;
         const float* ar = st + 8 * R * WROW + sub * CLS;
-        float4 w[2][R], a[2][MT];                     // the next four k are on their way while four are multiplied
-        auto fetch = [&](int kk, int b) {
-#pragma unroll
-            for (int j = 0; j < R; j++) w[b][j] = *(const float4*)(wr + j * 8 * WROW + kk);
-#pragma unroll
-            for (int m = 0; m < MT; m++) a[b][m] = *(const float4*)(ar + m * 4 * CLS + kk);
-        };
-        fetch(0, 0);
 #pragma unroll
         for (int kk = 0; kk < KS; kk += 4) {
-            const int b = kk / 4 & 1;
-            if (kk + 4 < KS) fetch(kk + 4, b ^ 1);
+            float4 w[R];
 #pragma unroll
-            for (int j = 0; j < R; j++)
+            for (int j = 0; j < R; j++) w[j] = *(const float4*)(wr + j * 8 * WROW + kk);
 #pragma unroll
-                for (int m = 0; m < MT; m++) acc[j][m] = fmaf(a[b][m].x, w[b][j].x, acc[j][m]);
+            for (int m = 0; m < MT; m++) {
+                const float4 a = *(const float4*)(ar + m * 4 * CLS + kk);
 #pragma unroll
-            for (int j = 0; j < R; j++)
-#pragma unroll
-                for (int m = 0; m < MT; m++) acc[j][m] = fmaf(a[b][m].y, w[b][j].y, acc[j][m]);
-#pragma unroll
-            for (int j = 0; j < R; j++)
-#pragma unroll
-                for (int m = 0; m < MT; m++) acc[j][m] = fmaf(a[b][m].z, w[b][j].z, acc[j][m]);
-#pragma unroll
-            for (int j = 0; j < R; j++)
-#pragma unroll
-                for (int m = 0; m < MT; m++) acc[j][m] = fmaf(a[b][m].w, w[b][j].w, acc[j][m]);
+                for (int j = 0; j < R; j++) {
+                    acc[j][m] = fmaf(a.x, w[j].x, acc[j][m]);
+                    acc[j][m] = fmaf(a.y, w[j].y, acc[j][m]);
+                    acc[j][m] = fmaf(a.z, w[j].z, acc[j][m]);
+                    acc[j][m] = fmaf(a.w, w[j].w, acc[j][m]);
+                }
+            }
         }
+        __syncwarp();
+        if (i + S::STAGES - 1 < total) { load_w(pa); load_a(pa); next(pa); }
+        cp_commit();
         if (++it < per_tile) continue;
         it = 0;
         const int n0 = tile / tiles_m * (16 * R), m0 = tile % tiles_m * MT;
@@ -210,13 +202,13 @@ gemm_tile_kernel(float* C, const float* A, const float* __restrict__ W, int M, i
     float* ring = smem + g * S::STAGES * S::STAGE;
     const int classes = class_count(K), rounds = class_rounds(K);
     constexpr int CPG = CLASSES / KG;                // classes of a group
-    const int per_class = rounds * (SEG / TK);
+    const int seg = segment(K), steps = seg / TK, per_class = rounds * steps;
     const int total = (KG == 1 ? classes : CPG) * per_class;
 
     const int lq = t & 3, lr = t >> 2;
     auto load = [&](int i) {
         const int c = g * CPG + i / per_class, it = i % per_class;
-        const int k = ((it / (SEG / TK)) * CLASSES + c) * SEG + (it % (SEG / TK)) * TK + 4 * lq;
+        const int k = (it / steps * CLASSES + c) * seg + it % steps * TK + 4 * lq;
         float* st = ring + (i % S::STAGES) * S::STAGE + 4 * lq;
 #pragma unroll
         for (int r = lr; r < BM; r += GT / 4) {
@@ -347,9 +339,10 @@ gemm_nt_kernel(TC* C, const TA* A, const TA* __restrict__ W,
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j] = tot[i][j] = 0.f;
 
+    const int seg = segment(K);
     for (int c = 0; c < class_count(K); c++) {
-    for (int s = c * SEG; s < K; s += SEG * CLASSES)
-    for (int k0 = s; k0 < s + SEG && k0 < K; k0 += BK) {
+    for (int s = c * seg; s < K; s += seg * CLASSES)
+    for (int k0 = s; k0 < s + seg && k0 < K; k0 += BK) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int k = k0 + lk + j;
@@ -446,9 +439,10 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, lo
     if (kind == 0) {
         const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128);
         const long long t64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
-        // up to 64 rows a narrow weight has too few tiles of 64 for the SMs (64 x 2,048 x 2,048: 58 us streamed, 78 by tiles; 64 x
+        // Eight chains are what tiles of 64 share out over a CTA's groups: up to K = 512 there is one, and tiles of 128 it is.
+        // Up to 64 rows a narrow weight has too few tiles of 64 for the SMs (64 x 2,048 x 2,048: 58 us streamed, 78 by tiles; 64 x
         // 16,384 x 2,048: 249 and 153); below 1.5 tiles of 128 an SM, tiles of 64 leave less of the last round empty
-        kind = M <= STREAM_MAX_M || (M <= 64 && 2 * t64 < sms) ? 1 : 2 * t128 >= 3 * sms ? 3 : 2;
+        kind = M <= STREAM_MAX_M || (M <= 64 && 2 * t64 < sms) ? 1 : K <= ONE_CHAIN || 2 * t128 >= 3 * sms ? 3 : 2;
     }
     if (kind == 3) return launch_tile<128, 128, 1, MODE>(C, A, W, M, N, K, lda, ldc, st);
     if (kind == 2) return launch_tile<64, 64, 4, MODE>(C, A, W, M, N, K, lda, ldc, st);
