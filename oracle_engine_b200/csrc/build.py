@@ -39,6 +39,7 @@ LIBRARIES = {
     "attention_split": ("attention_split.cu", []),
     "retention": ("retention.cu", []),
     "moe": ("moe.cu", []),
+    "moe_sparse": ("moe_sparse.cu", []),
     "stream": ("stream.cu", []),
     "gla": ("gla.cu", []),
     "attention_latent": ("attention_latent.cu", []),

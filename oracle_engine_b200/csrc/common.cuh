@@ -222,6 +222,18 @@ static inline bool oe_epilogue_ok(const OeEpilogue& e, int out_kind, int n_featu
            (e.w == nullptr || (e.ff > 0 && e.ld >= (n_features - e.from + e.ff - 1) / e.ff));
 }
 
+// An expert's gated unit from the float32 sums of its gate and up rows and the token's weight for it: 0 silu(g) u w; 1 the
+// clamped unit, shifted by one; 2 the weight on the expert's input, which both rows are linear in.
+__device__ __forceinline__ float oe_moe_unit(int unit, float g, float u, float w, float limit) {
+    if (unit == 1) {
+        g = fminf(g, limit);
+        u = fminf(fmaxf(u, -limit), limit);
+        return g / (1.f + expf(-1.702f * g)) * (u + 1.f) * w;
+    }
+    if (unit == 2) { g *= w; return g / (1.f + expf(-g)) * (u * w); }
+    return g / (1.f + expf(-g)) * u * w;
+}
+
 // Sum over a block in a fixed order (warp shuffles, then warp 0 over the warp totals);
 // every thread gets the result.  `red` holds 32 floats of shared memory.
 __device__ __forceinline__ float block_sum(float v, float* red) {

@@ -59,6 +59,21 @@ struct PairArgs {
     int tiles_m, tiles_n;          // tiles of 256 rows and of n_tile columns
 };
 
+// A product whose row tiles belong to experts (csrc/moe_sparse.cu sorts the rows): C[row] = unit or plain sums of A[row]
+// and the weights of the row tile's expert, which lie among all experts' in W.
+struct GroupArgs {
+    const int* tile_expert;        // the expert of every tile of 256 rows; null: one expert, `expert`, for all rows
+    const int* n_tiles;            // how many tiles there are (null: tiles_m), written by an earlier kernel
+    int expert;
+    int gate_up;                   // 1: the leader's half of a weight tile are gate rows, the other's the up rows that belong
+                                   // to them, F rows further down; C [M, ff] bf16.  0: n_tile rows of W, columns of one expert
+    int ff, F;                     // an expert's rows (gate_up) or columns, and all of them
+    const float* row_w;            // gate_up: a row's weight (row_w[row * row_w_ld])
+    long long row_w_ld;
+    int unit;                      // csrc/common.cuh: oe_moe_unit
+    float limit;
+};
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -222,10 +237,32 @@ __device__ __forceinline__ void emit16(const PairArgs& g, int row, int col0, flo
     }
 }
 
-// ACT: the product has an epilogue (common.cuh: OeEpilogue); a form of its own, so that the others stay as they are.
-template <bool ACT>
+// 16 consecutive columns (col0 ..) of output row `row` of an expert's gated unit.
+__device__ __forceinline__ void emit_unit(const PairArgs& g, const GroupArgs& q, int row, int col0, const uint32_t (&gate)[16], const uint32_t (&up)[16], float w) {
+    if (row >= g.M) return;
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = w != 0.f ? oe_moe_unit(q.unit, __uint_as_float(gate[j]), __uint_as_float(up[j]), w, q.limit) : 0.f;
+    bf16* dst = (bf16*)g.C + (long long)row * g.ldc + col0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {                          // ff is a multiple of 8
+        if (col0 + 8 * h >= q.ff) break;
+        uint32_t p[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            __nv_bfloat162 x = __floats2bfloat162_rn(v[8 * h + 2 * j], v[8 * h + 2 * j + 1]);
+            p[j] = *(uint32_t*)&x;
+        }
+        *(uint4*)(dst + 8 * h) = make_uint4(p[0], p[1], p[2], p[3]);
+    }
+}
+
+// KIND 1: the product has an epilogue (common.cuh: OeEpilogue); 2: its row tiles belong to experts (GroupArgs).  Forms of
+// their own, so that the plain one stays as it is.
+template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const PairArgs g) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const PairArgs g, const GroupArgs q) {
+    constexpr bool ACT = KIND == 1, GROUPED = KIND == 2;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int b_half_rows = g.n_tile / 2;
@@ -237,7 +274,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-    const int n_work = g.tiles_m * g.tiles_n;
+    int tiles_m = g.tiles_m;
     const int n_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
     uint32_t tmem_cols = 32;
     while ((int)tmem_cols < 2 * g.acc_cols) tmem_cols <<= 1;        // two accumulators
@@ -260,6 +297,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t tmem_base = *(volatile uint32_t*)&ctl->tmem_base;
 
     pdl_launch_dependents();
+    if (GROUPED) {
+        pdl_wait();                                        // the row tiles come from an earlier kernel
+        if (q.n_tiles) tiles_m = *(volatile const int*)q.n_tiles;
+    }
+    const int n_work = tiles_m * g.tiles_n;
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         // The whole warp runs the loop and waits; one elected lane issues the copies.
@@ -268,9 +310,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         uint32_t phase = 0;
         bool ok = true;
         for (int w = cluster_id; w < n_work && ok; w += n_clusters) {
-            const int tile_n = w / g.tiles_m, tile_m = w % g.tiles_m;
+            const int tile_n = w / tiles_m, tile_m = w % tiles_m;
             const int a_row = tile_m * (2 * BLOCK_M) + (int)rank * BLOCK_M;
-            const int b_row = tile_n * g.n_tile + (int)rank * b_half_rows;
+            int b_row = tile_n * g.n_tile + (int)rank * b_half_rows, b_col = 0;
+            if (GROUPED) {
+                const int e = q.tile_expert ? q.tile_expert[tile_m] : q.expert;
+                if (q.gate_up) b_row = (int)rank * q.F + e * q.ff + tile_n * b_half_rows;
+                else b_col = e * q.ff;
+            }
             // a short loop per k-block (no division, addresses carried along): see gemm_tcgen05.cu
             for (int i = 0, col = 0; i < n_kb; i++, col += BLOCK_K) {
                 if (!__all_sync(0xffffffffu, mbar_wait(&ctl->empty[s], phase ^ 1u, ctl, 1))) { ok = false; break; }
@@ -279,7 +326,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (leader) mbar_expect_tx(&ctl->full[s], (uint32_t)(2 * (A_TILE_BYTES + b_bytes)));
                     const uint32_t bar = in_leader(&ctl->full[s]);
                     tma_load_pair(a_dst, &map_a, bar, col, a_row);
-                    tma_load_pair(a_dst + A_TILE_BYTES, &map_b, bar, col, b_row);
+                    tma_load_pair(a_dst + A_TILE_BYTES, &map_b, bar, GROUPED ? col + b_col : col, b_row);
                 }
                 __syncwarp();
                 if (++s == g.stages) { s = 0; phase ^= 1u; }
@@ -330,7 +377,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         int lt = 0;
         bool first = true;
         for (int w = cluster_id; w < n_work; w += n_clusters, lt++) {
-            const int tile_n = w / g.tiles_m, tile_m = w % g.tiles_m;
+            const int tile_n = w / tiles_m, tile_m = w % tiles_m;
             const int row = tile_m * (2 * BLOCK_M) + (int)rank * BLOCK_M + row_in_cta;
             const int buf = lt & 1;
             OeGroupWeight kept;                            // of this thread's row, along the tile's columns
@@ -338,6 +385,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if (first) { pdl_wait(); first = false; }     // before the first access to C
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * g.acc_cols);
+            if (GROUPED && q.gate_up) {
+                // gate sums in the first half of the accumulator's columns, up sums in the second
+                const float rw = row < g.M ? q.row_w[(long long)row * q.row_w_ld] : 0.f;
+                for (int c0 = 0; c0 < b_half_rows; c0 += 16) {
+                    uint32_t gate[16], up[16];
+                    tmem_ld16(taddr + (uint32_t)c0, gate);
+                    tmem_ld16(taddr + (uint32_t)(b_half_rows + c0), up);
+                    tmem_ld_wait();
+                    emit_unit(g, q, row, tile_n * b_half_rows + c0, gate, up, rw);
+                }
+            } else
             for (int c0 = 0; c0 < g.n_tile; c0 += 32) {    // n_tile is a multiple of 16: the last group may be half
                 uint32_t r[2][16];
                 const bool two = c0 + 16 < g.n_tile;
@@ -400,6 +458,57 @@ int make_map(CUtensorMap* map, const void* ptr, long long rows, long long K, lon
 
 int g_clusters = -1;               // clusters of two CTAs that the device runs at once
 
+int prepare_device() {
+    const size_t smem_max = 227 * 1024;
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+        if (e != cudaSuccess) return (int)e;
+        attr_set = true;
+    }
+    if (g_clusters < 0) {
+        cudaLaunchConfig_t probe = {};
+        probe.gridDim = dim3(2); probe.blockDim = dim3(THREADS); probe.dynamicSmemBytes = smem_max;
+        int n = 0;
+        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<0>, &probe);
+        if (e != cudaSuccess) return (int)e;
+        if (n < 1) return OE_ERR_UNSUPPORTED;
+        g_clusters = n;
+    }
+    return 0;
+}
+
+// The tile width (a multiple of `step`) with the shortest rounds of clusters at the measured time of a
+// pair's k-block: 230, 249, 284, 310 and 365 ns from 128, 160, 192, 224 and 256 columns on, and a
+// width between two of these costs what the one below it costs (4096^3 with every width forced,
+// the roles as converged warps).  So 176 columns are the cheapest per column after 224..256, and
+// 8192 -> 3072 at 2,048 tokens takes 18 x 8 tiles of 176 (1.95 rounds of 74 clusters) rather than
+// 16 x 8 of 192 (1.73 rounds).
+int tile_width(long long tiles_m, int N, int limit, int step) {
+    long long best = -1;
+    int n_tile = limit;
+    for (int nt = limit; nt >= 128 && nt >= 32; nt -= step) {
+        const long long tiles = tiles_m * ((N + nt - 1) / nt);
+        static const int kb_ns[9] = {230, 230, 230, 230, 230, 249, 284, 310, 365};
+        const long long cost = ((tiles + g_clusters - 1) / g_clusters) * kb_ns[nt / 32];
+        if (best < 0 || cost < best) { best = cost; n_tile = nt; }
+    }
+    return n_tile;
+}
+
+size_t ring(PairArgs& g) {
+    const int n_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
+    const int b_bytes = (g.n_tile / 2) * BLOCK_K * 2;
+    const int stage_bytes = A_TILE_BYTES + ((b_bytes + 1023) & ~1023);
+    int stages = (200 * 1024) / stage_bytes;
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    if (stages > n_kb) stages = n_kb < 2 ? 2 : n_kb;
+    g.stages = stages;
+    return (size_t)stages * stage_bytes + sizeof(SharedCtl) + 1024;
+}
+
 }  // namespace
 
 extern "C" {
@@ -423,44 +532,15 @@ int oe_gemm_pair_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K
     if (out_kind < 0 || out_kind > 3 || (out_kind == 3 && (N & 1))) return OE_ERR_UNSUPPORTED;
     int rc = get_encode();
     if (rc) return rc;
-    const size_t smem_max = 227 * 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
-        if (e != cudaSuccess) return (int)e;
-        attr_set = true;
-    }
-    if (g_clusters < 0) {
-        cudaLaunchConfig_t probe = {};
-        probe.gridDim = dim3(2); probe.blockDim = dim3(THREADS); probe.dynamicSmemBytes = smem_max;
-        int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<false>, &probe);
-        if (e != cudaSuccess) return (int)e;
-        if (n < 1) return OE_ERR_UNSUPPORTED;
-        g_clusters = n;
-    }
+    if ((rc = prepare_device())) return rc;
     PairArgs g;
     g.C = C; g.ldc = ldc; g.M = M; g.N = N; g.K = K; g.out_kind = out_kind;
     g.epi = OeEpilogue{act, act_from, act_ff, act_ld, act_w};
     if (!oe_epilogue_ok(g.epi, out_kind, N)) return OE_ERR_UNSUPPORTED;
     g.tiles_m = (M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
-    // The tile width (a multiple of 16) with the shortest rounds of clusters at the measured time of a
-    // pair's k-block: 230, 249, 284, 310 and 365 ns from 128, 160, 192, 224 and 256 columns on, and a
-    // width between two of these costs what the one below it costs (4096^3 with every width forced,
-    // the roles as converged warps).  So 176 columns are the cheapest per column after 224..256, and
-    // 8192 -> 3072 at 2,048 tokens takes 18 x 8 tiles of 176 (1.95 rounds of 74 clusters) rather than
-    // 16 x 8 of 192 (1.73 rounds).
     int limit = 256;
     if (max_tile >= 32 && max_tile < limit) limit = max_tile / 16 * 16;
-    long long best = -1;
-    g.n_tile = limit;
-    for (int nt = limit; nt >= 128 && nt >= 32; nt -= 16) {
-        const long long tiles = (long long)g.tiles_m * ((N + nt - 1) / nt);
-        static const int kb_ns[9] = {230, 230, 230, 230, 230, 249, 284, 310, 365};
-        const long long cost = ((tiles + g_clusters - 1) / g_clusters) * kb_ns[nt / 32];
-        if (best < 0 || cost < best) { best = cost; g.n_tile = nt; }
-    }
+    g.n_tile = tile_width(g.tiles_m, N, limit, 16);
     if (max_tile <= -32 && max_tile >= -256 && max_tile % 16 == 0) g.n_tile = -max_tile;     // measurements: this width
     if (N < g.n_tile) g.n_tile = (N + 15) / 16 * 16;
     g.acc_cols = (g.n_tile + 31) / 32 * 32;
@@ -470,16 +550,46 @@ int oe_gemm_pair_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K
     CUtensorMap map_a, map_b;
     if ((rc = make_map(&map_a, A, M, K, lda, BLOCK_M))) return rc;
     if ((rc = make_map(&map_b, W, N, K, K, g.n_tile / 2))) return rc;
-    const int n_kb = (K + BLOCK_K - 1) / BLOCK_K;
-    const int b_bytes = (g.n_tile / 2) * BLOCK_K * 2;
-    const int stage_bytes = A_TILE_BYTES + ((b_bytes + 1023) & ~1023);
-    int stages = (200 * 1024) / stage_bytes;
-    if (stages > MAX_STAGES) stages = MAX_STAGES;
-    if (stages > n_kb) stages = n_kb < 2 ? 2 : n_kb;
-    g.stages = stages;
-    const size_t smem = (size_t)stages * stage_bytes + sizeof(SharedCtl) + 1024;
+    const size_t smem = ring(g);
     const int clusters = (int)(n_work < g_clusters ? n_work : g_clusters);
-    return oe_launch(g.epi.act ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, dim3(2 * clusters), dim3(THREADS), smem, st, map_a, map_b, g);
+    return oe_launch(g.epi.act ? gemm_pair_kernel<1> : gemm_pair_kernel<0>, dim3(2 * clusters), dim3(THREADS), smem, st, map_a, map_b, g, GroupArgs{});
+}
+
+// The products of a mixture's chosen experts.  The rows of A stand in tiles of 256 of one expert each: tile_expert (null: all
+// of `expert`) and n_tiles (null: every row counts) come from oe_moe_place; `likely` is the number of tiles to plan for.
+// gate_up 1: A [M, K], W [2 F, K], C [M, ff] bf16 = the gated unit of the expert's gate rows e ff .. and up rows F + e ff ..
+// with the row's weight; gate_up 0: A [M, ff], W [N, F], C [M, N] float32 (out_kind 1) or added to it (2), the sums over the
+// expert's columns e ff ..  An expert that is no multiple of ff rows from the start is given by `first` (its first row).
+int oe_gemm_pair_grouped_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K, long long lda, long long ldc, int gate_up, int out_kind,
+                              const int* tile_expert, const int* n_tiles, int likely, int first, int ff, int F, const float* row_w,
+                              long long row_w_ld, int unit, float limit, cudaStream_t st) {
+    if (M <= 0) return 0;
+    if (K <= 0 || (K % 8) || (lda % 8) || (((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15)) return OE_ERR_UNSUPPORTED;
+    if (ff < 16 || ff % 8 || F % 8 || F < ff || first < 0 || first % 8 || (tile_expert && first) || first + ff > F) return OE_ERR_UNSUPPORTED;
+    if (gate_up ? (row_w == nullptr || ldc % 8 || ldc < ff || unit < 0 || unit > 2) : (out_kind < 1 || out_kind > 2 || N < 32 || ldc < N || K != ff))
+        return OE_ERR_UNSUPPORTED;
+    int rc = get_encode();
+    if (rc || (rc = prepare_device())) return rc;
+    PairArgs g = {};
+    g.C = C; g.ldc = ldc; g.M = M; g.N = gate_up ? 2 * ff : N; g.K = K; g.out_kind = gate_up ? 0 : out_kind;
+    g.tiles_m = (M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
+    if (likely < 1 || likely > g.tiles_m) likely = g.tiles_m;
+    g.n_tile = tile_width(likely, g.N, 256, gate_up ? 32 : 16);
+    if (g.N < g.n_tile) g.n_tile = (g.N + 31) / 32 * 32;
+    g.acc_cols = (g.n_tile + 31) / 32 * 32;
+    g.tiles_n = (g.N + g.n_tile - 1) / g.n_tile;
+    const long long n_work = (long long)g.tiles_m * g.tiles_n;
+    if (n_work > 2147483647LL) return OE_ERR_UNSUPPORTED;
+    // The weights of `first` are reached by where the map begins; its extent keeps every load inside W.
+    CUtensorMap map_a, map_b;
+    if ((rc = make_map(&map_a, A, M, K, lda, BLOCK_M))) return rc;
+    if (gate_up) rc = make_map(&map_b, W + (size_t)first * K, 2LL * F - first, K, K, g.n_tile / 2);
+    else rc = make_map(&map_b, W + first, N, F - first, F, g.n_tile / 2);
+    if (rc) return rc;
+    const GroupArgs q = {tile_expert, n_tiles, 0, gate_up, ff, F, row_w, row_w_ld, unit, limit};
+    const size_t smem = ring(g);
+    const int clusters = (int)(n_work < g_clusters ? n_work : g_clusters);
+    return oe_launch(gemm_pair_kernel<2>, dim3(2 * clusters), dim3(THREADS), smem, st, map_a, map_b, g, q);
 }
 
 // Reads and clears the device-side error flag (0 = no wait ran out).

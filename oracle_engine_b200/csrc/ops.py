@@ -99,6 +99,12 @@ _SIGNATURES = {
         "oe_moe_dense_relu2": [_P, _P, _I, _I, _I, _I, _P],
         "oe_moe_dense_act": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P],
     },
+    "moe_sparse": {
+        "oe_moe_up_stream": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _I, _F, _P],
+        "oe_moe_down_stream": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _I, _P],
+        "oe_moe_place": [_P, _I, _I, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P, _P, _P, _I, _P],
+        "oe_moe_combine": [_P, _L, _P, _P, _I, _I, _I, _I, _P],
+    },
     "stream": {
         "oe_group_rmsnorm": [_P, _P, _L, _P, _I, _I, _I, _F, _P],
         "oe_group_rmsnorm_add": [_P, _P, _P, _I, _I, _I, _F, _F, _I, _P, _P],
@@ -1067,6 +1073,91 @@ def moe_dense_act(a: torch.Tensor, gu: torch.Tensor, dense: torch.Tensor, n_expe
     _check(_fn("moe", "oe_moe_dense_act", a.dtype)(_ptr(a), _ptr(gu), _ptr(dense), T, F, n_experts, ff, dense.shape[1],
                                                    int(bool(scale_input)), int(act == "clamped"), float(limit),
                                                    _stream()), "moe_dense_act")
+
+
+# ---------------------------------------------------------------------------------------- moe_sparse.cu
+
+_UNITS = {"silu": 0, "clamped": 1, "scale_input": 2}
+MOE_MAX_EXPERTS = 64         # experts and shared expert that the sparse kernels take; must equal MAX_GROUPS of moe_sparse.cu
+MOE_MAX_TOP = 8
+MOE_ROW_TILE = 256           # rows of a tile of the grouped product (gemm_tcgen05_pair.cu)
+
+
+def moe_sparse_supported(D: int, F: int, n_experts: int, ff: int, top: int) -> bool:
+    """Whether the kernels that compute the chosen experts alone take a mixture of these sizes (bfloat16)."""
+    shared = F - n_experts * ff
+    return (D % 8 == 0 and D >= 32 and F <= 64 * 2048 and ff % 8 == 0 and ff >= 16 and shared % 8 == 0 and (shared == 0 or shared >= 16)
+            and n_experts <= MOE_MAX_EXPERTS and top <= MOE_MAX_TOP)
+
+
+def _moe_operands(what, h, w, dense, out, n_experts, ff, columns):
+    _dev(h, w, dense, out)
+    _f32c(dense, "dense")
+    if h.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or h.stride(1) != 1 or not w.is_contiguous() or out.stride(1) != 1 \
+            or dense.shape[0] != h.shape[0] or dense.shape[1] < n_experts or columns < n_experts * ff \
+            or (columns > n_experts * ff and dense.shape[1] != n_experts + 1):
+        raise KernelError(f"{what}: shapes or types do not agree")
+
+
+def moe_up_stream(a: torch.Tensor, h: torch.Tensor, w: torch.Tensor, dense: torch.Tensor, n_experts: int, ff: int,
+                  unit: str = "silu", limit: float = 0.0) -> None:
+    """a [T, F] bfloat16 = the experts' gated units of h [T, D] (T <= 16) times the tokens' weights, of the experts that some
+    token chose (the others' columns are left as they are); w [2 F, D] as moe_dense_act has it: F gate rows, F up rows."""
+    T, F = a.shape
+    _moe_operands("moe_up_stream", h, w, dense, a, n_experts, ff, F)
+    if tuple(w.shape) != (2 * F, h.shape[1]) or h.shape[0] != T or a.dtype != torch.bfloat16 or not a.is_contiguous():
+        raise KernelError("moe_up_stream: a [T, F] contiguous and w [2 F, D] expected")
+    _check(_fn("moe_sparse", "oe_moe_up_stream")(_ptr(a), _ptr(h), _ptr(w), _ptr(dense), T, h.shape[1], F, n_experts, ff, dense.shape[1],
+                                                 h.stride(0), _UNITS[unit], float(limit), _stream()), "moe_up_stream", (T, F, h.shape[1]))
+
+
+def moe_down_stream(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, dense: torch.Tensor, n_experts: int, ff: int,
+                    accumulate: bool) -> None:
+    """out [T, N] float32 (+)= a [T, F] @ w [N, F].T over the columns of the experts that some token chose (T <= 16)."""
+    T, F = a.shape
+    _moe_operands("moe_down_stream", a, w, dense, out, n_experts, ff, F)
+    if w.shape[1] != F or tuple(out.shape) != (T, w.shape[0]) or out.dtype != torch.float32 or not a.is_contiguous():
+        raise KernelError("moe_down_stream: a [T, F] contiguous, w [N, F] and out float32 [T, N] expected")
+    _check(_fn("moe_sparse", "oe_moe_down_stream")(_ptr(out), _ptr(a), _ptr(w), _ptr(dense), T, w.shape[0], F, n_experts, ff, dense.shape[1],
+                                                   out.stride(0), int(bool(accumulate)), _stream()), "moe_down_stream", (T, w.shape[0], F))
+
+
+def moe_max_tiles(T: int, top: int, n_experts: int) -> int:
+    """The most row tiles that T tokens with `top` experts each can need."""
+    return T * top // MOE_ROW_TILE + n_experts
+
+
+def moe_place(dense: torch.Tensor, h: torch.Tensor, n_experts: int, top: int, xs: torch.Tensor, place: torch.Tensor, row_w: torch.Tensor,
+              tiles: torch.Tensor, counts: torch.Tensor) -> None:
+    """The (token, expert) pairs of `dense` sorted by expert: the rows of h copied into xs [max_tiles * 256, D], every expert's
+    rows from a multiple of 256 on; place int32 [T, top] the row of a token's j-th expert (-1: none), row_w the rows' weights,
+    tiles int32 [max_tiles + 1] every tile's expert and, last, how many tiles there are; counts: scratch."""
+    _dev(dense, h, xs, place, row_w, tiles, counts)
+    _f32c(dense, "dense")
+    _f32c(row_w, "row_w")
+    for t, n in ((place, "place"), (tiles, "tiles"), (counts, "counts")):
+        _i32(t, n)
+    T, D = h.shape
+    most = tiles.numel() - 1
+    if h.dtype != torch.bfloat16 or xs.dtype != torch.bfloat16 or h.stride(1) != 1 or not xs.is_contiguous() \
+            or tuple(xs.shape) != (most * MOE_ROW_TILE, D) or tuple(place.shape) != (T, top) or row_w.numel() < xs.shape[0] \
+            or counts.numel() < (T + 7) // 8 * n_experts or dense.shape[0] != T:
+        raise KernelError("moe_place: shapes or types do not agree")
+    _check(_fn("moe_sparse", "oe_moe_place")(_ptr(dense), T, n_experts, dense.shape[1], top, MOE_ROW_TILE, _ptr(counts), _ptr(h), h.stride(0), D,
+                                             _ptr(xs), _ptr(place), _ptr(row_w), _ptr(tiles), tiles.data_ptr() + 4 * most, most, _stream()),
+           "moe_place")
+
+
+def moe_combine(out: torch.Tensor, y: torch.Tensor, place: torch.Tensor, accumulate: bool) -> None:
+    """out[t] float32 (+)= the sum of y[place[t, j]] over j, in order."""
+    _dev(out, y, place)
+    _i32(place, "place")
+    T, D = out.shape
+    if out.dtype != torch.float32 or out.stride(1) != 1 or y.dtype != torch.float32 or not y.is_contiguous() or y.shape[1] != D \
+            or place.shape[0] != T:
+        raise KernelError("moe_combine: out [T, D] and y [rows, D] float32 expected")
+    _check(_fn("moe_sparse", "oe_moe_combine")(_ptr(out), out.stride(0), _ptr(y), _ptr(place), place.shape[1], T, D, int(bool(accumulate)),
+                                               _stream()), "moe_combine")
 
 
 # ---------------------------------------------------------------------------------------- stream.cu

@@ -160,6 +160,9 @@ def _pair():
         lib.oe_gemm_pair_bf16.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                                           c_int, c_int] + _EPILOGUE + [c_void_p]
         lib.oe_gemm_pair_bf16.restype = c_int
+        lib.oe_gemm_pair_grouped_bf16.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int,
+                                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_float, c_void_p]
+        lib.oe_gemm_pair_grouped_bf16.restype = c_int
         lib.oe_gemm_pair_error.restype = c_int
         _state["pair"] = lib
     return lib
@@ -250,6 +253,34 @@ def gemm(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool =
                                   counters.data_ptr() if split_k else None, counters.numel(), sms,
                                   *epilogue, ops._stream())
     ops._check(code, "gemm_tc", (M, N, K))
+
+
+def gemm_grouped(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, ff: int, tiles: torch.Tensor | None = None, likely: int = 0,
+                 first: int = 0, row_w: torch.Tensor | None = None, unit: str | None = None, limit: float = 0.0, accumulate: bool = False) -> None:
+    """The products of a mixture's chosen experts (csrc/gemm_tcgen05_pair.cu).  The rows of a stand in tiles of 256 of one
+    expert each; tiles (ops.moe_place; None: every row belongs to the one expert whose first row or column is `first`) names
+    the experts, `likely` is the number of tiles to plan for.
+    unit given: w [2 F, K] holds F gate rows and F up rows, out [rows, ff] bfloat16 = the expert's gated unit times row_w[row].
+    unit None: w [N, F], a [rows, ff], out [rows, N] float32 (+)= the sums over the expert's columns."""
+    M, K = a.shape
+    F = w.shape[0] // 2 if unit else w.shape[1]
+    N = w.shape[0]
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or a.stride(1) != 1 or not w.is_contiguous() or out.stride(1) != 1 \
+            or K != (w.shape[1] if unit else ff) or tuple(out.shape) != (M, ff if unit else N) \
+            or out.dtype != (torch.bfloat16 if unit else torch.float32) or (unit is None) != (row_w is None):
+        raise KernelError("gemm_grouped: shapes or types do not agree")
+    if row_w is not None and (row_w.dtype != torch.float32 or row_w.dim() != 1 or row_w.numel() < M):
+        raise KernelError("gemm_grouped: row_w must be float32, one value per row")
+    if tiles is not None:
+        ops._i32(tiles, "tiles")
+        if M != (tiles.numel() - 1) * ops.MOE_ROW_TILE:
+            raise KernelError("gemm_grouped: one entry of tiles per 256 rows, and their number behind them")
+    code = _pair().oe_gemm_pair_grouped_bf16(
+        out.data_ptr(), a.data_ptr(), w.data_ptr(), M, N, K, a.stride(0), out.stride(0), int(unit is not None), 2 if accumulate else 1,
+        None if tiles is None else tiles.data_ptr(), None if tiles is None else tiles.data_ptr() + 4 * (tiles.numel() - 1), int(likely), int(first),
+        int(ff), F, None if row_w is None else row_w.data_ptr(), 0 if row_w is None else row_w.stride(0), ops._UNITS[unit] if unit else 0,
+        float(limit), ops._stream())
+    ops._check(code, "gemm_pair_grouped", (M, N, K))
 
 
 def device_error() -> int:

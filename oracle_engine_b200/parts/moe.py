@@ -16,14 +16,16 @@ expert's, and only experts of the `keep` best runs can be chosen.
 Feed-forward `moe_relu2`: experts without a gate, E_e(h) = Wdown_e max(Wup_e h, 0)^2; by default the weights are the
 softmax over ALL experts, the chosen ones divided by their sum (+ 1e-20).
 
-How it is computed: the experts stand side by side.  One product with all gate and up matrices (the shared expert's
-behind the routed ones), one kernel that applies silu(gate) * up and multiplies each expert's columns by the token's
-weight for that expert (zero where it was not chosen, sigmoid(Wsg h) for the shared one), and one product with all
-down matrices side by side, which sums the chosen experts in its float32 accumulators.  The router and the shared
-gate are one small float32 product.  No token is moved and nothing depends on the host, so a step is the same
-kernels whatever the routing (and can be captured in a graph); the price is the products of the experts a token
-did not choose, experts / top times the arithmetic of the chosen ones, while the weights read are the same as
-soon as a step's tokens choose every expert between them.
+How it is computed: the experts stand side by side in two matrices, all gate and up rows (the shared expert's behind the
+routed ones) and all down columns; the router and the shared gate are one small float32 product, whose outcome (a weight
+per token and expert, zero where it was not chosen, sigmoid(Wsg h) for the shared one) stays on the device, so a step is
+the same kernels whatever the routing (and can be captured in a graph).  By the number of a step's tokens:
+
+* up to 16 (bfloat16): the weight-streaming products over the experts that some token chose (csrc/moe_sparse.cu);
+* from where it pays (`_sorted_pays`, bfloat16): the (token, expert) pairs sorted by expert and the grouped products over
+  them, the arithmetic of the chosen experts and what fills their last row tiles; the shared expert over all tokens;
+* else, in float32 and for sizes those do not take: one product with all gate and up matrices, one kernel that applies the
+  unit and multiplies each expert's columns by the token's weight, and one product with all down matrices.
 """
 from __future__ import annotations
 
@@ -33,6 +35,15 @@ from ..csrc import ops
 from .linear import chain_flags, matmul_act, matmul_nt
 from .registry import FEED_FORWARDS, Part
 from .spec import TensorDecl
+
+
+STREAM_TOKENS = 16           # a step's tokens up to which a mixture's products stream the chosen experts' weights
+
+
+def _sorted_pays(T: int, top: int, experts: int) -> bool:
+    """Whether sorting T tokens by expert saves at least a third of the rows that the products over all experts have: a
+    token's rows are its experts', and every expert's last tile of 256 rows is half empty on average."""
+    return 3 * (T * top + 128 * experts) <= 2 * T * experts
 
 
 def _route(rt, h, w_route, experts: int, top: int, has_gate, dense, ctx, weights, bias, groups) -> None:
@@ -104,6 +115,9 @@ class MoESwiGLU(Part):
                  **self.params.get("tensor_names", {})}
         self.names = {k: prefix + v for k, v in names.items()}
         self.F = self.E * self.ff + self.sff
+        self.unit = "clamped" if self.activation == "clamped" else "scale_input" if self.weight_on == "input" else "silu"
+        self.sparse = (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores
+                       and ops.moe_sparse_supported(self.D, self.F, self.E, self.ff, self.top))
         self.w_route = self.w_gu = self.w_down = self.bias = None
 
     def _expert_names(self):
@@ -155,12 +169,41 @@ class MoESwiGLU(Part):
         dense = self.rt.buffer("moe.dense", T, self.E + (1 if self.sff else 0), dtype=torch.float32)
         _route(self.rt, h, self.w_route, self.E, self.top, (True if self.shared_gate else "one") if self.sff else False,
                dense, ctx, self.router_weights, self.bias, self.groups)
+        aligned = h.stride(1) == 1 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
+        if self.sparse and aligned and T <= STREAM_TOKENS:
+            a = self.rt.buffer("moe.a", T, self.F)
+            ops.moe_up_stream(a, h, self.w_gu, dense, self.E, self.ff, self.unit, self.limit)
+            ops.moe_down_stream(residual, a, self.w_down, dense, self.E, self.ff, accumulate=not overwrite)
+            return
+        if self.sparse and aligned and _sorted_pays(T, self.top, self.E):
+            self._forward_sorted(h, residual, dense, overwrite)
+            return
         gu = self.rt.buffer("moe.gu", T, 2 * self.F)
         matmul_nt(self.rt, gu, h, self.w_gu)
         a = self.rt.buffer("moe.a", T, self.F)
         ops.moe_dense_act(a, gu, dense, self.E, self.ff, scale_input=self.weight_on == "input", act=self.activation,
                           limit=self.limit)
         matmul_nt(self.rt, residual, a, self.w_down, accumulate=not overwrite)
+
+
+    def _forward_sorted(self, h, residual, dense, overwrite: bool) -> None:
+        from ..csrc import ops_tc
+        rt, T, E, ff = self.rt, h.shape[0], self.E, self.ff
+        most = ops.moe_max_tiles(T, self.top, E)
+        likely = -(-T * self.top // ops.MOE_ROW_TILE) + E // 2
+        rows = most * ops.MOE_ROW_TILE
+        i32 = torch.int32
+        xs, place = rt.buffer("moe.xs", rows, self.D), rt.buffer("moe.place", T, self.top, dtype=i32)
+        row_w, tiles = rt.buffer("moe.row_w", rows, dtype=torch.float32), rt.buffer("moe.tiles", most + 1, dtype=i32)
+        ops.moe_place(dense, h, E, self.top, xs, place, row_w, tiles, rt.buffer("moe.counts", (T + 7) // 8 * E, dtype=i32))
+        a, y = rt.buffer("moe.a", rows, ff), rt.buffer("moe.y", rows, self.D, dtype=torch.float32)
+        ops_tc.gemm_grouped(a, xs, self.w_gu, ff, tiles, likely, row_w=row_w, unit=self.unit, limit=self.limit)
+        ops_tc.gemm_grouped(y, a, self.w_down, ff, tiles, likely)
+        ops.moe_combine(residual, y, place, accumulate=not overwrite)
+        if self.sff:
+            a = rt.buffer("moe.a", T, self.sff)
+            ops_tc.gemm_grouped(a, h, self.w_gu, self.sff, first=E * ff, row_w=dense[:, E], unit=self.unit, limit=self.limit)
+            ops_tc.gemm_grouped(residual, a, self.w_down, self.sff, first=E * ff, accumulate=True)
 
 
 @FEED_FORWARDS.register("moe_relu2")

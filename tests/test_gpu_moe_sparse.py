@@ -1,0 +1,123 @@
+"""Mixtures of experts: the kernels that compute the chosen experts alone, against the mixture in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _routing(T, E, top, shared, kind, g):
+    """Weights [T, E (+ 1)]: `top` experts a token, or all tokens the same ones, or some tokens none (padding rows)."""
+    dense = torch.zeros(T, E + int(shared))
+    for t in range(T):
+        if kind == "padding" and t % 3 == 1:
+            continue
+        chosen = torch.randperm(E, generator=g)[:top] if kind != "one" else torch.arange(E - top, E)
+        dense[t, chosen] = torch.rand(top, generator=g) + 0.1
+        if shared:
+            dense[t, E] = torch.rand(1, generator=g)
+    return dense
+
+
+def _unit(g, u, w, unit, limit):
+    if unit == "clamped":
+        g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+        return g * torch.sigmoid(1.702 * g) * (u + 1) * w
+    if unit == "scale_input":
+        g, u = g * w, u * w
+        return g * torch.sigmoid(g) * u
+    return g * torch.sigmoid(g) * u * w
+
+
+def _want(h, w_gu, w_down, dense, E, ff, unit, limit):
+    """(result, what an error of one bfloat16 rounding of every unit can move it by): 64 bits."""
+    F = w_down.shape[1]
+    gu = h.double() @ w_gu.double().T
+    w = torch.cat([dense[:, :E].repeat_interleave(ff, 1), dense[:, E:].expand(-1, F - E * ff)], 1).double()
+    a = torch.where(w != 0, _unit(gu[:, :F], gu[:, F:], w, unit, limit), 0.0)
+    return a @ w_down.double().T, a.abs() @ w_down.double().abs().T
+
+
+SIZES = [(8, 2, 64, 0, 64, 48), (3, 1, 24, 40, 136, 50), (64, 8, 16, 16, 72, 256), (5, 3, 152, 0, 520, 200), (1, 1, 40, 0, 64, 40)]
+CASES = [("spread", "silu"), ("one", "clamped"), ("padding", "scale_input")]
+
+
+@pytest.mark.parametrize("E,top,ff,sff,D,N", SIZES)
+@pytest.mark.parametrize("kind,unit", CASES)
+def test_streamed_experts(E, top, ff, sff, D, N, kind, unit):
+    from oracle_engine_b200.csrc import ops
+    F = E * ff + sff
+    g = torch.Generator().manual_seed(E * 1000 + ff)
+    w_gu, w_down = (torch.randn(2 * F, D, generator=g) * 0.2).bfloat16().to(DEV), (torch.randn(N, F, generator=g) * 0.2).bfloat16().to(DEV)
+    for T in (1, 2, 8, 9, 16):
+        dense = _routing(T, E, top, sff > 0, kind, g).to(DEV)
+        wide = torch.randn(T, D + 8, generator=g).bfloat16().to(DEV)
+        h = wide[:, :D]
+        a = torch.full((T, F), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.moe_up_stream(a, h, w_gu, dense, E, ff, unit, 1.5)
+        base = torch.randn(T, N, generator=g).to(DEV)
+        out, added = torch.full((T, N), 7.0, device=DEV), base.clone()
+        ops.moe_down_stream(out, a, w_down, dense, E, ff, accumulate=False)
+        ops.moe_down_stream(added, a, w_down, dense, E, ff, accumulate=True)
+        want, scale = _want(h, w_gu, w_down, dense, E, ff, unit, 1.5)
+        # a unit is rounded once to bfloat16 (2^-9) behind float32 sums of at most D products
+        assert ((out.double() - want).abs() <= 2.0 ** -8 * scale + 1e-4).all()
+        assert torch.equal(added, base + out)
+        # a token's result does not depend on which experts its neighbours chose
+        ops.moe_up_stream(a[:1], h[:1], w_gu, dense[:1], E, ff, unit, 1.5)
+        one = torch.empty(1, N, device=DEV)
+        ops.moe_down_stream(one, a[:1], w_down, dense[:1], E, ff, accumulate=False)
+        if T <= 8:
+            assert torch.equal(one[0], out[0])
+
+
+@pytest.mark.parametrize("E,top,ff,sff,D,N", SIZES)
+@pytest.mark.parametrize("kind,unit", CASES)
+@pytest.mark.parametrize("T", [1, 31, 257, 700])
+def test_sorted_experts(E, top, ff, sff, D, N, kind, unit, T):
+    from oracle_engine_b200.csrc import ops, ops_tc
+    F = E * ff + sff
+    g = torch.Generator().manual_seed(E * 1000 + ff + T)
+    w_gu, w_down = (torch.randn(2 * F, D, generator=g) * 0.2).bfloat16().to(DEV), (torch.randn(N, F, generator=g) * 0.2).bfloat16().to(DEV)
+    dense = _routing(T, E, top, sff > 0, kind, g).to(DEV)
+    h = torch.randn(T, D, generator=g).bfloat16().to(DEV)
+    most = ops.moe_max_tiles(T, top, E)
+    rows = most * 256
+    xs = torch.full((rows, D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    place, tiles = torch.empty(T, top, dtype=torch.int32, device=DEV), torch.empty(most + 1, dtype=torch.int32, device=DEV)
+    row_w, counts = torch.full((rows,), float("nan"), device=DEV), torch.empty((T + 7) // 8 * E, dtype=torch.int32, device=DEV)
+    ops.moe_place(dense, h, E, top, xs, place, row_w, tiles, counts)
+    # the rows stand by expert, in order of the tokens, every expert from a tile's edge on
+    at, expert_of, want_place = 0, [], torch.full((T, top), -1, dtype=torch.int32)
+    seen = [0] * T
+    d = dense.cpu()
+    for e in range(E):
+        mine = torch.nonzero(d[:, e]).flatten().tolist()
+        for i, t in enumerate(mine):
+            want_place[t, seen[t]] = at + i
+            seen[t] += 1
+            assert torch.equal(xs[at + i], h[t]) and float(row_w[at + i]) == float(d[t, e])
+        n = -(-len(mine) // 256)
+        expert_of += [e] * n
+        at += n * 256
+    assert torch.equal(place.cpu(), want_place)
+    assert int(tiles[-1]) == len(expert_of) and tiles[:len(expert_of)].tolist() == expert_of
+    a, y = torch.empty(rows, ff, dtype=torch.bfloat16, device=DEV), torch.empty(rows, N, device=DEV)
+    ops_tc.gemm_grouped(a, xs, w_gu, ff, tiles, row_w=row_w, unit=unit, limit=1.5)
+    ops_tc.gemm_grouped(y, a, w_down, ff, tiles, likely=1)
+    base = torch.randn(T, N, generator=g).to(DEV)
+    for accumulate in (False, True):
+        out = base.clone()
+        if N % 4:
+            with pytest.raises(ops.KernelError):
+                ops.moe_combine(out, y, place, accumulate)
+            return
+        ops.moe_combine(out, y, place, accumulate)
+        if sff:
+            s = torch.empty(T, sff, dtype=torch.bfloat16, device=DEV)
+            ops_tc.gemm_grouped(s, h, w_gu, sff, first=E * ff, row_w=dense[:, E], unit=unit, limit=1.5)
+            ops_tc.gemm_grouped(out, s, w_down, sff, first=E * ff, accumulate=True)
+        want, scale = _want(h, w_gu, w_down, dense, E, ff, unit, 1.5)
+        got = out.double() - (base.double() if accumulate else 0.0)
+        assert ((got - want).abs() <= 2.0 ** -8 * scale + 1e-4).all()
+    assert ops_tc.device_error() == 0
