@@ -32,13 +32,20 @@ _CHAIN_FLAGS = {
 }
 
 
+# Products that are given no flags, in the other decoders' longer chains of short kernels, start early and trigger late: behind
+# a kernel of any kind they then wait beside it, and nothing starts on the SMs they still stream through (us a decode step
+# with none / 1 / 2 / 3 of the flags: Fuvipel 487 / 517 / 476 / 460, Fovirax 676 / 751 / 661 / 626, Mavinex 619 / 629 / 619 / 611,
+# one sequence, 8 layers, width 2,048; at 8 sequences 1 to 3 % between none and both).
+DEFAULT_FLAGS = START_EARLY | TRIGGER_LATE
+
+
 def chain_flags(product: str, n_tokens: int) -> int:
     """START_EARLY / TRIGGER_LATE for one of a block's four products in a step of n_tokens rows."""
     return _CHAIN_FLAGS[product][0 if n_tokens <= 8 else 1]
 
 
 def matmul_nt(rt, out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool = False,
-              early: int = 0, then: torch.Tensor | None = None) -> None:
+              early: int = DEFAULT_FLAGS, then: torch.Tensor | None = None) -> None:
     """early: START_EARLY and TRIGGER_LATE flags (above); other kernels ignore them.
     then: the weight matrix of the product that runs after this one (a hint, see ops_tc.gemm)."""
     if rt.dtype == torch.bfloat16 and rt.tensor_cores:
@@ -50,7 +57,7 @@ def matmul_nt(rt, out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulat
 
 
 def matmul_act(rt, out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, act: str, group_weights: tuple | None = None,
-               early: int = 0) -> None:
+               early: int = DEFAULT_FLAGS) -> None:
     """out = act(a @ w.T), act "gelu" or "relu2", out of the compute dtype; with group_weights (float32 [T, groups], ff;
     "relu2" only) column c times weights[:, c // ff].  Where a tensor-core product takes the shapes the activation is its
     epilogue, on the float32 sums; else it is a kernel of its own."""
