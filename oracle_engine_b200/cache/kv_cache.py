@@ -129,9 +129,8 @@ class KVCache:
         if not self.slots.is_held(slot):
             raise ValueError(f"slot {slot} is not held (freed twice, or never allocated)")
         for g in self.groups:
-            row = g.tables[slot]
-            for i in np.nonzero(row >= 0)[0]:
-                g.pool.release(int(row[i]))
+            row = g.tables[slot, :int(g.hi[slot])]       # nothing is mapped behind hi
+            g.pool.release_all(row[row >= 0].tolist())
             row[:] = -1
             g.lo[slot] = g.hi[slot] = 0
         self.version += 1
@@ -167,22 +166,24 @@ class KVCache:
                 lo_page = g.need.first_position(cur) // PAGE          # oldest key the first new query reads
             first_needed_page[g.index] = lo_page
             row = g.tables[slot]
-            releasable = int(((row[:lo_page] >= 0).sum()))
-            want = [p for p in range(lo_page, pages_for(new_len)) if row[p] < 0]
-            if len(want) > g.pool.n_free + releasable:
+            releasable = int(((row[:lo_page] >= 0).sum())) if lo_page else 0
+            want = int((row[lo_page:need_hi] < 0).sum())
+            if want > g.pool.n_free + releasable:
                 raise CacheFull(f"cache group {g.index} ({g.need.kind}) has {g.pool.n_free} free pages, "
-                                f"{len(want)} more are needed; size the cache for more tokens")
+                                f"{want} more are needed; size the cache for more tokens")
         for g in self.groups:
             row = g.tables[slot]
             lo_page = first_needed_page[g.index]
-            for p in np.nonzero(row[:lo_page] >= 0)[0]:
-                g.pool.release(int(row[p]))
-                row[p] = -1
-                changed = True
-            for p in range(lo_page, pages_for(new_len)):
-                if row[p] < 0:
-                    row[p] = g.pool.alloc()
+            if lo_page:
+                old = np.nonzero(row[:lo_page] >= 0)[0]
+                if old.size:
+                    g.pool.release_all(row[old].tolist())
+                    row[old] = -1
                     changed = True
+            new = lo_page + np.nonzero(row[lo_page:need_hi] < 0)[0]
+            if new.size:
+                row[new] = g.pool.alloc_many(new.size)
+                changed = True
             g.lo[slot] = lo_page
             g.hi[slot] = max(int(g.hi[slot]), pages_for(new_len))
         if changed:

@@ -63,6 +63,25 @@ class PagePool:
         self._used.add(p)
         return p
 
+    def alloc_many(self, n: int) -> list:
+        """The pages that n calls of alloc would give, in that order."""
+        if n > len(self._free):
+            raise CacheFull(f"{n} cache pages are wanted, {len(self._free)} of {self.n} are free")
+        if n <= 0:
+            return []
+        pages = self._free[:-n - 1:-1]
+        del self._free[-n:]
+        self._used.update(pages)
+        return pages
+
+    def release_all(self, pages: list) -> None:
+        """release() of every page, in order; nothing is released if one of them is not in use."""
+        if len(set(pages)) != len(pages) or not self._used.issuperset(pages):
+            bad = next((p for p in pages if p not in self._used), None)
+            raise ValueError(f"page {bad} is not in use (released twice?)" if bad is not None else "a page is released twice")
+        self._used.difference_update(pages)
+        self._free.extend(pages)
+
     def release(self, page: int) -> None:
         if page not in self._used:
             raise ValueError(f"page {page} is not in use (released twice?)")

@@ -132,6 +132,8 @@ _SIGNATURES = {
     "sampling": {
         "oe_argmax_rows": [_P, _P, _I, _I, _P],
         "oe_argmax_rows_wide": [_P, _P, _P, _P, _I, _I, _P],
+        "oe_zero_rows": [_P, _I, _L, _I, _P],
+        "oe_sampler_start": [_P, _P, _P, _P, _I, _I, _L, _I, _P, _P],
         "oe_sample_rows": [_P, _P, _P, _I, _I, _F, _I, _F, _F, _I, _P, _P, _P, _P, _I, _I, _P],
     },
 }
@@ -1490,3 +1492,31 @@ def sample_rows(logits: torch.Tensor, out: torch.Tensor, row_slot: torch.Tensor,
         _ptr(logits), _ptr(out), _ptr(row_slot), logits.shape[0], logits.shape[1], float(temperature), int(top_k),
         float(top_p), float(repeat_penalty), int(repeat_last_n), _ptr(rng_seed), _ptr(rng_counter), _ptr(hist),
         _ptr(hist_count), cap, int(record), _stream()), "sample_rows")
+
+
+def row_table(tensors) -> tuple:
+    """What zero_rows takes of a list of contiguous tensors [slots, ...]: their addresses and the bytes of a row on the
+    device, and the largest row's bytes."""
+    rows = [t[0].numel() * t.element_size() for t in tensors]
+    if any(not t.is_contiguous() or n % 4 for t, n in zip(tensors, rows)):
+        raise KernelError("zero_rows: tensors must be contiguous, their rows a multiple of 4 bytes")
+    table = torch.tensor([[t.data_ptr(), n] for t, n in zip(tensors, rows)], dtype=torch.int64).to(tensors[0].device)
+    return table, max(rows)
+
+
+def zero_rows(table: torch.Tensor, largest: int, row: int) -> None:
+    """Zeroes row `row` of every tensor of `table` (row_table), in one launch."""
+    _check(_fn("sampling", "oe_zero_rows")(_ptr(table), table.shape[0], int(largest), int(row), _stream()), "zero_rows")
+
+
+def sampler_start(rng_seed: torch.Tensor, rng_counter: torch.Tensor, hist: torch.Tensor, hist_count: torch.Tensor, slot: int, seed: int,
+                  count: int, ring) -> None:
+    """The sampler's state of `slot` at a sequence's start, in one launch: seed, no draws yet, `count` recorded tokens and,
+    unless `ring` is None (a numpy int32 array as long as the history), the history itself."""
+    _dev(rng_seed, rng_counter, hist, hist_count)
+    if not 0 <= slot < rng_seed.numel():
+        raise IndexError(f"slot {slot} of {rng_seed.numel()}")
+    if ring is not None and (str(ring.dtype) != "int32" or ring.shape != (hist.shape[1],) or not ring.flags["C_CONTIGUOUS"]):
+        raise KernelError("sampler_start: ring must be a contiguous int32 array of the history's length")
+    _check(_fn("sampling", "oe_sampler_start")(_ptr(rng_seed), _ptr(rng_counter), _ptr(hist), _ptr(hist_count), int(hist.shape[1]), int(slot), int(seed),
+                                               int(count), None if ring is None else ring.ctypes.data, _stream()), "sampler_start")

@@ -549,9 +549,49 @@ int launch_cluster(float* logits, int* out, const int* row_slot, int rows, int V
                              repeat_pen, repeat_last, state, record);
 }
 
+// Row `row` of every tensor of a table of (address, bytes of a row), four bytes at a time.  grid (pieces, tensors)
+__global__ void __launch_bounds__(256)
+zero_rows_kernel(const long long* table, int row) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long bytes = table[2 * blockIdx.y + 1];
+    unsigned* p = (unsigned*)(table[2 * blockIdx.y] + (long long)row * bytes);
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < bytes / 4; i += (long long)gridDim.x * 256) p[i] = 0u;
+}
+
+// A sequence's first sampler state.  The recorded tokens come as a kernel argument: no copy to the device.
+struct Ring { int id[PENALTY_CAP]; };
+__global__ void __launch_bounds__(PENALTY_CAP)
+sampler_start_kernel(long long* rng_seed, int* rng_counter, int* hist, int* hist_count, int slot, long long seed, int count, int cap,
+                     int with_ring, const __grid_constant__ Ring ring) {
+    pdl_launch_dependents();
+    pdl_wait();
+    if (threadIdx.x == 0) { rng_seed[slot] = seed; rng_counter[slot] = 0; hist_count[slot] = count; }
+    if (with_ring && (int)threadIdx.x < cap) hist[(size_t)slot * cap + threadIdx.x] = ring.id[threadIdx.x];
+}
+
 }  // namespace
 
 extern "C" {
+
+int oe_zero_rows(const long long* table, int n, long long largest, int row, cudaStream_t st) {
+    if (n <= 0) return 0;
+    if (n > 65535 || row < 0 || largest < 0) return OE_ERR_UNSUPPORTED;
+    long long pieces = (largest / 4 + 1023) / 1024;
+    if (pieces < 1) pieces = 1;
+    if (pieces > 64) pieces = 64;
+    return oe_launch(zero_rows_kernel, dim3((unsigned)pieces, n), dim3(256), 0, st, table, row);
+}
+
+// ring: null, or `cap` token ids in host memory, read before the call returns.
+int oe_sampler_start(long long* rng_seed, int* rng_counter, int* hist, int* hist_count, int cap, int slot, long long seed, int count,
+                     const int* ring, cudaStream_t st) {
+    if (cap < 1 || cap > PENALTY_CAP || slot < 0) return OE_ERR_UNSUPPORTED;
+    Ring r = {};
+    if (ring) for (int i = 0; i < cap; i++) r.id[i] = ring[i];
+    return oe_launch(sampler_start_kernel, dim3(1), dim3(PENALTY_CAP), 0, st, rng_seed, rng_counter, hist, hist_count, slot, seed, count, cap,
+                     ring != nullptr ? 1 : 0, r);
+}
 
 // Wide rows in two stages; scratch: rows * 32 floats and rows * 32 ints.
 int oe_argmax_rows_wide(const float* logits, int* out, float* part_val, int* part_idx, int rows, int V, cudaStream_t st) {

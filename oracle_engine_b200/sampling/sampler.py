@@ -9,6 +9,7 @@ batch.  The kernels are in csrc/sampling.cu.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from ..csrc import ops
@@ -29,21 +30,18 @@ class Sampler:
     def start_sequence(self, slot: int, seed: int, prompt, params) -> None:
         """Seeds the slot's generator and records the prompt without its last token, as
         the reference does before generating (core/engine.cpp:118-122)."""
-        self.rng_seed[slot] = int(seed)
-        self.rng_counter[slot] = 0
-        recorded = list(prompt[:-1])
-        if params.repeat_penalty > 1.0 and recorded:
+        ring, count = None, 0
+        recorded = len(prompt) - 1
+        if params.repeat_penalty > 1.0 and recorded > 0:
             if params.repeat_last_n > HISTORY_CAPACITY:
                 raise ValueError(f"repeat_last_n {params.repeat_last_n} exceeds the {HISTORY_CAPACITY} tokens kept")
-            tail = recorded[-HISTORY_CAPACITY:]
-            count = len(recorded)
-            ring = torch.zeros(HISTORY_CAPACITY, dtype=torch.int32)
-            for j, tok in enumerate(tail):
-                ring[(count - len(tail) + j) % HISTORY_CAPACITY] = int(tok)
-            self.hist[slot].copy_(ring)
-            self.hist_count[slot] = count
-        else:
-            self.hist_count[slot] = 0
+            tail = np.asarray(prompt[max(0, recorded - HISTORY_CAPACITY):recorded], dtype=np.int32)
+            count = recorded
+            ring = np.zeros(HISTORY_CAPACITY, dtype=np.int32)
+            ring[(count - tail.size + np.arange(tail.size)) % HISTORY_CAPACITY] = tail
+        if not -2 ** 63 <= int(seed) < 2 ** 63:
+            raise OverflowError(f"seed {seed} does not fit 64 bits")
+        ops.sampler_start(self.rng_seed, self.rng_counter, self.hist, self.hist_count, slot, seed, count, ring)
 
     def sample(self, logits: torch.Tensor, row_slot: torch.Tensor, params, out: torch.Tensor | None = None):
         """logits float32 [R, V] (overwritten unless greedy without penalty); row_slot int32 [R].
