@@ -121,6 +121,9 @@ _SIGNATURES = {
         "oe_attn_latent": [_P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _L, _P],
         "oe_head_matmul": [_P, _L, _L, _P, _L, _L, _P, _I, _I, _I, _I, _P],
     },
+    "delta_step": {
+        "oe_delta_step": [_P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P],
+    },
     "recurrent": {
         "oe_short_conv_prepare": [_P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P],
         "oe_conv_state_update": [_P, _P, _I, _I, _I, _P, _P, _I, _P],
@@ -1397,6 +1400,30 @@ def delta_rule_scan(o, state, qkv, gb, ctx, kv_heads: int, heads: int, dk: int, 
     _check(_fn("recurrent", "oe_delta_rule_scan")(_ptr(o), _ptr(state), _ptr(qkv), _ptr(gb), _ptr(ctx.seq_slot),
                                                   _ptr(ctx.cu_q), ctx.n_seqs, kv_heads, heads, dk, dv, _stream()),
            "delta_rule_scan")
+
+
+def delta_step_supported(kv_heads: int, heads: int, dk: int, dv: int, taps: int) -> bool:
+    """Whether delta_step takes these sizes (csrc/delta_step.cu: oe_delta_step_supported)."""
+    return (kv_heads >= 1 and heads % kv_heads == 0 and heads // kv_heads <= 8 and 4 <= dv <= 256 and dv % 4 == 0 and dk >= 1
+            and 1 <= taps <= 8 and dk % 2 == 0 and dk <= 16 * (256 // (dv // 4)) and 2 * dk + dv <= 768)
+
+
+def delta_step(y, state, conv_state, proj, conv_w, A_log, dt_bias, norm_w, ctx, kv_heads: int, heads: int, dk: int, dv: int, q_scale: float,
+               eps: float) -> None:
+    """short_conv_prepare, conv_state_update, delta_rule_scan and head_gate (per-head norm, silu of the gate columns of
+    proj) for a step in which every sequence brings one token, in one launch; y bfloat16 [T, H dv]."""
+    _dev(y, state, conv_state, proj, conv_w, A_log, dt_bias, norm_w)
+    for t, n in ((state, "state"), (conv_state, "conv_state"), (proj, "proj"), (conv_w, "conv_w"), (A_log, "A_log"), (dt_bias, "dt_bias"),
+                 (norm_w, "norm_w")):
+        _f32c(t, n)
+    C, taps = 2 * kv_heads * dk + heads * dv, conv_w.shape[1]
+    if tuple(state.shape[1:]) != (heads, dk, dv) or conv_w.shape[0] != C or proj.shape[1] < C + heads * dv + 2 * heads \
+            or tuple(conv_state.shape[1:]) != (max(taps - 1, 1), C) or y.dtype != torch.bfloat16 or not y.is_contiguous() \
+            or tuple(y.shape) != (proj.shape[0], heads * dv) or A_log.numel() != heads or dt_bias.numel() != heads or norm_w.numel() != dv:
+        raise KernelError("delta_step: shapes do not agree")
+    _check(_fn("delta_step", "oe_delta_step")(_ptr(y), _ptr(state), _ptr(conv_state), _ptr(proj), proj.shape[1], _ptr(conv_w), taps, _ptr(A_log),
+                                              _ptr(dt_bias), _ptr(norm_w), _ptr(ctx.seq_slot), _ptr(ctx.cu_q), ctx.n_seqs, kv_heads, heads, dk, dv,
+                                              float(q_scale), float(eps), _stream()), "delta_step")
 
 
 def token_shift_mix(out, h, mu, prev_state, ctx) -> None:

@@ -66,6 +66,9 @@ class GatedDelta(Part):
         self.conv_w = torch.cat([f32(get(n[k])) for k in ("q_conv", "k_conv", "v_conv")], 0).contiguous()
         self.A_log, self.dt_bias, self.norm_w = f32(get(n["A_log"])), f32(get(n["dt_bias"])), f32(get(n["norm"]))
         self.w_o = to(get(n["o"]))
+        # a decode step's mixer in one launch (the 32-bit path keeps the walk whose bits do not depend on how a sequence is cut)
+        self.one_launch = (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores
+                           and ops.delta_step_supported(self.G, self.H, self.dk, self.dv, self.taps))
 
     def state_need(self):
         return {"S": StateNeed((self.H, self.dk, self.dv), torch.float32),
@@ -97,6 +100,12 @@ class GatedDelta(Part):
         buf = self.rt.buffer
         proj = buf("delta.proj", T, self.P, dtype=f32)
         matmul_nt(self.rt, proj, h, self.w_in)
+        if self.one_launch and ctx.all_decode and ctx.n_tokens == ctx.n_seqs:
+            y = buf("delta.y", T, vv)
+            ops.delta_step(y, state["S"], state["conv"], proj, self.conv_w, self.A_log, self.dt_bias, self.norm_w, ctx, self.G, self.H,
+                           self.dk, self.dv, self.dk ** -0.5, self.eps)
+            matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
+            return
         qkv = buf("delta.qkv", T, self.C, dtype=f32)
         gb = buf("delta.gb", T, 2 * self.H, dtype=f32)
         ops.short_conv_prepare(qkv, gb, proj, self.conv_w, state["conv"], self.A_log, self.dt_bias, ctx, self.G,
