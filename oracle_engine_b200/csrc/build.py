@@ -36,6 +36,7 @@ LIBRARIES = {
     "sampling": ("sampling.cu", []),
     "rowwise": ("rowwise.cu", []),
     "recurrent": ("recurrent.cu", []),
+    "delta_chunks": ("delta_chunks.cu", []),
     "delta_step": ("delta_step.cu", []),
     "attention_split": ("attention_split.cu", []),
     "retention": ("retention.cu", []),

@@ -124,6 +124,9 @@ _SIGNATURES = {
     "delta_step": {
         "oe_delta_step": [_P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P],
     },
+    "delta_chunks": {
+        "oe_delta_chunks": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    },
     "recurrent": {
         "oe_short_conv_prepare": [_P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P],
         "oe_conv_state_update": [_P, _P, _I, _I, _I, _P, _P, _I, _P],
@@ -1424,6 +1427,30 @@ def delta_step(y, state, conv_state, proj, conv_w, A_log, dt_bias, norm_w, ctx, 
     _check(_fn("delta_step", "oe_delta_step")(_ptr(y), _ptr(state), _ptr(conv_state), _ptr(proj), proj.shape[1], _ptr(conv_w), taps, _ptr(A_log),
                                               _ptr(dt_bias), _ptr(norm_w), _ptr(ctx.seq_slot), _ptr(ctx.cu_q), ctx.n_seqs, kv_heads, heads, dk, dv,
                                               float(q_scale), float(eps), _stream()), "delta_step")
+
+
+def delta_chunks_supported(kv_heads: int, heads: int, dk: int, dv: int) -> bool:
+    """Whether delta_chunks takes these sizes (csrc/delta_chunks.cu: oe_delta_chunks_supported)."""
+    return kv_heads >= 1 and heads % kv_heads == 0 and dk in (64, 128) and dv % 16 == 0 and 16 <= dv <= 4096
+
+
+def delta_chunks_floats(ctx, heads: int, dk: int, dv: int) -> int:
+    """Floats of scratch that delta_chunks needs for a step."""
+    return (ctx.n_tokens // 32 + ctx.n_seqs) * heads * (32 * (3 * dk + dv + 32) + 4)
+
+
+def delta_chunks(o, state, blocks, qkv, gb, ctx, kv_heads: int, heads: int, dk: int, dv: int) -> None:
+    """delta_rule_scan in chunks of 32 tokens: the same recurrence, its float32 sums in another order."""
+    _dev(o, state, blocks, qkv, gb)
+    for t, n in ((o, "o"), (state, "state"), (blocks, "blocks"), (qkv, "qkv"), (gb, "gb")):
+        _f32c(t, n)
+    T = qkv.shape[0]
+    if tuple(state.shape[1:]) != (heads, dk, dv) or tuple(o.shape) != (T, heads * dv) or T != ctx.n_tokens \
+            or qkv.shape[1] != 2 * kv_heads * dk + heads * dv or tuple(gb.shape) != (T, 2 * heads) \
+            or blocks.numel() < delta_chunks_floats(ctx, heads, dk, dv):
+        raise KernelError("delta_chunks: shapes do not agree")
+    _check(_fn("delta_chunks", "oe_delta_chunks")(_ptr(o), _ptr(state), _ptr(blocks), _ptr(qkv), _ptr(gb), _ptr(ctx.seq_slot), _ptr(ctx.cu_q), T,
+                                                  ctx.n_seqs, kv_heads, heads, dk, dv, _stream()), "delta_chunks")
 
 
 def token_shift_mix(out, h, mu, prev_state, ctx) -> None:

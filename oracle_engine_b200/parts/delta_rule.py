@@ -22,6 +22,9 @@ from .linear import matmul_nt
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
+CHUNKS_FROM = 64             # tokens of a step's longest sequence from which its scan goes in chunks
+CHUNKS_MAX_TOKENS = 16384     # (the chunks' scratch is 36 KB a token at 16 heads of 128 x 128)
+
 _NAMES = {"q": "mix.q", "k": "mix.k", "v": "mix.v", "q_conv": "mix.q.conv", "k_conv": "mix.k.conv",
           "v_conv": "mix.v.conv", "b": "mix.b", "a": "mix.a", "A_log": "mix.A_log", "dt_bias": "mix.dt_bias",
           "g": "mix.g", "norm": "mix.norm", "o": "mix.o"}
@@ -70,6 +73,9 @@ class GatedDelta(Part):
         self.one_launch = (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores
                            and ops.delta_step_supported(self.G, self.H, self.dk, self.dv, self.taps))
 
+        self.chunks = (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores
+                       and ops.delta_chunks_supported(self.G, self.H, self.dk, self.dv))
+
     def state_need(self):
         return {"S": StateNeed((self.H, self.dk, self.dv), torch.float32),
                 "conv": StateNeed((max(self.taps - 1, 1), self.C), torch.float32)}
@@ -112,7 +118,11 @@ class GatedDelta(Part):
                                self.H, self.dk, self.dv, self.dk ** -0.5)
         ops.conv_state_update(state["conv"], proj, self.C, self.taps, ctx)
         o = buf("delta.o", T, vv, dtype=f32)
-        ops.delta_rule_scan(o, state["S"], qkv, gb, ctx, self.G, self.H, self.dk, self.dv)
+        if self.chunks and CHUNKS_FROM <= ctx.max_qlen and T <= CHUNKS_MAX_TOKENS:
+            blocks = buf("delta.blocks", ops.delta_chunks_floats(ctx, self.H, self.dk, self.dv), dtype=f32)
+            ops.delta_chunks(o, state["S"], blocks, qkv, gb, ctx, self.G, self.H, self.dk, self.dv)
+        else:
+            ops.delta_rule_scan(o, state["S"], qkv, gb, ctx, self.G, self.H, self.dk, self.dv)
         y = buf("delta.y", T, vv)
         ops.head_gate(y, o, proj[:, self.C:self.C + vv], self.norm_w, self.H, self.dv, True, "silu", self.eps)
         matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
