@@ -56,6 +56,7 @@ _SIGNATURES = {
         "oe_tanh_rows": [_P, _P, _L, _P],
         "oe_head_gate": [_P, _P, _L, _P, _L, _P, _I, _I, _I, _I, _I, _I, _F, _P],
         "oe_rot_norm_kv_write": [_P, _L, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P],
+        "oe_scaled_add_norm": [_P, _P, _P, _P, _P, _F, _F, _F, _P, _I, _I, _F, _P],
         "oe_scaled_add": [_P, _P, _P, _P, _F, _F, _F, _L, _I, _P],
     },
     "attention_split": {
@@ -503,6 +504,25 @@ def scaled_add(dst: torch.Tensor, y0: torch.Tensor, vec: torch.Tensor | None = N
         raise KernelError("scaled_add: y0 and y1 of dst's shape and vec of its width expected")
     _check(_fn("rowwise", "oe_scaled_add")(_ptr(dst), _ptr(y0), _ptr(y1), _ptr(vec), float(mult), float(c0), float(c1),
                                            rows, D, _stream()), "scaled_add")
+
+
+def scaled_add_norm_supported(dst: torch.Tensor, *others) -> bool:
+    D = dst.shape[1]
+    return dst.is_cuda and D % 4 == 0 and D <= 4096 and all(t is None or t.data_ptr() % 16 == 0 for t in (dst,) + others)
+
+
+def scaled_add_norm(out: torch.Tensor, dst: torch.Tensor, y0: torch.Tensor, w: torch.Tensor, eps: float, vec: torch.Tensor | None = None,
+                    mult: float = 1.0, c0: float = 1.0, y1: torch.Tensor | None = None, c1: float = 0.0) -> None:
+    """scaled_add(dst, y0, vec, mult, c0, y1, c1), then out = rmsnorm(dst, w, eps) as bfloat16, in one launch."""
+    _dev(out, dst, y0, y1, vec, w)
+    for t, n in ((dst, "dst"), (y0, "y0"), (w, "w")) + (((y1, "y1"),) if y1 is not None else ()) + (((vec, "vec"),) if vec is not None else ()):
+        _f32c(t, n)
+    rows, D = dst.shape
+    if y0.shape != dst.shape or (y1 is not None and y1.shape != dst.shape) or (vec is not None and vec.numel() != D) or w.numel() != D \
+            or out.shape != dst.shape or out.dtype != torch.bfloat16 or not out.is_contiguous():
+        raise KernelError("scaled_add_norm: y0, y1 and out of dst's shape, vec and w of its width expected")
+    _check(_fn("rowwise", "oe_scaled_add_norm")(_ptr(out), _ptr(dst), _ptr(y0), _ptr(y1), _ptr(vec), float(mult), float(c0), float(c1), _ptr(w),
+                                                rows, D, float(eps), _stream()), "scaled_add_norm")
 
 
 # ---------------------------------------------------------------------------------------- attention_split.cu

@@ -347,6 +347,70 @@ int rot_norm_launch(T* qk, long long row_stride, const float* inv_freq, int rot_
 }
 
 
+// dst += mult * vec * (c0 y0 + c1 y1) and y = norm(dst) * w in one pass over the stream, a block a row (D a multiple of 4 up
+// to 4,096, kept in registers): the norm that reads what a sublayer's output was just added to.  Bound by the bytes: 1,500
+// rows of 2,048, two outputs, 15 us as two launches of which the second reads the stream again.
+__global__ void __launch_bounds__(256)
+scaled_add_norm_kernel(bf16* out, float* dst, const float* y0, const float* y1, const float* __restrict__ vec, float mult, float c0,
+                       float c1, const float* __restrict__ w, int D, float eps) {
+    __shared__ float red[32];
+    constexpr int KEEP = 4;
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t row = (size_t)blockIdx.x * D;
+    const int n4 = D / 4;
+    float4 x[KEEP];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < KEEP; j++) {
+        const int i = threadIdx.x + j * 256;
+        x[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i >= n4) continue;
+        const float4 a = reinterpret_cast<const float4*>(y0 + row)[i], d = reinterpret_cast<const float4*>(dst + row)[i];
+        float4 v = make_float4(c0 * a.x, c0 * a.y, c0 * a.z, c0 * a.w);
+        if (y1) {
+            const float4 b = reinterpret_cast<const float4*>(y1 + row)[i];
+            v.x = fmaf(c1, b.x, v.x); v.y = fmaf(c1, b.y, v.y); v.z = fmaf(c1, b.z, v.z); v.w = fmaf(c1, b.w, v.w);
+        }
+        float4 s = make_float4(mult, mult, mult, mult);
+        if (vec) {
+            const float4 q = reinterpret_cast<const float4*>(vec)[i];
+            s.x *= q.x; s.y *= q.y; s.z *= q.z; s.w *= q.w;
+        }
+        x[j] = make_float4(fmaf(s.x, v.x, d.x), fmaf(s.y, v.y, d.y), fmaf(s.z, v.z, d.z), fmaf(s.w, v.w, d.w));
+        reinterpret_cast<float4*>(dst + row)[i] = x[j];
+        ss += x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
+    }
+    ss = block_sum(ss, red);
+    const float s = 1.f / sqrtf(ss / (float)D + eps);
+#pragma unroll
+    for (int j = 0; j < KEEP; j++) {
+        const int i = threadIdx.x + j * 256;
+        if (i >= n4) continue;
+        const float4 g = reinterpret_cast<const float4*>(w)[i];
+        const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[j].x * s * g.x, x[j].y * s * g.y), __floats2bfloat162_rn(x[j].z * s * g.z, x[j].w * s * g.w)};
+        reinterpret_cast<uint2*>(out + row)[i] = *reinterpret_cast<const uint2*>(h);
+    }
+}
+
+__global__ void __launch_bounds__(256)
+scaled_add4_kernel(float4* dst, const float4* y0, const float4* y1, const float4* __restrict__ vec, float mult, float c0, float c1, int rows, int n4) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int r = blockIdx.y; r < rows; r += gridDim.y)
+        for (int i = blockIdx.x * 256 + threadIdx.x; i < n4; i += gridDim.x * 256) {
+            const size_t at = (size_t)r * n4 + i;
+            const float4 a = y0[at], d = dst[at];
+            float4 v = make_float4(c0 * a.x, c0 * a.y, c0 * a.z, c0 * a.w), s = make_float4(mult, mult, mult, mult);
+            if (y1) {
+                const float4 b = y1[at];
+                v.x = fmaf(c1, b.x, v.x); v.y = fmaf(c1, b.y, v.y); v.z = fmaf(c1, b.z, v.z); v.w = fmaf(c1, b.w, v.w);
+            }
+            if (vec) { const float4 q = vec[i]; s.x *= q.x; s.y *= q.y; s.z *= q.z; s.w *= q.w; }
+            dst[at] = make_float4(fmaf(s.x, v.x, d.x), fmaf(s.y, v.y, d.y), fmaf(s.z, v.z, d.z), fmaf(s.w, v.w, d.w));
+        }
+}
+
 __global__ void __launch_bounds__(256)
 scaled_add_kernel(float* dst, const float* y0, const float* y1, const float* __restrict__ vec, float mult, float c0,
                   float c1, size_t total, int D) {
@@ -368,10 +432,24 @@ int oe_scaled_add(float* dst, const float* y0, const float* y1, const float* vec
                   long long rows, int D, cudaStream_t st) {
     if (rows <= 0) return 0;
     if (D < 1) return OE_ERR_UNSUPPORTED;
+    if (D % 4 == 0 && rows <= 2147483647LL && (((uintptr_t)dst | (uintptr_t)y0 | (uintptr_t)y1 | (uintptr_t)vec) & 15) == 0) {
+        // four values a thread and no division per value (2,048 columns: 4,096 rows 34 us with one value a thread)
+        const int n4 = D / 4;
+        return oe_launch(scaled_add4_kernel, dim3((n4 + 255) / 256, (unsigned)(rows < 65535 ? rows : 65535)), dim3(256), 0, st, (float4*)dst,
+                         (const float4*)y0, (const float4*)y1, (const float4*)vec, mult, c0, c1, (int)rows, n4);
+    }
     const size_t total = (size_t)rows * D;
     size_t blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     return oe_launch(scaled_add_kernel, dim3((unsigned)blocks), dim3(256), 0, st, dst, y0, y1, vec, mult, c0, c1, total, D);
+}
+
+int oe_scaled_add_norm(bf16* out, float* dst, const float* y0, const float* y1, const float* vec, float mult, float c0, float c1, const float* w,
+                       int rows, int D, float eps, cudaStream_t st) {
+    if (rows <= 0) return 0;
+    if (D < 4 || D % 4 || D > 4096) return OE_ERR_UNSUPPORTED;
+    if ((((uintptr_t)dst | (uintptr_t)y0 | (uintptr_t)y1 | (uintptr_t)vec | (uintptr_t)w) & 15) || ((uintptr_t)out & 7)) return OE_ERR_UNSUPPORTED;
+    return oe_launch(scaled_add_norm_kernel, dim3(rows), dim3(256), 0, st, out, dst, y0, y1, vec, mult, c0, c1, w, D, eps);
 }
 
 int oe_cast_rows_bf16(bf16* y, const float* x, long long total, cudaStream_t st) {

@@ -256,24 +256,32 @@ class PreNormScaledBlock:
     def first_weights(self):
         return _first_weights(self.mixer)
 
-    def _sublayer(self, part, key, h, x, *args):
+    def _sublayer(self, part, key, h, x, *args, norm=None):
+        """Adds the sublayer's scaled output; returns norm.forward(x) of the new stream where a norm is given."""
         vec = self.scales.vec.get(key)
+        fused = norm if hasattr(norm, "after_scaled_add") else None
         if getattr(part, "can_scale", False):
+            if fused is not None and getattr(part, "can_norm", False):
+                return part.forward(h, x, *args, scale=(self.mult, vec), norm=fused)
             part.forward(h, x, *args, scale=(self.mult, vec))
-            return
+            return norm.forward(x) if norm is not None else None
         y = self.rt.buffer("sublayer_out", *x.shape, dtype=torch.float32)
         if getattr(part, "can_overwrite", False):
             part.forward(h, y, *args, overwrite=True)
         else:
             y.zero_()
             part.forward(h, y, *args)
+        if fused is not None:
+            return fused.after_scaled_add(x, y, vec, self.mult)
         ops.scaled_add(x, y, vec, self.mult)
+        return norm.forward(x) if norm is not None else None
 
     def forward(self, x, ctx, cache, state, owns_cache=True):
         self.rt.next_weights = None
-        self._sublayer(self.mixer, "mixer", self.mixer_norm.forward(x), x, ctx, cache, state, owns_cache)
+        h = self._sublayer(self.mixer, "mixer", self.mixer_norm.forward(x), x, ctx, cache, state, owns_cache,
+                           norm=self.ffn_norm if self.feed_forward is not None else None)
         if self.feed_forward is not None:
-            self._sublayer(self.feed_forward, "ffn", self.ffn_norm.forward(x), x, ctx)
+            self._sublayer(self.feed_forward, "ffn", h, x, ctx)
 
 
 class TokenSide(Part):

@@ -51,6 +51,15 @@ class RMSNorm(Part):
             ops.rmsnorm(y, x, self.weight, self.eps)
         return y
 
+    def after_scaled_add(self, x, y0, vec, mult, c0=1.0, y1=None, c1=0.0):
+        """x += mult * vec * (c0 y0 + c1 y1), then forward(x): in one kernel on the bfloat16 path where it takes the sizes."""
+        if self.groups == 1 and self.rt.dtype != x.dtype and ops.scaled_add_norm_supported(x, y0, y1, vec, self.weight):
+            y = self.rt.empty(*x.shape)
+            ops.scaled_add_norm(y, x, y0, self.weight, self.eps, vec, mult, c0, y1, c1)
+            return y
+        ops.scaled_add(x, y0, vec, mult, c0, y1, c1)
+        return self.forward(x)
+
     def add_into(self, dst, y, coef: float = 1.0, accumulate: bool = True, keep_cast: bool = False) -> None:
         """dst (+)= coef * norm(y); dst and y float32 of one shape.  keep_cast: on the bfloat16 path the kernel
         also leaves the new dst rounded to bfloat16 for the sublayer that reads it next (Runtime.activations)."""

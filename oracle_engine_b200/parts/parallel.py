@@ -49,7 +49,7 @@ class ParallelMixers(Part):
         self.weighted = self.coefs[0] is not None
         if any((c is not None) != self.weighted for c in self.coefs):
             raise ValueError("parallel_mixers: either every branch has an output norm or none has")
-        self.can_scale = self.weighted
+        self.can_scale = self.can_norm = self.weighted
         if sum(1 for _, m, _ in self.branches if m.cache_need() is not None) > 1:
             raise ValueError("parallel_mixers: only one branch may keep a paged cache")
         self.graph_safe = all(getattr(m, "graph_safe", False) for _, m, _ in self.branches)
@@ -140,7 +140,7 @@ class ParallelMixers(Part):
             out.append((y, self.out_w[tag]))
         return out
 
-    def _forward_weighted(self, h, residual, ctx, cache, state, owns_cache, overwrite, scale):
+    def _forward_weighted(self, h, residual, ctx, cache, state, owns_cache, overwrite, scale, norm=None):
         mult, vec = scale if scale is not None else (1.0, None)
         if overwrite:
             residual.zero_()
@@ -151,16 +151,21 @@ class ParallelMixers(Part):
             ys.append(y)
         for i in range(0, len(ys), 2):               # two outputs a kernel
             two = i + 1 < len(ys)
+            if norm is not None and i + 2 >= len(ys):
+                return norm.after_scaled_add(residual, ys[i], vec, mult, self.coefs[i], ys[i + 1] if two else None,
+                                             self.coefs[i + 1] if two else 0.0)
             ops.scaled_add(residual, ys[i], vec, mult, self.coefs[i], ys[i + 1] if two else None,
                            self.coefs[i + 1] if two else 0.0)
 
-    def forward(self, h, residual, ctx, cache, state, owns_cache=True, overwrite: bool = False, scale=None):
+    def forward(self, h, residual, ctx, cache, state, owns_cache=True, overwrite: bool = False, scale=None,
+                norm=None):
         """overwrite: the output is written into `residual` (float32) instead of added.  scale = (m, s): the output
         is multiplied by the constant m and, per channel, by the float32 vector s (or None) before it is added
-        (the weighted form only)."""
+        (the weighted form only).  norm (the weighted form only): a norm with `after_scaled_add`; its output for the new
+        residual is returned."""
         if self.weighted:
-            return self._forward_weighted(h, residual, ctx, cache, state, owns_cache, overwrite, scale)
-        if scale is not None:
+            return self._forward_weighted(h, residual, ctx, cache, state, owns_cache, overwrite, scale, norm)
+        if scale is not None or norm is not None:
             raise ValueError("parallel_mixers: branches with output norms take no scale")
         coef = 1.0 / len(self.branches)
         y = self.rt.buffer("parallel.branch_out", h.shape[0], self.D, dtype=torch.float32)
