@@ -341,6 +341,8 @@ attn_split_mma_kernel(const Args a) {
     }
 }
 
+constexpr int MAX_SPLITS = 256;
+
 // One block per (token, head): the splits' sums put together in split order.  Maxima are in units of log2(e).
 __global__ void __launch_bounds__(128)
 attn_split_merge_kernel(bf16* out, const float* partial, int n_splits, const int* __restrict__ seq_qlen, int H,
@@ -354,33 +356,44 @@ attn_split_merge_kernel(bf16* out, const float* partial, int n_splits, const int
         return;
     }
     const float* p = partial + (size_t)blockIdx.x * n_splits * (DV + 2);
+    // Every split's weight at once, a lane a split, and then sums whose loads do not wait for one another: split after split
+    // the two passes were chains of 17 loads each (4 of the 11 us of a decode step's attention at 1,024 keys).  A split
+    // without a key has weight zero and its sums, which nothing has written, are not used.
+    __shared__ float f[MAX_SPLITS], f_inv;
     // a sink counts as one more split: maximum sinks[h] (in units of log2(e)), denominator 1, no values
     const float sk = sinks ? sinks[blockIdx.x % H] * 1.4426950408889634f : -INFINITY;
-    float m = sk;
-    for (int s = 0; s < n_splits; s++) m = fmaxf(m, p[(size_t)s * (DV + 2) + DV]);
-    float l = sinks ? exp2f(sk - m) : 0.f;
-    for (int s = 0; s < n_splits; s++) {
-        const float ms = p[(size_t)s * (DV + 2) + DV];
-        if (ms != -INFINITY) l += exp2f(ms - m) * p[(size_t)s * (DV + 2) + DV + 1];
+    if (threadIdx.x < 32) {
+        float m = sk;
+        for (int s = threadIdx.x; s < n_splits; s += 32) m = fmaxf(m, p[(size_t)s * (DV + 2) + DV]);
+        m = warp_max(m);
+        float l = 0.f;
+        for (int s = threadIdx.x; s < n_splits; s += 32) {
+            const float ms = p[(size_t)s * (DV + 2) + DV], ls = p[(size_t)s * (DV + 2) + DV + 1];
+            const float w = ms != -INFINITY ? exp2f(ms - m) : 0.f;
+            f[s] = w;
+            if (ms != -INFINITY) l = fmaf(w, ls, l);
+        }
+        l = warp_sum(l) + (sinks ? exp2f(sk - m) : 0.f);
+        if (threadIdx.x == 0) f_inv = l > 0.f ? 1.f / l : 0.f;
     }
-    float inv = l > 0.f ? 1.f / l : 0.f;
+    __syncthreads();
+    auto sum = [&](int d) {
+        float acc = 0.f;
+#pragma unroll 8
+        for (int s = 0; s < n_splits; s++) {
+            const float w = f[s], v = p[(size_t)s * (DV + 2) + d];
+            acc = fmaf(w, w != 0.f ? v : 0.f, acc);
+        }
+        return acc;
+    };
+    float inv = f_inv;
     const int gt = blockIdx.x / H, gh = blockIdx.x % H;          // token and head
     if (gate_mode == OE_GATE_HEAD) inv *= oe_sigmoid_gate(gate, gate_stride, gate_mode, gt, gh, H, DV, 0);
     if (unrot_cos != nullptr) {
         // the sequence's one token stands at position seq_start; a thread takes a pair (d, d + DV/2) and turns it back
         const size_t at = (size_t)seq_start[blockIdx.x / H] * (DV / 2);
         for (int d = threadIdx.x; d < DV / 2; d += blockDim.x) {
-            float u = 0.f, v = 0.f;
-            for (int s = 0; s < n_splits; s++) {
-                const float ms = p[(size_t)s * (DV + 2) + DV];
-                if (ms != -INFINITY) {
-                    const float f = exp2f(ms - m);
-                    u = fmaf(f, p[(size_t)s * (DV + 2) + d], u);
-                    v = fmaf(f, p[(size_t)s * (DV + 2) + d + DV / 2], v);
-                }
-            }
-            u *= inv;
-            v *= inv;
+            const float u = sum(d) * inv, v = sum(d + DV / 2) * inv;
             const float c = unrot_cos[at + d], sn = unrot_sin[at + d];
             out[(size_t)blockIdx.x * DV + d] = __float2bfloat16_rn(u * c + v * sn);
             out[(size_t)blockIdx.x * DV + d + DV / 2] = __float2bfloat16_rn(v * c - u * sn);
@@ -388,12 +401,7 @@ attn_split_merge_kernel(bf16* out, const float* partial, int n_splits, const int
         return;
     }
     for (int d = threadIdx.x; d < DV; d += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < n_splits; s++) {
-            const float ms = p[(size_t)s * (DV + 2) + DV];
-            if (ms != -INFINITY) acc = fmaf(exp2f(ms - m), p[(size_t)s * (DV + 2) + d], acc);
-        }
-        acc *= inv;
+        float acc = sum(d) * inv;
         if (gate_mode == OE_GATE_VALUE) acc *= oe_sigmoid_gate(gate, gate_stride, gate_mode, gt, gh, H, DV, d);
         out[(size_t)blockIdx.x * DV + d] = __float2bfloat16_rn(acc);
     }
@@ -413,7 +421,7 @@ int oe_attn_split_mma(bf16* out, const bf16* q, long long q_stride, const bf16* 
                       long long gate_stride, int gate_mode, cudaStream_t st) {
     if (n_seqs <= 0 || max_qlen <= 0) return 0;
     if (KVH < 1 || H % KVH || H / KVH > NWARPS * 16 || n_seqs > 65535 || KVH > 65535) return OE_ERR_UNSUPPORTED;
-    if (n_splits > 1 && (max_qlen != 1 || partial == nullptr)) return OE_ERR_UNSUPPORTED;
+    if (n_splits > 1 && (max_qlen != 1 || partial == nullptr || n_splits > MAX_SPLITS)) return OE_ERR_UNSUPPORTED;
     Args a;
     a.out = out; a.q = q; a.q_stride = q_stride; a.kcache = kcache; a.vcache = vcache; a.tables = tables;
     a.max_pages = max_pages; a.cu_q = cu_q; a.seq_start = seq_start; a.seq_qlen = seq_qlen;
