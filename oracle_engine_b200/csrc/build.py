@@ -36,6 +36,7 @@ LIBRARIES = {
     "sampling": ("sampling.cu", []),
     "rowwise": ("rowwise.cu", []),
     "recurrent": ("recurrent.cu", []),
+    "decay_chunks": ("decay_chunks.cu", []),
     "delta_chunks": ("delta_chunks.cu", []),
     "delta_step": ("delta_step.cu", []),
     "attention_split": ("attention_split.cu", []),

@@ -128,6 +128,9 @@ _SIGNATURES = {
     "delta_chunks": {
         "oe_delta_chunks": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     },
+    "decay_chunks": {
+        "oe_decay_chunks": [_P, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _P],
+    },
     "recurrent": {
         "oe_short_conv_prepare": [_P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _P],
         "oe_conv_state_update": [_P, _P, _I, _I, _I, _P, _P, _I, _P],
@@ -1499,9 +1502,8 @@ def last_rows_to_state(state, h, ctx) -> None:
            "last_rows_to_state")
 
 
-def decay_scan(o, state, r, k, v, z, u, w0, ctx, heads: int, d: int) -> None:
-    """Per sequence and head, over the step's tokens in order: o = (S + diag(u) k v^T)^T r;
-    S <- diag(w) S + k v^T with w = exp(-exp(z + w0)).  r, k, v, z: float32 [T, H d] with one common row stride."""
+def _decay_operands(o, state, r, k, v, z, u, w0, heads: int, d: int) -> int:
+    """The row stride that r, k, v and z share."""
     _dev(o, state, r, k, v, z, u, w0)
     for t, n in ((o, "o"), (state, "state"), (u, "u"), (w0, "w0")):
         _f32c(t, n)
@@ -1513,9 +1515,37 @@ def decay_scan(o, state, r, k, v, z, u, w0, ctx, heads: int, d: int) -> None:
     if tuple(state.shape[1:]) != (heads, d, d) or tuple(o.shape) != (T, heads * d) or u.numel() != heads * d \
             or w0.numel() != heads * d:
         raise KernelError("decay_scan: shapes do not agree")
+    return stride
+
+
+def decay_scan(o, state, r, k, v, z, u, w0, ctx, heads: int, d: int) -> None:
+    """Per sequence and head, over the step's tokens in order: o = (S + diag(u) k v^T)^T r;
+    S <- diag(w) S + k v^T with w = exp(-exp(z + w0)).  r, k, v, z: float32 [T, H d] with one common row stride."""
+    stride = _decay_operands(o, state, r, k, v, z, u, w0, heads, d)
     _check(_fn("recurrent", "oe_decay_scan")(_ptr(o), _ptr(state), _ptr(r), _ptr(k), _ptr(v), _ptr(z), stride, _ptr(u),
                                              _ptr(w0), _ptr(ctx.seq_slot), _ptr(ctx.cu_q), ctx.n_seqs, heads, d,
                                              _stream()), "decay_scan")
+
+
+def decay_chunks_supported(d: int) -> bool:
+    """Whether decay_chunks takes heads of this size."""
+    return d in (64, 128)
+
+
+def decay_chunks_floats(ctx, heads: int, d: int) -> int:
+    """Floats of scratch that decay_chunks needs for a step."""
+    return (ctx.n_tokens // 32 + ctx.n_seqs) * heads * (32 * (3 * d + 32) + d)
+
+
+def decay_chunks(o, state, blocks, r, k, v, z, u, w0, ctx, heads: int, d: int) -> None:
+    """decay_scan in chunks of 32 tokens: the same recurrence, its float32 sums in another order."""
+    stride = _decay_operands(o, state, r, k, v, z, u, w0, heads, d)
+    _f32c(blocks, "blocks")
+    if r.shape[0] != ctx.n_tokens or blocks.numel() < decay_chunks_floats(ctx, heads, d):
+        raise KernelError("decay_chunks: shapes do not agree")
+    _check(_fn("decay_chunks", "oe_decay_chunks")(_ptr(o), _ptr(state), _ptr(blocks), _ptr(r), _ptr(k), _ptr(v), _ptr(z), stride, _ptr(u), _ptr(w0),
+                                                  _ptr(ctx.seq_slot), _ptr(ctx.cu_q), ctx.n_tokens, ctx.n_seqs, heads, d, _stream()),
+           "decay_chunks")
 
 
 _argmax_scratch: dict = {}

@@ -19,6 +19,20 @@ from .linear import matmul_nt
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
+CHUNKS_MAX_TOKENS = 16384    # (the chunks' scratch is 29 KB a token at 32 heads of 64)
+
+
+def chunked(tokens: int, longest: int, heads: int, d: int) -> bool:
+    """Whether the scan of a step goes in chunks (csrc/decay_chunks.cu) or walks (csrc/recurrent.cu).  One sequence alone is
+    bound by its chain of tokens or chunks, many by the additions, which the chunks have more of.  us, walk / chunks, 32 heads
+    of 64: one sequence of 64 25 / 26, 96 36 / 31, 256 90 / 61, 1,111 379 / 227; 8 of 300 234 / 244, 16 of 64 91 / 103, 32 of
+    40 115 / 189; 4 of 1 to 4,096 2,129 / 614.  8 heads of 128: one of 48 27 / 28, 64 35 / 28, 1,111 553 / 157; 8 of 300
+    220 / 154, 16 of 64 99 / 74."""
+    if longest < 64 or tokens > CHUNKS_MAX_TOKENS:
+        return False
+    return d >= 128 or (longest >= 96 and tokens * heads <= 96 * longest)
+
+
 _MIXES = ("r", "k", "v", "g", "w")
 _NAMES = {"r": "r", "k": "k", "v": "v", "g": "g", "w1": "w1", "w2": "w2", "w0": "w0", "u": "u", "norm": "norm", "o": "o",
           **{"mu_" + s: "mu." + s for s in _MIXES}}
@@ -95,7 +109,13 @@ class DecayTimeMix(Part):
         ops.tanh_rows(th, low)
         matmul_nt(self.rt, z, th, self.w["w2"])
         o = buf("mix.o", T, hd, dtype=f32)
-        ops.decay_scan(o, state["S"], r, k, v, z, self.u, self.w0, ctx, self.H, self.d)
+        # prompts in chunks (the 32-bit path keeps the walk whose bits do not depend on how a sequence is cut)
+        if self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores and ops.decay_chunks_supported(self.d) \
+                and chunked(T, ctx.max_qlen, self.H, self.d):
+            blocks = buf("mix.blocks", ops.decay_chunks_floats(ctx, self.H, self.d), dtype=f32)
+            ops.decay_chunks(o, state["S"], blocks, r, k, v, z, self.u, self.w0, ctx, self.H, self.d)
+        else:
+            ops.decay_scan(o, state["S"], r, k, v, z, self.u, self.w0, ctx, self.H, self.d)
         y = buf("mix.y", T, hd)
         ops.head_gate(y, o, g, self.norm_w, self.H, self.d, True, "silu", self.eps)
         matmul_nt(self.rt, residual, y, self.w["o"], accumulate=not overwrite)
