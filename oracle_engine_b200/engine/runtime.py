@@ -43,6 +43,7 @@ class Runtime:
     # that runs first puts them here, the others find them.  While a CUDA graph is captured they are the graph's memory.
     pass_store: dict = field(default_factory=dict, repr=False)
     _buffers: dict = field(default_factory=dict, repr=False)
+    _side: object = None               # the second stream of `fork`
     _cast_turn: int = 0
 
     def empty(self, *shape, dtype=None) -> torch.Tensor:
@@ -69,6 +70,27 @@ class Runtime:
             flat = torch.empty(max(n + n // 4, 1), dtype=dtype, device=self.device)
             self._buffers[key] = flat
         return flat[:n].view(*shape)
+
+    def fork(self, first, second) -> None:
+        """first() on the current stream and second() beside it on a second one, both behind what the current stream holds;
+        what follows on the current stream waits for both.  Only while a CUDA graph is captured, where they become two
+        branches of the graph.  What both touch must be made before, and every tensor that second() is handed or that is read
+        afterwards must be the current stream's own and outlive the call; what second() allocates for itself is taken from
+        the graph's memory of the second stream, which only later calls of second() use again."""
+        if not torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("fork: only while a CUDA graph is captured")
+        if self._side is None:
+            self._side = torch.cuda.Stream(self.device)
+        main, begin, end = torch.cuda.current_stream(self.device), torch.cuda.Event(), torch.cuda.Event()
+        begin.record(main)
+        self._side.wait_event(begin)
+        try:
+            with torch.cuda.stream(self._side):
+                second()
+            first()
+        finally:
+            end.record(self._side)             # the capture ends on the current stream, whatever happened
+            main.wait_event(end)
 
     def activations(self, x: torch.Tensor) -> torch.Tensor:
         """The float32 residual stream as a sublayer's input: itself on the 32-bit path (the sublayer

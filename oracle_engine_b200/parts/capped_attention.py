@@ -26,6 +26,7 @@ _NAMES = {"q": "q", "k": "k", "v": "v", "o": "o"}
 @MIXERS.register("capped_attention")
 class CappedAttention(Part):
     graph_safe = True
+    runs_beside = True
     can_overwrite = True
     """params: hidden_size, num_heads, num_kv_heads, key_dim, value_dim, scale, softcap (0 or None: no cap),
     window (0 or None: all keys), chunk (0 or None: no chunks; not with a window), reads_cache (no Wk and Wv), position

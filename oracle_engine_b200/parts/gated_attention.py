@@ -28,6 +28,7 @@ _NAMES = {"q": "q", "k": "k", "v": "v", "g": "g", "o": "o", "q_norm": "q.norm", 
 @MIXERS.register("gated_attention")
 class GatedAttention(Part):
     graph_safe = True
+    runs_beside = True
     can_overwrite = True
     """params: hidden_size, num_heads, num_kv_heads, key_dim, value_dim, scale, eps, window (0 or None: all keys), chunk
     (chunks of positions instead of a window), position (a `rotary` encoding whose head_dim is the number of turned

@@ -19,10 +19,13 @@ from __future__ import annotations
 
 import torch
 
-from ..csrc import ops
+from ..csrc import ops, ops_tc
 from .linear import chain_flags, matmul_nt
 from .registry import MIXERS, Part
 from .spec import TensorDecl
+
+
+FORK_TOKENS = 16             # rows of a captured decode step up to which two branches run beside each other
 
 
 @MIXERS.register("parallel_mixers")
@@ -53,6 +56,8 @@ class ParallelMixers(Part):
         if sum(1 for _, m, _ in self.branches if m.cache_need() is not None) > 1:
             raise ValueError("parallel_mixers: only one branch may keep a paged cache")
         self.graph_safe = all(getattr(m, "graph_safe", False) for _, m, _ in self.branches)
+        self.two_streams = runtime.device.type == "cuda" and len(self.branches) == 2 \
+            and all(vars(type(m)).get("runs_beside", False) for _, m, _ in self.branches)
         self.out_w = {}
         self.w_joined, self.columns = None, []
 
@@ -128,27 +133,42 @@ class ParallelMixers(Part):
             y.zero_()
             m.forward(h, y, ctx, cache, own, owns_cache, **projected)
 
+    def _branches_into(self, ys, h, ctx, cache, state, owns_cache) -> None:
+        """Every branch's output in its own buffer of `ys`.  Two branches of a decode step that is being captured become two
+        branches of the graph: their kernels are short and their chains independent, so the shorter chain runs in what the
+        longer one leaves idle.  Only up to 16 rows: products of more share the one-SM tcgen05 kernel's split-K workspace.
+        Measured with 8 layers of width 2,048, one after the other / beside (a prompt and 24 decode steps): Fovirax, one
+        sequence of 1,500 tokens, 18.74 / 16.47 ms; Fuvipel, one of 1,111, two of eight layers with branches,
+        14.30 / 13.33 ms; Mavinex, eight of up to 900, 25.85 / 25.52 ms."""
+        projected = self._projected(h)
+
+        def run(i):
+            self._branch_into(i, ys[i], h, ctx, cache, state, owns_cache, projected[i])
+        if self.two_streams and h.shape[0] <= min(FORK_TOKENS, ops_tc.SKINNY_MAX_TOKENS) and ctx.all_decode \
+                and torch.cuda.is_current_stream_capturing():
+            self.rt.fork(lambda: run(0), lambda: run(1))
+            return
+        for i in range(len(ys)):
+            run(i)
+
+    def _outputs(self, h):
+        return [self.rt.buffer(f"parallel.branch_out{i}", h.shape[0], self.D, dtype=torch.float32) for i in range(len(self.branches))]
+
     def normed_outputs(self, h, ctx, cache, state, owns_cache=True):
         """[(a branch's output [T, hidden] float32, its norm's weight)]: the caller norms each with `eps` and takes their
         mean.  None where the branches are not two with output norms."""
         if self.weighted or len(self.branches) != 2:
             return None
-        out = []
-        for i, (projected, (tag, _, _)) in enumerate(zip(self._projected(h), self.branches)):
-            y = self.rt.buffer(f"parallel.branch_out{i}", h.shape[0], self.D, dtype=torch.float32)
-            self._branch_into(i, y, h, ctx, cache, state, owns_cache, projected)
-            out.append((y, self.out_w[tag]))
-        return out
+        ys = self._outputs(h)
+        self._branches_into(ys, h, ctx, cache, state, owns_cache)
+        return [(y, self.out_w[tag]) for y, (tag, _, _) in zip(ys, self.branches)]
 
     def _forward_weighted(self, h, residual, ctx, cache, state, owns_cache, overwrite, scale, norm=None):
         mult, vec = scale if scale is not None else (1.0, None)
         if overwrite:
             residual.zero_()
-        ys = []
-        for i, projected in enumerate(self._projected(h)):
-            y = self.rt.buffer(f"parallel.branch_out{i}", h.shape[0], self.D, dtype=torch.float32)
-            self._branch_into(i, y, h, ctx, cache, state, owns_cache, projected)
-            ys.append(y)
+        ys = self._outputs(h)
+        self._branches_into(ys, h, ctx, cache, state, owns_cache)
         for i in range(0, len(ys), 2):               # two outputs a kernel
             two = i + 1 < len(ys)
             if norm is not None and i + 2 >= len(ys):
@@ -168,7 +188,7 @@ class ParallelMixers(Part):
         if scale is not None or norm is not None:
             raise ValueError("parallel_mixers: branches with output norms take no scale")
         coef = 1.0 / len(self.branches)
-        y = self.rt.buffer("parallel.branch_out", h.shape[0], self.D, dtype=torch.float32)
-        for i, (projected, (tag, _, _)) in enumerate(zip(self._projected(h), self.branches)):
-            self._branch_into(i, y, h, ctx, cache, state, owns_cache, projected)
+        ys = self._outputs(h)
+        self._branches_into(ys, h, ctx, cache, state, owns_cache)
+        for i, (y, (tag, _, _)) in enumerate(zip(ys, self.branches)):
             ops.rmsnorm_add(residual, y, self.out_w[tag], self.eps, coef, accumulate=not (overwrite and i == 0))

@@ -110,6 +110,10 @@ HEADS = Registry("output head")
 class Part:
     """Base of every part: holds params, prefix and runtime; no weights by default."""
     kind = "?"
+    # Whether a forward pass of the part writes only its residual, its own cache and state and memory that it asks the
+    # runtime for: then another part's forward may run beside it on a second stream (Runtime.fork).  Not inherited: a class
+    # says it of its own forward.
+    runs_beside = False
 
     def __init__(self, params: dict, prefix: str, runtime):
         self.params = dict(params)

@@ -28,6 +28,7 @@ CHUNK_FROM = 16         # a step whose longest sequence brings fewer tokens goes
 @MIXERS.register("retention")
 class Retention(Part):
     graph_safe = True
+    runs_beside = True
     can_overwrite = True
     """params: hidden_size, num_heads, key_dim, value_dim, decay (one number per head), eps (of the read-out's
     norm), position (a `rotary` encoding whose head_dim is the number of turned dimensions, or None),

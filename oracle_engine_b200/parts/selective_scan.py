@@ -43,6 +43,7 @@ def segment_plan(C: int, N: int, n_seqs: int, longest: int) -> tuple | None:
 @MIXERS.register("selective_scan")
 class SelectiveScan(Part):
     graph_safe = True
+    runs_beside = True
     can_overwrite = True
     """params: hidden_size, inner (C), state (N), dt_rank, conv_taps, tensor_names (optional overrides)."""
 

@@ -27,6 +27,7 @@ _NAMES = {"q": "q", "k": "k", "g": "g", "o": "o"}
 @MIXERS.register("sink_attention")
 class SinkAttention(Part):
     graph_safe = True
+    runs_beside = True
     """params: hidden_size, num_heads, num_kv_heads, head_dim, scale, eps (of the q/k norm), position (a
     `rotary_pairs` encoding or None), window (0 = all keys), gate (True: the output gate sigmoid(Wg h)),
     tensor_names (optional overrides)."""

@@ -41,6 +41,7 @@ _NAMES = {"r": "r", "k": "k", "v": "v", "g": "g", "w1": "w1", "w2": "w2", "w0": 
 @MIXERS.register("decay_time_mix")
 class DecayTimeMix(Part):
     graph_safe = True
+    runs_beside = True
     """params: hidden_size, num_heads, head_dim, eps (of the read-out's norm), decay_rank (the rank of the
     decay's two-matrix projection; None: the shape of `w1` in the file gives it), tensor_names (optional
     overrides)."""
