@@ -210,11 +210,12 @@ head_matmul_rows_kernel(TO* out, long long ldo, long long out_hs, const bf16* a,
         const uint4 wv = *(const uint4*)(wr + k);
         if (!waited) { pdl_wait(); waited = true; }   // the weights do not depend on the kernel before
         const __nv_bfloat162* wp = (const __nv_bfloat162*)&wv;
+        uint4 xs[HR_TOK];                             // all asked for at once; tokens behind the last repeat it
+#pragma unroll
+        for (int i = 0; i < HR_TOK; i++) xs[i] = *(const uint4*)(ar + (size_t)min(i, nt - 1) * lda + k);
 #pragma unroll
         for (int i = 0; i < HR_TOK; i++) {
-            if (i >= nt) break;
-            const uint4 xv = *(const uint4*)(ar + (size_t)i * lda + k);
-            const __nv_bfloat162* xp = (const __nv_bfloat162*)&xv;
+            const __nv_bfloat162* xp = (const __nv_bfloat162*)&xs[i];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const float2 x = __bfloat1622float2(xp[j]), y = __bfloat1622float2(wp[j]);

@@ -125,12 +125,10 @@ moe_down_stream_kernel(float* out, const bf16* a, const bf16* __restrict__ w, co
     const int n_chunks = (F + CHUNK - 1) / CHUNK;
     const bool whole = ff % CHUNK == 0;               // a chunk belongs to one group
     pdl_wait();
-    if (threadIdx.x <= E) {
-        bool on = false;
-        if ((int)threadIdx.x < W)
-            for (int m = 0; m < M; m++) on |= dense[(size_t)m * W + threadIdx.x] != 0.f;
-        used[threadIdx.x] = on;
-    }
+    if (threadIdx.x <= E) used[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < M * W; i += WARPS * 32)        // a weight a thread: token after token the loads were a chain
+        if (dense[i] != 0.f && i % W <= E) used[i % W] = 1;
     __syncthreads();
     // the warp's chunks with a column that counts, in order
     int count = 0;
