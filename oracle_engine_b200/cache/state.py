@@ -49,7 +49,9 @@ class StateStore:
         tensors = list(self._tensors.values())
         if not tensors:
             return
-        if not tensors[0].is_cuda or any(t[0].numel() * t.element_size() % 4 for t in tensors):
+        # a store of a few tensors, the sampler's four, is filled one by one: the launch of zero_rows before a short prompt
+        # cost more than four fills (a 41-token request of the 3B shape 37.41 and 37.22 ms)
+        if not tensors[0].is_cuda or len(tensors) <= 8 or any(t[0].numel() * t.element_size() % 4 for t in tensors):
             for t in tensors:
                 t[slot].zero_()
             return
