@@ -35,15 +35,34 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// The norm between two products, without a kernel of its own.  The first product (out_kind 2) adds into the float32 stream x
+// and knows 16 channels of the new x: it leaves bf16(x w) and the 16 channels' sum of squares.  The second product multiplies
+// those rows, and each of its CTAs adds up the squares while it streams its weights and scales its sums by
+// 1 / sqrt(mean(x^2) + eps): the roundings are those of a norm kernel (one to bfloat16, of the weighted value).  For one or
+// two tokens, where a launch is a twentieth of the time between two products (csrc/ops_tc.py: SCALED_MAX_TOKENS); a CTA's
+// share of the squares grows with the tokens, at 8 tokens to 6 % of its weights.
+struct SkinnyNorm {
+    const float* weight;           // not null: this product leaves the rows
+    bf16* rows;                    // [M, N]
+    float* squares;                // [M, N / 16]
+    const float* in_squares;       // not null: A are such rows, [M, n_parts] their squares
+    int n_parts;
+    float eps;
+};
+
 // NT: 8-token tiles, 1 (M <= 8) or 2 (M <= 16); WARPS: warps per CTA (they split K);
 // UNROLL: 64-wide k chunks whose weight loads a warp has in flight at once.
-// ACT: the product has an epilogue (common.cuh: OeEpilogue); a form of its own, so that the others stay as they are.
-template <int NT, int WARPS, int UNROLL, bool ACT>
+// FORM 1: the product has an epilogue (common.cuh: OeEpilogue); FORM 2: a norm stands before or behind it (SkinnyNorm); forms
+// of their own, so that the plain one stays as it is.
+template <int NT, int WARPS, int UNROLL, int FORM>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_skinny_kernel(void* C, const bf16* A, const bf16* __restrict__ W,
-                   int M, int N, int K, long long lda, long long ldc, int out_kind, int late_trigger, const OeEpilogue epi) {
+                   int M, int N, int K, long long lda, long long ldc, int out_kind, int late_trigger, const OeEpilogue epi, const SkinnyNorm nrm) {
+    constexpr bool ACT = FORM == 1;
     __shared__ float red[WARPS][ROWS][8 * NT + 1];
     __shared__ float total[ROWS][8 * NT + 1];
+    __shared__ float scale[FORM == 2 ? 8 * NT : 1];
+    extern __shared__ __align__(16) float squares[];          // FORM 2 that reads scaled rows: [M][nrm.n_parts]
     if (!late_trigger) pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -61,6 +80,15 @@ gemm_skinny_kernel(void* C, const bf16* A, const bf16* __restrict__ W,
     for (int n = 0; n < NT; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     bool waited = false;
+    // behind the kernel before; the rows' sums of squares are asked for here and awaited behind the products
+    auto arrive = [&]() {
+        pdl_wait();
+        if (FORM == 2 && nrm.in_squares != nullptr) {
+            for (int i = threadIdx.x; i < M * nrm.n_parts / 4; i += WARPS * 32)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(squares + 4 * i)),
+                             "l"(nrm.in_squares + 4 * i) : "memory");
+        }
+    };
 
     for (int c = c_begin; c < c_end; c += UNROLL) {
         uint4 wa[UNROLL][2], wb[UNROLL][2];
@@ -74,7 +102,7 @@ gemm_skinny_kernel(void* C, const bf16* A, const bf16* __restrict__ W,
                 wb[u][hh] = (kv && rv1) ? ld_weight(w1 + k8) : zero;
             }
         }
-        if (!waited) { pdl_wait(); waited = true; }      // activations come from the kernel before
+        if (!waited) { arrive(); waited = true; }        // activations come from the kernel before
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) {
 #pragma unroll
@@ -92,7 +120,7 @@ gemm_skinny_kernel(void* C, const bf16* A, const bf16* __restrict__ W,
             }
         }
     }
-    if (!waited) pdl_wait();
+    if (!waited) arrive();
     // late_trigger: the kernel after this one may be scheduled only now, when this CTA has streamed
     // its weights, so that its CTAs do not sit on the SMs while this kernel still needs them
     if (late_trigger) pdl_launch_dependents();
@@ -105,7 +133,16 @@ gemm_skinny_kernel(void* C, const bf16* A, const bf16* __restrict__ W,
         red[warp][g + 8][n * 8 + t * 2] = acc[n][2];
         red[warp][g + 8][n * 8 + t * 2 + 1] = acc[n][3];
     }
+    if (FORM == 2) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
+    if (FORM == 2 && nrm.in_squares != nullptr) {
+        for (int tok = warp; tok < M; tok += WARPS) {
+            float s = 0.f;
+            for (int i = lane; i < nrm.n_parts; i += 32) s += squares[tok * nrm.n_parts + i];
+            s = warp_sum(s);
+            if (lane == 0) scale[tok] = 1.f / sqrtf(s / (float)K + nrm.eps);
+        }
+    }
     for (int idx = threadIdx.x; idx < ROWS * 8 * NT; idx += WARPS * 32) {
         const int r = idx % ROWS, tok = idx / ROWS;
         float s = 0.f;
@@ -117,38 +154,47 @@ gemm_skinny_kernel(void* C, const bf16* A, const bf16* __restrict__ W,
     for (int idx = threadIdx.x; idx < ROWS * 8 * NT; idx += WARPS * 32) {
         const int r = idx % ROWS, tok = idx / ROWS;
         const int row = row0 + r;
+        if (FORM == 2 && nrm.weight != nullptr) {             // N is a multiple of 16: every row of the CTA counts
+            float x = 0.f;
+            if (tok < M) {
+                float* at = (float*)C + (size_t)tok * ldc + row;
+                x = *at + total[r][tok];
+                *at = x;
+                nrm.rows[(size_t)tok * N + row] = __float2bfloat16_rn(x * nrm.weight[row]);
+            }
+            x *= x;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (r == 0 && tok < M) nrm.squares[(size_t)tok * gridDim.x + blockIdx.x] = x;
+            continue;
+        }
         if (tok >= M || row >= N) continue;
-        const float v = total[r][tok];
+        float v = total[r][tok];
+        if (FORM == 2) v *= scale[tok];
         if (out_kind == 0) ((bf16*)C)[(size_t)tok * ldc + row] = __float2bfloat16_rn(ACT ? oe_epilogue_one(epi, v, tok, row) : v);
         else if (out_kind == 1) ((float*)C)[(size_t)tok * ldc + row] = v;
         else if (out_kind == 2) ((float*)C)[(size_t)tok * ldc + row] += v;
         else if (!(r & 1)) {
-            const float up = total[r + 1][tok];
+            const float up = FORM == 2 ? total[r + 1][tok] * scale[tok] : total[r + 1][tok];
             ((bf16*)C)[(size_t)tok * ldc + (row >> 1)] = __float2bfloat16_rn((v / (1.f + expf(-v))) * up);
         }
     }
 }
 
-}  // namespace
-
-extern "C" {
-
-int oe_gemm_skinny_supported(const void* A, const void* W, int M, int N, int K, long long lda) {
-    if (M <= 0 || M > 16 || N <= 0 || K <= 0) return 0;
-    if ((K % 8) || (lda % 8)) return 0;
-    if (((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return 0;
-    return 1;
+bool skinny_supported(const void* A, const void* W, int M, int N, int K, long long lda) {
+    if (M <= 0 || M > 16 || N <= 0 || K <= 0) return false;
+    if ((K % 8) || (lda % 8)) return false;
+    if (((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return false;
+    return true;
 }
 
-// out_kind: 0 bf16, 1 float32, 2 float32 accumulate, 3 bf16 silu(gate)*up on interleaved rows (C is [M, N/2]).
-// early: bit 0 start early, bit 1 trigger late (see below).  act ..: what happens to the sums (common.cuh: OeEpilogue).
-int oe_gemm_skinny_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K, long long lda, long long ldc,
-                        int out_kind, int early, int act, int act_from, const float* act_w, int act_ff, long long act_ld,
-                        cudaStream_t st) {
-    if (!oe_gemm_skinny_supported(A, W, M, N, K, lda)) return OE_ERR_UNSUPPORTED;
+int launch_skinny(void* C, const bf16* A, const bf16* W, int M, int N, int K, long long lda, long long ldc, int out_kind, int early,
+                  const OeEpilogue epi, const SkinnyNorm nrm, cudaStream_t st) {
+    if (!skinny_supported(A, W, M, N, K, lda)) return OE_ERR_UNSUPPORTED;
     if (out_kind < 0 || out_kind > 3 || (out_kind == 3 && (N & 1))) return OE_ERR_UNSUPPORTED;
-    const OeEpilogue epi = {act, act_from, act_ff, act_ld, act_w};
     if (!oe_epilogue_ok(epi, out_kind, N)) return OE_ERR_UNSUPPORTED;
+    const bool normed = nrm.weight != nullptr || nrm.in_squares != nullptr;
+    const size_t smem = nrm.in_squares != nullptr ? (size_t)M * nrm.n_parts * 4 : 0;
     const int blocks = (N + ROWS - 1) / ROWS;
     // early bit 0: the kernel may start (and request its first weights) while the kernel before it
     // drains.  early bit 1: this kernel releases the kernel after it only when its CTAs have
@@ -164,11 +210,9 @@ int oe_gemm_skinny_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int
     // Warps and loads in flight per shape: matrices with many rows do best with small CTAs, long rows
     // with more loads in flight.
 #define OE_SKINNY_LAUNCH(NT, WARPS, UNROLL)                                                                        \
-    return epi.act                                                                                                 \
-        ? oe_launch_ex((early & 1) != 0, gemm_skinny_kernel<NT, WARPS, UNROLL, true>, dim3(blocks), dim3(WARPS * 32), 0, st, C, \
-                       A, W, M, N, K, lda, ldc, out_kind, (early >> 1) & 1, epi)                                   \
-        : oe_launch_ex((early & 1) != 0, gemm_skinny_kernel<NT, WARPS, UNROLL, false>, dim3(blocks), dim3(WARPS * 32), 0, st, C, \
-                       A, W, M, N, K, lda, ldc, out_kind, (early >> 1) & 1, epi)
+    return oe_launch_ex((early & 1) != 0, normed ? gemm_skinny_kernel<NT, WARPS, UNROLL, NT == 1 ? 2 : 0>          \
+                                          : epi.act ? gemm_skinny_kernel<NT, WARPS, UNROLL, 1> : gemm_skinny_kernel<NT, WARPS, UNROLL, 0>, \
+                        dim3(blocks), dim3(WARPS * 32), smem, st, C, A, W, M, N, K, lda, ldc, out_kind, (early >> 1) & 1, epi, nrm)
     if (M > 8) {
         // 9 to 16 tokens, chosen inside the 28-layer decode step (16 sequences: 2.11 ms with 8 warps x 3 loads
         // for every shape, 1.96 ms with these)
@@ -183,6 +227,31 @@ int oe_gemm_skinny_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int
     if (K > 4096) OE_SKINNY_LAUNCH(1, 8, 4);
     OE_SKINNY_LAUNCH(1, 8, 2);
 #undef OE_SKINNY_LAUNCH
+}
+
+}  // namespace
+
+extern "C" {
+
+int oe_gemm_skinny_supported(const void* A, const void* W, int M, int N, int K, long long lda) { return skinny_supported(A, W, M, N, K, lda); }
+
+// out_kind: 0 bf16, 1 float32, 2 float32 accumulate, 3 bf16 silu(gate)*up on interleaved rows (C is [M, N/2]).
+// early: bit 0 start early, bit 1 trigger late (see below).  act ..: what happens to the sums (common.cuh: OeEpilogue).
+int oe_gemm_skinny_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K, long long lda, long long ldc,
+                        int out_kind, int early, int act, int act_from, const float* act_w, int act_ff, long long act_ld,
+                        cudaStream_t st) {
+    return launch_skinny(C, A, W, M, N, K, lda, ldc, out_kind, early, OeEpilogue{act, act_from, act_ff, act_ld, act_w}, SkinnyNorm{}, st);
+}
+
+// The product before a norm (weight, rows, squares) or behind it (in_squares, n_parts, eps); see SkinnyNorm.
+int oe_gemm_skinny_norm_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K, long long lda, long long ldc, int out_kind, int early,
+                             const float* weight, bf16* rows, float* squares, const float* in_squares, int n_parts, float eps, cudaStream_t st) {
+    if (M > 8) return OE_ERR_UNSUPPORTED;
+    if (weight != nullptr ? (out_kind != 2 || N % ROWS || rows == nullptr || squares == nullptr || in_squares != nullptr)
+                          : (in_squares == nullptr || out_kind == 2 || n_parts * ROWS != K || n_parts % 4 || ((uintptr_t)in_squares & 15)
+                             || (long long)M * n_parts * 4 > 32768))
+        return OE_ERR_UNSUPPORTED;
+    return launch_skinny(C, A, W, M, N, K, lda, ldc, out_kind, early, OeEpilogue{}, SkinnyNorm{weight, rows, squares, in_squares, n_parts, eps}, st);
 }
 
 }  // extern "C"

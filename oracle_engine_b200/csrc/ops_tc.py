@@ -175,6 +175,9 @@ def _skinny():
         lib.oe_gemm_skinny_bf16.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                                             c_int, c_int] + _EPILOGUE + [c_void_p]
         lib.oe_gemm_skinny_bf16.restype = c_int
+        lib.oe_gemm_skinny_norm_bf16.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int,
+                                                 c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p]
+        lib.oe_gemm_skinny_norm_bf16.restype = c_int
         _state["skinny"] = lib
     return lib
 
@@ -182,9 +185,30 @@ def _skinny():
 NEXT_WEIGHTS_L2_BYTES = 8 << 20     # see gemm(then=)
 
 
+class ScaledRows:
+    """The rows of an RMS norm whose last step is still to come: rows = bf16(x w) [M, D] and, per token, the sums of squares of
+    x's 16-channel pieces, squares float32 [M, D / 16].  `gemm` takes it in place of a and scales its sums by
+    1 / sqrt(mean(x^2) + eps)."""
+
+    def __init__(self, rows: torch.Tensor, squares: torch.Tensor, eps: float):
+        self.rows, self.squares, self.eps, self.shape = rows, squares, float(eps), rows.shape
+
+
+SCALED_MAX_TOKENS = 2               # A request of 41 tokens and 24 steps, 3B shape, one sequence: 37.22 ms with norm kernels, 35.54
+                                    # without; 8 sequences of 512 and 48 steps 103.0 and 105.3 (every CTA reads all squares)
+SCALED_MAX_BYTES = 32768            # of the squares, which every CTA of the product behind the norm keeps in shared memory
+
+
+def scaled_rows_supported(M: int, D: int, weight: torch.Tensor) -> bool:
+    """Whether the norm of a stream [M, D] may be left to the products around it: both have to go to the weight-streaming
+    kernel, whose CTAs own 16 channels each."""
+    return 0 < M <= min(SCALED_MAX_TOKENS, SKINNY_MAX_TOKENS) and D % 64 == 0 and M * (D // 16) * 4 <= SCALED_MAX_BYTES \
+        and weight.dtype == torch.float32 and weight.is_contiguous() and weight.numel() == D
+
+
 def gemm(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool = False, split_k: bool = True,
          swiglu: bool = False, kernel: str = "auto", early: int = 0, then: torch.Tensor | None = None,
-         act: str | None = None, act_from: int = 0, group_weights: tuple | None = None) -> None:
+         act: str | None = None, act_from: int = 0, group_weights: tuple | None = None, leave: tuple | None = None) -> None:
     """out (+)= a @ w.T, a [M, K] and w [N, K] bfloat16; out bfloat16 or float32 [M, N].
 
     swiglu: w's rows alternate gate and up rows (g0, u0, g1, u1, ...) and out [M, N/2]
@@ -201,6 +225,9 @@ def gemm(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool =
     after this one; when this kernel's own loads are out it asks the first 8 MB of it into the L2, so that the
     memory does not idle through its epilogue and the next kernel's set-up (decode step of the 28-layer 3B shape,
     ms, without / 4 / 8 / 12 / 32 MB: 32 sequences 2.62 / 2.57 / 2.56 / 2.56 / 2.63, 64: 2.96 / 2.91 / 2.89 / 2.89 / 3.01)."""
+    scaled, norm_of = (a, None) if isinstance(a, ScaledRows) else (None, leave)
+    if scaled is not None:
+        a = scaled.rows
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N // 2 if swiglu else N):
@@ -234,6 +261,17 @@ def gemm(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool =
             epilogue[2:] = [gw.data_ptr(), int(ff), gw.stride(0)]
     elif group_weights is not None:
         raise KernelError("gemm: group weights come with an activation")
+    if scaled is not None or norm_of is not None:
+        if act is not None or kernel != "auto" or not uses_skinny(M, N, K, kind):
+            raise KernelError("gemm: a norm beside a product goes with the weight-streaming kernel only")
+        weight, left = norm_of if norm_of is not None else (None, None)
+        code = _skinny().oe_gemm_skinny_norm_bf16(
+            out.data_ptr(), a.data_ptr(), w.data_ptr(), M, N, K, a.stride(0), out.stride(0), kind, int(early),
+            None if left is None else weight.data_ptr(), None if left is None else left.rows.data_ptr(),
+            None if left is None else left.squares.data_ptr(), None if scaled is None else scaled.squares.data_ptr(),
+            0 if scaled is None else scaled.squares.shape[1], 0.0 if scaled is None else scaled.eps, ops._stream())
+        ops._check(code, "gemm_skinny", (M, N, K))
+        return
     if kernel == "skinny" or (kernel == "auto" and uses_skinny(M, N, K, kind)):
         code = _skinny().oe_gemm_skinny_bf16(out.data_ptr(), a.data_ptr(), w.data_ptr(), M, N, K, a.stride(0),
                                              out.stride(0), kind, int(early), *epilogue, ops._stream())

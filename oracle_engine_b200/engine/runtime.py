@@ -39,6 +39,11 @@ class Runtime:
     # add_into(..., keep_cast=True)): (address of the stream, the copy).  `activations` takes it instead of casting
     # again; the model clears it when a forward pass starts.
     cast_cache: tuple | None = None
+    # The norm that reads the stream next and nothing else does before it, set by the model and the block while a sublayer
+    # runs whose last product may do the norm's work (`leave_normed`), and what that product left: (address of the stream,
+    # the norm, its rows).  The norm's forward takes it; both are of one step.
+    next_norm: object = None
+    normed: tuple | None = None
     # Tensors that parts of different layers share during ONE forward pass (a history of the stream, say): the part
     # that runs first puts them here, the others find them.  While a CUDA graph is captured they are the graph's memory.
     pass_store: dict = field(default_factory=dict, repr=False)
@@ -91,6 +96,20 @@ class Runtime:
         finally:
             end.record(self._side)             # the capture ends on the current stream, whatever happened
             main.wait_event(end)
+
+    def leave_normed(self, out: torch.Tensor):
+        """For a product that adds into `out`: (weight, rows to fill) if the norm behind it can be left to the products around
+        it (csrc/ops_tc.py: ScaledRows), else None."""
+        norm = self.next_norm
+        if norm is None or out.dtype != torch.float32 or not out.is_contiguous():
+            return None
+        from ..csrc import ops_tc
+        M, D = out.shape
+        if not ops_tc.scaled_rows_supported(M, D, norm.weight):
+            return None
+        left = ops_tc.ScaledRows(self.empty(M, D), self.empty(M, D // 16, dtype=torch.float32), norm.eps)
+        self.normed = (out.data_ptr(), norm, left)
+        return norm.weight, left
 
     def activations(self, x: torch.Tensor) -> torch.Tensor:
         """The float32 residual stream as a sublayer's input: itself on the 32-bit path (the sublayer

@@ -88,6 +88,7 @@ class GQAAttention(Part):
         return self.w_qkv
 
     joint_weight = "w_qkv"         # parts/block.py: JoinedInput
+    takes_scaled = True            # its input goes to one product (Runtime.leave_normed)
 
     def forward(self, h, residual, ctx, cache, state, owns_cache=True, projected=None):
         """projected: Wqkv h (Wq h first), computed by the caller; the rotation works in it."""

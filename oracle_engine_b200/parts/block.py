@@ -19,8 +19,25 @@ from .registry import BLOCKS, Part
 from .spec import TensorDecl
 
 
+def leaves_to(before, norm, behind):
+    """`norm`, if the part before it ends in a product that adds into the stream, and the part behind it begins with one
+    product that reads nothing else: then those two do the norm's work where they can (Runtime.leave_normed)."""
+    def says(part, name):               # of its own class: a subclass may read its input in other ways
+        value = vars(type(part)).get(name, False)
+        return value.fget(part) if isinstance(value, property) else value
+    return norm if says(before, "takes_scaled") and says(norm, "can_be_left") and says(behind, "takes_scaled") else None
+
+
 @BLOCKS.register("pre_norm")
 class PreNormBlock:
+    def first_norm(self):
+        """The norm of the block's input, if the products around it may do its work, else None."""
+        return leaves_to(self.mixer, self.mixer_norm, self.mixer)
+
+    def last_part(self):
+        """The part that adds into the stream last."""
+        return self.mixer if self.feed_forward is None else self.feed_forward
+
     def __init__(self, mixer, feed_forward, mixer_norm, ffn_norm):
         self.mixer = mixer
         self.feed_forward = feed_forward
@@ -37,17 +54,21 @@ class PreNormBlock:
     def forward(self, x, ctx, cache, state, owns_cache=True):
         rt = getattr(self.mixer, "rt", None)
         after = getattr(rt, "next_weights", None)          # what the model says comes after this block
+        norm_after = getattr(rt, "next_norm", None)
         h = self.mixer_norm.forward(x)
         if rt is not None:
             rt.next_weights = _first_weights(self.feed_forward) if self.feed_forward is not None else after
+            rt.next_norm = leaves_to(self.mixer, self.ffn_norm, self.feed_forward) if self.feed_forward is not None \
+                else norm_after
         self.mixer.forward(h, x, ctx, cache, state, owns_cache)
         if self.feed_forward is not None:
             h = self.ffn_norm.forward(x)
             if rt is not None:
                 rt.next_weights = after
+                rt.next_norm = norm_after
             self.feed_forward.forward(h, x, ctx)
         if rt is not None:
-            rt.next_weights = None
+            rt.next_weights = rt.next_norm = None
 
 
 class JoinedInput(Part):

@@ -43,6 +43,9 @@ class SwiGLU(Part):
             self.w_gu = torch.cat([gate, up], 0)
         self.w_down = to(get(self.names["down"]))
 
+    # its input goes to one product on the tensor-core path (Runtime.leave_normed)
+    takes_scaled = property(lambda self: self.fused)
+
     def weight_bytes(self):
         return sum(t.numel() * t.element_size() for t in (self.w_gu, self.w_down) if t is not None)
 
@@ -55,7 +58,7 @@ class SwiGLU(Part):
     def forward(self, h, residual, ctx):
         T = h.shape[0]
         a = self.rt.empty(T, self.FF)
-        if self.fused:
+        if self.fused:                      # (h may be ScaledRows, see takes_scaled)
             from ..csrc import ops_tc
             ops_tc.gemm(a, h, self.w_gu, swiglu=True, early=chain_flags("ffn_in", T), then=self.w_down)
         else:

@@ -50,8 +50,12 @@ def matmul_nt(rt, out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulat
     then: the weight matrix of the product that runs after this one (a hint, see ops_tc.gemm)."""
     if rt.dtype == torch.bfloat16 and rt.tensor_cores:
         from ..csrc import ops_tc
-        if ops_tc.gemm_supported(a, w, out):
-            ops_tc.gemm(out, a, w, accumulate=accumulate, early=int(early), then=then)
+        scaled = isinstance(a, ops_tc.ScaledRows)
+        if scaled or ops_tc.gemm_supported(a, w, out):
+            leave = rt.leave_normed(out) if accumulate else None
+            if leave is not None:           # what comes next is a product with many CTAs, not a norm
+                early |= TRIGGER_LATE
+            ops_tc.gemm(out, a, w, accumulate=accumulate, early=int(early), then=then, leave=leave)
             return
     ops.gemm_simple(out, a, w, accumulate=accumulate)
 

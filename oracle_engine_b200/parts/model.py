@@ -149,6 +149,7 @@ class DecoderModel:
         return x
 
     def run_entries(self, x, ctx, cache_views, state_views, lo: int, hi: int) -> None:
+        self.rt.next_norm = self.rt.normed = None
         if lo == 0:
             self.rt.cast_cache = None          # nothing of an earlier pass is taken for this one's stream
         for i in range(lo, hi):
@@ -158,10 +159,18 @@ class DecoderModel:
             nxt = self.layers[self.schedule[i + 1].layer] if i + 1 < len(self.schedule) else None
             first = getattr(nxt, "first_weights", None)
             self.rt.next_weights = first() if first is not None else None
+            # and the norm that reads the stream behind this entry, if nothing else does first (the next entry of this run)
+            self.rt.next_norm = self._norm_between(e, self.schedule[i + 1]) if i + 1 < hi else None
             if e.before is not None:
                 self.stream_parts[e.before[0]].forward(x, ctx, **dict(e.before[1]))
             self.layers[e.layer].forward(x, ctx, cache_views[owner], state_views[i], e.cache_from is None)
-        self.rt.next_weights = None
+        self.rt.next_weights = self.rt.next_norm = self.rt.normed = None
+
+    def _norm_between(self, entry, following):
+        """The norm between two entries that the products around it may do the work of, else None."""
+        a, b = self.layers[entry.layer], self.layers[following.layer]
+        norm = b.first_norm() if following.before is None and hasattr(b, "first_norm") and hasattr(a, "last_part") else None
+        return norm if norm is not None and block.leaves_to(a.last_part(), norm, b.mixer) is norm else None
 
     def logits(self, x, ctx):
         if ctx.n_want == 0:
