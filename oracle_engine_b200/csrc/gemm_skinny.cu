@@ -38,9 +38,9 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
 // The norm between two products, without a kernel of its own.  The first product (out_kind 2) adds into the float32 stream x
 // and knows 16 channels of the new x: it leaves bf16(x w) and the 16 channels' sum of squares.  The second product multiplies
 // those rows, and each of its CTAs adds up the squares while it streams its weights and scales its sums by
-// 1 / sqrt(mean(x^2) + eps): the roundings are those of a norm kernel (one to bfloat16, of the weighted value).  For one or
-// two tokens, where a launch is a twentieth of the time between two products (csrc/ops_tc.py: SCALED_MAX_TOKENS); a CTA's
-// share of the squares grows with the tokens, at 8 tokens to 6 % of its weights.
+// 1 / sqrt(mean(x^2) + eps): the roundings are those of a norm kernel (one to bfloat16, of the weighted value).  For up
+// to four tokens (csrc/ops_tc.py: SCALED_MAX_TOKENS): the squares that every CTA reads grow with the tokens, at 8 to 6 % of
+// its weights.
 struct SkinnyNorm {
     const float* weight;           // not null: this product leaves the rows
     bf16* rows;                    // [M, N]

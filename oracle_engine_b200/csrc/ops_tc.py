@@ -194,8 +194,9 @@ class ScaledRows:
         self.rows, self.squares, self.eps, self.shape = rows, squares, float(eps), rows.shape
 
 
-SCALED_MAX_TOKENS = 2               # A request of 41 tokens and 24 steps, 3B shape, one sequence: 37.22 ms with norm kernels, 35.54
-                                    # without; 8 sequences of 512 and 48 steps 103.0 and 105.3 (every CTA reads all squares)
+SCALED_MAX_TOKENS = 4               # Requests of 41 tokens and 24 steps, 3B shape, with norm kernels / without: one sequence 37.17 /
+                                    # 35.48 ms, two 38.05 / 36.38, four 39.03 / 37.85; 8 sequences of 512 tokens and 48 steps
+                                    # 103.0 / 105.3 (every CTA reads all squares)
 SCALED_MAX_BYTES = 32768            # of the squares, which every CTA of the product behind the norm keeps in shared memory
 
 
