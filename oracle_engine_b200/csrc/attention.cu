@@ -38,9 +38,10 @@ struct Running {
 #pragma unroll
         for (int i = 0; i < NI; i++) acc[i] = 0.f;
     }
-    // one chunk more: its maximum (-inf: it has no key for this row), its sum and its weighted values
+    // one chunk more: its maximum, its sum and its weighted values.  Without a key for this row the maximum is -inf and the
+    // sum zero; with keys whose scores are all NaN the maximum, which passes NaN over, is -inf as well, but not the sum
     __device__ __forceinline__ void join(float mc, float lc, const float (&ac)[NI]) {
-        if (mc == -INFINITY) return;
+        if (mc == -INFINITY && lc == 0.f) return;
         const float m_new = fmaxf(m, mc);
         const float a = expf(m - m_new), b = expf(mc - m_new);
         l = fmaf(l, a, __fmul_rn(lc, b));

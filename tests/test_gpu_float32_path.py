@@ -107,3 +107,25 @@ def test_attention_gives_the_same_bits_by_both_kernels(dtype, H, KVH, hd, window
                 e = torch.exp(s - s.max())
                 o = (e @ rd(vs[b][lo:p + 1, h // G])) / (e.sum() + (math.exp(-s.max()) if sink else 0.0))
                 assert (got[h] - o).abs().max() <= (2e-5 if dtype == torch.float32 else 2.0 ** -8 * o.abs().max() + 2e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("window", [0, 16])
+def test_a_key_of_nan_reaches_the_queries_that_see_it_and_no_others(dtype, kind, sink, window):
+    """Keys of NaN: alone in what a query sees of a chunk, beside other keys of their chunk, and in a chunk that is full."""
+    from oracle_engine_b200.csrc import ops
+    H, KVH, hd, n = 4, 2, 64, 128
+    for nans in ((32, 33), (40, 41), (0, 1), (64, 96)):
+        cache = _rand(n // 64, 2, KVH, 64, hd, seed=7)
+        keys = cache[:, 0].transpose(1, 2).reshape(n, KVH, hd)
+        keys[nans[0]:nans[1]] = float("nan")
+        cache[:, 0] = keys.view(n // 64, 64, KVH, hd).transpose(1, 2)
+        i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)                       # noqa: E731
+        out = torch.full((n, H * hd), 7.0, dtype=dtype, device=DEV)
+        ops.attn_paged(out, _rand(n, H * hd, seed=8).to(dtype), cache.to(dtype), i32([[0, 1]]), i32([0] * n), i32(range(n)), H, KVH, hd, window,
+                       hd ** -0.5, sink, kind)
+        sees = torch.tensor([p >= nans[0] and (window == 0 or nans[1] - 1 > p - window) for p in range(n)])
+        got = out.cpu()
+        assert torch.isnan(got[sees]).all() and torch.isfinite(got[~sees]).all()
