@@ -79,8 +79,8 @@ attn_prompt_kernel(T* out, const T* q, int q_stride, const T* cache, const int* 
     float* qs = vs + 32 * hp;                                 // [ROWS][hp]
     float* ps = qs + ROWS * hp;                               // [WARPS][32][RB]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kvh = blockIdx.x, G = H / KVH;
-    const long long row0 = (long long)blockIdx.y * ROWS, n_rows = (long long)n_tokens * G;
+    const int kvh = blockIdx.x % KVH, G = H / KVH;
+    const long long row0 = (long long)(blockIdx.x / KVH) * ROWS, n_rows = (long long)n_tokens * G;
     pdl_launch_dependents();
     pdl_wait();
     const int t0 = (int)(row0 / G), t1 = (int)((min(row0 + ROWS, n_rows) - 1) / G);
@@ -214,7 +214,7 @@ attn_token_kernel(T* out, const T* q, int q_stride, const T* cache, const int* _
     __shared__ float pm[WARPS][RB], pl[WARPS][RB];
     extern __shared__ __align__(16) float part[];             // [WARPS][RB][32 NI]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kvh = blockIdx.x, t = blockIdx.y, G = H / KVH;
+    const int kvh = blockIdx.x % KVH, t = blockIdx.x / KVH, G = H / KVH;
     pdl_launch_dependents();
     pdl_wait();
     const int b = tok_seq[t];
@@ -324,26 +324,26 @@ int launch_sized(T* out, const T* q, int q_stride, const T* cache, const int* ta
     // A prompt CTA loads a chunk once for 64 rows of one sequence, chunk after chunk; with few tokens a sequence most of its
     // rows would idle, and with few CTAs most SMs: a CTA a token walks eight chunks at a time.
     const bool by_token = kind == 1 || (kind == 0 && (n_tokens <= 4LL * n_seqs || tiles * KVH < 74));
-    if ((by_token ? (long long)n_tokens : tiles) > 65535) {
-        if (kind || tiles > 65535) return OE_ERR_UNSUPPORTED;
-        return launch_sized<T, NI>(out, q, q_stride, cache, tables, max_pages, tok_seq, tok_pos, n_tokens, n_seqs, H, KVH, hd, window, scale, sink, 2, st);
-    }
+    // a grid of one dimension, the KV heads of a token or tile side by side: the others end at 65,535
+    const long long ctas = (by_token ? (long long)n_tokens : tiles) * KVH;
+    if (ctas > 2147483647LL) return OE_ERR_UNSUPPORTED;
+    const dim3 grid((unsigned)ctas);
     if (by_token) {
         const bool quads = hd % 4 == 0 && ((uintptr_t)cache & 15) == 0;
         const size_t bytes = (size_t)WARPS * RB * NI * 32 * 4;
         cudaError_t e = cudaFuncSetAttribute(quads ? attn_token_kernel<T, NI, true> : attn_token_kernel<T, NI, false>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return (int)e;
-        if (quads) return oe_launch(attn_token_kernel<T, NI, true>, dim3(KVH, n_tokens), dim3(WARPS * 32), bytes, st, out, q, q_stride, cache, tables,
+        if (quads) return oe_launch(attn_token_kernel<T, NI, true>, grid, dim3(WARPS * 32), bytes, st, out, q, q_stride, cache, tables,
                                   max_pages, tok_seq, tok_pos, H, KVH, hd, window, scale, sink);
-        return oe_launch(attn_token_kernel<T, NI, false>, dim3(KVH, n_tokens), dim3(WARPS * 32), bytes, st, out, q, q_stride, cache, tables,
+        return oe_launch(attn_token_kernel<T, NI, false>, grid, dim3(WARPS * 32), bytes, st, out, q, q_stride, cache, tables,
                          max_pages, tok_seq, tok_pos, H, KVH, hd, window, scale, sink);
     }
     const int hp = (hd + 3) / 4 * 4;
     const size_t bytes = (size_t)(32 * (hp + 4) + 32 * hp + ROWS * hp + WARPS * 32 * RB) * 4;
     cudaError_t e = cudaFuncSetAttribute(attn_prompt_kernel<T, NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
-    return oe_launch(attn_prompt_kernel<T, NI>, dim3(KVH, (unsigned)tiles), dim3(WARPS * 32), bytes, st, out, q, q_stride, cache, tables, max_pages,
+    return oe_launch(attn_prompt_kernel<T, NI>, grid, dim3(WARPS * 32), bytes, st, out, q, q_stride, cache, tables, max_pages,
                      tok_seq, tok_pos, n_tokens, H, KVH, hd, window, scale, sink);
 }
 

@@ -129,3 +129,18 @@ def test_a_key_of_nan_reaches_the_queries_that_see_it_and_no_others(dtype, kind,
         sees = torch.tensor([p >= nans[0] and (window == 0 or nans[1] - 1 > p - window) for p in range(n)])
         got = out.cpu()
         assert torch.isnan(got[sees]).all() and torch.isfinite(got[~sees]).all()
+
+
+@pytest.mark.parametrize("T,seqs,kind", [(530000, 1, 0), (66000, 66000, 0), (66000, 1, 1)])
+def test_attention_of_more_tokens_than_a_grid_s_second_dimension_holds(T, seqs, kind):
+    """66,250 tiles of 64 rows, and a CTA per token for 66,000 tokens; the tokens repeat a few."""
+    from oracle_engine_b200.csrc import ops
+    H, hd = 8, 2
+    q, cache = _rand(5, H * hd, seed=9), _rand(1, 2, 1, 64, hd, seed=10)
+    tables = torch.zeros(seqs, 1, dtype=torch.int32, device=DEV)
+    at = torch.arange(T, device=DEV) % 5
+    seq = (torch.arange(T, device=DEV) % seqs).int()
+    few, many = torch.empty(5, H * hd, device=DEV), torch.empty(T, H * hd, device=DEV)
+    ops.attn_paged(few, q, cache, tables[:1], torch.zeros(5, dtype=torch.int32, device=DEV), torch.arange(5, dtype=torch.int32, device=DEV), H, 1, hd, 0, 1.0)
+    ops.attn_paged(many, q[at], cache, tables, seq, at.int(), H, 1, hd, 0, 1.0, False, kind)
+    assert torch.equal(many, few[at])
