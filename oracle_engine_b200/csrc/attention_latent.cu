@@ -270,10 +270,11 @@ int launch_hm(TO* out, long long ldo, long long out_hs, const T* a, long long ld
     if (n_tokens <= 0) return 0;
     if (H < 1 || H > 65535 || N < 1 || K < 1) return OE_ERR_UNSUPPORTED;
     const int tz = (n_tokens + HM_TOK - 1) / HM_TOK;
-    if (tz > 32767) return OE_ERR_UNSUPPORTED;
+    if (tz > 65535) return OE_ERR_UNSUPPORTED;
     if constexpr (sizeof(T) == 2) {
-        if (K % 8 == 0 && lda % 8 == 0 && a_hs % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0)
-            return oe_launch(head_matmul_rows_kernel<TO>, dim3((N + HR_ROWS - 1) / HR_ROWS, H, (n_tokens + HR_TOK - 1) / HR_TOK), dim3(128), 0, st,
+        const int tr = (n_tokens + HR_TOK - 1) / HR_TOK;      // half as many tokens a block: its grid ends sooner
+        if (tr <= 65535 && K % 8 == 0 && lda % 8 == 0 && a_hs % 8 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0)
+            return oe_launch(head_matmul_rows_kernel<TO>, dim3((N + HR_ROWS - 1) / HR_ROWS, H, tr), dim3(128), 0, st,
                              out, ldo, out_hs, (const bf16*)a, lda, a_hs, (const bf16*)w, n_tokens, N, K);
     }
     return oe_launch(head_matmul_kernel<T, TO>, dim3((N + 7) / 8, H, tz), dim3(256), 0, st, out, ldo, out_hs, a, lda, a_hs, w,

@@ -33,3 +33,18 @@ def test_head_matmul_rows(T, H, N, K, out_dtype):
     shifted = torch.einsum("thk,hnk->thn", wide[:, :, 1:K + 1].double(), w.double())
     scale = torch.einsum("thk,hnk->thn", wide[:, :, 1:K + 1].double().abs(), w.double().abs())
     assert ((off.double() - shifted).abs() <= bound(shifted, scale)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_as_many_tokens_as_the_blocks_of_sixteen_reach(dtype):
+    """32,768 blocks of 16 tokens: beyond what blocks of eight reach, and not refused."""
+    from oracle_engine_b200.csrc import ops
+    T, K = 32767 * 16 + 1, 8
+    few = torch.randn(7, 1, K, generator=torch.Generator().manual_seed(3)).to(dtype).to(DEV)
+    w = torch.randn(1, 3, K, generator=torch.Generator().manual_seed(4)).to(dtype).to(DEV)
+    at = torch.arange(T, device=DEV) % 7
+    out = torch.empty(T, 1, 3, device=DEV)
+    ops.head_matmul(out, few[at], w)
+    want = torch.einsum("thk,hnk->thn", few.double(), w.double())
+    bound = K * 2.0 ** -24 * torch.einsum("thk,hnk->thn", few.double().abs(), w.double().abs())
+    assert ((out.double() - want[at]).abs() <= bound[at]).all()
