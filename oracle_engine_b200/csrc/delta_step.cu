@@ -5,8 +5,8 @@
 // and the convolution's kept rows moved on by one.
 //
 // A step of one sequence is bound by its launches and the round trips to memory in each (16 heads of 128 x 128: 4 launches
-// of 2 to 4 us for 1 MB of state): here a CTA has one head of one sequence, asks for its state and the kept rows before it
-// waits for the projection, and keeps the state in registers, four columns and up to 16 rows a thread.  The heads that share
+// of 2 to 4 us for 1 MB of state): here a CTA has one head of one sequence, has its state and the kept rows brought into the
+// L2 before it waits for the projection, and keeps the state in registers, four columns and up to 16 rows a thread.  The heads that share
 // a key head are a cluster: the last one to have read the kept rows of q and k lets the first one overwrite them.
 #include "common.cuh"
 
@@ -14,6 +14,7 @@ namespace {
 
 constexpr int THREADS = 256, MAX_ROWS = 16, MAX_KEPT = 7, MAX_CHANNELS = 3;     // rows a thread, kept rows, channels a thread
 
+__device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
@@ -33,15 +34,24 @@ delta_step_kernel(bf16* y, float* state, float* conv_state, const float* proj, i
     float* vec = smem;                                // [q: dk | k: dk | v: dv]
     float* part = vec + 2 * dk + dv;                  // [groups][dv]
     float* S = state + ((size_t)slot * H + h) * dk * dv;
+    const int C = 2 * G * dk + H * dv, channels = 2 * dk + dv;
+    auto channel = [&](int c) { return c < dk ? g * dk + c : c < 2 * dk ? G * dk + g * dk + (c - dk) : 2 * G * dk + h * dv + (c - 2 * dk); };
+    float* kept = conv_state + (size_t)slot * (taps - 1) * C;
+    // An earlier kernel of the stream may still write both (a slot's reset, this kernel a token earlier): they are read behind
+    // the wait, and before it only asked into the L2, 128 bytes at a time.  (Reading them before it saved 0.4 us a layer: six of
+    // eight layers of width 2,048, one sequence, 393 and 396 us a decode step.)
+    for (int i = tid; i < dk * dv / 32; i += THREADS) prefetch_l2(S + 32 * i);
+    if (tid % 32 == 0)
+        for (int c = tid; c < channels; c += THREADS)
+            for (int j = 0; j < taps - 1; j++) prefetch_l2(kept + (size_t)j * C + channel(c));
+    pdl_wait();
+    pdl_launch_dependents();
     float4 s[MAX_ROWS];
 #pragma unroll
     for (int i = 0; i < MAX_ROWS; i++) {
         const int r = rg + groups * i;
         s[i] = works && r < dk ? *(const float4*)(S + (size_t)r * dv + 4 * cq) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const int C = 2 * G * dk + H * dv, channels = 2 * dk + dv;
-    auto channel = [&](int c) { return c < dk ? g * dk + c : c < 2 * dk ? G * dk + g * dk + (c - dk) : 2 * G * dk + h * dv + (c - 2 * dk); };
-    float* kept = conv_state + (size_t)slot * (taps - 1) * C;
     float old[MAX_CHANNELS][MAX_KEPT];
 #pragma unroll
     for (int e = 0; e < MAX_CHANNELS; e++) {
@@ -49,8 +59,6 @@ delta_step_kernel(bf16* y, float* state, float* conv_state, const float* proj, i
 #pragma unroll
         for (int j = 0; j < MAX_KEPT; j++) old[e][j] = c < channels && j < taps - 1 ? kept[(size_t)j * C + channel(c)] : 0.f;
     }
-    pdl_wait();
-    pdl_launch_dependents();
     const float* row = proj + (size_t)t * P;
     const float beta = 1.f / (1.f + expf(-row[C + H * dv + h]));
     const float decay = expf(-expf(A_log[h]) * softplus_f(row[C + H * dv + H + h] + dt_bias[h]));
