@@ -16,7 +16,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import TensorDecl, mask_span, span_need, visible_keys, visible_pairs
 
@@ -101,4 +101,4 @@ class CappedAttention(Part):
         from . import attention_dispatch as ad
         ad.split_mixer_core(self.rt, o, qkv, cos, sin, self.rot, kc, vc, cache.tables, ctx, self.H, self.G, self.dk,
                             self.dv, self.span, self.scale, self.cap, owns_cache)
-        matmul_nt(self.rt, residual, o, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, o, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
@@ -110,7 +110,7 @@ class GatedDelta(Part):
             y = buf("delta.y", T, vv)
             ops.delta_step(y, state["S"], state["conv"], proj, self.conv_w, self.A_log, self.dt_bias, self.norm_w, ctx, self.G, self.H,
                            self.dk, self.dv, self.dk ** -0.5, self.eps)
-            matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
+            matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))
             return
         qkv = buf("delta.qkv", T, self.C, dtype=f32)
         gb = buf("delta.gb", T, 2 * self.H, dtype=f32)
@@ -125,4 +125,4 @@ class GatedDelta(Part):
             ops.delta_rule_scan(o, state["S"], qkv, gb, ctx, self.G, self.H, self.dk, self.dv)
         y = buf("delta.y", T, vv)
         ops.head_gate(y, o, proj[:, self.C:self.C + vv], self.norm_w, self.H, self.dv, True, "silu", self.eps)
-        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

@@ -8,7 +8,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import chain_flags, matmul_act, matmul_nt
+from .linear import chain_flags, matmul_act, matmul_nt, output_flags
 from .registry import FEED_FORWARDS, Part
 from .spec import TensorDecl
 
@@ -168,4 +168,4 @@ class PolyNormMLP(Part):
         matmul_nt(self.rt, z, h, self.w_up)
         a = self.rt.buffer("polynorm.a", T, self.FF)
         ops.poly_norm(a, z, self.coef, self.eps)
-        matmul_nt(self.rt, residual, a, self.w_down, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, a, self.w_down, accumulate=not overwrite, early=output_flags(self.w_down))

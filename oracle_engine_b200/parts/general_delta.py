@@ -21,7 +21,7 @@ import math
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
@@ -104,4 +104,4 @@ class GeneralDelta(Part):
         ops.gdelta_scan(o, state["S"], packed, proj[:, 2 * C:3 * C], ctx, self.H, self.d, self.d)
         y = buf("gdelta.y", T, C)
         ops.head_gate(y, o, proj[:, 3 * C:4 * C], self.norm_w, self.H, self.d, True, "sigmoid", self.eps)
-        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

@@ -14,7 +14,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
@@ -118,4 +118,4 @@ class GatedLinearAttention(Part):
                      self.tau, segments=self._segments(ctx))
         y = buf("gla.y", T, vv)
         ops.head_gate(y, o, proj[:, 2 * qk + vv:2 * qk + 2 * vv], self.norm_w, self.H, self.dv, True, "silu", self.eps)
-        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

@@ -22,7 +22,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import chain_flags, matmul_nt
+from .linear import chain_flags, matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import TensorDecl, mask_span, span_need, visible_keys, visible_pairs
 
@@ -218,4 +218,4 @@ class LatentAttention(Part):
             y = buf("latent.y", T, H * dv)
             ops.head_gate(y, o, proj[:, self.off_g:self.off_g + H * dv], None, H, dv, False, "sigmoid")
             o = y
-        matmul_nt(self.rt, residual, o, self.w["o"], accumulate=not overwrite)
+        matmul_nt(self.rt, residual, o, self.w["o"], accumulate=not overwrite, early=output_flags(self.w["o"]))

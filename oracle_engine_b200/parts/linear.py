@@ -34,9 +34,20 @@ _CHAIN_FLAGS = {
 
 # Products that are given no flags, in the other decoders' longer chains of short kernels, start early and trigger late: behind
 # a kernel of any kind they then wait beside it, and nothing starts on the SMs they still stream through (us a decode step
-# with none / 1 / 2 / 3 of the flags: Fuvipel 487 / 517 / 476 / 460, Fovirax 676 / 751 / 661 / 626, Mavinex 619 / 629 / 619 / 611,
-# one sequence, 8 layers, width 2,048; at 8 sequences 1 to 3 % between none and both).
+# with none / 1 / 2 / 3 of the flags, one sequence, 8 layers, width 2,048: Fuvipel 487 / 517 / 476 / 460, Fovirax
+# 676 / 751 / 661 / 626, Mavinex 619 / 629 / 619 / 611, Pusunex 678 / 689 / 680 / 651, Bogupel 444 / 498 / 430 / 423; at 8 to 16
+# sequences mostly 1 to 4 % between none and both).  Goridra has none of them.
 DEFAULT_FLAGS = START_EARLY | TRIGGER_LATE
+
+
+def output_flags(w: torch.Tensor) -> int:
+    """Of a product that ends a mixer or feed-forward and is not in the table: as the default, but it starts early only while each
+    of its CTAs, of 16 weight rows, can have an SM of 148 to itself.  More of them behind an attention or a scan sat on the SMs
+    that the other chains still needed.  us a decode step at width 3,072, none of the flags / the default everywhere / this:
+    Bogupel, 1 sequence 588 / 628 / 568, 4 710 / 785 / 645, 16 1,003 / 1,096 / 942; Fovirax, 4 1,043 / 1,069 / 1,003, 8
+    1,182 / 1,298 / 1,259, 16 1,744 / 1,550 / 1,485; Fuvipel, 1 600 / 603 / 593; Pusunex, 1 954 / 924 / 930; up to width 2,048 it
+    is the default."""
+    return DEFAULT_FLAGS if w.shape[0] <= 16 * 148 else TRIGGER_LATE
 
 
 def chain_flags(product: str, n_tokens: int) -> int:

@@ -32,7 +32,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import chain_flags, matmul_act, matmul_nt
+from .linear import chain_flags, matmul_act, matmul_nt, output_flags
 from .registry import FEED_FORWARDS, Part
 from .spec import TensorDecl
 
@@ -183,7 +183,7 @@ class MoESwiGLU(Part):
         a = self.rt.buffer("moe.a", T, self.F)
         ops.moe_dense_act(a, gu, dense, self.E, self.ff, scale_input=self.weight_on == "input", act=self.activation,
                           limit=self.limit)
-        matmul_nt(self.rt, residual, a, self.w_down, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, a, self.w_down, accumulate=not overwrite, early=output_flags(self.w_down))
 
 
     def _forward_sorted(self, h, residual, dense, overwrite: bool) -> None:

@@ -17,7 +17,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
@@ -95,4 +95,4 @@ class Retention(Part):
                            self.H, self.dk, self.dv, scratch=scratch)
         y = self.rt.buffer("retention.y", T, vv)
         ops.head_gate(y, o, proj[:, 2 * qk + vv:], None, self.H, self.dv, True, "silu", self.eps)
-        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, y, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

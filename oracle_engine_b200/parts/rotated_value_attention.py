@@ -21,7 +21,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import CacheNeed, TensorDecl
 
@@ -131,4 +131,4 @@ class RotatedValueAttention(Part):
         from . import attention_dispatch as ad
         ad.split_attend(self.rt, o, q, kc, vc, cache.tables, ctx, self.H, self.G, self.dk, self.dv, self.window, self.scale,
                         0.0, self.sinks, unrotate=value_tables)      # the turn back happens where the result is stored
-        matmul_nt(self.rt, residual, o, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, o, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

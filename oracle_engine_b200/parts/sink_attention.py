@@ -17,7 +17,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import TensorDecl, attention_cache_need
 
@@ -107,4 +107,4 @@ class SinkAttention(Part):
             y = self.rt.buffer("sink.y", T, qw)
             ops.head_gate(y, o, qkg[:, qw + kw:], None, self.H, self.hd, False, "sigmoid")
             o = y
-        matmul_nt(self.rt, residual, o, self.w_o, accumulate=not overwrite)
+        matmul_nt(self.rt, residual, o, self.w_o, accumulate=not overwrite, early=output_flags(self.w_o))

@@ -15,7 +15,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .linear import matmul_nt
+from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
@@ -119,4 +119,4 @@ class DecayTimeMix(Part):
             ops.decay_scan(o, state["S"], r, k, v, z, self.u, self.w0, ctx, self.H, self.d)
         y = buf("mix.y", T, hd)
         ops.head_gate(y, o, g, self.norm_w, self.H, self.d, True, "silu", self.eps)
-        matmul_nt(self.rt, residual, y, self.w["o"], accumulate=not overwrite)
+        matmul_nt(self.rt, residual, y, self.w["o"], accumulate=not overwrite, early=output_flags(self.w["o"]))

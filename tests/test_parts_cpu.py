@@ -100,3 +100,10 @@ def test_logger_levels_and_format():
     assert len(out.getvalue().splitlines()) == 2
     with pytest.raises(ValueError):
         lg.set_level("loud")
+
+
+def test_an_output_product_starts_early_only_while_its_ctas_have_an_sm_each():
+    from oracle_engine_b200.parts.linear import DEFAULT_FLAGS, START_EARLY, TRIGGER_LATE, output_flags
+    rows = lambda n: torch.empty(n, 64, device="meta")                                    # noqa: E731
+    assert output_flags(rows(16)) == output_flags(rows(148 * 16)) == DEFAULT_FLAGS
+    assert output_flags(rows(148 * 16 + 1)) == TRIGGER_LATE and DEFAULT_FLAGS & START_EARLY
