@@ -26,6 +26,40 @@ def test_a_slot_s_rows_of_every_tensor_and_no_others_are_zeroed():
         store.reset(5)
 
 
+def test_a_reset_goes_through_one_launch_where_rows_are_whole_words(monkeypatch):
+    """Of few tensors as of many; a tensor added later is among the next reset's; rows of odd bytes are filled one by one."""
+    from oracle_engine_b200.cache.state import StateStore
+    from oracle_engine_b200.csrc import ops
+    from oracle_engine_b200.parts.spec import StateNeed
+    launches, zero_rows = [], ops.zero_rows
+    monkeypatch.setattr(ops, "zero_rows", lambda *a: (launches.append(a[0].shape[0]), zero_rows(*a)))
+    store, tensors, want = StateStore(3, DEV), [], []
+    for i, (shape, dtype) in enumerate([((1,), torch.int32), ((4097,), torch.float32), ((2, 3), torch.bfloat16)] * 4 + [((5,), torch.bfloat16)]):
+        tensors.append(store.add(i, "t", StateNeed(shape, dtype)))
+        for t in tensors:
+            t.fill_(3)
+        store.reset(1)
+        if i < 12:
+            want.append(i + 1)
+        assert launches == want
+        for t in tensors:
+            assert (t[1] == 0).all() and (t[[0, 2]] == 3).all()
+
+
+@pytest.mark.parametrize("sizes", [[1], [4], [1023, 1, 70000], [2 ** 20 + 3] + [5] * 40])
+def test_rows_of_a_table_are_zeroed(sizes):
+    """Rows of one word and of more words than the pieces of the grid take at once, of many tensors; the rows around them stay."""
+    from oracle_engine_b200.csrc import ops
+    tensors = [torch.full((3, n), 7, dtype=torch.int32, device=DEV) for n in sizes]
+    table, largest = ops.row_table(tensors)
+    for row in (0, 2):
+        ops.zero_rows(table, largest, row)
+    for t in tensors:
+        assert (t[[0, 2]] == 0).all() and (t[1] == 7).all()
+    with pytest.raises(ops.KernelError):
+        ops.row_table([torch.empty(2, 3, dtype=torch.bfloat16, device=DEV)])
+
+
 @pytest.mark.parametrize("n,penalty", [(1, 1.3), (2, 1.3), (100, 1.3), (257, 1.3), (600, 1.3), (100, 1.0)])
 def test_the_sampler_s_state_at_a_sequence_s_start(n, penalty):
     from oracle_engine_b200.cache.state import StateStore
