@@ -1457,9 +1457,12 @@ def delta_chunks_supported(kv_heads: int, heads: int, dk: int, dv: int) -> bool:
     return kv_heads >= 1 and heads % kv_heads == 0 and dk in (64, 128) and dv % 16 == 0 and 16 <= dv <= 4096
 
 
+SCAN_CHUNK = 32              # tokens of a chunk of the scans in chunks (csrc/delta_chunks.cu, csrc/decay_chunks.cu: CH)
+
+
 def delta_chunks_floats(ctx, heads: int, dk: int, dv: int) -> int:
     """Floats of scratch that delta_chunks needs for a step."""
-    return (ctx.n_tokens // 32 + ctx.n_seqs) * heads * (32 * (3 * dk + dv + 32) + 4)
+    return (ctx.n_tokens // SCAN_CHUNK + ctx.n_seqs) * heads * (32 * (3 * dk + dv + 32) + 4)
 
 
 def delta_chunks(o, state, blocks, qkv, gb, ctx, kv_heads: int, heads: int, dk: int, dv: int) -> None:
@@ -1534,7 +1537,7 @@ def decay_chunks_supported(d: int) -> bool:
 
 def decay_chunks_floats(ctx, heads: int, d: int) -> int:
     """Floats of scratch that decay_chunks needs for a step."""
-    return (ctx.n_tokens // 32 + ctx.n_seqs) * heads * (32 * (3 * d + 32) + d)
+    return (ctx.n_tokens // SCAN_CHUNK + ctx.n_seqs) * heads * (32 * (3 * d + 32) + d)
 
 
 def decay_chunks(o, state, blocks, r, k, v, z, u, w0, ctx, heads: int, d: int) -> None:

@@ -19,6 +19,8 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from ..csrc.ops import SCAN_CHUNK
+
 
 @dataclass
 class SequenceStep:
@@ -41,9 +43,13 @@ class StepPlan:
     seq_qlen: np.ndarray            # [B] int32
     cu_q: np.ndarray                # [B+1] int32
     want_rows: np.ndarray           # [n_want] int32 rows of the packed token list
-    max_qlen: int
+    max_qlen: int                   # the most tokens a sequence brings, or a bound for it (a captured step's padded size)
     max_kvlen: int
     all_decode: bool                # every sequence brings exactly one token
+    # the step's own lengths, without padding: what a part's forward pass chooses by them is part of a captured step's key
+    # (Part.step_choice)
+    longest: int = 0                # the most tokens a sequence brings
+    scan_chunks: int = 0            # pieces of SCAN_CHUNK tokens that its sequences make, each sequence's last one padded
 
 
 def build_plan(seqs: list, starts: list, pad_seqs: int = 0, pad_tokens: int = 0,
@@ -85,7 +91,8 @@ def build_plan(seqs: list, starts: list, pad_seqs: int = 0, pad_tokens: int = 0,
         seq_slot=seq_slot, seq_start=seq_start, seq_qlen=seq_qlen, cu_q=cu_q,
         want_rows=np.asarray(want, dtype=np.int32), max_qlen=max(qlens, default=0),
         max_kvlen=max((st + n for st, n in zip(starts, qlens)), default=0),
-        all_decode=all(n == 1 for n in qlens) and B > 0)
+        all_decode=all(n == 1 for n in qlens) and B > 0, longest=max(qlens, default=0),
+        scan_chunks=sum((n + SCAN_CHUNK - 1) // SCAN_CHUNK for n in qlens))
 
 
 # Steps are classed by the longest sequence they touch: kernels may be chosen by the class, and a
@@ -118,6 +125,9 @@ class StepContext:
     max_kvlen: int
     all_decode: bool
     context_class: int = 0          # context_class() of the longest sequence (kernels may choose by it)
+    n_real_tokens: int = 0          # without padding, and the two below of the sequences as they are (see StepPlan)
+    longest: int = 0
+    scan_chunks: int = 0
 
 
 class StepBuffers:
@@ -195,4 +205,5 @@ class StepBuffers:
             n_tokens=self.n_tokens, n_seqs=self.n_seqs, n_want=self.n_want, token_ids=v[0], tok_seq=v[1],
             tok_pos=v[2], seq_slot=v[3], seq_start=v[4], seq_qlen=v[5], cu_q=v[6], want_rows=v[7], tables=tabs,
             max_qlen=plan.max_qlen, max_kvlen=plan.max_kvlen, all_decode=plan.all_decode,
-            context_class=context_class(plan.max_kvlen))
+            context_class=context_class(plan.max_kvlen), n_real_tokens=plan.n_real_tokens, longest=plan.longest,
+            scan_chunks=plan.scan_chunks)

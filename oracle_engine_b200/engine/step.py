@@ -92,7 +92,8 @@ class Stepper:
         self._stages = model.stages()
         self.use_graphs = bool(use_graphs and any(safe for safe, _, _ in self._stages))
         self._graphs: dict[tuple, _DecodeGraph] = {}      # (padded batch size, long context) -> graph
-        self._token_graphs: dict[tuple, _DecodeGraph] = {}    # (padded tokens, batch size, wanted rows; context class) -> graph
+        # (padded tokens, batch size, wanted rows; context class, what the parts choose by the lengths) -> graph
+        self._token_graphs: dict[tuple, _DecodeGraph] = {}
         self._eager_buffers: dict[tuple, StepBuffers] = {}
         self.launch_counter = None         # set by the bench to count kernel launches
 
@@ -238,7 +239,8 @@ class Stepper:
         return all_logits
 
     def _step_graph_tokens(self, seqs, starts, n_tokens: int, token_arrays=None):
-        """A short step that is no decode step, through a graph of its padded shape.  Everything a kernel's
+        """A short step that is no decode step, through a graph of its padded shape and of what the model's parts choose by
+        its sequences' lengths (DecoderModel.step_choice).  Everything else a kernel's
         launch depends on is the graph's: the token count and the batch size are padded (padding tokens
         belong to no sequence, padding sequences bring no token), the longest sequence's share of the
         step counts as the whole padded step, and the wanted rows are padded with row 0 (to the padded
@@ -251,7 +253,7 @@ class Stepper:
         if n_want > max(bb, MAX_GRAPH_WANTED_ROWS):            # a graph keeps its logits buffer: [rows, vocabulary] float32
             return self._step_eager(seqs, starts, None, token_arrays)
         wb = bb if n_want <= bb else min(tb, MAX_GRAPH_WANTED_ROWS)
-        gkey = (tb, bb, wb, context_class(plan.max_kvlen))
+        gkey = (tb, bb, wb, context_class(plan.max_kvlen), self.model.step_choice(plan))
         g = self._token_graphs.get(gkey)
         if g is None:
             if len(self._token_graphs) >= MAX_TOKEN_GRAPHS:     # shapes beyond these run directly

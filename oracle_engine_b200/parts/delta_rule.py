@@ -22,8 +22,21 @@ from .linear import matmul_nt, output_flags
 from .registry import MIXERS, Part
 from .spec import StateNeed, TensorDecl
 
-CHUNKS_FROM = 64             # tokens of a step's longest sequence from which its scan goes in chunks
-CHUNKS_MAX_TOKENS = 16384     # (the chunks' scratch is 36 KB a token at 16 heads of 128 x 128)
+CHUNKS_FROM = 96              # tokens of a step's longest sequence from which its scan goes in chunks
+CHUNKS_MAX_TOKENS = 16384     # (the chunks' scratch is 36 KB a token at 16 heads of 128 x 128; in a captured step, which keeps it, at most 27 MB)
+
+
+def chunked(tokens: int, longest: int, chunks: int, heads: int, dv: int) -> bool:
+    """Whether the scan of a step (its padded tokens; the most tokens a sequence brings; the chunks that its sequences make)
+    goes in chunks (csrc/delta_chunks.cu) or walks (csrc/recurrent.cu).  In chunks the chain is shorter, but there is more to
+    compute, a CTA (16 columns of a head) fills an SM, and a sequence of one token makes a whole chunk: it pays while the
+    chunks of all sequences, shared out over 148 SMs, are no more than 1.25 times the longest sequence's.  us, walk / chunks,
+    16 heads of 128 x 128: one sequence of 64 26 / 27, 96 38 / 32, 256 98 / 58, 1,111 416 / 256, 4,096 1,525 / 999; 2 of 300
+    168 / 145 (not taken), 4 of 300 208 / 305, 8 of 5 10 / 57, 8 of 300 217 / 579, 32 of 40 113 / 472; one of 192 beside 31 of
+    1 97 / 271.  8 heads: one of 1,111 415 / 213, 2 of 300 114 / 79, 8 of 300 208 / 306, one of 192 beside 7 of 1 89 / 53,
+    beside 31 90 / 133; 24 heads: one of 256 114 / 113 (not taken); 16 of 64 x 64: one of 1,111 300 / 229, 8 of 300 163 / 255."""
+    return CHUNKS_FROM <= longest and tokens <= CHUNKS_MAX_TOKENS and heads * (dv // 16) * chunks <= 185 * -(-longest // ops.SCAN_CHUNK)
+
 
 _NAMES = {"q": "mix.q", "k": "mix.k", "v": "mix.v", "q_conv": "mix.q.conv", "k_conv": "mix.k.conv",
           "v_conv": "mix.v.conv", "b": "mix.b", "a": "mix.a", "A_log": "mix.A_log", "dt_bias": "mix.dt_bias",
@@ -53,6 +66,7 @@ class GatedDelta(Part):
         self.P = self.C + self.H * self.dv + 2 * self.H                     # + gate, beta, a
         self.names = {k: prefix + v for k, v in {**_NAMES, **self.params.get("tensor_names", {})}.items()}
         self.w_in = self.w_o = None
+        self.one_launch = self.chunks = False          # set with the weights
 
     def tensors(self):
         n, qk, vv = self.names, self.G * self.dk, self.H * self.dv
@@ -75,6 +89,9 @@ class GatedDelta(Part):
 
         self.chunks = (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores
                        and ops.delta_chunks_supported(self.G, self.H, self.dk, self.dv))
+
+    def step_choice(self, step) -> bool:
+        return self.chunks and chunked(step.n_tokens, step.longest, step.scan_chunks, self.H, self.dv)
 
     def state_need(self):
         return {"S": StateNeed((self.H, self.dk, self.dv), torch.float32),
@@ -118,7 +135,7 @@ class GatedDelta(Part):
                                self.H, self.dk, self.dv, self.dk ** -0.5)
         ops.conv_state_update(state["conv"], proj, self.C, self.taps, ctx)
         o = buf("delta.o", T, vv, dtype=f32)
-        if self.chunks and CHUNKS_FROM <= ctx.max_qlen and T <= CHUNKS_MAX_TOKENS:
+        if self.step_choice(ctx):
             blocks = buf("delta.blocks", ops.delta_chunks_floats(ctx, self.H, self.dk, self.dv), dtype=f32)
             ops.delta_chunks(o, state["S"], blocks, qkv, gb, ctx, self.G, self.H, self.dk, self.dv)
         else:

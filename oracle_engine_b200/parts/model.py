@@ -9,7 +9,7 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .registry import BLOCKS, EMBEDDINGS, FEED_FORWARDS, HEADS, MIXERS, NORMS, POSITIONS, STREAM_PARTS
+from .registry import BLOCKS, EMBEDDINGS, FEED_FORWARDS, HEADS, MIXERS, NORMS, POSITIONS, STREAM_PARTS, Part
 from .spec import ModelSpec, TensorDecl
 
 # importing the modules registers the built-in parts
@@ -37,6 +37,8 @@ class DecoderModel:
                              for name, ps in spec.stream_parts.items()}
         self._keep_embedding = any(getattr(p, "needs_embedding_output", False) for p in self.stream_parts.values())
         self.embedding_state = {}          # the embedding's per-slot state tensors, bound by the engine
+        self._choosers = [p for layer in self.layers for p in layer.parts()
+                          if getattr(type(p), "step_choice", Part.step_choice) is not Part.step_choice]
 
     def _build_layer(self, ls):
         mparams = dict(ls.mixer.params)
@@ -127,6 +129,10 @@ class DecoderModel:
         return total + self.head.flops(0, n_want)
 
     # ------------------------------------------------------------------ one step
+    def step_choice(self, step) -> tuple:
+        """What the parts choose by the real lengths of a step's sequences (Part.step_choice)."""
+        return tuple(p.step_choice(step) for p in self._choosers)
+
     def forward(self, ctx, cache_views, state_views):
         """Runs the step's tokens through the schedule; returns float32 logits
         [n_want, vocab] at ctx.want_rows, or None if nothing is wanted."""

@@ -129,6 +129,12 @@ class Part:
     def cache_need(self):
         return None
 
+    def step_choice(self, step):
+        """What the forward pass chooses by the real lengths of a step's sequences (`step`: its StepPlan or StepContext, with
+        `longest`, `scan_chunks` and `n_real_tokens`), which the padded sizes of a captured step do not tell: hashable, part of
+        that step's key.  None: nothing."""
+        return None
+
     def state_need(self):
         return {}
 

@@ -22,15 +22,19 @@ from .spec import StateNeed, TensorDecl
 CHUNKS_MAX_TOKENS = 16384    # (the chunks' scratch is 29 KB a token at 32 heads of 64)
 
 
-def chunked(tokens: int, longest: int, heads: int, d: int) -> bool:
-    """Whether the scan of a step goes in chunks (csrc/decay_chunks.cu) or walks (csrc/recurrent.cu).  One sequence alone is
-    bound by its chain of tokens or chunks, many by the additions, which the chunks have more of.  us, walk / chunks, 32 heads
-    of 64: one sequence of 64 25 / 26, 96 36 / 31, 256 90 / 61, 1,111 379 / 227; 8 of 300 234 / 244, 16 of 64 91 / 103, 32 of
-    40 115 / 189; 4 of 1 to 4,096 2,129 / 614.  8 heads of 128: one of 48 27 / 28, 64 35 / 28, 1,111 553 / 157; 8 of 300
-    220 / 154, 16 of 64 99 / 74."""
-    if longest < 64 or tokens > CHUNKS_MAX_TOKENS:
+def chunked(tokens: int, real: int, longest: int, chunks: int, heads: int, d: int) -> bool:
+    """Whether the scan of a step (its tokens with padding and without; the most tokens a sequence brings; the chunks that its
+    sequences make) goes in chunks (csrc/decay_chunks.cu) or walks (csrc/recurrent.cu).  One sequence alone is bound by its
+    chain of tokens or chunks, many by the additions, which the chunks have more of, the more the emptier a sequence's last
+    chunk is: they pay while the chunks of all sequences, shared out over 148 SMs, are no more than 3 times the longest
+    sequence's, and with heads of 128 also where two thirds of them are filled.  us, walk / chunks, 32 heads of 64: one sequence
+    of 64 25 / 26, 96 36 / 31, 256 90 / 61, 1,111 379 / 226; 2 of 300 169 / 79, 4 of 300 216 / 145 (not taken), 8 of 5 12 / 35,
+    8 of 300 233 / 244, 16 of 64 90 / 103, 32 of 40 115 / 189; one of 192 beside 7 of 1 89 / 58, beside 31 92 / 115; 4 of 1 to
+    4,096 2,041 / 618.  8 heads of 128: one of 48 27 / 28, 64 35 / 28, 1,111 554 / 157; 8 of 5 12 / 40, 8 of 300 219 / 154, 16 of
+    64 99 / 74; 16 heads of 128: one of 192 beside 31 of 1 110 / 137."""
+    if longest < (64 if d >= 128 else 96) or tokens > CHUNKS_MAX_TOKENS:
         return False
-    return d >= 128 or (longest >= 96 and tokens * heads <= 96 * longest)
+    return heads * (d // 16) * chunks <= 444 * -(-longest // ops.SCAN_CHUNK) or (d >= 128 and 2 * ops.SCAN_CHUNK * chunks <= 3 * real)
 
 
 _MIXES = ("r", "k", "v", "g", "w")
@@ -76,6 +80,10 @@ class DecayTimeMix(Part):
             raise ValueError(f"{n['w2']}: {self.w['w2'].shape[1]} columns, but {n['w1']} has {self.rank} rows")
         self.w0, self.u, self.norm_w = f32(get(n["w0"])), f32(get(n["u"])).reshape(-1), f32(get(n["norm"]))
 
+    def step_choice(self, step) -> bool:
+        return (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores and ops.decay_chunks_supported(self.d)
+                and chunked(step.n_tokens, step.n_real_tokens, step.longest, step.scan_chunks, self.H, self.d))
+
     def state_need(self):
         return {"S": StateNeed((self.H, self.d, self.d), torch.float32), "prev": StateNeed((self.D,), torch.float32)}
 
@@ -111,8 +119,7 @@ class DecayTimeMix(Part):
         matmul_nt(self.rt, z, th, self.w["w2"])
         o = buf("mix.o", T, hd, dtype=f32)
         # prompts in chunks (the 32-bit path keeps the walk whose bits do not depend on how a sequence is cut)
-        if self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores and ops.decay_chunks_supported(self.d) \
-                and chunked(T, ctx.max_qlen, self.H, self.d):
+        if self.step_choice(ctx):
             blocks = buf("mix.blocks", ops.decay_chunks_floats(ctx, self.H, self.d), dtype=f32)
             ops.decay_chunks(o, state["S"], blocks, r, k, v, z, self.u, self.w0, ctx, self.H, self.d)
         else:
