@@ -9,6 +9,8 @@ batch.  The kernels are in csrc/sampling.cu.
 """
 from __future__ import annotations
 
+from array import array
+
 import numpy as np
 import torch
 
@@ -35,12 +37,21 @@ class Sampler:
         if params.repeat_penalty > 1.0 and recorded > 0:
             if params.repeat_last_n > HISTORY_CAPACITY:
                 raise ValueError(f"repeat_last_n {params.repeat_last_n} exceeds the {HISTORY_CAPACITY} tokens kept")
-            tail = np.asarray(prompt[max(0, recorded - HISTORY_CAPACITY):recorded], dtype=np.int32)
+            tail = prompt[max(0, recorded - HISTORY_CAPACITY):recorded]
+            try:
+                tail = np.frombuffer(array("i", tail), dtype=np.int32)
+            except TypeError:                      # whatever else int() takes; ids beyond 32 bits raise OverflowError
+                tail = np.frombuffer(array("i", [int(t) for t in tail]), dtype=np.int32)
             count = recorded
             ring = np.zeros(HISTORY_CAPACITY, dtype=np.int32)
             ring[(count - tail.size + np.arange(tail.size)) % HISTORY_CAPACITY] = tail
         if not -2 ** 63 <= int(seed) < 2 ** 63:
             raise OverflowError(f"seed {seed} does not fit 64 bits")
+        if not self.hist.is_cuda:
+            self.rng_seed[slot], self.rng_counter[slot], self.hist_count[slot] = int(seed), 0, count
+            if ring is not None:
+                self.hist[slot] = torch.from_numpy(ring)
+            return
         ops.sampler_start(self.rng_seed, self.rng_counter, self.hist, self.hist_count, slot, seed, count, ring)
 
     def sample(self, logits: torch.Tensor, row_slot: torch.Tensor, params, out: torch.Tensor | None = None):

@@ -81,3 +81,14 @@ def test_the_sampler_s_state_at_a_sequence_s_start(n, penalty):
         assert sampler.hist[2].tolist() == want
     with pytest.raises(OverflowError):
         sampler.start_sequence(0, 1 << 63, prompt, GenParams())
+
+
+def test_a_prompt_on_the_device_is_recorded_as_a_list_is():
+    from oracle_engine_b200.cache.state import StateStore
+    from oracle_engine_b200.sampling.params import GenParams
+    from oracle_engine_b200.sampling.sampler import Sampler
+    sampler = Sampler(StateStore(2, DEV), DEV)
+    prompt = [3 * i for i in range(300)]
+    sampler.start_sequence(0, 1, prompt, GenParams())
+    sampler.start_sequence(1, 1, torch.tensor(prompt, device=DEV), GenParams())
+    assert torch.equal(sampler.hist[0], sampler.hist[1]) and sampler.hist_count.tolist() == [299, 299]

@@ -49,3 +49,33 @@ def test_ids_of_any_kind_become_the_array_that_numpy_makes():
     for tokens in (["a"], [None]):
         with pytest.raises((TypeError, ValueError)):
             _id_array(tokens)
+
+
+@pytest.mark.parametrize("n", [1, 2, 100, 257, 600])
+def test_a_sequence_s_start_records_prompts_of_any_kind(n):
+    """On the host as on the device; the ids may come in whatever int() takes them from."""
+    import torch
+
+    from oracle_engine_b200.cache.state import StateStore
+    from oracle_engine_b200.sampling.params import GenParams
+    from oracle_engine_b200.sampling.sampler import HISTORY_CAPACITY, Sampler
+    ids = [7 * i % 1000 for i in range(n)]
+    want = [0] * HISTORY_CAPACITY
+    for i, t in enumerate(ids[:-1]):
+        want[i % HISTORY_CAPACITY] = t
+    for prompt in (ids, tuple(ids), np.asarray(ids), np.asarray(ids, dtype=np.int16), torch.tensor(ids), [torch.tensor(i) for i in ids],
+                   [float(i) for i in ids], [str(i) for i in ids]):
+        sampler = Sampler(StateStore(3, "cpu"), "cpu")
+        sampler.hist.fill_(5)
+        sampler.start_sequence(1, -9, prompt, GenParams())
+        assert (int(sampler.rng_seed[1]), int(sampler.rng_counter[1]), int(sampler.hist_count[1])) == (-9, 0, n - 1)
+        assert sampler.hist[1].tolist() == (want if n > 1 else [5] * HISTORY_CAPACITY) and (sampler.hist[[0, 2]] == 5).all()
+
+
+def test_ids_that_do_not_fit_are_not_recorded_as_others():
+    from oracle_engine_b200.cache.state import StateStore
+    from oracle_engine_b200.sampling.params import GenParams
+    from oracle_engine_b200.sampling.sampler import Sampler
+    for prompt in ([2 ** 32 + 5, 1], np.asarray([2 ** 32 + 5, 1])):
+        with pytest.raises(OverflowError):
+            Sampler(StateStore(1, "cpu"), "cpu").start_sequence(0, 1, prompt, GenParams())
