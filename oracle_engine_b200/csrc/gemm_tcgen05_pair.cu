@@ -57,6 +57,7 @@ struct PairArgs {
     int out_kind;                  // 0 bf16 store, 1 float32 store, 2 float32 accumulate, 3 bf16 silu(gate)*up
     OeEpilogue epi;                // what happens to the sums before a bf16 store (out_kind 0)
     int tiles_m, tiles_n;          // tiles of 256 rows and of n_tile columns
+    int band;                      // row tiles of a band (place_of)
 };
 
 // A product whose row tiles belong to experts (csrc/moe_sparse.cu sorts the rows): C[row] = unit or plain sums of A[row]
@@ -184,13 +185,9 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// Where work item w lies: bands of BAND row tiles, within a band a column of its tiles after the other.  The 74 clusters that
-// run at once then share some 8 row tiles and 9 column tiles, 17 tiles' operands, and a band's activations stay in the L2
-// while the weights go by; with all row tiles of one column first, a prompt step whose activations outgrow the L2 read them
-// again for every column (17,133 x 4,096 activations, 28,672 weight rows: 16 GB instead of 2 GB a product).
-constexpr int BAND = 8;
-__device__ __forceinline__ void place_of(int w, int tiles_m, int tiles_n, int& tile_m, int& tile_n) {
-    const int band = w / (BAND * tiles_n), first = band * BAND, rows = min(BAND, tiles_m - first), in = w - first * tiles_n;
+// Where work item w lies: bands of `band` row tiles, within a band a column of its tiles after the other.
+__device__ __forceinline__ void place_of(int w, int band, int tiles_m, int tiles_n, int& tile_m, int& tile_n) {
+    const int first = w / (band * tiles_n) * band, rows = min(band, tiles_m - first), in = w - first * tiles_n;
     tile_m = first + in % rows;
     tile_n = in / rows;
 }
@@ -322,7 +319,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         bool ok = true;
         for (int w = cluster_id; w < n_work && ok; w += n_clusters) {
             int tile_m, tile_n;
-            place_of(w, tiles_m, g.tiles_n, tile_m, tile_n);
+            place_of(w, g.band, tiles_m, g.tiles_n, tile_m, tile_n);
             const int a_row = tile_m * (2 * BLOCK_M) + (int)rank * BLOCK_M;
             int b_row = tile_n * g.n_tile + (int)rank * b_half_rows, b_col = 0;
             if (GROUPED) {
@@ -390,7 +387,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         bool first = true;
         for (int w = cluster_id; w < n_work; w += n_clusters, lt++) {
             int tile_m, tile_n;
-            place_of(w, tiles_m, g.tiles_n, tile_m, tile_n);
+            place_of(w, g.band, tiles_m, g.tiles_n, tile_m, tile_n);
             const int row = tile_m * (2 * BLOCK_M) + (int)rank * BLOCK_M + row_in_cta;
             const int buf = lt & 1;
             OeGroupWeight kept;                            // of this thread's row, along the tile's columns
@@ -511,6 +508,17 @@ int tile_width(long long tiles_m, int N, int limit, int step) {
     return n_tile;
 }
 
+// Row tiles of a band.  Of eight: the 74 clusters that run at once share some 8 row tiles and 9 column tiles, 17 tiles'
+// operands, and a band's activations stay in the L2 while the weights go by; with all row tiles of one column first, activations
+// that outgrow the L2 come from memory again for every column.  While they fit, all rows first reads the weights once and not
+// once a band, unless those are few beside the activations.  Time with bands of eight / all rows first, activations of
+// 25, 38, 50, 61, 74 and 105 MB (K = 3,072): 5,120 weight rows 1.03, 1.05, 1.03, 0.97, 0.90, 0.81, 16,384 1.06, 1.07, 1.05, 1.02, 0.96,
+// 0.86; 28,672 x 4,096, 34, 41, 50, 57 MB: 1.05, 1.05, 0.99, 0.97; 3,072 x 3,072, 15 to 105 MB: 0.95 to 1.00, 0.81; 2,048 x 2,048,
+// 10 to 70 MB: 0.94 to 0.98; 3,072 x 8,192, 39 to 281 MB: 0.89, 1.01, 1.01, 1.00, 0.97 ... 0.82.
+int band_of(const PairArgs& g) {
+    return 2LL * g.M * g.K > 56000000LL || 2LL * g.N <= 3LL * g.K ? 8 : g.tiles_m;
+}
+
 size_t ring(PairArgs& g) {
     const int n_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
     const int b_bytes = (g.n_tile / 2) * BLOCK_K * 2;
@@ -563,6 +571,7 @@ int oe_gemm_pair_bf16(void* C, const bf16* A, const bf16* W, int M, int N, int K
     CUtensorMap map_a, map_b;
     if ((rc = make_map(&map_a, A, M, K, lda, BLOCK_M))) return rc;
     if ((rc = make_map(&map_b, W, N, K, K, g.n_tile / 2))) return rc;
+    g.band = band_of(g);
     const size_t smem = ring(g);
     const int clusters = (int)(n_work < g_clusters ? n_work : g_clusters);
     return oe_launch(g.epi.act ? gemm_pair_kernel<1> : gemm_pair_kernel<0>, dim3(2 * clusters), dim3(THREADS), smem, st, map_a, map_b, g, GroupArgs{});
@@ -600,6 +609,7 @@ int oe_gemm_pair_grouped_bf16(void* C, const bf16* A, const bf16* W, int M, int 
     else rc = make_map(&map_b, W + first, N, F - first, F, g.n_tile / 2);
     if (rc) return rc;
     const GroupArgs q = {tile_expert, n_tiles, 0, gate_up, ff, F, row_w, row_w_ld, unit, limit};
+    g.band = 8;                                            // every row tile has weights of its own
     const size_t smem = ring(g);
     const int clusters = (int)(n_work < g_clusters ? n_work : g_clusters);
     return oe_launch(gemm_pair_kernel<2>, dim3(2 * clusters), dim3(THREADS), smem, st, map_a, map_b, g, q);
