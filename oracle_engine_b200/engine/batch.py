@@ -77,11 +77,13 @@ def build_plan(seqs: list, starts: list, pad_seqs: int = 0, pad_tokens: int = 0,
         tok_pos[row:row + n] = np.arange(st, st + n, dtype=np.int32)
         seq_slot[b], seq_start[b], seq_qlen[b] = s.slot, st, n
         cu_q[b + 1] = row + n
-        if len(s.want):
-            if min(s.want) < 0 or max(s.want) >= n:
-                bad = next(w for w in s.want if not 0 <= w < n)
-                raise ValueError(f"sequence {b}: wanted place {bad} is outside its {n} tokens")
-            want.extend([row + w for w in s.want])
+        if len(s.want) > 4 and min(s.want) >= 0 and max(s.want) < n:
+            want.extend([row + w for w in s.want])       # a text to be scored
+        else:
+            for w in s.want:
+                if not 0 <= w < n:
+                    raise ValueError(f"sequence {b}: wanted place {w} is outside its {n} tokens")
+                want.append(row + w)
         row += n
     cu_q[B + 1:] = row
     if want_all_rows:
