@@ -8,22 +8,9 @@
 // chunk, still a chain); 8 heads of 128 x 128 553 and 157 us.  Errors against 64 bits as the walk's (5.2e-7 both).  Here
 // decay_chunk_prepare_kernel makes a chunk's decayed vectors and its 32 x 32 scores for all chunks and heads side by side, and
 // decay_chunk_scan_kernel carries 16 columns of a head's state, in registers, from chunk to chunk.
-#include "common.cuh"
+#include "scan_chunks.cuh"
 
 namespace {
-
-constexpr int CH = 32;                 // tokens of a chunk
-constexpr int COLS = 16;               // columns of the state that a CTA of the scan carries
-constexpr int GROUPS = 16;             // threads that share a column, each d / 16 rows of it
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-
-// The chunks of sequence b stand behind those of the sequences before it.
-__device__ __forceinline__ int chunks_of(const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int b) {
-    return seq_slot[b] < 0 ? 0 : (cu_q[b + 1] - cu_q[b] + CH - 1) / CH;
-}
 
 // What the scan reads of a chunk and head: [Kd: CH d | Qd: CH d | V: CH d | M: CH CH | the chunk's decays: d].
 __host__ __device__ __forceinline__ size_t block_floats(int d) { return (size_t)CH * (3 * d + CH) + d; }
@@ -194,15 +181,16 @@ int launch(float* o, float* state, float* blocks, const float* r, const float* k
 
 extern "C" {
 
+int oe_decay_chunks_supported(int d) { return d == 64 || d == 128; }
+
 // blocks: scratch of at least (n_tokens / 32 + n_seqs) H (32 (3 d + 32) + d) floats, 16-byte aligned.  r, k, v, z: rows of
 // `stride` floats, [T, H d].  d 64 or 128.
 int oe_decay_chunks(float* o, float* state, float* blocks, const float* r, const float* k, const float* v, const float* z, long long stride,
                     const float* u, const float* w0, const int* seq_slot, const int* cu_q, int n_tokens, int n_seqs, int H, int d, cudaStream_t st) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
-    if (H < 1 || H > 65535 || n_seqs > 65535 || ((uintptr_t)blocks & 15)) return OE_ERR_UNSUPPORTED;
+    if (!oe_decay_chunks_supported(d) || H < 1 || H > 65535 || n_seqs > 65535 || ((uintptr_t)blocks & 15)) return OE_ERR_UNSUPPORTED;
     if (d == 64) return launch<64>(o, state, blocks, r, k, v, z, stride, u, w0, seq_slot, cu_q, n_tokens, n_seqs, H, st);
-    if (d == 128) return launch<128>(o, state, blocks, r, k, v, z, stride, u, w0, seq_slot, cu_q, n_tokens, n_seqs, H, st);
-    return OE_ERR_UNSUPPORTED;
+    return launch<128>(o, state, blocks, r, k, v, z, stride, u, w0, seq_slot, cu_q, n_tokens, n_seqs, H, st);
 }
 
 }  // extern "C"

@@ -11,22 +11,9 @@
 // 64 CTAs of which a scheduler had one or two warps).  Here delta_chunk_solve_kernel does what does not depend on the state
 // for all chunks and heads side by side, and delta_chunk_scan_kernel carries 16 columns of a head's state, in registers,
 // from chunk to chunk: the chain has 32 times fewer links.  Products of decays are formed as such, without dividing.
-#include "common.cuh"
+#include "scan_chunks.cuh"
 
 namespace {
-
-constexpr int CH = 32;                 // tokens of a chunk
-constexpr int COLS = 16;               // columns of the state that a CTA of the scan carries
-constexpr int GROUPS = 16;             // threads that share a column, each dk / 16 rows of it
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-
-// The chunks of sequence b stand behind those of the sequences before it.
-__device__ __forceinline__ int chunks_of(const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int b) {
-    return seq_slot[b] < 0 ? 0 : (cu_q[b + 1] - cu_q[b] + CH - 1) / CH;
-}
 
 // What the scan reads of a chunk and head, one block of floats: [W: CH dk | Kd: CH dk | Qg: CH dk | Uv: CH dv | M: CH CH | G: 4].
 __host__ __device__ __forceinline__ size_t block_floats(int dk, int dv) { return (size_t)CH * (3 * dk + dv + CH) + 4; }

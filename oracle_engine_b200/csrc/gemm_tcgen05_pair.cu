@@ -63,9 +63,8 @@ struct PairArgs {
 // A product whose row tiles belong to experts (csrc/moe_sparse.cu sorts the rows): C[row] = unit or plain sums of A[row]
 // and the weights of the row tile's expert, which lie among all experts' in W.
 struct GroupArgs {
-    const int* tile_expert;        // the expert of every tile of 256 rows; null: one expert, `expert`, for all rows
+    const int* tile_expert;        // the expert of every tile of 256 rows; null: one expert for all rows, the one the weights begin with
     const int* n_tiles;            // how many tiles there are (null: tiles_m), written by an earlier kernel
-    int expert;
     int gate_up;                   // 1: the leader's half of a weight tile are gate rows, the other's the up rows that belong
                                    // to them, F rows further down; C [M, ff] bf16.  0: n_tile rows of W, columns of one expert
     int ff, F;                     // an expert's rows (gate_up) or columns, and all of them
@@ -323,7 +322,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const int a_row = tile_m * (2 * BLOCK_M) + (int)rank * BLOCK_M;
             int b_row = tile_n * g.n_tile + (int)rank * b_half_rows, b_col = 0;
             if (GROUPED) {
-                const int e = q.tile_expert ? q.tile_expert[tile_m] : q.expert;
+                const int e = q.tile_expert ? q.tile_expert[tile_m] : 0;
                 if (q.gate_up) b_row = (int)rank * q.F + e * q.ff + tile_n * b_half_rows;
                 else b_col = e * q.ff;
             }
@@ -608,7 +607,7 @@ int oe_gemm_pair_grouped_bf16(void* C, const bf16* A, const bf16* W, int M, int 
     if (gate_up) rc = make_map(&map_b, W + (size_t)first * K, 2LL * F - first, K, K, g.n_tile / 2);
     else rc = make_map(&map_b, W + first, N, F - first, F, g.n_tile / 2);
     if (rc) return rc;
-    const GroupArgs q = {tile_expert, n_tiles, 0, gate_up, ff, F, row_w, row_w_ld, unit, limit};
+    const GroupArgs q = {tile_expert, n_tiles, gate_up, ff, F, row_w, row_w_ld, unit, limit};
     g.band = 8;                                            // every row tile has weights of its own
     const size_t smem = ring(g);
     const int clusters = (int)(n_work < g_clusters ? n_work : g_clusters);

@@ -123,12 +123,15 @@ _SIGNATURES = {
         "oe_head_matmul": [_P, _L, _L, _P, _L, _L, _P, _I, _I, _I, _I, _P],
     },
     "delta_step": {
+        "oe_delta_step_supported": [_I, _I, _I, _I, _I],
         "oe_delta_step": [_P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P],
     },
     "delta_chunks": {
+        "oe_delta_chunks_supported": [_I, _I, _I, _I],
         "oe_delta_chunks": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     },
     "decay_chunks": {
+        "oe_decay_chunks_supported": [_I],
         "oe_decay_chunks": [_P, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     },
     "recurrent": {
@@ -1429,9 +1432,8 @@ def delta_rule_scan(o, state, qkv, gb, ctx, kv_heads: int, heads: int, dk: int, 
 
 
 def delta_step_supported(kv_heads: int, heads: int, dk: int, dv: int, taps: int) -> bool:
-    """Whether delta_step takes these sizes (csrc/delta_step.cu: oe_delta_step_supported)."""
-    return (kv_heads >= 1 and heads % kv_heads == 0 and heads // kv_heads <= 8 and 4 <= dv <= 256 and dv % 4 == 0 and dk >= 1
-            and 1 <= taps <= 8 and dk % 2 == 0 and dk <= 16 * (256 // (dv // 4)) and 2 * dk + dv <= 768)
+    """Whether delta_step takes these sizes."""
+    return bool(_fn("delta_step", "oe_delta_step_supported")(kv_heads, heads, dk, dv, taps))
 
 
 def delta_step(y, state, conv_state, proj, conv_w, A_log, dt_bias, norm_w, ctx, kv_heads: int, heads: int, dk: int, dv: int, q_scale: float,
@@ -1453,8 +1455,8 @@ def delta_step(y, state, conv_state, proj, conv_w, A_log, dt_bias, norm_w, ctx, 
 
 
 def delta_chunks_supported(kv_heads: int, heads: int, dk: int, dv: int) -> bool:
-    """Whether delta_chunks takes these sizes (csrc/delta_chunks.cu: oe_delta_chunks_supported)."""
-    return kv_heads >= 1 and heads % kv_heads == 0 and dk in (64, 128) and dv % 16 == 0 and 16 <= dv <= 4096
+    """Whether delta_chunks takes these sizes."""
+    return bool(_fn("delta_chunks", "oe_delta_chunks_supported")(kv_heads, heads, dk, dv))
 
 
 SCAN_CHUNK = 32              # tokens of a chunk of the scans in chunks (csrc/delta_chunks.cu, csrc/decay_chunks.cu: CH)
@@ -1532,7 +1534,7 @@ def decay_scan(o, state, r, k, v, z, u, w0, ctx, heads: int, d: int) -> None:
 
 def decay_chunks_supported(d: int) -> bool:
     """Whether decay_chunks takes heads of this size."""
-    return d in (64, 128)
+    return bool(_fn("decay_chunks", "oe_decay_chunks_supported")(d))
 
 
 def decay_chunks_floats(ctx, heads: int, d: int) -> int:

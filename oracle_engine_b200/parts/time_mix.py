@@ -61,6 +61,7 @@ class DecayTimeMix(Part):
             raise ValueError("decay_time_mix: head_dim up to 256 is supported")
         self.names = {k: prefix + v for k, v in {**_NAMES, **self.params.get("tensor_names", {})}.items()}
         self.w = {}
+        self.chunks = False            # set with the weights
 
     def tensors(self):
         n, hd = self.names, self.H * self.d
@@ -79,10 +80,11 @@ class DecayTimeMix(Part):
         if self.w["w2"].shape[1] != self.rank:
             raise ValueError(f"{n['w2']}: {self.w['w2'].shape[1]} columns, but {n['w1']} has {self.rank} rows")
         self.w0, self.u, self.norm_w = f32(get(n["w0"])), f32(get(n["u"])).reshape(-1), f32(get(n["norm"]))
+        # (the 32-bit path keeps the walk whose bits do not depend on how a sequence is cut)
+        self.chunks = self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores and ops.decay_chunks_supported(self.d)
 
     def step_choice(self, step) -> bool:
-        return (self.rt.dtype == torch.bfloat16 and self.rt.tensor_cores and ops.decay_chunks_supported(self.d)
-                and chunked(step.n_tokens, step.n_real_tokens, step.longest, step.scan_chunks, self.H, self.d))
+        return self.chunks and chunked(step.n_tokens, step.n_real_tokens, step.longest, step.scan_chunks, self.H, self.d)
 
     def state_need(self):
         return {"S": StateNeed((self.H, self.d, self.d), torch.float32), "prev": StateNeed((self.D,), torch.float32)}
@@ -118,7 +120,6 @@ class DecayTimeMix(Part):
         ops.tanh_rows(th, low)
         matmul_nt(self.rt, z, th, self.w["w2"])
         o = buf("mix.o", T, hd, dtype=f32)
-        # prompts in chunks (the 32-bit path keeps the walk whose bits do not depend on how a sequence is cut)
         if self.step_choice(ctx):
             blocks = buf("mix.blocks", ops.decay_chunks_floats(ctx, self.H, self.d), dtype=f32)
             ops.decay_chunks(o, state["S"], blocks, r, k, v, z, self.u, self.w0, ctx, self.H, self.d)
