@@ -58,8 +58,8 @@ class PreNormBlock:
         h = self.mixer_norm.forward(x)
         if rt is not None:
             rt.next_weights = _first_weights(self.feed_forward) if self.feed_forward is not None else after
-            rt.next_norm = leaves_to(self.mixer, self.ffn_norm, self.feed_forward) if self.feed_forward is not None \
-                else norm_after
+            if rt.leaving and self.feed_forward is not None:
+                rt.next_norm = leaves_to(self.mixer, self.ffn_norm, self.feed_forward)
         self.mixer.forward(h, x, ctx, cache, state, owns_cache)
         if self.feed_forward is not None:
             h = self.ffn_norm.forward(x)

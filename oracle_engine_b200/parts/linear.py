@@ -63,7 +63,7 @@ def matmul_nt(rt, out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulat
         from ..csrc import ops_tc
         scaled = isinstance(a, ops_tc.ScaledRows)
         if scaled or ops_tc.gemm_supported(a, w, out):
-            leave = rt.leave_normed(out) if accumulate else None
+            leave = rt.leave_normed(out) if accumulate and rt.leaving else None
             if leave is not None:           # what comes next is a product with many CTAs, not a norm
                 early |= TRIGGER_LATE
             ops_tc.gemm(out, a, w, accumulate=accumulate, early=int(early), then=then, leave=leave)

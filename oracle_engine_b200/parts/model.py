@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from ..csrc import ops
+from ..csrc import ops, ops_tc
 from .registry import BLOCKS, EMBEDDINGS, FEED_FORWARDS, HEADS, MIXERS, NORMS, POSITIONS, STREAM_PARTS, Part
 from .spec import ModelSpec, TensorDecl
 
@@ -156,6 +156,7 @@ class DecoderModel:
 
     def run_entries(self, x, ctx, cache_views, state_views, lo: int, hi: int) -> None:
         self.rt.next_norm = self.rt.normed = None
+        self.rt.leaving = self.rt.tensor_cores and x.shape[0] <= ops_tc.SCALED_MAX_TOKENS
         if lo == 0:
             self.rt.cast_cache = None          # nothing of an earlier pass is taken for this one's stream
         for i in range(lo, hi):
@@ -166,11 +167,12 @@ class DecoderModel:
             first = getattr(nxt, "first_weights", None)
             self.rt.next_weights = first() if first is not None else None
             # and the norm that reads the stream behind this entry, if nothing else does first (the next entry of this run)
-            self.rt.next_norm = self._norm_between(e, self.schedule[i + 1]) if i + 1 < hi else None
+            self.rt.next_norm = self._norm_between(e, self.schedule[i + 1]) if self.rt.leaving and i + 1 < hi else None
             if e.before is not None:
                 self.stream_parts[e.before[0]].forward(x, ctx, **dict(e.before[1]))
             self.layers[e.layer].forward(x, ctx, cache_views[owner], state_views[i], e.cache_from is None)
         self.rt.next_weights = self.rt.next_norm = self.rt.normed = None
+        self.rt.leaving = False
 
     def _norm_between(self, entry, following):
         """The norm between two entries that the products around it may do the work of, else None."""

@@ -47,9 +47,11 @@ class RMSNorm(Part):
     can_be_left = property(lambda self: self.groups == 1)
 
     def forward(self, x):
-        left, self.rt.normed = self.rt.normed, None
-        if left is not None and left[0] == x.data_ptr() and left[1] is self:
-            return left[2]
+        left = self.rt.normed
+        if left is not None:
+            self.rt.normed = None
+            if left[0] == x.data_ptr() and left[1] is self:
+                return left[2]
         y = self.rt.empty(*x.shape)
         if self.groups > 1:
             ops.group_rmsnorm(y, x, self.weight, self.eps, self.groups)

@@ -72,3 +72,21 @@ def test_a_decoder_uses_it(batch, monkeypatch):
     assert sum(used[:6]) == (5 if batch <= 4 else 0)                       # two norms a layer but the first and the last
     other = run(lambda self, out: None)
     assert torch.isfinite(mine).all() and ((mine - other).norm() / other.norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("tokens", [4, 5, 300])
+def test_passes_of_more_rows_do_not_look_for_it(tokens, monkeypatch):
+    """What a pass launched kernel by kernel would pay for on the host in every layer."""
+    from oracle_engine_b200.config.base import get_architecture
+    from oracle_engine_b200.engine.batch import SequenceStep
+    from oracle_engine_b200.engine.engine import Engine
+    from oracle_engine_b200.engine.runtime import Runtime
+    from oracle_engine_b200.parts import block
+    cfg = get_architecture("LlamaForCausalLM").config_cls.from_dict(dict(
+        architectures=["LlamaForCausalLM"], vocab_size=256, hidden_size=256, num_hidden_layers=3, num_attention_heads=4, num_key_value_heads=2,
+        head_dim=64, intermediate_size=512, rms_norm_eps=1e-5, max_position_embeddings=512, tie_word_embeddings=True))
+    eng, calls = Engine.from_config(cfg, seed=3, std=0.1, dtype="bfloat16", max_tokens=1024, use_graphs=False), []
+    for owner, name in ((block, "leaves_to"), (Runtime, "leave_normed")):
+        monkeypatch.setattr(owner, name, lambda *a, f=getattr(owner, name): (calls.append(1), f(*a))[1])
+    out = eng.step([SequenceStep(eng.alloc(), [t % 256 for t in range(tokens)], [tokens - 1])])
+    assert torch.isfinite(out).all() and bool(calls) == (tokens <= 4)
