@@ -31,7 +31,10 @@ _BUCKETS = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256)
 # tokens mixed) is captured as well, per padded token count, padded batch size and context class: launched
 # one by one its 230 kernels cost the host 3.1 ms, twice what the device needs for them.
 GRAPH_STEP_TOKENS = 256
-EARLY_LAUNCH_MAX_TOKENS = 512       # steps of more tokens launch their kernels without programmatic stream serialization
+# Steps of more tokens launch their kernels without programmatic stream serialization (_step_eager says why); of a model with a
+# mixture of experts those of more than a captured step's.
+EARLY_LAUNCH_MAX_TOKENS = 512
+EARLY_LAUNCH_MAX_TOKENS_MIXTURE = GRAPH_STEP_TOKENS
 MAX_TOKEN_GRAPHS = 64
 MAX_GRAPH_WANTED_ROWS = 64
 _TOKEN_BUCKETS = (16, 32, 64, 128, 256)
@@ -189,7 +192,10 @@ class Stepper:
         # about once in ten to forty steps, for minutes, in three designs; without it 100 such steps in a row ran
         # through.  What the early starts win is in the chains of short kernels of small steps (a third of a decode step),
         # where nothing of the kind was ever seen; on a prompt step of thousands of tokens they win 3 %.
-        calm = plan.n_tokens > EARLY_LAUNCH_MAX_TOKENS
+        # One run of prompts of 270 to 1,500 tokens (mixtures of experts at width 3,072, the products of every expert and of
+        # the chosen ones in turn) stood still as well, for half an hour, at 330 tokens or more, and the cause is not known:
+        # such a model's steps start nothing early beyond what is captured.
+        calm = plan.n_tokens > (EARLY_LAUNCH_MAX_TOKENS_MIXTURE if self.model.has_mixture else EARLY_LAUNCH_MAX_TOKENS)
         if calm:
             _build.set_early_launch(False)
         try:

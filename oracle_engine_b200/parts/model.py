@@ -37,6 +37,7 @@ class DecoderModel:
                              for name, ps in spec.stream_parts.items()}
         self._keep_embedding = any(getattr(p, "needs_embedding_output", False) for p in self.stream_parts.values())
         self.embedding_state = {}          # the embedding's per-slot state tensors, bound by the engine
+        self.has_mixture = any(getattr(p, "mixture", False) for layer in self.layers for p in layer.parts())
         self._choosers = [p for layer in self.layers for p in layer.parts()
                           if getattr(type(p), "step_choice", Part.step_choice) is not Part.step_choice]
 

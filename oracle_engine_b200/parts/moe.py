@@ -72,6 +72,7 @@ def _groups(raw, experts: int, top: int):
 @FEED_FORWARDS.register("moe_swiglu")
 class MoESwiGLU(Part):
     graph_safe = True
+    mixture = True
     can_overwrite = True
     """params: hidden_size, num_experts, top, expert_size, shared_size (0 or None: no shared expert), router_weights
     ("softmax", the default: the softmax over the chosen logits alone; "sigmoid": each chosen expert's own
@@ -209,6 +210,7 @@ class MoESwiGLU(Part):
 @FEED_FORWARDS.register("moe_relu2")
 class MoEReLU2(Part):
     graph_safe = True
+    mixture = True
     can_overwrite = True
     """params: hidden_size, num_experts, top, expert_size, groups (None, or {"count", "keep"}), router_weights
     ("softmax_all", the default, "softmax" or "sigmoid", as csrc/ops.py: moe_route), tensor_names (optional overrides of

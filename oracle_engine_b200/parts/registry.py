@@ -115,6 +115,8 @@ class Part:
     # says it of its own forward.
     runs_beside = False
 
+    mixture = False                # a mixture of experts
+
     def __init__(self, params: dict, prefix: str, runtime):
         self.params = dict(params)
         self.prefix = prefix
