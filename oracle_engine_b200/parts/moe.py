@@ -21,10 +21,11 @@ routed ones) and all down columns; the router and the shared gate are one small 
 per token and expert, zero where it was not chosen, sigmoid(Wsg h) for the shared one) stays on the device, so a step is
 the same kernels whatever the routing (and can be captured in a graph).  By the number of a step's tokens:
 
-* up to 16 (bfloat16): the weight-streaming products over the experts that some token chose (csrc/moe_sparse.cu);
+* few beside the experts (`_stream_pays`, up to 16, bfloat16): the weight-streaming products over the experts that some token
+  chose (csrc/moe_sparse.cu);
 * from where it pays (`_sorted_pays`, bfloat16): the (token, expert) pairs sorted by expert and the grouped products over
   them, the arithmetic of the chosen experts and what fills their last row tiles; the shared expert over all tokens;
-* else, in float32 and for sizes those do not take: one product with all gate and up matrices, one kernel that applies the
+* else, between the two, in float32 and for sizes those do not take: one product with all gate and up matrices, one kernel that applies the
   unit and multiplies each expert's columns by the token's weight, and one product with all down matrices.
 """
 from __future__ import annotations
@@ -37,13 +38,29 @@ from .registry import FEED_FORWARDS, Part
 from .spec import TensorDecl
 
 
-STREAM_TOKENS = 16           # a step's tokens up to which a mixture's products stream the chosen experts' weights
+STREAM_TOKENS = 16           # the most tokens that the kernels which stream the chosen experts' weights take
 
 
-def _sorted_pays(T: int, top: int, experts: int) -> bool:
-    """Whether sorting T tokens by expert saves at least a third of the rows that the products over all experts have: a
-    token's rows are its experts', and every expert's last tile of 256 rows is half empty on average."""
-    return 3 * (T * top + 128 * experts) <= 2 * T * experts
+def _stream_pays(T: int, top: int, experts: int) -> bool:
+    """Whether T tokens choose few enough of the experts for the kernels that stream the chosen ones' weights; they read at a
+    lower rate than the products over all experts, and tokens that choose differently leave little to skip.  us a decode step,
+    streamed / all experts, 8 experts of which a token has 2, 8 layers: Fovirax, width 2,048, 2 tokens 530 / 601, 4 607 / 620, 6
+    696 / 661, 8 778 / 696, 16 959 / 846, width 3,072, 2 851 / 966, 4 974 / 998, 6 1,072 / 1,035, 16 1,482 / 1,332; Mavinex, width 2,048, 2
+    534 / 610, 4 634 / 658, 6 695 / 696, 8 703 / 681, 16 925 / 825; Pusunex, 4 732 / 756, 6 790 / 797, 8 810 / 794, 16 972 / 905.
+    (Bogupel with random weights, whose tokens all choose alike, 8 494 / 559.)"""
+    return T <= STREAM_TOKENS and T * top <= experts
+
+
+def _sorted_pays(T: int, top: int, experts: int, D: int, ff: int) -> bool:
+    """Whether sorting T tokens by expert saves at least a third of the rows that the products over all experts have (a
+    token's rows are its experts', and every expert's last tile of 256 rows is half empty on average), and 130 GFLOP, 0.1 ms: the
+    four launches more take 60 us a layer on the host, and as much on the device for what is not the products.  ms a prompt
+    step, sorted / all experts, 8 layers: width 1,024 (experts of 704), 2,000 tokens (48 GFLOP) 3.60 / 3.46 Fovirax, 3.26 / 3.13 Mavinex;
+    2,048 (1,408), 700 (55) 3.64 / 3.35, 3.33 / 3.00, 1,000 (86) 3.84 / 3.88, 3.16 / 3.31, 1,500 (138) 4.92 / 4.93, 3.71 / 4.11; 3,072
+    (2,048), 512 (77) 4.03 / 3.87, 3.38 / 3.38, 700 (120) 4.62 / 4.66, 3.62 / 3.97, Pusunex 4.74 / 4.57, 1,000 (188) 5.23 / 5.67,
+    4.25 / 4.92, 5.14 / 5.43."""
+    saved = T * experts - (T * top + 128 * experts)
+    return 3 * saved >= T * experts and 6.0 * saved * D * ff >= 130e9
 
 
 def _route(rt, h, w_route, experts: int, top: int, has_gate, dense, ctx, weights, bias, groups) -> None:
@@ -171,12 +188,12 @@ class MoESwiGLU(Part):
         _route(self.rt, h, self.w_route, self.E, self.top, (True if self.shared_gate else "one") if self.sff else False,
                dense, ctx, self.router_weights, self.bias, self.groups)
         aligned = h.stride(1) == 1 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
-        if self.sparse and aligned and T <= STREAM_TOKENS:
+        if self.sparse and aligned and _stream_pays(T, self.top, self.E):
             a = self.rt.buffer("moe.a", T, self.F)
             ops.moe_up_stream(a, h, self.w_gu, dense, self.E, self.ff, self.unit, self.limit)
             ops.moe_down_stream(residual, a, self.w_down, dense, self.E, self.ff, accumulate=not overwrite)
             return
-        if self.sparse and aligned and _sorted_pays(T, self.top, self.E):
+        if self.sparse and aligned and _sorted_pays(T, self.top, self.E, self.D, self.ff):
             self._forward_sorted(h, residual, dense, overwrite)
             return
         gu = self.rt.buffer("moe.gu", T, 2 * self.F)

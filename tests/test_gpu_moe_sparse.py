@@ -38,7 +38,8 @@ def _want(h, w_gu, w_down, dense, E, ff, unit, limit):
     return a @ w_down.double().T, a.abs() @ w_down.double().abs().T
 
 
-SIZES = [(8, 2, 64, 0, 64, 48), (3, 1, 24, 40, 136, 50), (64, 8, 16, 16, 72, 256), (5, 3, 152, 0, 520, 200), (1, 1, 40, 0, 64, 40)]
+SIZES = [(8, 2, 64, 0, 64, 48), (3, 1, 24, 40, 136, 50), (64, 8, 16, 16, 72, 256), (5, 3, 152, 0, 520, 200), (1, 1, 40, 0, 64, 40),
+         (3, 2, 24, 104, 136, 52)]
 CASES = [("spread", "silu"), ("one", "clamped"), ("padding", "scale_input")]
 
 
@@ -67,8 +68,7 @@ def test_streamed_experts(E, top, ff, sff, D, N, kind, unit):
         ops.moe_up_stream(a[:1], h[:1], w_gu, dense[:1], E, ff, unit, 1.5)
         one = torch.empty(1, N, device=DEV)
         ops.moe_down_stream(one, a[:1], w_down, dense[:1], E, ff, accumulate=False)
-        if T <= 8:
-            assert torch.equal(one[0], out[0])
+        assert torch.equal(one[0], out[0])
 
 
 @pytest.mark.parametrize("E,top,ff,sff,D,N", SIZES)
@@ -108,11 +108,13 @@ def test_sorted_experts(E, top, ff, sff, D, N, kind, unit, T):
     base = torch.randn(T, N, generator=g).to(DEV)
     for accumulate in (False, True):
         out = base.clone()
-        if N % 4:
+        if N % 4:                                             # the adding kernel refuses the width: by hand, for what is behind it
             with pytest.raises(ops.KernelError):
                 ops.moe_combine(out, y, place, accumulate)
-            return
-        ops.moe_combine(out, y, place, accumulate)
+            rows_of = torch.where(place.long()[:, :, None] >= 0, y[place.long().clamp(min=0)], 0.0).sum(1)
+            out = base + rows_of if accumulate else rows_of
+        else:
+            ops.moe_combine(out, y, place, accumulate)
         if sff:
             s = torch.empty(T, sff, dtype=torch.bfloat16, device=DEV)
             ops_tc.gemm_grouped(s, h, w_gu, sff, first=E * ff, row_w=dense[:, E], unit=unit, limit=1.5)
@@ -121,3 +123,42 @@ def test_sorted_experts(E, top, ff, sff, D, N, kind, unit, T):
         got = out.double() - (base.double() if accumulate else 0.0)
         assert ((got - want).abs() <= 2.0 ** -8 * scale + 1e-4).all()
     assert ops_tc.device_error() == 0
+
+
+@pytest.mark.parametrize("design", ["fovirax", "mavinex", "bogupel"])
+def test_a_decoder_by_every_form(design, tmp_path, monkeypatch):
+    """Prompts sorted by expert or through all experts, decode steps streamed or through all experts."""
+    import importlib
+    from oracle_engine_b200.engine.batch import SequenceStep
+    from oracle_engine_b200.engine.engine import Engine
+    from oracle_engine_b200.parts import moe
+    models = importlib.import_module(design + "_models")
+    folder = models.write(tmp_path, models.REAL, 11)
+    used, forward_sorted = [], moe.MoESwiGLU._forward_sorted
+    monkeypatch.setattr(moe.MoESwiGLU, "_forward_sorted", lambda *a: (used.append("sorted"), forward_sorted(*a)))
+    from oracle_engine_b200.csrc import ops
+    for name in ("moe_up_stream", "moe_dense_act"):
+        monkeypatch.setattr(ops, name, lambda *a, n=name, f=getattr(ops, name), **k: (used.append(n), f(*a, **k)))
+
+    def logits(sort, stream, dtype="bfloat16"):
+        monkeypatch.setattr(moe, "_sorted_pays", lambda *a: sort)
+        monkeypatch.setattr(moe, "_stream_pays", lambda T, top, experts: stream and T <= moe.STREAM_TOKENS)
+        eng = Engine.from_pretrained(folder, dtype=dtype, max_tokens=2048, use_graphs=False)
+        slots, out = [eng.alloc() for _ in range(3)], []
+        used.clear()
+        out.append(eng.step([SequenceStep(s, [(31 * b + 7 * j) % 90 for j in range(150 + 70 * b)], [0, 149]) for b, s in enumerate(slots)]).clone())
+        forms = [set(used)]
+        used.clear()
+        for i in range(3):
+            out.append(eng.step([SequenceStep(s, [(13 * i + b) % 90], [0]) for b, s in enumerate(slots)]).clone())
+        eng.check_device_errors()
+        return torch.cat(out), forms + [set(used)]
+    plain, forms = logits(False, False)
+    assert forms == [{"moe_dense_act"}, {"moe_dense_act"}]
+    other, forms = logits(True, True)
+    assert forms == [{"sorted"}, {"moe_up_stream"}]
+    # no further from the 32-bit path than the products over all experts are, whose units' inputs are rounded once more; in the
+    # median, as a token near a tie may choose another expert in a later layer
+    exact, _ = logits(False, False, "float32")
+    off = lambda t: ((t - exact).norm(dim=1) / exact.norm(dim=1)).median().item()          # noqa: E731
+    assert torch.isfinite(other).all() and off(other) < 1.3 * off(plain) + 1e-3
