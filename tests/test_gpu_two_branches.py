@@ -43,6 +43,29 @@ def test_branches_beside_each_other(design, dtype, batch, tmp_path, monkeypatch)
     assert torch.isfinite(beside).all() and torch.equal(beside, after)
 
 
+@pytest.mark.parametrize("design", DESIGNS)
+@pytest.mark.parametrize("batch", [1, 8, 16])
+def test_branches_of_a_wide_model(design, batch, monkeypatch):
+    """Width 2,048, four layers, 300 tokens a sequence: products of hundreds of CTAs and attention by split keys beside a scan."""
+    import bench
+    from oracle_engine_b200.config.base import get_architecture
+    from oracle_engine_b200.engine.batch import SequenceStep
+    from oracle_engine_b200.engine.engine import Engine
+    from oracle_engine_b200.parts import parallel
+    raw = getattr(bench, design + "_shape")(2048, 4, 4096)
+    config = get_architecture(raw["architecture"]).config_cls.from_dict(raw)
+
+    def logits():
+        eng = Engine.from_config(config, seed=3, dtype="bfloat16", max_tokens=16 * 384)
+        slots = [eng.alloc() for _ in range(batch)]
+        eng.step([SequenceStep(s, [(31 * b + 7 * j) % 4096 for j in range(300 - b)], []) for b, s in enumerate(slots)])
+        return torch.stack([eng.step([SequenceStep(s, [(13 * i + b) % 4096], [0]) for b, s in enumerate(slots)]).clone() for i in range(5)])
+    beside = logits()
+    monkeypatch.setattr(parallel, "FORK_TOKENS", 0)
+    after = logits()
+    assert torch.isfinite(beside).all() and torch.equal(beside, after)
+
+
 def test_only_in_a_capture():
     from oracle_engine_b200.engine.runtime import Runtime
     with pytest.raises(RuntimeError, match="captured"):
