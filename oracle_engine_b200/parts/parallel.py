@@ -105,7 +105,7 @@ class ParallelMixers(Part):
         return None
 
     def step_choice(self, step):
-        return tuple(m.step_choice(step) for _, m, _ in self.branches)
+        return tuple(getattr(m, "step_choice", lambda step: None)(step) for _, m, _ in self.branches)
 
     def state_need(self):
         return {f"{tag}.{name}": need for tag, m, _ in self.branches for name, need in m.state_need().items()}

@@ -34,6 +34,9 @@ Mixer  (MIXERS; e.g. attention)
     feed-forward also with `joint_epilogue(h, ctx)`, can have their first products computed as one by an arrangement
     that gives both the same input (parts/block.py: JoinedInput; parts/parallel.py for mixers side by side)
 
+    optional: a mixer or feed-forward whose forward chooses by the real lengths of a step's sequences says so in
+    step_choice(step) (Part.step_choice); one that is a mixture of experts has `mixture = True`
+
     optional: a mixer made of mixers with output norms may hand those outputs over unnormed, with the norms' weights
     (`normed_outputs`, `eps`); an arrangement that norms the sum then does all of it in one kernel
 

@@ -68,3 +68,26 @@ def test_steps_of_one_padded_shape_and_other_scans_have_other_keys():
     choice = {n: model.step_choice(_plan(lens, pad_seqs=4, pad_tokens=256)) for n, lens in steps.items()}
     assert choice["short"] == choice["few"] != choice["long"] == choice["one"]
     assert choice["long"] == ((None, True), True, (None, True)) and choice["short"] == ((None, False), False, (None, False))
+
+
+def test_a_branch_that_says_nothing_of_its_choice_chooses_nothing():
+    """A mixer needs what the interface names; it need not derive from Part."""
+    from types import SimpleNamespace
+
+    from oracle_engine_b200.engine.runtime import Runtime
+    from oracle_engine_b200.parts import parallel
+    from oracle_engine_b200.parts.registry import MIXERS
+
+    @MIXERS.register("says_nothing")
+    class SaysNothing:
+        def __init__(self, params, prefix, runtime):
+            pass
+
+        def cache_need(self):
+            return None
+    branches = [{"tag": t, "kind": "says_nothing", "prefix": t, "params": {}, "coef": 1.0} for t in "ab"]
+    try:
+        both = parallel.ParallelMixers({"hidden_size": 8, "branches": branches}, "", Runtime(torch.bfloat16, torch.device("cpu")))
+        assert both.step_choice(SimpleNamespace(n_tokens=3, longest=3, scan_chunks=1, n_real_tokens=3)) == (None, None)
+    finally:
+        MIXERS.unregister("says_nothing")
