@@ -358,7 +358,8 @@ attn_split_merge_kernel(bf16* out, const float* partial, int n_splits, const int
     const float* p = partial + (size_t)blockIdx.x * n_splits * (DV + 2);
     // Every split's weight at once, a lane a split, and then sums whose loads do not wait for one another: split after split
     // the two passes were chains of 17 loads each (4 of the 11 us of a decode step's attention at 1,024 keys).  A split
-    // without a key has weight zero and its sums, which nothing has written, are not used.
+    // without a key has the weight -1 and its sums, which nothing has written, are not used; one whose weight is merely too
+    // small for float32 is, as an infinite value of its keys times zero is no number.
     __shared__ float f[MAX_SPLITS], f_inv;
     // a sink counts as one more split: maximum sinks[h] (in units of log2(e)), denominator 1, no values
     const float sk = sinks ? sinks[blockIdx.x % H] * 1.4426950408889634f : -INFINITY;
@@ -369,7 +370,7 @@ attn_split_merge_kernel(bf16* out, const float* partial, int n_splits, const int
         float l = 0.f;
         for (int s = threadIdx.x; s < n_splits; s += 32) {
             const float ms = p[(size_t)s * (DV + 2) + DV], ls = p[(size_t)s * (DV + 2) + DV + 1];
-            const float w = ms != -INFINITY ? exp2f(ms - m) : 0.f;
+            const float w = ms != -INFINITY ? exp2f(ms - m) : -1.f;
             f[s] = w;
             if (ms != -INFINITY) l = fmaf(w, ls, l);
         }
@@ -382,7 +383,7 @@ attn_split_merge_kernel(bf16* out, const float* partial, int n_splits, const int
 #pragma unroll 8
         for (int s = 0; s < n_splits; s++) {
             const float w = f[s], v = p[(size_t)s * (DV + 2) + d];
-            acc = fmaf(w, w != 0.f ? v : 0.f, acc);
+            acc = w == -1.f ? acc : fmaf(w, v, acc);
         }
         return acc;
     };
