@@ -138,7 +138,10 @@ constexpr int PENALTY_CAP = 256;                    // the longest history whose
 
 // The repeat penalty over the last `repeat_last` recorded tokens, for those in [lo, hi), by the whole block: the first of
 // equal tokens is penalised once for each of them.  (One thread going through the history took 1.2 us a token.)
-__device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, int repeat_last, const SampleState& st, int* s_ids) {
+// hit: null, or per thread of the block a mask, zeroed by it before, in which the changed places are marked: place
+// lo + stride j + t is bit j of hit[t].
+__device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, int repeat_last, const SampleState& st, int* s_ids,
+                         unsigned* hit = nullptr, int stride = 1) {
     const int count = st.hist_count[slot];
     int n = count < repeat_last ? count : repeat_last;
     if (n > st.hist_cap) n = st.hist_cap;
@@ -156,6 +159,7 @@ __device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, i
         float v = x[id];
         for (int i = 0; i < times; i++) v = v > 0.f ? v / repeat_pen : v * repeat_pen;
         x[id] = v;
+        if (hit != nullptr) atomicOr(&hit[(id - lo) % stride], 1u << ((id - lo) / stride));
     }
     __syncthreads();
 }
@@ -292,13 +296,21 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
 
 // ------------------------------------------------------------------------------------------------------------------
 // The same chain for wide rows (a temperature above zero): a cluster of eight CTAs per row, the row's values in registers
-// (up to 32 a thread) from the first pass to the draw.  With one block per row the row came from the L2 again for each of
-// the 62 passes of the two threshold searches: 1.35 ms for 128,256 tokens whatever the number of rows.  Here a pass is a
-// few compares in registers, one exchange of every warp's sums through the cluster's shared memory and one cluster
-// barrier; it settles two bits of a threshold (three candidates), and a search ends as soon as the tokens it keeps are
-// known: top-k when a candidate keeps exactly k, top-p when one token is left between the bounds.
+// (up to 32 a thread) from the first pass to the draw.  What bounds it is the number of exchanges between the CTAs (a cluster
+// barrier and what stands on both sides of it, 1.2 us each), not the row's bytes.
+//   * The usual case, a top-k of at most as many tokens as the cluster has warps (128): the k-th largest of the warps' maxima
+//     is a lower bound of the k-th largest value, and few values are at or above it (about 50 for k = 40 where the order of the
+//     tokens is unrelated to their values).  Those go to the first CTA with the exchange of the softmax's sums, which ends the
+//     row alone by comparing them all with one another: two exchanges in all.  8 rows of 128,256: 33.3 -> 15.6 us a launch.
+//   * Otherwise, or where more values are at or above the bound than there is room for, passes over the registers: one
+//     settles two bits of a threshold (three candidates), and a search ends as soon as the tokens it keeps are known: top-k
+//     when a candidate keeps exactly k, top-p when one token is left between the bounds.
+// With one block per row the row came from the L2 again for each of the 62 passes of the two searches: 1.35 ms for 128,256
+// tokens whatever the number of rows.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int CL = 8, CT = 512, CW = CT / 32;        // CTAs of a cluster, threads and warps of a CTA
+constexpr int SEG = 16, FEW = 1024;                  // values at or above the bound: room for a warp's and for all of them
+constexpr int KEPT = 1 << 30;                        // marks a kept token's index
 
 struct __align__(16) Sums { float a[4]; unsigned n[4]; };
 
@@ -362,14 +374,32 @@ __device__ __forceinline__ Sums cluster_sums(Sums v, Sums (*box)[CL * CW], int& 
     return t;
 }
 
+__device__ __forceinline__ void record_token(int token, int row, int slot, int* out, const SampleState& st, int record) {
+    out[row] = token;
+    if (record) {
+        st.rng_counter[slot] += 1;
+        if (st.hist != nullptr) {
+            const int c = st.hist_count[slot];
+            st.hist[(size_t)slot * st.hist_cap + (c % st.hist_cap)] = token;
+            st.hist_count[slot] = c + 1;
+        }
+    }
+}
+
 template <int EPT>
 __global__ void __launch_bounds__(CT)
 sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float temperature, int top_k, float top_p, float repeat_pen,
                       int repeat_last, SampleState st, int record) {
     __shared__ Sums box[2][CL * CW];
+    __shared__ float2 s_seg[CL * CW][SEG];            // of the first CTA: per warp of the cluster its (value, index) at or above the bound
+    __shared__ float2 s_few[FEW];                     // the same side by side
+    __shared__ int2 s_place[CL * CW];                 // of a warp's values in s_few: the first, how many
+    __shared__ unsigned s_hit[CT];
     __shared__ int s_ids[PENALTY_CAP];
     __shared__ float s_part[EPT * CW], s_excl[EPT * CW], s_total[CL];
     __shared__ int s_entry, s_last[CL], s_warp_last[CW];
+    __shared__ float s_bound;
+    __shared__ unsigned s_cut;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = (int)cluster_rank(), row = blockIdx.y;
     pdl_launch_dependents();
@@ -380,29 +410,147 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     const int slice = EPT * CT, base = rank * slice;  // this CTA's values are base + 512 j + tid
     int turn = 0;
 
-    cluster_barrier();                                // every CTA of the cluster is there before its memory is written
-
-    // repeat penalty, of the tokens in this CTA's slice
-    if (repeat_pen > 1.f && st.hist != nullptr) penalise(x, base, min(base + slice, V), slot, repeat_pen, repeat_last, st, s_ids);
-
-    // temperature, softmax
-    const float inv_t = temperature == 1.f ? 1.f : 1.f / temperature;
     float v[EPT];
-    Sums sums = {};
-    float mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < EPT; j++) {
         const int i = base + j * CT + tid;
         v[j] = i < V ? x[i] : -INFINITY;
     }
+    // repeat penalty, of the tokens in this CTA's slice, while the values are on their way; what it changes is read again
+    if (repeat_pen > 1.f && st.hist != nullptr) {
+        s_hit[tid] = 0u;
+        __syncthreads();
+        penalise(x, base, min(base + slice, V), slot, repeat_pen, repeat_last, st, s_ids, s_hit, CT);
+        const unsigned again = s_hit[tid];
+        if (again != 0u) {
+#pragma unroll
+            for (int j = 0; j < EPT; j++) if (again >> j & 1u) v[j] = x[base + j * CT + tid];
+        }
+    }
+
+    // temperature, softmax
+    const float inv_t = temperature == 1.f ? 1.f : 1.f / temperature;
+    Sums sums = {};
+    float mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < EPT; j++) { v[j] *= inv_t; mx = fmaxf(mx, v[j]); }
+    cluster_barrier();                                // every CTA of the cluster is there before its memory is written
     sums.a[0] = mx;
     mx = cluster_sums<true>(sums, box, turn).a[0];
+    // the bound: the top_k-th largest of the warps' maxima.  At least top_k values are at or above it.
+    const bool by_bound = top_k > 0 && top_k < V && top_k <= CL * CW;
+    float least = INFINITY;                           // exponentials from here on are marked: a little below the bound's, so
+    if (by_bound) {                                   // that whatever rounds to the bound's probability is among them
+        const Sums* maxima = box[turn ^ 1];
+        if (tid < CL * CW) {
+            const float own = maxima[tid].a[0];
+            int above = 0, from_it_on = 0;
+#pragma unroll 16
+            for (int i = 0; i < CL * CW; i++) { const float m = maxima[i].a[0]; above += m > own ? 1 : 0; from_it_on += m >= own ? 1 : 0; }
+            if (above < top_k && top_k <= from_it_on) s_bound = own;
+        }
+        __syncthreads();
+        least = fmaxf(expf(s_bound - mx) * 0.9999f, 1e-45f);
+    }
     sums = {};
+    unsigned marked = 0u;
 #pragma unroll
-    for (int j = 0; j < EPT; j++) { v[j] = base + j * CT + tid < V ? expf(v[j] - mx) : 0.f; sums.a[0] += v[j]; }
-    const float inv = 1.f / cluster_sums<false>(sums, box, turn).a[0];
+    for (int j = 0; j < EPT; j++) {
+        v[j] = base + j * CT + tid < V ? expf(v[j] - mx) : 0.f;
+        marked |= v[j] >= least ? 1u << j : 0u;
+        sums.a[0] += v[j];
+    }
+    if (by_bound) {
+        const int mine = __popc(marked), all = __reduce_add_sync(0xffffffffu, mine);
+        if (all > 0 && all <= SEG) {
+            int at = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, at, o); if (lane >= o) at += u; }
+            at -= mine;
+            const unsigned here = (unsigned)__cvta_generic_to_shared(&s_seg[rank * CW + warp][0]);
+            unsigned there;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(0));
+#pragma unroll
+            for (int j = 0; j < EPT; j++) {
+                if (marked >> j & 1u) {
+                    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(there + 8u * at), "f"(v[j]),
+                                 "f"(__int_as_float(base + j * CT + tid)) : "memory");
+                    at++;
+                }
+            }
+        }
+        if (lane == 0) { sums.n[0] = all; sums.n[1] = all > SEG ? 1u : 0u; }
+    }
+    const Sums softmax = cluster_sums<false>(sums, box, turn);
+    const float inv = 1.f / softmax.a[0];
+
+    // (a sum that is no number takes the passes, which choose no token)
+    if (by_bound && softmax.n[1] == 0u && softmax.n[0] <= FEW && softmax.a[0] >= 1.f) {
+        if (rank != 0) return;                        // nothing is written to another CTA any more
+        const int n = (int)softmax.n[0];
+        // side by side, in the warps' order
+        if (warp == 0) {
+            const Sums* of = box[turn ^ 1];
+            int count[CL * CW / 32], before = 0;
+#pragma unroll
+            for (int i = 0; i < CL * CW / 32; i++) { count[i] = (int)of[lane * (CL * CW / 32) + i].n[0]; before += count[i]; }
+            int scan = before;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, scan, o); if (lane >= o) scan += u; }
+            before = scan - before;
+#pragma unroll
+            for (int i = 0; i < CL * CW / 32; i++) { s_place[lane * (CL * CW / 32) + i] = make_int2(before, count[i]); before += count[i]; }
+        }
+        if (tid == 0) { s_cut = 0u; s_entry = 0x7fffffff; }
+        __syncthreads();
+        {
+            static_assert(CT == 4 * CL * CW, "four threads a warp's values");
+            const int2 place = s_place[tid >> 2];
+            for (int i = tid & 3; i < place.y; i += 4) { const float2 c = s_seg[tid >> 2][i]; s_few[place.x + i] = make_float2(c.x * inv, c.y); }
+        }
+        __syncthreads();
+        // kept by top-k: fewer than top_k are above it; the cut of top-p: the largest value with which the mass reaches top_p
+        for (int i = tid; i < n; i += CT) {
+            const float p = s_few[i].x;
+            int above = 0;
+            float mass = 0.f;
+            for (int j = 0; j < n; j++) { const float q = s_few[j].x; above += q > p ? 1 : 0; mass += q >= p ? q : 0.f; }
+            if (above < top_k) {
+                if (top_p < 1.f && mass >= top_p) atomicMax(&s_cut, __float_as_uint(p));
+                s_few[i].y = __int_as_float(__float_as_int(s_few[i].y) | KEPT);
+            }
+        }
+        __syncthreads();
+        const unsigned cut = s_cut;
+        const float u = uniform_from_counter((unsigned long long)st.rng_seed[slot], (unsigned long long)st.rng_counter[slot]);
+        // the draw: the first kept token, by index, whose running mass exceeds u x the kept mass
+        int last_kept = -1;
+        for (int i = tid; i < n; i += CT) {
+            const float2 c = s_few[i];
+            const int id = __float_as_int(c.y);
+            if (!(id & KEPT) || __float_as_uint(c.x) < cut) continue;
+            float run = 0.f, total = 0.f;
+            for (int j = 0; j < n; j++) {
+                const float2 o = s_few[j];
+                const int other = __float_as_int(o.y);
+                const float q = (other & KEPT) && __float_as_uint(o.x) >= cut ? o.x : 0.f;
+                total += q;
+                run += other <= id ? q : 0.f;
+            }
+            if (run > u * total) atomicMin(&s_entry, id & ~KEPT);
+            last_kept = max(last_kept, id & ~KEPT);
+        }
+        __syncthreads();
+        if (s_entry == 0x7fffffff) {                  // rounding left u x the mass at or beyond the last one: the last kept token
+            if (tid == 0) s_last[0] = -1;
+            __syncthreads();
+            if (last_kept >= 0) atomicMax(&s_last[0], last_kept);
+            __syncthreads();
+            if (tid == 0) s_entry = s_last[0];
+        }
+        if (tid == 0) record_token(s_entry, row, slot, out, st, record);
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < EPT; j++) v[j] *= inv;
 
@@ -528,18 +676,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
         box[turn][0].a[0] = __int_as_float(l);
     }
     cluster_barrier();
-    if (rank == 0 && tid == 0) {
-        const int token = __float_as_int(box[turn][0].a[0]);
-        out[row] = token;
-        if (record) {
-            st.rng_counter[slot] += 1;
-            if (st.hist != nullptr) {
-                const int c = st.hist_count[slot];
-                st.hist[(size_t)slot * st.hist_cap + (c % st.hist_cap)] = token;
-                st.hist_count[slot] = c + 1;
-            }
-        }
-    }
+    if (rank == 0 && tid == 0) record_token(__float_as_int(box[turn][0].a[0]), row, slot, out, st, record);
 }
 
 template <int EPT>
