@@ -12,8 +12,9 @@
 // Role of the reference's `ops::matmul` / `gemm_q` (core/ops.cpp:207-289,
 // core/gguf_parser.cpp:919-997): out[m,n] = A[m,k] . B[n,k]^T.
 //
-// Three kernels: `gemm_stream_kernel` for a few rows (bound by the weights' bytes), `gemm_tile_kernel` for more (bound
-// by the multiply-adds), both float32 with 16-byte aligned rows, and `gemm_nt_kernel` for everything else.
+// Four kernels: `gemm_stream_kernel` for a few rows (bound by the weights' bytes), `gemm_tile_kernel` for some dozens and
+// `gemm_wide_kernel` for more (bound by the multiply-adds), all float32 with 16-byte aligned rows, and `gemm_nt_kernel` for
+// everything else.
 #include "common.cuh"
 
 namespace {
@@ -174,10 +175,10 @@ gemm_stream_kernel(float* C, const float* A, const float* __restrict__ W, int M,
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Many rows.  256 threads of 8 x 8 outputs: a tile of 128 x 128 (KG = 1), or of 64 x 64 whose classes are shared out over
-// KG = 4 groups of 64 threads (small products, for which tiles of 128 would leave SMs idle).  Stages of 16 values of k come
-// by cp.async as they lie in memory; a thread reads four k at a time of its rows (rows 20 words apart: no bank conflicts
-// between the eight lanes that differ), 16 16-byte loads for 256 multiply-adds.
+// Some dozens of rows of a wide weight.  256 threads of 8 x 8 outputs: a tile of 64 x 64 whose classes are shared out over
+// KG = 4 groups of 64 threads.  Stages of 16 values of k come by cp.async as they lie in memory; a thread reads four k at a
+// time of its rows (rows 20 words apart: no bank conflicts between the eight lanes that differ), 16 16-byte loads for 256
+// multiply-adds.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int TK = 16, TROW = TK + 4;
 
@@ -185,7 +186,7 @@ template <int BM, int BN, int KG>
 struct TileShape {
     static constexpr int STAGE = (BM + BN) * TROW, STAGES = 3;
     static constexpr size_t RING = (size_t)KG * STAGES * STAGE * 4;
-    static constexpr size_t BYTES = RING + (KG > 1 ? (size_t)KG * BM * BN * 4 : 0);   // the first of a group's two classes
+    static constexpr size_t BYTES = RING + (size_t)KG * BM * BN * 4;                  // the first of a group's two classes
 };
 
 template <int BM, int BN, int KG, int MODE>
@@ -203,7 +204,7 @@ gemm_tile_kernel(float* C, const float* A, const float* __restrict__ W, int M, i
     const int classes = class_count(K), rounds = class_rounds(K);
     constexpr int CPG = CLASSES / KG;                // classes of a group
     const int seg = segment(K), steps = seg / TK, per_class = rounds * steps;
-    const int total = (KG == 1 ? classes : CPG) * per_class;
+    const int total = CPG * per_class;
 
     const int lq = t & 3, lr = t >> 2;
     auto load = [&](int i) {
@@ -225,11 +226,11 @@ gemm_tile_kernel(float* C, const float* A, const float* __restrict__ W, int M, i
     pdl_wait();
 #pragma unroll
     for (int i = 0; i < S::STAGES - 1; i++) { if (i < total) load(i); cp_commit(); }
-    float acc[8][8], tot[KG == 1 ? 8 : 1][8];
+    float acc[8][8];
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) { acc[i][j] = 0.f; if (KG == 1) tot[KG == 1 ? i : 0][j] = 0.f; }
+        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
     float* kept = smem + KG * S::STAGES * S::STAGE + g * BM * BN;
     const int row = 32 * wm + ty, col = 64 * wn + tx;
 
@@ -265,12 +266,7 @@ gemm_tile_kernel(float* C, const float* A, const float* __restrict__ W, int M, i
         }
         if (++it < per_class) continue;
         it = 0;                                       // a class is complete
-        if (KG == 1) {
-#pragma unroll
-            for (int ii = 0; ii < 8; ii++)
-#pragma unroll
-                for (int j = 0; j < 8; j++) { tot[KG == 1 ? ii : 0][j] = c == 0 ? acc[ii][j] : tot[KG == 1 ? ii : 0][j] + acc[ii][j]; acc[ii][j] = 0.f; }
-        } else if (c == 0) {
+        if (c == 0) {
 #pragma unroll
             for (int ii = 0; ii < 8; ii++)
 #pragma unroll
@@ -278,39 +274,233 @@ gemm_tile_kernel(float* C, const float* A, const float* __restrict__ W, int M, i
         }
         c++;
     }
-    if constexpr (KG > 1) {
-        // the second classes go where the stages were; then every thread adds up a share of the outputs
-        cp_wait<0>();
-        __syncthreads();
-        float* second = smem + g * BM * BN;
-        static_assert(KG == 1 || (size_t)KG * BM * BN * 4 <= S::RING, "the ring holds the second classes");
+    // the second classes go where the stages were; then every thread adds up a share of the outputs
+    cp_wait<0>();
+    __syncthreads();
+    float* second = smem + g * BM * BN;
+    static_assert((size_t)KG * BM * BN * 4 <= S::RING, "the ring holds the second classes");
 #pragma unroll
-        for (int ii = 0; ii < 8; ii++)
+    for (int ii = 0; ii < 8; ii++)
 #pragma unroll
-            for (int j = 0; j < 8; j++) second[(row + 4 * ii) * BN + col + 8 * j] = acc[ii][j];
-        __syncthreads();
-        const float* first = smem + KG * S::STAGES * S::STAGE;
-        for (int e = threadIdx.x; e < BM * BN; e += 256) {
-            const int m = m0 + e / BN, n = n0 + e % BN;
-            if (m >= M || n >= N) continue;
-            float v = first[e];
-            for (int q = 1; q < classes; q++) v += ((q & 1) ? smem : first)[(q >> 1) * BM * BN + e];
-            float* o = C + (size_t)m * ldc + n;
-            *o = MODE == 1 ? *o + v : v;
+        for (int j = 0; j < 8; j++) second[(row + 4 * ii) * BN + col + 8 * j] = acc[ii][j];
+    __syncthreads();
+    const float* first = smem + KG * S::STAGES * S::STAGE;
+    for (int e = threadIdx.x; e < BM * BN; e += 256) {
+        const int m = m0 + e / BN, n = n0 + e % BN;
+        if (m >= M || n >= N) continue;
+        float v = first[e];
+        for (int q = 1; q < classes; q++) v += ((q & 1) ? smem : first)[(q >> 1) * BM * BN + e];
+        float* o = C + (size_t)m * ldc + n;
+        *o = MODE == 1 ? *o + v : v;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// Many rows, tiles of 128 x 128.  Four warps multiply, 16 x 8 outputs a thread; four others load (setmaxnreg gives the first
+// the others' registers); two CTAs an SM.  A thread of 8 x 8 outputs reads 16 values from shared memory for 64 products, at
+// which the two take the same time; 16 x 8 read 24 for 128.  Stages of 16 k lie transposed, k by k, so that a thread's values
+// of one k are 16-byte pieces; the loading warps turn 4 x 4 values in registers.  Loaded by the multiplying warps themselves the
+// same kernel was a quarter slower, with cp.async of 4 bytes as with 16-byte loads.  The products are done two rows at a time
+// (fma.rn.f32x2: each half is rounded as by itself), which leaves issue slots to the loads from shared memory.
+// KG = 1: a single chain (K up to 512).  KG = 4, 8: the classes of a tile are shared out over the CTAs of a cluster, class
+// p KG + rank in phase p; behind each phase every CTA adds up its share of the rows, class by class, from the shared memory
+// of all.  468 rows, tiles of 8 x 8 outputs before -> now: 2,048 -> 16,384 997 -> 734 us (43 TFLOP/s; the multiply-adds of
+// tiles that are full to the last row would take 470), 2,048 -> 3,072 228 -> 162, 2,048 -> 2,048 156 -> 118, 8,192 -> 2,048
+// 578 -> 406.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int WT = 128, WLD = WT;
+
+struct WideShape {
+    static constexpr int STAGE = 2 * TK * WLD;
+    static constexpr size_t BYTES = ((size_t)2 * STAGE + 2 * WT * TK + WT * WT) * 4;      // 112 KB: two CTAs an SM, no more
+};
+
+__device__ __forceinline__ unsigned long long two(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 halves(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 load_shared_of(const float* local, unsigned rank) {
+    const unsigned here = (unsigned)__cvta_generic_to_shared(local);
+    unsigned there;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(there) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// Four neighbouring outputs of a row.
+template <int MODE>
+__device__ __forceinline__ void store4(float* C, float4 v, int m, int n, int M, int N, long long ldc, bool vec) {
+    if (m >= M) return;
+    float* o = C + (size_t)m * ldc + n;
+    if (vec && n + 4 <= N) {
+        if (MODE == 1) v = add4(*(const float4*)o, v);
+        *(float4*)o = v;
+        return;
+    }
+    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) if (n + i < N) o[i] = MODE == 1 ? o[i] + e[i] : e[i];
+}
+
+__device__ __forceinline__ void named_sync(int id) { asm volatile("barrier.cta.sync %0, 256;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id) { asm volatile("barrier.cta.arrive %0, 256;" ::"r"(id) : "memory"); }
+constexpr int FULL = 1, FREE = 3;                    // the barriers of stage s: FULL + s, FREE + s
+
+template <int KG, int MODE>
+__global__ void __launch_bounds__(256, 2)
+gemm_wide_kernel(float* C, const float* A, const float* __restrict__ W, int M, int N, int K, long long lda, long long ldc, int tiles_m) {
+    extern __shared__ __align__(16) float smem[];
+    float4* landing = (float4*)(smem + 2 * WideShape::STAGE);        // what the loading threads have asked for, [piece][thread]
+    float* sums = smem + 2 * WideShape::STAGE + 2 * WT * TK;         // a class's sums, [row][column]
+    const int tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
+    const int rank = KG == 1 ? 0 : (int)(blockIdx.x % KG), tile = blockIdx.x / KG;
+    const int m0 = tile % tiles_m * WT, n0 = tile / tiles_m * WT;
+    const int seg = segment(K), steps = seg / TK, per_class = class_rounds(K) * steps;
+    const int phases = KG == 1 ? 1 : CLASSES / KG, total = phases * per_class;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (KG > 1) cluster_barrier();                   // every CTA of the cluster is there before its memory is read
+
+    if (threadIdx.x >= 128) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        // k 4 lk .. 4 lk + 3 of rows 4 lr .. 4 lr + 3
+        const int lr = lane & 7 | warp << 3, lk = lane >> 3;
+        const float* a_at = A + (size_t)(m0 + 4 * lr) * lda;
+        const float* w_at = W + (size_t)(n0 + 4 * lr) * K;
+        const int a_rows = M - m0 - 4 * lr, w_rows = N - n0 - 4 * lr;
+        auto ask = [&](int i) {
+            const int c = i / per_class * KG + rank, it = i % per_class;
+            const int k = (it / steps * CLASSES + c) * seg + it % steps * TK + 4 * lk;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const bool on = k < K && r < a_rows;
+                cp_async16((float*)(landing + r * 128 + tid), on ? a_at + r * lda + k : A, on);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const bool on = k < K && r < w_rows;
+                cp_async16((float*)(landing + (4 + r) * 128 + tid), on ? w_at + (size_t)r * K + k : W, on);
+            }
+        };
+        auto turn = [&](const float4* from, float* st) {
+            const float4 p0 = from[0], p1 = from[128], p2 = from[256], p3 = from[384];
+            float* to = st + 4 * lk * WLD + 4 * lr;
+            *(float4*)to = make_float4(p0.x, p1.x, p2.x, p3.x);
+            *(float4*)(to + WLD) = make_float4(p0.y, p1.y, p2.y, p3.y);
+            *(float4*)(to + 2 * WLD) = make_float4(p0.z, p1.z, p2.z, p3.z);
+            *(float4*)(to + 3 * WLD) = make_float4(p0.w, p1.w, p2.w, p3.w);
+        };
+        ask(0);
+        for (int i = 0; i < total; i++) {
+            // two stages may lie ahead of the multiplying warps, which meet the other CTAs behind the first class
+            if (KG > 1 && i == per_class + 2) cluster_barrier();
+            cp_commit();
+            cp_wait<0>();
+            if (i >= 2) named_sync(FREE + (i & 1));
+            float* st = smem + (i & 1) * WideShape::STAGE;
+            turn(landing + tid, st);
+            turn(landing + 512 + tid, st + TK * WLD);
+            named_arrive(FULL + (i & 1));
+            if (i + 1 < total) ask(i + 1);            // (a thread reads only what it has asked for)
         }
-    } else
-#pragma unroll
-    for (int ii = 0; ii < 8; ii++) {
-        const int m = m0 + row + 4 * ii;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int n = n0 + col + 8 * j;
-            if (n >= N) continue;
-            float* o = C + (size_t)m * ldc + n;
-            const float v = tot[KG == 1 ? ii : 0][j];
-            *o = MODE == 1 ? *o + v : v;
+        if (KG > 1) {                                 // the barriers of the multiplying warps that are left
+            for (int b = phases > 1 ? 1 : 0; b < 2 * phases; b++) cluster_barrier();
         }
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    // outputs (row + 16 i + r, col + 32 j + c), i, r, c < 4, j < 2
+    const int row = (warp >> 1) * 64 + (lane >> 3) * 4, col = (warp & 1) * 64 + (lane & 7) * 4;
+    unsigned long long acc[8][8];                    // rows 2 p, 2 p + 1 of the thread's sixteen; columns
+#pragma unroll
+    for (int p = 0; p < 8; p++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[p][j] = 0ull;
+    constexpr int SHARE = KG == 1 ? 1 : WT * WT / KG / 128 / 4;      // 16-byte pieces of the tile that a thread adds up
+    float4 share[SHARE];
+
+    const bool vec = (ldc & 3) == 0 && ((size_t)C & 15) == 0;
+
+    int it = 0, phase = 0;
+    for (int i = 0; i < total; i++) {
+        named_sync(FULL + (i & 1));
+        const float* as = smem + (i & 1) * WideShape::STAGE + row;
+        const float* ws = smem + (i & 1) * WideShape::STAGE + TK * WLD + col;
+#pragma unroll
+        for (int kk = 0; kk < TK; kk++) {
+            unsigned long long a[8], b[8];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const ulonglong2 v = *(const ulonglong2*)(as + kk * WLD + 16 * q);
+                a[2 * q] = v.x; a[2 * q + 1] = v.y;
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float4 v = *(const float4*)(ws + kk * WLD + 32 * q);
+                b[4 * q] = two(v.x, v.x); b[4 * q + 1] = two(v.y, v.y); b[4 * q + 2] = two(v.z, v.z); b[4 * q + 3] = two(v.w, v.w);
+            }
+#pragma unroll
+            for (int p = 0; p < 8; p++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) fma2(acc[p][j], a[p], b[j]);
+        }
+        if (i + 2 < total) named_arrive(FREE + (i & 1));
+        if (++it < per_class) continue;
+        it = 0;                                       // a class is complete
+        const bool first = phase++ == 0;
+        if (KG > 1 && !first) cluster_barrier();      // the class before has been read
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                float2 h[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) { h[c] = halves(acc[p][4 * j + c]); acc[p][4 * j + c] = 0ull; }
+                const float4 even = make_float4(h[0].x, h[1].x, h[2].x, h[3].x), odd = make_float4(h[0].y, h[1].y, h[2].y, h[3].y);
+                const int r = row + 16 * (p >> 1) + 2 * (p & 1), c = col + 32 * j;
+                if (KG == 1) {
+                    store4<MODE>(C, even, m0 + r, n0 + c, M, N, ldc, vec);
+                    store4<MODE>(C, odd, m0 + r + 1, n0 + c, M, N, ldc, vec);
+                } else {
+                    float4* to = (float4*)(sums + r * WT + c);
+                    to[0] = even; to[WT / 4] = odd;
+                }
+            }
+        }
+        if (KG > 1) {
+            cluster_barrier();
+#pragma unroll
+            for (int e = 0; e < SHARE; e++) {
+                const int place = rank * (WT * WT / KG) + (e * 128 + tid) * 4;
+                float4 v = load_shared_of(sums + place, 0);
+                if (!first) v = add4(share[e], v);
+#pragma unroll
+                for (int g = 1; g < KG; g++) v = add4(v, load_shared_of(sums + place, g));
+                share[e] = v;
+            }
+        }
+    }
+    if (KG > 1) {
+#pragma unroll
+        for (int e = 0; e < SHARE; e++) {
+            const int place = rank * (WT * WT / KG) + (e * 128 + tid) * 4;
+            store4<MODE>(C, share[e], m0 + place / WT, n0 + place % WT, M, N, ldc, vec);
+        }
+        cluster_barrier();                            // no CTA leaves while its memory is read
     }
 }
 
@@ -424,9 +614,23 @@ int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, l
     return oe_launch(gemm_tile_kernel<BM_, BN_, KG, MODE>, grid, dim3(256), bytes, st, C, A, W, M, N, K, lda, ldc);
 }
 
+template <int KG, int MODE>
+int launch_wide(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, cudaStream_t st) {
+    if ((KG == 1) != (K <= ONE_CHAIN)) return OE_ERR_UNSUPPORTED;
+    constexpr size_t bytes = WideShape::BYTES;
+    cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<KG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return (int)e;
+    const int tiles_m = (M + WT - 1) / WT;
+    const long long ctas = (long long)tiles_m * ((N + WT - 1) / WT) * KG;
+    if (tiles_m > 65535 || ctas > 0x7fffffffll) return OE_ERR_UNSUPPORTED;
+    if (KG == 1) return oe_launch(gemm_wide_kernel<KG, MODE>, dim3((unsigned)ctas), dim3(256), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m);
+    return oe_launch_cluster(gemm_wide_kernel<KG, MODE>, KG, dim3((unsigned)ctas), dim3(256), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m);
+}
+
 constexpr int STREAM_MAX_M = 32;
 
-// kind: 0 by size, else 1 streaming, 2 tiles of 64, 3 tiles of 128, 4 the general kernel (tests).
+// kind: 0 by size, else 1 streaming, 2 tiles of 64, 3 tiles of 128, 4 the general kernel, 5, 6 tiles of 128 whose classes
+// four, eight CTAs share (tests).
 template <int MODE>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int kind, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
@@ -436,15 +640,22 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, lo
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128);
     if (kind == 0) {
-        const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128);
-        const long long t64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
-        // Eight chains are what tiles of 64 share out over a CTA's groups: up to K = 512 there is one, and tiles of 128 it is.
-        // Up to 64 rows a narrow weight has too few tiles of 64 for the SMs (64 x 2,048 x 2,048: 58 us streamed, 78 by tiles; 64 x
-        // 16,384 x 2,048: 249 and 153); below 1.5 tiles of 128 an SM, tiles of 64 leave less of the last round empty
-        kind = M <= STREAM_MAX_M || (M <= 64 && 2 * t64 < sms) ? 1 : K <= ONE_CHAIN || 2 * t128 >= 3 * sms ? 3 : 2;
+        // Up to 64 rows a tile of 128 is half empty.  A weight of few rows is streamed (2,048 x 2,048: 48 rows 51 us, 55 by tiles of
+        // 128; 64 rows 68 and 55); with two CTAs an SM for eight shares of every tile, tiles of 128 (40 x 3,072 x 3,072: 78 us, 92
+        // streamed, 113 by tiles of 64); a weight of more rows has tiles of 64 enough for all SMs (64 x 16,384 x 2,048: 156 us, 197 by
+        // tiles of 128).  From 65 rows on tiles of 128 are faster at every size tried.
+        kind = M <= STREAM_MAX_M || (M <= 48 && t128 <= 16) ? 1 : M > 64 || K <= ONE_CHAIN || 8 * t128 <= 2 * sms ? 3 : 2;
     }
-    if (kind == 3) return launch_tile<128, 128, 1, MODE>(C, A, W, M, N, K, lda, ldc, st);
+    if (kind == 3) {
+        // eight shares of a tile while four would not fill the SMs (192 x 4,096 x 4,096, 64 tiles: 211 us, 240 with four; 300 rows, 96
+        // tiles: 301 and 301; 468 x 16,384 x 2,048: 769 and 734: a share's adding up costs what it costs)
+        if (K <= ONE_CHAIN) return launch_wide<1, MODE>(C, A, W, M, N, K, lda, ldc, st);
+        kind = 4 * t128 <= 2 * sms ? 6 : 5;
+    }
+    if (kind == 5) return launch_wide<4, MODE>(C, A, W, M, N, K, lda, ldc, st);
+    if (kind == 6) return launch_wide<8, MODE>(C, A, W, M, N, K, lda, ldc, st);
     if (kind == 2) return launch_tile<64, 64, 4, MODE>(C, A, W, M, N, K, lda, ldc, st);
     if (M == 1) return launch_stream_rows<1, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
     if (M == 2) return launch_stream_rows<2, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
@@ -461,7 +672,7 @@ int oe_gemm_simple_f32(void* C, const float* A, const float* W, int M, int N, in
     if (out_kind == 2) return launch_f32<1>((float*)C, A, W, M, N, K, lda, ldc, 0, st);
     return launch_f32<0>((float*)C, A, W, M, N, K, lda, ldc, 0, st);
 }
-// The same through one kernel of the three, whatever the size: they give the same bits.
+// The same through one kernel, whatever the size: they give the same bits.
 int oe_gemm_simple_kind_f32(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc,
                             int accumulate, int kind, cudaStream_t st) {
     if (accumulate) return launch_f32<1>(C, A, W, M, N, K, lda, ldc, kind, st);

@@ -319,7 +319,7 @@ def gemm_simple(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate:
 
     a [M, K] and w [N, K] of one dtype (float32 or bfloat16); out [M, N] of that dtype or
     float32; accumulate needs a float32 out.  kind (float32 only): 0 the kernel is chosen by size, 1 weight streaming,
-    2 tiles of 64, 3 tiles of 128, 4 the general one; the same bits."""
+    2 tiles of 64, 3 tiles of 128, 4 the general one, 5 and 6 tiles of 128 (K > 512) that 4 and 8 CTAs share; the same bits."""
     _dev(out, a, w)
     M, K = a.shape
     N = w.shape[0]
