@@ -12,7 +12,7 @@
 // Role of the reference's `ops::matmul` / `gemm_q` (core/ops.cpp:207-289,
 // core/gguf_parser.cpp:919-997): out[m,n] = A[m,k] . B[n,k]^T.
 //
-// Four kernels: `gemm_stream_kernel` for a few rows (bound by the weights' bytes), `gemm_tile_kernel` for some dozens and
+// Four kernels: `gemm_rows_kernel` for a few rows (bound by the weights' bytes), `gemm_tile_kernel` for some dozens and
 // `gemm_wide_kernel` for more (bound by the multiply-adds), all float32 with 16-byte aligned rows, and `gemm_nt_kernel` for
 // everything else.
 #include "common.cuh"
@@ -35,141 +35,123 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ------------------------------------------------------------------------------------------------------------------
-// A few rows.  A warp owns 8 R weight rows and four classes (lane = row mod 8 and class), two warps share a set of rows, a
-// CTA of four warps has 16 R rows, and CTAs walk over the tiles of rows.  Every warp has a ring of its own: a stage is KS
-// values of k of its rows and classes (4 KS consecutive bytes a row and class) and the same k of MT rows of A; the ring
-// runs on from tile to tile, so that loads stay in flight while a tile's classes are added up.  A lane reads its weights
-// and A's values from the stage (rows four words apart from a multiple of 32: no eight lanes meet in a bank).  The next
-// stage is asked for behind the products: before them it cost 5 to 15 %.
+// A few rows: bound by the weights' bytes.  A CTA takes tiles of 16 weight rows in turn, a stage at a time: 512 k of every row,
+// that is 2 KB in one piece from memory, where the eight classes lie side by side.  Two warps multiply, a lane rows rl and
+// rl + 8 of one class (A's values, four fifths of what was read from shared memory when a lane had one row, are read once for
+// two); two warps load the weights and one the rows of A, so that the ring runs on from tile to tile.  Rows four words apart
+// from a multiple of 32: no eight lanes meet in a bank.  In the decode step of the 1B shape (3 rows), against a kernel whose
+// warps loaded 128 bytes of every other segment for themselves: 8,192 -> 2,048 43.5 -> 21.5 us (67 MB), 2,048 -> 2,048
+// 9.5 -> 5.2, 2,048 -> 3,072 12.4 -> 10, 2,048 -> 16,384 34.7 -> 32.8 (134 MB).
 // ------------------------------------------------------------------------------------------------------------------
-template <int R, int MT>
-struct StreamShape {
-    static constexpr int KS = R == 1 && MT <= 4 ? 32 : 16;                                 // k per stage and class
-    static constexpr int CLS = KS;                                           // words between two classes of a row
-    static constexpr int WROW = 4 * CLS + 4;                                     // words of a weight row in a stage
-    static constexpr int STAGE = 8 * R * WROW + MT * 4 * CLS;                    // floats
-    static constexpr int PER_SM = R == 4 ? 1 : 2;                                // CTAs an SM
-    static constexpr int BUDGET = ((PER_SM == 1 ? 208 : 104) * 1024 - 16 * R * CLASSES * MT * 4) / (4 * STAGE * 4);
-    static constexpr int STAGES = BUDGET > 10 ? 10 : BUDGET;
-    static constexpr size_t BYTES = (size_t)(4 * STAGES * STAGE + 16 * R * CLASSES * MT) * 4;
-};
+constexpr int RT = 16, RK = 512, RPITCH = RK + 4;    // weight rows of a tile, k of a stage, words between a stage's rows
 
-template <int R, int MT, int MODE>
-__global__ void __launch_bounds__(128)
-gemm_stream_kernel(float* C, const float* A, const float* __restrict__ W, int M, int N, int K, long long lda, long long ldc,
-                   int tiles_m, int tiles) {
-    using S = StreamShape<R, MT>;
-    constexpr int KS = S::KS, WROW = S::WROW, CLS = S::CLS;
-    const int seg = segment(K), steps = seg / KS;
+template <int MT, int S>
+struct RowsShape {
+    static constexpr int STAGE = (RT + MT) * RPITCH;
+    static constexpr size_t BYTES = ((size_t)S * STAGE + CLASSES * RT * MT) * 4;
+};
+__device__ __forceinline__ void rows_sync(int id) { asm volatile("barrier.cta.sync %0, 160;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void rows_arrive(int id) { asm volatile("barrier.cta.arrive %0, 160;" ::"r"(id) : "memory"); }
+
+template <int MT, int S, int MODE>
+__global__ void __launch_bounds__(160)
+gemm_rows_kernel(float* C, const float* A, const float* __restrict__ W, int M, int N, int K, long long lda, long long ldc,
+                 int tiles_m, int tiles) {
+    constexpr int STAGE = RowsShape<MT, S>::STAGE;
+    constexpr int READY = 1, TAKEN = 1 + S, PAIR = 1 + 2 * S;      // barriers: of stage s READY + s, TAKEN + s; of the multiplying warps
     extern __shared__ __align__(16) float smem[];
+    float* part = smem + S * STAGE;                  // [class][row][MT]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int half = warp & 1, group = warp >> 1;    // classes 4 half .. 4 half + 3; rows 8 R group .. of the tile
-    const int rl = lane & 7, sub = lane >> 3;
-    float* ring = smem + warp * S::STAGES * S::STAGE;
-    float* part = smem + 4 * S::STAGES * S::STAGE;   // [class][row of the tile][MT]
-    const int per_tile = class_rounds(K) * steps;
+    const int per_tile = (K + RK - 1) / RK;
     const int mine = tiles > (int)blockIdx.x ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int total = mine * per_tile;
 
-    // what a lane loads in each stage: 16 bytes (k 4 lq .. 4 lq + 3) of class ls of weight rows lr, lr + LROWS, ...
-    constexpr int LQ = KS / 4, LROWS = 8 / LQ;       // 16-byte pieces a row and class; rows a load instruction covers
-    const int lq = lane % LQ, ls = lane / LQ % 4, lr = lane / LQ / 4;
-    struct Place {                                   // where the next stage comes from and goes
-        int tile, it, stage;
-    };
-    auto next = [&](Place& p) {
-        if (++p.it == per_tile) { p.it = 0; p.tile += gridDim.x; }
-        if (++p.stage == S::STAGES) p.stage = 0;
-    };
-    auto k_of = [&](const Place& p) { return (p.it / steps * CLASSES + 4 * half + ls) * seg + p.it % steps * KS + 4 * lq; };
-    auto load_w = [&](const Place& p) {
-        const int n0 = p.tile / tiles_m * (16 * R) + group * 8 * R, k = k_of(p);
-        float* st = ring + p.stage * S::STAGE + ls * CLS + 4 * lq;
-        const float* src = W + (size_t)n0 * K + k;
+    if (warp >= 2) {
+        const bool weights = warp < 4;               // two warps load the weights, which no kernel writes, one the rows of A
+        if (!weights) pdl_wait();
+        for (int i = 0; i < total + S - 1; i++) {
+            if (i < total) {
+                if (i >= S) rows_sync(TAKEN + i % S);
+                const int tile = blockIdx.x + i / per_tile * (int)gridDim.x, k0 = i % per_tile * RK;
+                const int pieces = min(RK, K - k0) / 4;             // of 16 bytes in a row
+                float* st = smem + i % S * STAGE;
+                if (weights) {
+                    const int n0 = tile / tiles_m * RT, rows = min(RT, N - n0);
+                    const float* from = W + (size_t)n0 * K + k0;
+                    for (int p = (threadIdx.x & 31); p < pieces; p += 32) {
 #pragma unroll
-        for (int r0 = 0; r0 < 8 * R; r0 += LROWS) {
-            const int r = r0 + lr;
-            const bool on = k < K && n0 + r < N;
-            cp_async16(st + r * WROW, on ? src + (size_t)r * K : W, on);
-        }
-    };
-    auto load_a = [&](const Place& p) {
-        const int m0 = p.tile % tiles_m * MT, k = k_of(p);
-        float* st = ring + p.stage * S::STAGE + 8 * R * WROW + ls * CLS + 4 * lq;
+                        for (int r = warp - 2; r < RT; r += 2) if (r < rows) cp_async16(st + r * RPITCH + 4 * p, from + (size_t)r * K + 4 * p, true);
+                    }
+                } else {
+                    const int m0 = tile % tiles_m * MT, rows = min(MT, M - m0);
+                    const float* from = A + (size_t)m0 * lda + k0;
+                    for (int p = lane; p < pieces; p += 32) {
 #pragma unroll
-        for (int r0 = 0; r0 < MT; r0 += LROWS) {
-            const int m = r0 + lr;
-            if (m < MT) {
-                const bool on = k < K && m0 + m < M;
-                cp_async16(st + m * 4 * CLS, on ? A + (size_t)(m0 + m) * lda + k : W, on);
-            }
-        }
-    };
-    // the first weights are asked for while the kernel before this one drains
-    Place pw = {(int)blockIdx.x, 0, 0}, pa = pw;
-#pragma unroll
-    for (int i = 0; i < S::STAGES - 1; i++) if (i < total) { load_w(pw); next(pw); }
-    pdl_wait();
-#pragma unroll
-    for (int i = 0; i < S::STAGES - 1; i++) {
-        if (i < total) { load_a(pa); next(pa); }
-        cp_commit();
-    }
-    float acc[R][MT];
-#pragma unroll
-    for (int j = 0; j < R; j++)
-#pragma unroll
-        for (int m = 0; m < MT; m++) acc[j][m] = 0.f;
-
-    int it = 0, tile = blockIdx.x, stage = 0;
-    for (int i = 0; i < total; i++) {
-        cp_wait<S::STAGES - 2>();
-        __syncwarp();                                 // the stage is there, and the one before it is free
-        const float* st = ring + stage * S::STAGE;
-        if (++stage == S::STAGES) stage = 0;
-        const float* wr = st + rl * WROW + sub * CLS;
-        const float* ar = st + 8 * R * WROW + sub * CLS;
-#pragma unroll
-        for (int kk = 0; kk < KS; kk += 4) {
-            float4 w[R];
-#pragma unroll
-            for (int j = 0; j < R; j++) w[j] = *(const float4*)(wr + j * 8 * WROW + kk);
-#pragma unroll
-            for (int m = 0; m < MT; m++) {
-                const float4 a = *(const float4*)(ar + m * 4 * CLS + kk);
-#pragma unroll
-                for (int j = 0; j < R; j++) {
-                    acc[j][m] = fmaf(a.x, w[j].x, acc[j][m]);
-                    acc[j][m] = fmaf(a.y, w[j].y, acc[j][m]);
-                    acc[j][m] = fmaf(a.z, w[j].z, acc[j][m]);
-                    acc[j][m] = fmaf(a.w, w[j].w, acc[j][m]);
+                        for (int m = 0; m < MT; m++) if (m < rows) cp_async16(st + (RT + m) * RPITCH + 4 * p, from + (size_t)m * lda + 4 * p, true);
+                    }
                 }
             }
+            cp_commit();
+            if (i >= S - 1) {
+                cp_wait<S - 1>();
+                rows_arrive(READY + (i - (S - 1)) % S);
+            }
         }
-        __syncwarp();
-        if (i + S::STAGES - 1 < total) { load_w(pa); load_a(pa); next(pa); }
-        cp_commit();
+        if (weights) pdl_wait();
+        return;
+    }
+    pdl_wait();
+    // a lane: rows rl and rl + 8, class c
+    const int rl = lane & 7, c = 4 * warp + (lane >> 3), seg = segment(K), classes = class_count(K);
+    float acc[2][MT];
+#pragma unroll
+    for (int m = 0; m < MT; m++) acc[0][m] = acc[1][m] = 0.f;
+    int it = 0, tile = blockIdx.x;
+    for (int i = 0; i < total; i++) {
+        const int left = K - (it * CLASSES + c) * seg, n = left < 0 ? 0 : left < seg ? left : seg;    // values of this lane's class
+        rows_sync(READY + i % S);
+        const float* w0 = smem + i % S * STAGE + rl * RPITCH + c * seg;
+        const float* a0 = smem + i % S * STAGE + RT * RPITCH + c * seg;
+        auto four = [&](int k) {
+            const float4 u = *(const float4*)(w0 + k), v = *(const float4*)(w0 + 8 * RPITCH + k);
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                const float4 a = *(const float4*)(a0 + m * RPITCH + k);
+                acc[0][m] = fmaf(a.x, u.x, acc[0][m]); acc[1][m] = fmaf(a.x, v.x, acc[1][m]);
+                acc[0][m] = fmaf(a.y, u.y, acc[0][m]); acc[1][m] = fmaf(a.y, v.y, acc[1][m]);
+                acc[0][m] = fmaf(a.z, u.z, acc[0][m]); acc[1][m] = fmaf(a.z, v.z, acc[1][m]);
+                acc[0][m] = fmaf(a.w, u.w, acc[0][m]); acc[1][m] = fmaf(a.w, v.w, acc[1][m]);
+            }
+        };
+        if (__all_sync(0xffffffffu, n == 64)) {
+#pragma unroll
+            for (int k = 0; k < 64; k += 4) four(k);
+        } else {
+            for (int k = 0; k < n; k += 4) four(k);
+            __syncwarp();
+        }
+        if (i + S < total) rows_arrive(TAKEN + i % S);
         if (++it < per_tile) continue;
         it = 0;
-        const int n0 = tile / tiles_m * (16 * R), m0 = tile % tiles_m * MT;
+        const int n0 = tile / tiles_m * RT, m0 = tile % tiles_m * MT;
         tile += gridDim.x;
-        float* p = part + ((4 * half + sub) * 16 * R + group * 8 * R + rl) * MT;
 #pragma unroll
-        for (int j = 0; j < R; j++)
-#pragma unroll
-            for (int m = 0; m < MT; m++) { p[j * 8 * MT + m] = acc[j][m]; acc[j][m] = 0.f; }
-        __syncthreads();
-        const int classes = class_count(K);
-        for (int e = threadIdx.x; e < 16 * R * MT; e += 128) {
-            const int r = e % (16 * R), m = e / (16 * R);
+        for (int m = 0; m < MT; m++) {
+            part[(c * RT + rl) * MT + m] = acc[0][m];
+            part[(c * RT + rl + 8) * MT + m] = acc[1][m];
+            acc[0][m] = acc[1][m] = 0.f;
+        }
+        asm volatile("barrier.cta.sync %0, 64;" ::"r"(PAIR) : "memory");
+        for (int e = threadIdx.x; e < RT * MT; e += 64) {
+            const int r = e % RT, m = e / RT;
             float v = part[r * MT + m];
-            for (int c = 1; c < classes; c++) v += part[(c * 16 * R + r) * MT + m];
+            for (int q = 1; q < classes; q++) v += part[(q * RT + r) * MT + m];
             if (n0 + r < N && m0 + m < M) {
                 float* o = C + (size_t)(m0 + m) * ldc + n0 + r;
                 *o = MODE == 1 ? *o + v : v;
             }
         }
-        __syncthreads();
+        asm volatile("barrier.cta.sync %0, 64;" ::"r"(PAIR) : "memory");
     }
     pdl_launch_dependents();
 }
@@ -586,23 +568,23 @@ int launch(TC* C, const TA* A, const TA* W, int M, int N, int K, long long lda, 
     return launch_rc;
 }
 
-template <int R, int MT, int MODE>
-int launch_stream(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int sms, cudaStream_t st) {
-    constexpr size_t bytes = StreamShape<R, MT>::BYTES;
-    static_assert(StreamShape<R, MT>::STAGES >= 3, "stages");
-    cudaError_t e = cudaFuncSetAttribute(gemm_stream_kernel<R, MT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+template <int MT, int S, int MODE>
+int launch_rows(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int most, cudaStream_t st) {
+    constexpr size_t bytes = RowsShape<MT, S>::BYTES;
+    cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<MT, S, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
-    const int tiles_m = (M + MT - 1) / MT, tiles = tiles_m * ((N + 16 * R - 1) / (16 * R));
-    const int most = StreamShape<R, MT>::PER_SM * sms, grid = tiles < most ? tiles : most;
-    return oe_launch(gemm_stream_kernel<R, MT, MODE>, dim3(grid), dim3(128), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m, tiles);
+    const int tiles_m = (M + MT - 1) / MT, tiles = tiles_m * ((N + RT - 1) / RT);
+    return oe_launch(gemm_rows_kernel<MT, S, MODE>, dim3(tiles < most ? tiles : most), dim3(160), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m, tiles);
 }
 template <int MT, int MODE>
-int launch_stream_rows(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int sms, cudaStream_t st) {
-    // Weight rows a lane: A's values are read from shared memory once for R rows, so more of them help as soon as there are
-    // tiles for every SM.
-    if (MT > 2 && N >= 64 * sms) return launch_stream<4, MT, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
-    if (N >= 32 * sms) return launch_stream<2, MT, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
-    return launch_stream<1, MT, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+int launch_rows_for(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int sms, cudaStream_t st) {
+    // While the tiles leave an SM each, one CTA with a deep ring; beyond, two an SM (8 x 2,048 x 8,192: 43 us with the deep ring,
+    // 45 with two stages, 16 rows 82 and 53; 3 x 128,256 x 2,048: 265 and 202).
+    constexpr int DEEP = MT == 8 ? 4 : 5;
+    const long long tiles = (long long)((M + MT - 1) / MT) * ((N + RT - 1) / RT);
+    if (tiles > 0x7fffffffll) return OE_ERR_UNSUPPORTED;
+    if (tiles <= sms) return launch_rows<MT, DEEP, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+    return launch_rows<MT, 2, MODE>(C, A, W, M, N, K, lda, ldc, 2 * sms, st);
 }
 template <int BM_, int BN_, int KG, int MODE>
 int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, cudaStream_t st) {
@@ -627,9 +609,9 @@ int launch_wide(float* C, const float* A, const float* W, int M, int N, int K, l
     return oe_launch_cluster(gemm_wide_kernel<KG, MODE>, KG, dim3((unsigned)ctas), dim3(256), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m);
 }
 
-constexpr int STREAM_MAX_M = 32;
+constexpr int ROWS_MAX_M = 32;
 
-// kind: 0 by size, else 1 streaming, 2 tiles of 64, 3 tiles of 128, 4 the general kernel, 5, 6 tiles of 128 whose classes
+// kind: 0 by size, else 1 few rows, 2 tiles of 64, 3 tiles of 128, 4 the general kernel, 5, 6 tiles of 128 whose classes
 // four, eight CTAs share (tests).
 template <int MODE>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int kind, cudaStream_t st) {
@@ -642,11 +624,12 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, lo
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128);
     if (kind == 0) {
-        // Up to 64 rows a tile of 128 is half empty.  A weight of few rows is streamed (2,048 x 2,048: 48 rows 51 us, 55 by tiles of
-        // 128; 64 rows 68 and 55); with two CTAs an SM for eight shares of every tile, tiles of 128 (40 x 3,072 x 3,072: 78 us, 92
-        // streamed, 113 by tiles of 64); a weight of more rows has tiles of 64 enough for all SMs (64 x 16,384 x 2,048: 156 us, 197 by
-        // tiles of 128).  From 65 rows on tiles of 128 are faster at every size tried.
-        kind = M <= STREAM_MAX_M || (M <= 48 && t128 <= 16) ? 1 : M > 64 || K <= ONE_CHAIN || 8 * t128 <= 2 * sms ? 3 : 2;
+        // Up to 64 rows a tile of 128 is half empty.  A weight of few rows is streamed (64 x 2,048 x 8,192: 174 us, 191 by tiles of
+        // 128, 297 by tiles of 64; 40 x 3,072 x 3,072: 70, 79, 113; 48 x 2,048 x 2,048: 41, 56, 80); beyond that, while there are two
+        // CTAs an SM for eight shares of every tile, tiles of 128 (64 x 3,072 x 3,072: 137 us streamed by the kernel before, 80, 119); a
+        // weight of more rows has tiles of 64 enough for all SMs (64 x 16,384 x 2,048: 156 us, 197 by tiles of 128; 32 rows 154
+        // streamed, 150).  From 65 rows on tiles of 128 are faster at every size tried.
+        kind = M <= ROWS_MAX_M || (M <= 64 && M * t128 <= 1024) ? 1 : M > 64 || K <= ONE_CHAIN || 8 * t128 <= 2 * sms ? 3 : 2;
     }
     if (kind == 3) {
         // eight shares of a tile while four would not fill the SMs (192 x 4,096 x 4,096, 64 tiles: 211 us, 240 with four; 300 rows, 96
@@ -657,10 +640,10 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, lo
     if (kind == 5) return launch_wide<4, MODE>(C, A, W, M, N, K, lda, ldc, st);
     if (kind == 6) return launch_wide<8, MODE>(C, A, W, M, N, K, lda, ldc, st);
     if (kind == 2) return launch_tile<64, 64, 4, MODE>(C, A, W, M, N, K, lda, ldc, st);
-    if (M == 1) return launch_stream_rows<1, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
-    if (M == 2) return launch_stream_rows<2, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
-    if (M <= 4) return launch_stream_rows<4, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
-    return launch_stream_rows<8, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+    if (M == 1) return launch_rows_for<1, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+    if (M == 2) return launch_rows_for<2, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+    if (M <= 4) return launch_rows_for<4, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+    return launch_rows_for<8, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
 }
 
 }  // namespace

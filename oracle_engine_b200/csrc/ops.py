@@ -318,7 +318,7 @@ def gemm_simple(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate:
     the shapes (csrc/gemm_simple.cu).
 
     a [M, K] and w [N, K] of one dtype (float32 or bfloat16); out [M, N] of that dtype or
-    float32; accumulate needs a float32 out.  kind (float32 only): 0 the kernel is chosen by size, 1 weight streaming,
+    float32; accumulate needs a float32 out.  kind (float32 only): 0 the kernel is chosen by size, 1 a few rows,
     2 tiles of 64, 3 tiles of 128, 4 the general one, 5 and 6 tiles of 128 (K > 512) that 4 and 8 CTAs share; the same bits."""
     _dev(out, a, w)
     M, K = a.shape
