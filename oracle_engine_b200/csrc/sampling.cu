@@ -138,10 +138,7 @@ constexpr int PENALTY_CAP = 256;                    // the longest history whose
 
 // The repeat penalty over the last `repeat_last` recorded tokens, for those in [lo, hi), by the whole block: the first of
 // equal tokens is penalised once for each of them.  (One thread going through the history took 1.2 us a token.)
-// hit: null, or per thread of the block a mask, zeroed by it before, in which the changed places are marked: place
-// lo + stride j + t is bit j of hit[t].
-__device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, int repeat_last, const SampleState& st, int* s_ids,
-                         unsigned* hit = nullptr, int stride = 1) {
+__device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, int repeat_last, const SampleState& st, int* s_ids) {
     const int count = st.hist_count[slot];
     int n = count < repeat_last ? count : repeat_last;
     if (n > st.hist_cap) n = st.hist_cap;
@@ -159,7 +156,6 @@ __device__ void penalise(float* x, int lo, int hi, int slot, float repeat_pen, i
         float v = x[id];
         for (int i = 0; i < times; i++) v = v > 0.f ? v / repeat_pen : v * repeat_pen;
         x[id] = v;
-        if (hit != nullptr) atomicOr(&hit[(id - lo) % stride], 1u << ((id - lo) / stride));
     }
     __syncthreads();
 }
@@ -301,7 +297,7 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
 //   * The usual case, a top-k of at most as many tokens as the cluster has warps (128): the k-th largest of the warps' maxima
 //     is a lower bound of the k-th largest value, and few values are at or above it (about 50 for k = 40 where the order of the
 //     tokens is unrelated to their values).  Those go to the first CTA with the exchange of the softmax's sums, which ends the
-//     row alone by comparing them all with one another: two exchanges in all.  8 rows of 128,256: 33.3 -> 15.6 us a launch.
+//     row alone by comparing them all with one another: two exchanges in all.  8 rows of 128,256: 34 -> 15 us a launch (12 without the repeat penalty).
 //   * Otherwise, or where more values are at or above the bound than there is room for, passes over the registers: one
 //     settles two bits of a threshold (three candidates), and a search ends as soon as the tokens it keeps are known: top-k
 //     when a candidate keeps exactly k, top-p when one token is left between the bounds.
@@ -315,9 +311,9 @@ constexpr int KEPT = 1 << 30;                        // marks a kept token's ind
 struct __align__(16) Sums { float a[4]; unsigned n[4]; };
 
 __device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_barrier() { cluster_arrive(); cluster_wait(); }
 __device__ __forceinline__ void store_remote(void* local, unsigned rank, float4 v) {
     const unsigned here = (unsigned)__cvta_generic_to_shared(local);
     unsigned there;
@@ -374,14 +370,14 @@ __device__ __forceinline__ Sums cluster_sums(Sums v, Sums (*box)[CL * CW], int& 
     return t;
 }
 
-__device__ __forceinline__ void record_token(int token, int row, int slot, int* out, const SampleState& st, int record) {
+// drawn, recorded: what the slot's counters hold.
+__device__ __forceinline__ void record_token(int token, int row, int slot, int drawn, int recorded, int* out, const SampleState& st, int record) {
     out[row] = token;
     if (record) {
-        st.rng_counter[slot] += 1;
+        st.rng_counter[slot] = drawn + 1;
         if (st.hist != nullptr) {
-            const int c = st.hist_count[slot];
-            st.hist[(size_t)slot * st.hist_cap + (c % st.hist_cap)] = token;
-            st.hist_count[slot] = c + 1;
+            st.hist[(size_t)slot * st.hist_cap + (recorded % st.hist_cap)] = token;
+            st.hist_count[slot] = recorded + 1;
         }
     }
 }
@@ -397,7 +393,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     __shared__ unsigned s_hit[CT];
     __shared__ int s_ids[PENALTY_CAP];
     __shared__ float s_part[EPT * CW], s_excl[EPT * CW], s_total[CL];
-    __shared__ int s_entry, s_last[CL], s_warp_last[CW];
+    __shared__ int s_entry, s_again, s_last[CL], s_warp_last[CW];
     __shared__ float s_bound;
     __shared__ unsigned s_cut;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -405,26 +401,53 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     pdl_launch_dependents();
     pdl_wait();
     const int slot = row_slot[row];
-    if (slot < 0) { if (rank == 0 && tid == 0) out[row] = -1; return; }      // the whole cluster
     float* x = logits + (size_t)row * V;
     const int slice = EPT * CT, base = rank * slice;  // this CTA's values are base + 512 j + tid
     int turn = 0;
-
     float v[EPT];
 #pragma unroll
     for (int j = 0; j < EPT; j++) {
         const int i = base + j * CT + tid;
         v[j] = i < V ? x[i] : -INFINITY;
     }
-    // repeat penalty, of the tokens in this CTA's slice, while the values are on their way; what it changes is read again
+    if (slot < 0) { if (rank == 0 && tid == 0) out[row] = -1; return; }      // the whole cluster
+    cluster_arrive();                                 // (waited for before another CTA's memory is written)
+    const unsigned long long seed = (unsigned long long)st.rng_seed[slot];
+    const int drawn = st.rng_counter[slot], recorded = st.hist != nullptr ? st.hist_count[slot] : 0;
+    // Repeat penalty, while the values are on their way: the recorded tokens in this CTA's slice are marked, and the thread that
+    // has a marked one penalises it, as often as it was recorded.
     if (repeat_pen > 1.f && st.hist != nullptr) {
+        int n = recorded < repeat_last ? recorded : repeat_last;
+        if (n > st.hist_cap) n = st.hist_cap;
+        // place p of the ring holds one of the last n if it lies less than n places, going round, before the next one's
+        int id = -1;
+        if (tid < st.hist_cap) {
+            id = st.hist[(size_t)slot * st.hist_cap + tid];
+            int back = recorded % st.hist_cap - tid;
+            if (back <= 0) back += st.hist_cap;
+            if (back > n) id = -1;
+        }
+        if (id < base || id >= min(base + slice, V)) id = -1;
         s_hit[tid] = 0u;
+        if (tid < PENALTY_CAP) s_ids[tid] = id;
+        if (tid == 0) s_again = 0;
         __syncthreads();
-        penalise(x, base, min(base + slice, V), slot, repeat_pen, repeat_last, st, s_ids, s_hit, CT);
-        const unsigned again = s_hit[tid];
-        if (again != 0u) {
+        if (id >= 0) {
+            const unsigned bit = 1u << ((id - base) / CT);
+            if (atomicOr(&s_hit[(id - base) % CT], bit) & bit) s_again = 1;
+        }
+        __syncthreads();
+        for (unsigned mine = s_hit[tid]; mine != 0u; mine &= mine - 1u) {
+            const int at = __ffs(mine) - 1, token = base + at * CT + tid;
+            int times = s_again ? 0 : 1;
+            if (s_again) for (int i = 0; i < PENALTY_CAP; i++) times += s_ids[i] == token ? 1 : 0;
+            float p = 0.f;
 #pragma unroll
-            for (int j = 0; j < EPT; j++) if (again >> j & 1u) v[j] = x[base + j * CT + tid];
+            for (int j = 0; j < EPT; j++) p = j == at ? v[j] : p;
+            for (int i = 0; i < times; i++) p = p > 0.f ? p / repeat_pen : p * repeat_pen;
+            x[token] = p;
+#pragma unroll
+            for (int j = 0; j < EPT; j++) v[j] = j == at ? p : v[j];
         }
     }
 
@@ -434,7 +457,8 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     float mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < EPT; j++) { v[j] *= inv_t; mx = fmaxf(mx, v[j]); }
-    cluster_barrier();                                // every CTA of the cluster is there before its memory is written
+    __syncwarp();
+    cluster_wait();
     sums.a[0] = mx;
     mx = cluster_sums<true>(sums, box, turn).a[0];
     // the bound: the top_k-th largest of the warps' maxima.  At least top_k values are at or above it.
@@ -522,7 +546,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
         }
         __syncthreads();
         const unsigned cut = s_cut;
-        const float u = uniform_from_counter((unsigned long long)st.rng_seed[slot], (unsigned long long)st.rng_counter[slot]);
+        const float u = uniform_from_counter(seed, (unsigned long long)drawn);
         // the draw: the first kept token, by index, whose running mass exceeds u x the kept mass
         int last_kept = -1;
         for (int i = tid; i < n; i += CT) {
@@ -548,7 +572,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
             __syncthreads();
             if (tid == 0) s_entry = s_last[0];
         }
-        if (tid == 0) record_token(s_entry, row, slot, out, st, record);
+        if (tid == 0) record_token(s_entry, row, slot, drawn, recorded, out, st, record);
         return;
     }
 #pragma unroll
@@ -643,7 +667,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
 #pragma unroll
     for (int c = 0; c < CL; c++) { if (c == rank) from = total; total += s_total[c]; }
     float to = from + s_total[rank];
-    const float u = uniform_from_counter((unsigned long long)st.rng_seed[slot], (unsigned long long)st.rng_counter[slot]);
+    const float u = uniform_from_counter(seed, (unsigned long long)drawn);
     const float r = u * total;
     int pick = -1;
     if (from <= r && r < to) {                        // one CTA at most
@@ -676,7 +700,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
         box[turn][0].a[0] = __int_as_float(l);
     }
     cluster_barrier();
-    if (rank == 0 && tid == 0) record_token(__float_as_int(box[turn][0].a[0]), row, slot, out, st, record);
+    if (rank == 0 && tid == 0) record_token(__float_as_int(box[turn][0].a[0]), row, slot, drawn, recorded, out, st, record);
 }
 
 template <int EPT>
