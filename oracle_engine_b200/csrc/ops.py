@@ -146,7 +146,7 @@ _SIGNATURES = {
         "oe_argmax_rows": [_P, _P, _I, _I, _P],
         "oe_argmax_rows_wide": [_P, _P, _P, _P, _I, _I, _P],
         "oe_zero_rows": [_P, _I, _L, _I, _P],
-        "oe_sampler_start": [_P, _P, _P, _P, _I, _I, _L, _I, _P, _P],
+        "oe_sampler_start": [_P, _P, _P, _P, _I, _I, _L, _I, _P, _I, _P],
         "oe_sample_rows": [_P, _P, _P, _I, _I, _F, _I, _F, _F, _I, _P, _P, _P, _P, _I, _I, _P],
     },
 }
@@ -1584,23 +1584,27 @@ def sample_rows(logits: torch.Tensor, out: torch.Tensor, row_slot: torch.Tensor,
                 rng_counter: torch.Tensor, hist: torch.Tensor | None, hist_count: torch.Tensor | None,
                 record: bool = True) -> None:
     """One token per row of float32 logits (overwritten), by the reference's sampling chain."""
-    _dev(logits, out, row_slot, rng_seed, rng_counter, hist, hist_count)
-    _i32(out, "out")
-    _i32(row_slot, "row_slot")
-    _i32(rng_counter, "rng_counter")
-    if rng_seed.dtype != torch.int64:
+    if not (logits.is_cuda and out.is_cuda and row_slot.is_cuda and rng_seed.is_cuda and rng_counter.is_cuda):
+        raise KernelError("kernel arguments must be CUDA tensors")
+    i32 = torch.int32
+    if not (out.dtype is i32 and row_slot.dtype is i32 and rng_counter.dtype is i32 and out.is_contiguous() and row_slot.is_contiguous()
+            and rng_counter.is_contiguous()):
+        raise KernelError("out, row_slot and rng_counter must be contiguous int32 tensors")
+    if rng_seed.dtype is not torch.int64:
         raise KernelError("sample_rows: rng_seed must be int64")
-    if logits.dtype != torch.float32 or not logits.is_contiguous():
+    if logits.dtype is not torch.float32 or not logits.is_contiguous():
         raise KernelError("sample_rows: logits must be contiguous float32")
-    cap = 0
+    cap, ring, recorded = 0, None, None
     if hist is not None:
+        _dev(hist, hist_count)
         _i32(hist, "hist")
         _i32(hist_count, "hist_count")
-        cap = hist.shape[1]
+        cap, ring, recorded = hist.shape[1], hist.data_ptr(), hist_count.data_ptr()
+    rows, width = logits.shape
     _check(_fn("sampling", "oe_sample_rows")(
-        _ptr(logits), _ptr(out), _ptr(row_slot), logits.shape[0], logits.shape[1], float(temperature), int(top_k),
-        float(top_p), float(repeat_penalty), int(repeat_last_n), _ptr(rng_seed), _ptr(rng_counter), _ptr(hist),
-        _ptr(hist_count), cap, int(record), _stream()), "sample_rows")
+        logits.data_ptr(), out.data_ptr(), row_slot.data_ptr(), rows, width, float(temperature), int(top_k), float(top_p),
+        float(repeat_penalty), int(repeat_last_n),
+        rng_seed.data_ptr(), rng_counter.data_ptr(), ring, recorded, cap, int(record), _stream()), "sample_rows")
 
 
 def row_table(tensors) -> tuple:
@@ -1619,13 +1623,14 @@ def zero_rows(table: torch.Tensor, largest: int, row: int) -> None:
 
 
 def sampler_start(rng_seed: torch.Tensor, rng_counter: torch.Tensor, hist: torch.Tensor, hist_count: torch.Tensor, slot: int, seed: int,
-                  count: int, ring) -> None:
+                  count: int, tail) -> None:
     """The sampler's state of `slot` at a sequence's start, in one launch: seed, no draws yet, `count` recorded tokens and,
-    unless `ring` is None (a numpy int32 array as long as the history), the history itself."""
+    unless `tail` is None (an array.array of C ints: the last of those tokens), the history itself."""
     _dev(rng_seed, rng_counter, hist, hist_count)
     if not 0 <= slot < rng_seed.numel():
         raise IndexError(f"slot {slot} of {rng_seed.numel()}")
-    if ring is not None and (str(ring.dtype) != "int32" or ring.shape != (hist.shape[1],) or not ring.flags["C_CONTIGUOUS"]):
-        raise KernelError("sampler_start: ring must be a contiguous int32 array of the history's length")
-    _check(_fn("sampling", "oe_sampler_start")(_ptr(rng_seed), _ptr(rng_counter), _ptr(hist), _ptr(hist_count), int(hist.shape[1]), int(slot), int(seed),
-                                               int(count), None if ring is None else ring.ctypes.data, _stream()), "sampler_start")
+    if tail is not None and (tail.typecode != "i" or tail.itemsize != 4):
+        raise KernelError("sampler_start: tail must be an array of C ints")
+    address, n = (None, 0) if tail is None else tail.buffer_info()
+    _check(_fn("sampling", "oe_sampler_start")(rng_seed.data_ptr(), rng_counter.data_ptr(), hist.data_ptr(), hist_count.data_ptr(), hist.shape[1],
+                                               int(slot), int(seed), int(count), address, n, _stream()), "sampler_start")

@@ -744,14 +744,15 @@ int oe_zero_rows(const long long* table, int n, long long largest, int row, cuda
     return oe_launch(zero_rows_kernel, dim3((unsigned)pieces, n), dim3(256), 0, st, table, row);
 }
 
-// ring: null, or `cap` token ids in host memory, read before the call returns.
+// tail: null, or the last `n_tail` (up to `cap`) of the `count` recorded tokens in host memory, read before the call returns; they
+// go where a ring of `cap` places has them, the other places are zero.  null: the history stays as it is.
 int oe_sampler_start(long long* rng_seed, int* rng_counter, int* hist, int* hist_count, int cap, int slot, long long seed, int count,
-                     const int* ring, cudaStream_t st) {
-    if (cap < 1 || cap > PENALTY_CAP || slot < 0) return OE_ERR_UNSUPPORTED;
+                     const int* tail, int n_tail, cudaStream_t st) {
+    if (cap < 1 || cap > PENALTY_CAP || slot < 0 || n_tail < 0 || n_tail > cap || (tail && n_tail > count)) return OE_ERR_UNSUPPORTED;
     Ring r = {};
-    if (ring) for (int i = 0; i < cap; i++) r.id[i] = ring[i];
+    if (tail) for (int i = 0, at = (count - n_tail) % cap; i < n_tail; i++, at = at + 1 == cap ? 0 : at + 1) r.id[at] = tail[i];
     return oe_launch(sampler_start_kernel, dim3(1), dim3(PENALTY_CAP), 0, st, rng_seed, rng_counter, hist, hist_count, slot, seed, count, cap,
-                     ring != nullptr ? 1 : 0, r);
+                     tail != nullptr ? 1 : 0, r);
 }
 
 // Wide rows in two stages; scratch: rows * 32 floats and rows * 32 ints.

@@ -32,27 +32,27 @@ class Sampler:
     def start_sequence(self, slot: int, seed: int, prompt, params) -> None:
         """Seeds the slot's generator and records the prompt without its last token, as
         the reference does before generating (core/engine.cpp:118-122)."""
-        ring, count = None, 0
+        tail, count = None, 0
         recorded = len(prompt) - 1
         if params.repeat_penalty > 1.0 and recorded > 0:
             if params.repeat_last_n > HISTORY_CAPACITY:
                 raise ValueError(f"repeat_last_n {params.repeat_last_n} exceeds the {HISTORY_CAPACITY} tokens kept")
-            tail = prompt[max(0, recorded - HISTORY_CAPACITY):recorded]
-            try:
-                tail = np.frombuffer(array("i", tail), dtype=np.int32)
-            except TypeError:                      # whatever else int() takes; ids beyond 32 bits raise OverflowError
-                tail = np.frombuffer(array("i", [int(t) for t in tail]), dtype=np.int32)
             count = recorded
-            ring = np.zeros(HISTORY_CAPACITY, dtype=np.int32)
-            ring[(count - tail.size + np.arange(tail.size)) % HISTORY_CAPACITY] = tail
+            ids = prompt[max(0, recorded - HISTORY_CAPACITY):recorded]
+            try:
+                tail = array("i", ids)
+            except TypeError:                      # whatever else int() takes; ids beyond 32 bits raise OverflowError
+                tail = array("i", [int(t) for t in ids])
         if not -2 ** 63 <= int(seed) < 2 ** 63:
             raise OverflowError(f"seed {seed} does not fit 64 bits")
-        if not self.hist.is_cuda:
-            self.rng_seed[slot], self.rng_counter[slot], self.hist_count[slot] = int(seed), 0, count
-            if ring is not None:
-                self.hist[slot] = torch.from_numpy(ring)
+        if self.hist.is_cuda:
+            ops.sampler_start(self.rng_seed, self.rng_counter, self.hist, self.hist_count, slot, int(seed), count, tail)
             return
-        ops.sampler_start(self.rng_seed, self.rng_counter, self.hist, self.hist_count, slot, seed, count, ring)
+        self.rng_seed[slot], self.rng_counter[slot], self.hist_count[slot] = int(seed), 0, count
+        if tail is not None:
+            ring = np.zeros(HISTORY_CAPACITY, dtype=np.int32)
+            ring[(count - len(tail) + np.arange(len(tail))) % HISTORY_CAPACITY] = tail
+            self.hist[slot] = torch.from_numpy(ring)
 
     def sample(self, logits: torch.Tensor, row_slot: torch.Tensor, params, out: torch.Tensor | None = None):
         """logits float32 [R, V] (overwritten unless greedy without penalty); row_slot int32 [R].
