@@ -425,20 +425,24 @@ attn_mma_kernel(const AttnArgs a) {
 // ---------------------------------------------------------------------------------------
 // Decoded tokens, one CTA per (sequence, KV head), the WARPS of the CTA split the keys.
 // Every warp holds the same 16 query rows (the G heads of the group for the one new token),
-// walks half pages (32 keys) warp, warp + NW, ... of the sequence through a double buffer of
+// walks tiles of TB keys (half pages, or quarters) warp, warp + NW, ... of the sequence through a double buffer of
 // its own (cp.async, no CTA-wide barrier in the loop) and keeps its own running softmax; at
 // the end the warps' partial results are added in warp order through shared memory.  The
 // kernel also rotates q and the new token's k and writes k and v to the cache (as the fused
 // path of attn_mma_kernel does), so a decode step needs one attention launch and no scratch
 // in global memory.  For batches whose (sequence, KV head) pairs alone give enough CTAs.
 // ---------------------------------------------------------------------------------------
-constexpr int TB = 32;                          // keys per tile of a warp
-constexpr int TB_BYTES = TB * ROW_BYTES;
-constexpr int WARP_STAGE_BYTES = 2 * TB_BYTES;  // K and V
+template <int TB>                                // keys per tile of a warp: 32 or 16
+struct Tile {
+    static constexpr int BYTES = TB * ROW_BYTES, STAGE_BYTES = 2 * BYTES;      // K and V
+};
+constexpr size_t warps_bytes(int nw, int st, int tb) { return (size_t)nw * st * 2 * tb * ROW_BYTES; }
 
-__device__ __forceinline__ void load_half_page(uint8_t* ks, uint8_t* vs, const bf16* cache, int page, int half, int kvh, int KVH, int lane) {
-    const bf16* kg = cache + (((size_t)page * 2 + 0) * KVH + kvh) * (size_t)(BN * HD) + (size_t)half * TB * HD;
-    const bf16* vg = cache + (((size_t)page * 2 + 1) * KVH + kvh) * (size_t)(BN * HD) + (size_t)half * TB * HD;
+// Tile `tile` of a sequence (tiles of TB keys, BN / TB to a page).
+template <int TB>
+__device__ __forceinline__ void load_tile(uint8_t* ks, uint8_t* vs, const bf16* cache, int page, int part, int kvh, int KVH, int lane) {
+    const bf16* kg = cache + (((size_t)page * 2 + 0) * KVH + kvh) * (size_t)(BN * HD) + (size_t)part * TB * HD;
+    const bf16* vg = cache + (((size_t)page * 2 + 1) * KVH + kvh) * (size_t)(BN * HD) + (size_t)part * TB * HD;
     constexpr int CHUNKS = TB * HD / 8;
 #pragma unroll
     for (int c0 = 0; c0 < CHUNKS; c0 += 32) {
@@ -472,9 +476,10 @@ __device__ __forceinline__ float ld_peer_f32(const float* p, uint32_t rank) {
     return v;
 }
 
-template <int NW, int ST>
+template <int NW, int ST, int TB>
 __global__ void __launch_bounds__(NW * 32, 1)
 attn_decode_warps_kernel(const AttnArgs a) {
+    constexpr int TB_BYTES = Tile<TB>::BYTES, WARP_STAGE_BYTES = Tile<TB>::STAGE_BYTES, PARTS = BN / TB;
     constexpr int WARP_BYTES = ST * WARP_STAGE_BYTES;
     static_assert(ST >= 2 && (NW + 1) * 16 * (HD + 2) * 4 <= NW * WARP_BYTES, "the merge scratch shares the staging buffers");
     extern __shared__ __align__(16) uint8_t smem[];
@@ -515,7 +520,7 @@ attn_decode_warps_kernel(const AttnArgs a) {
         if (pre < n_my) {
             const int hp = hp_lo + gw + pre * stride;
             uint8_t* st = mine + (size_t)pre * WARP_STAGE_BYTES;
-            load_half_page(st, st + TB_BYTES, a.cache, trow[hp >> 1], hp & 1, kvh, a.KVH, lane);
+            load_tile<TB>(st, st + TB_BYTES, a.cache, trow[hp / PARTS], hp % PARTS, kvh, a.KVH, lane);
         }
         cp_async_commit();
     }
@@ -717,7 +722,7 @@ attn_decode_warps_kernel(const AttnArgs a) {
         __syncwarp();                                       // every lane has read the stage: refill it
         if (it + ST < n_my) {
             const int hn = hp + ST * stride;
-            load_half_page(ks_cur, vs_cur, a.cache, trow[hn >> 1], hn & 1, kvh, a.KVH, lane);
+            load_tile<TB>(ks_cur, vs_cur, a.cache, trow[hn / PARTS], hn % PARTS, kvh, a.KVH, lane);
         }
         cp_async_commit();
         stage = stage + 1 == ST ? 0 : stage + 1;
@@ -951,6 +956,10 @@ int oe_attn_decode_fused_bf16(bf16* out, const bf16* qkv, long long qkv_stride, 
 // one launch, no scratch.  Needs G = H/KVH <= 16.  shape = warps * 16 + ring depth; the forms
 // built here: 6 x 2 (a CTA fills an SM: up to about two CTAs for every SM), 4 x 3 (the same with
 // a deeper ring), 2 x 3 (two CTAs an SM) and 1 x 3 (four CTAs an SM: large batches).  0: 6 x 2.
+// In the last two each of these warps is a pair that shares its tiles, 16 keys each: a long sequence among short ones is a
+// chain of tiles, and a tile's scores, softmax and sums are what a warp takes 1.3 us for (ms a step of the 28-layer model, one
+// warp a tile / two: 64 sequences of 33 to 480 tokens 2.644 / 2.539, of 512 2.877 / 2.820, 48 of 33 to 480 2.546 / 2.437, 32 of 33 to
+// 480 2.411 / 2.357, of 300 to 1,400 2.851 / 2.766).  6 x 2 as 8 x 3 tiles of 16 keys is slower: 8 sequences of 512 1.627 and 1.643.
 // cluster: 1, or how many CTAs (a thread-block cluster, up to 8) share one (sequence, KV head).
 // Returns OE_ERR_UNSUPPORTED for a form that is not built or does not fit an SM at this head size.
 int oe_attn_decode_warps_bf16(bf16* out, const bf16* qkv, long long qkv_stride, const float* cos_tab,
@@ -970,34 +979,34 @@ int oe_attn_decode_warps_bf16(bf16* out, const bf16* qkv, long long qkv_stride, 
     if (cluster < 1 || cluster > 8) return OE_ERR_UNSUPPORTED;
     a.cluster = cluster;
     if (shape == 0) shape = 6 * 16 + 2;
-    if (shape == 6 * 16 + 2 && 6 * 2 * WARP_STAGE_BYTES > 220 * 1024) shape = 3 * 16 + 2;    // large heads
-#define OE_WARPS_LAUNCH(NW, ST)                                                                                    \
-    if (shape == NW * 16 + ST) {                                                                                  \
-        constexpr size_t smem = (size_t)NW * ST * WARP_STAGE_BYTES;                                               \
+    if (shape == 6 * 16 + 2 && warps_bytes(6, 2, 32) > 220 * 1024) shape = 3 * 16 + 2;    // large heads
+#define OE_WARPS_LAUNCH(SHAPE, NW, ST, TB)                                                                         \
+    if (shape == SHAPE) {                                                                                         \
+        constexpr size_t smem = warps_bytes(NW, ST, TB);                                                          \
         if (smem > 220 * 1024) return OE_ERR_UNSUPPORTED;                                                         \
         static bool attr_set = false;                                                                             \
         if (!attr_set) {                                                                                          \
-            cudaError_t e = cudaFuncSetAttribute(attn_decode_warps_kernel<NW, ST>,                                \
+            cudaError_t e = cudaFuncSetAttribute(attn_decode_warps_kernel<NW, ST, TB>,                            \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
             if (e != cudaSuccess) return (int)e;                                                                  \
             attr_set = true;                                                                                      \
         }                                                                                                         \
         if (cluster > 1)                                                                                          \
-            return oe_launch_cluster(attn_decode_warps_kernel<NW, ST>, (unsigned)cluster, dim3(cluster, KVH, n_seqs), \
+            return oe_launch_cluster(attn_decode_warps_kernel<NW, ST, TB>, (unsigned)cluster, dim3(cluster, KVH, n_seqs), \
                                      dim3(NW * 32), smem, st, a);                                                  \
-        return oe_launch(attn_decode_warps_kernel<NW, ST>, dim3(1, KVH, n_seqs), dim3(NW * 32), smem, st, a);     \
+        return oe_launch(attn_decode_warps_kernel<NW, ST, TB>, dim3(1, KVH, n_seqs), dim3(NW * 32), smem, st, a); \
     }
-    OE_WARPS_LAUNCH(6, 2)
-    OE_WARPS_LAUNCH(3, 2)
-    OE_WARPS_LAUNCH(4, 3)
-    OE_WARPS_LAUNCH(2, 3)
-    OE_WARPS_LAUNCH(1, 3)
+    OE_WARPS_LAUNCH(6 * 16 + 2, 6, 2, 32)
+    OE_WARPS_LAUNCH(3 * 16 + 2, 3, 2, 32)
+    OE_WARPS_LAUNCH(4 * 16 + 3, 4, 3, 32)
+    OE_WARPS_LAUNCH(2 * 16 + 3, 4, 3, 16)
+    OE_WARPS_LAUNCH(1 * 16 + 3, 2, 3, 16)
 #undef OE_WARPS_LAUNCH
     return OE_ERR_UNSUPPORTED;
 }
 
 // Bytes of shared memory one CTA of a form takes (how many share an SM follows from it).
-int oe_attn_decode_warps_smem(int shape) { return (shape / 16) * (shape % 16) * WARP_STAGE_BYTES; }
+int oe_attn_decode_warps_smem(int shape) { return (int)warps_bytes(shape / 16, shape % 16, 32); }
 
 }  // extern "C"
 

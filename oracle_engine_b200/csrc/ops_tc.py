@@ -540,8 +540,8 @@ def decode_warps_shape(n_seqs: int, context_class: int, head_dim: int, n_kv_head
     CTAs are all resident at once (at head size 128 one CTA an SM for up to 148 pairs, then two,
     then four); with more pairs than that, short contexts take the smallest CTAs.  Long contexts
     leave the one-warp form out (a lone warp's arithmetic shows there) and, past one round, take
-    the form whose last round of CTAs is fullest.  Measured (us; 24 heads over 8 KV heads of 128; 6x2 / 2x3 /
-    1x3 / the one-warp kernel with one staged page):
+    the form whose last round of CTAs is fullest.  Measured before a pair of warps shared each tile of the last two (us; 24
+    heads over 8 KV heads of 128; 6x2 / 2x3 / 1x3 / the one-warp kernel with one staged page):
     600 keys:   16 sequences 10.5 / 14.0 / 20.6 / -,  24: 19.2 / 15.0 / 22.8 / -,  32: 21.2 / 16.1 / 24.2 / -,
                 48: 31.5 / 31.4 / 24.9 / 35.2,  64: 41.9 / 33.1 / 31.3 / 37.8,  128: 74.1 / 64.1 / 55.3 / 74.2
     2,100 keys: 24: 46.0 / 40.0 / 67.3,  32: 48.3 / 49.0 / 70.5,  48: 71.9 / 83.8 / 73.9,  64: 95.1 / 87.2 / 96.4,
