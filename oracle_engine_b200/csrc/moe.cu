@@ -31,14 +31,19 @@ __device__ __forceinline__ void route_token(const float* zr, int t, int lane, in
                                             const float* __restrict__ bias, int n_groups, int keep, unsigned* kept) {
     const int W = E + (has_gate ? 1 : 0);
     float* drow = dense + (size_t)t * W;
-    for (int e = lane; e < W; e += 32) drow[e] = 0.f;
-    if (tok_seq[t] < 0) {
+    // up to 64 experts a lane keeps its two weights and stores them once (stored as chosen and multiplied in place behind it, a
+    // weight was read back from the L2); more are zeroed first
+    const bool few = E <= 64;
+    const bool pads = tok_seq[t] < 0;
+    if (!few || pads) for (int e = lane; e < W; e += 32) drow[e] = 0.f;
+    if (pads) {
         for (int j = lane; j < top; j += 32) {
             if (idx) idx[(size_t)t * top + j] = 0;
             if (wt) wt[(size_t)t * top + j] = 0.f;
         }
         return;
     }
+    float own[2] = {0.f, 0.f};
     __syncwarp();
     // what the choice goes by: a logit (its order is the softmax's), or sigmoid + bias
     auto score = [&](int e) {
@@ -93,9 +98,13 @@ __device__ __forceinline__ void route_token(const float* zr, int t, int lane, in
         if (j == 0) zmax = best;
         const float p = mode == 1 ? 1.f / (1.f + expf(-(bias ? zr[bi] : best))) : expf(best - zmax);
         sum += p;
+        if ((bi & 31) == lane) {
+            if (bi < 32) own[0] = p;
+            else if (bi < 64) own[1] = p;
+        }
         if (lane == 0) {
             if (idx) idx[(size_t)t * top + j] = bi;
-            drow[bi] = p;
+            if (!few) drow[bi] = p;
             if (wt) wt[(size_t)t * top + j] = p;
         }
     }
@@ -109,8 +118,13 @@ __device__ __forceinline__ void route_token(const float* zr, int t, int lane, in
         total = warp_sum(total);
         inv = 1.f / total / (sum / total + 1e-20f);
     }
-    for (int i = 0, e = lane; e < E; e += 32, i++)
-        if (taken >> i & 1u) drow[e] *= inv;
+    if (few) {
+        if (lane < E) drow[lane] = taken & 1u ? own[0] * inv : 0.f;
+        if (lane + 32 < E) drow[lane + 32] = taken & 2u ? own[1] * inv : 0.f;
+    } else {
+        for (int i = 0, e = lane; e < E; e += 32, i++)
+            if (taken >> i & 1u) drow[e] *= inv;
+    }
     if (wt) for (int j = lane; j < top; j += 32) wt[(size_t)t * top + j] *= inv;
     if (has_gate && lane == 0) drow[E] = has_gate == 2 ? 1.f : 1.f / (1.f + expf(-zr[E]));
 }
@@ -140,16 +154,24 @@ moe_router_kernel(const bf16* h, long long ldh, const bf16* __restrict__ w, int 
     __shared__ float part[ROUTER_WARPS][TOK][ROWS];
     __shared__ float z[TOK][ROWS];
     __shared__ unsigned kept_runs[TOK][32];
-    pdl_launch_dependents();
-    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.x * TOK;
+    // a lane's first columns of all rows, which no kernel writes, are asked for before the wait
+    constexpr bool AHEAD = ROWS <= 16 && TOK == 1;
+    const int first = (warp * 32 + lane) * 8;
+    uint4 ahead[AHEAD ? ROWS : 1];
+    if (AHEAD) {
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) ahead[AHEAD ? r : 0] = r < R && first < D ? *reinterpret_cast<const uint4*>(w + (size_t)r * D + first) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    pdl_launch_dependents();
+    pdl_wait();
     float acc[TOK][ROWS];
 #pragma unroll
     for (int i = 0; i < TOK; i++)
 #pragma unroll
         for (int r = 0; r < ROWS; r++) acc[i][r] = 0.f;
-    for (int c = (warp * 32 + lane) * 8; c < D; c += ROUTER_WARPS * 256) {
+    for (int c = first; c < D; c += ROUTER_WARPS * 256) {
         float x[TOK][8];
 #pragma unroll
         for (int i = 0; i < TOK; i++) {
@@ -162,7 +184,7 @@ moe_router_kernel(const bf16* h, long long ldh, const bf16* __restrict__ w, int 
 #pragma unroll
         for (int r = 0; r < ROWS; r++) {
             if (r >= R) break;
-            const uint4 v = *reinterpret_cast<const uint4*>(w + (size_t)r * D + c);
+            const uint4 v = AHEAD && c == first ? ahead[AHEAD ? r : 0] : *reinterpret_cast<const uint4*>(w + (size_t)r * D + c);
             const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
             for (int j = 0; j < 4; j++) {

@@ -46,21 +46,16 @@ moe_up_stream_kernel(bf16* a, const bf16* h, const bf16* __restrict__ w, const f
     __shared__ float red[WARPS][ROWS][8 * NT + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int col0 = blockIdx.x * 8, grp = group_of(col0, E, ff);
-    pdl_wait();                                   // the routing comes from the kernel before
-    float mine = 0.f;
-    if (lane < M && grp < W) mine = dense[(size_t)lane * W + grp];
-    if (!__any_sync(0xffffffffu, mine != 0.f)) { pdl_launch_dependents(); return; }      // every warp alike
+    // The shared expert's columns come first: every token uses them, so that their first weights are asked for while the kernel
+    // before this one still routes.
+    const int col0 = (gridDim.x - 1 - blockIdx.x) * 8, grp = group_of(col0, E, ff);
     const bf16* w0 = w + (size_t)(col0 + g) * D;
     const bf16* w1 = w0 + (size_t)F * D;
     const int n_chunks = (D + CHUNK - 1) / CHUNK, per = (n_chunks + WARPS - 1) / WARPS;
     const int c_begin = warp * per, c_end = min(n_chunks, c_begin + per);
-    float acc[NT][4];
-#pragma unroll
-    for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    uint4 wa[UNROLL][2], wb[UNROLL][2];
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    for (int c = c_begin; c < c_end; c += UNROLL) {
-        uint4 wa[UNROLL][2], wb[UNROLL][2];
+    auto weights = [&](int c) {
 #pragma unroll
         for (int u = 0; u < UNROLL; u++)
 #pragma unroll
@@ -70,6 +65,18 @@ moe_up_stream_kernel(bf16* a, const bf16* h, const bf16* __restrict__ w, const f
                 wa[u][hh] = kv ? ld_weight(w0 + k8) : zero;
                 wb[u][hh] = kv ? ld_weight(w1 + k8) : zero;
             }
+    };
+    const bool shared = grp >= E;
+    if (shared) weights(c_begin);
+    pdl_wait();                                   // the routing comes from the kernel before
+    float mine = 0.f;
+    if (lane < M && grp < W) mine = dense[(size_t)lane * W + grp];
+    if (!__any_sync(0xffffffffu, mine != 0.f)) { pdl_launch_dependents(); return; }      // every warp alike
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    for (int c = c_begin; c < c_end; c += UNROLL) {
+        if (!shared || c > c_begin) weights(c);
         __syncwarp();                             // all loads are asked for before the first is used
 #pragma unroll
         for (int u = 0; u < UNROLL; u++)
