@@ -131,6 +131,12 @@ moe_down_stream_kernel(float* out, const bf16* a, const bf16* __restrict__ w, co
     const bf16* w1 = w + (size_t)(rv1 ? row0 + g + 8 : 0) * F;
     const int n_chunks = (F + CHUNK - 1) / CHUNK;
     const bool whole = ff % CHUNK == 0;               // a chunk belongs to one group
+    // the shared expert's columns count whatever is chosen: into the L2 while the kernel before this one drains
+    if (W > E)
+        for (int c = E * ff / CHUNK + warp * 2 + (lane >> 4); c < n_chunks; c += 2 * WARPS) {
+            const int row = row0 + (lane & 15);
+            if (row < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (size_t)row * F + c * CHUNK));
+        }
     pdl_wait();
     if (threadIdx.x <= E) used[threadIdx.x] = 0;
     __syncthreads();
