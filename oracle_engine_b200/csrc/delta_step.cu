@@ -44,6 +44,15 @@ delta_step_kernel(bf16* y, float* state, float* conv_state, const float* proj, i
     if (tid % 32 == 0)
         for (int c = tid; c < channels; c += THREADS)
             for (int j = 0; j < taps - 1; j++) prefetch_l2(kept + (size_t)j * C + channel(c));
+    // what no kernel writes: read before the wait, since it has left the L2 since the step before
+    float tap[MAX_CHANNELS][MAX_KEPT + 1];
+#pragma unroll
+    for (int e = 0; e < MAX_CHANNELS; e++) {
+        const int c = tid + e * THREADS;
+#pragma unroll
+        for (int j = 0; j <= MAX_KEPT; j++) tap[e][j] = c < channels && j < taps ? conv_w[(size_t)channel(c) * taps + j] : 0.f;
+    }
+    const float a_log = A_log[h], dt = dt_bias[h], out_w = tid < dv ? norm_w[tid] : 0.f;
     pdl_wait();
     pdl_launch_dependents();
     float4 s[MAX_ROWS];
@@ -61,7 +70,7 @@ delta_step_kernel(bf16* y, float* state, float* conv_state, const float* proj, i
     }
     const float* row = proj + (size_t)t * P;
     const float beta = 1.f / (1.f + expf(-row[C + H * dv + h]));
-    const float decay = expf(-expf(A_log[h]) * softplus_f(row[C + H * dv + H + h] + dt_bias[h]));
+    const float decay = expf(-expf(a_log) * softplus_f(row[C + H * dv + H + h] + dt));
     const float gate = tid < dv ? row[C + (size_t)h * dv + tid] : 0.f;
     float now[MAX_CHANNELS];
 #pragma unroll
@@ -72,8 +81,11 @@ delta_step_kernel(bf16* y, float* state, float* conv_state, const float* proj, i
         now[e] = row[ch];
         float acc = 0.f;
 #pragma unroll
-        for (int j = 0; j < MAX_KEPT; j++) if (j < taps - 1) acc = fmaf(conv_w[(size_t)ch * taps + j], old[e][j], acc);
-        vec[c] = silu_f(fmaf(conv_w[(size_t)ch * taps + taps - 1], now[e], acc));
+        for (int j = 0; j < MAX_KEPT; j++) if (j < taps - 1) acc = fmaf(tap[e][j], old[e][j], acc);
+        float last = 0.f;
+#pragma unroll
+        for (int j = 0; j <= MAX_KEPT; j++) last = j == taps - 1 ? tap[e][j] : last;
+        vec[c] = silu_f(fmaf(last, now[e], acc));
     }
     // every CTA of the cluster has read the kept rows of q and k
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -120,7 +132,7 @@ delta_step_kernel(bf16* y, float* state, float* conv_state, const float* proj, i
     if (tid < dv) for (int q = 0; q < groups; q++) out += part[q * dv + tid];
     const float ss = block_sum(out * out, red);
     const float scale = 1.f / sqrtf(ss / (float)dv + eps);
-    if (tid < dv) y[((size_t)t * H + h) * dv + tid] = __float2bfloat16_rn(out * scale * norm_w[tid] * silu_f(gate));
+    if (tid < dv) y[((size_t)t * H + h) * dv + tid] = __float2bfloat16_rn(out * scale * out_w * silu_f(gate));
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 #pragma unroll
     for (int e = 0; e < MAX_CHANNELS; e++) {

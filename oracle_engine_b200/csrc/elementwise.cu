@@ -67,12 +67,17 @@ __global__ void __launch_bounds__(NT)
 rmsnorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, int D, float eps) {
     __shared__ float red[32];
     constexpr int KEEP = 4;
+    const float4* wr = (const float4*)w;
+    const int n4 = D / 4;
+    // A decode step's norm is a chain of round trips: the gains, which no kernel writes and which have left the L2 since the step
+    // before, are asked for before the wait and not behind the sum (8 sequences of 512 tokens, 57 norms a step: 1.623 -> 1.612 ms).
     pdl_launch_dependents();
+    float4 gain[KEEP];
+#pragma unroll
+    for (int j = 0; j < KEEP; j++) gain[j] = (int)threadIdx.x + j * NT < n4 ? wr[threadIdx.x + j * NT] : make_float4(0.f, 0.f, 0.f, 0.f);
     pdl_wait();
     const float4* xr = (const float4*)(x + (size_t)blockIdx.x * D);
-    const float4* wr = (const float4*)w;
     T* yr = y + (size_t)blockIdx.x * D;
-    const int n4 = D / 4;
     float4 keep[KEEP];
     float ss = 0.f;
 #pragma unroll
@@ -91,7 +96,7 @@ rmsnorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, int D, flo
     for (int j = 0; j < KEEP; j++) {
         const int i = threadIdx.x + j * NT;
         if (i < n4) {
-            const float4 g = wr[i];
+            const float4 g = gain[j];
             Out4<T>::store(yr + 4 * i, (keep[j].x * s) * g.x, (keep[j].y * s) * g.y, (keep[j].z * s) * g.z, (keep[j].w * s) * g.w);
         }
     }
@@ -185,12 +190,19 @@ __global__ void __launch_bounds__(NT)
 layernorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, const float* __restrict__ b, int D, float eps) {
     __shared__ float red[32];
     constexpr int KEEP = 4;
+    const float4 *wr = (const float4*)w, *br = (const float4*)b;
+    const int n4 = D / 4;
     pdl_launch_dependents();
+    float4 gain[KEEP], shift[KEEP];                    // as in rmsnorm_vec_kernel
+#pragma unroll
+    for (int j = 0; j < KEEP; j++) {
+        const int i = threadIdx.x + j * NT;
+        gain[j] = shift[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n4) { gain[j] = wr[i]; shift[j] = br[i]; }
+    }
     pdl_wait();
     const float4* xr = (const float4*)(x + (size_t)blockIdx.x * D);
-    const float4 *wr = (const float4*)w, *br = (const float4*)b;
     T* yr = y + (size_t)blockIdx.x * D;
-    const int n4 = D / 4;
     float4 keep[KEEP];
     float sum = 0.f, sq = 0.f;
 #pragma unroll
@@ -209,7 +221,7 @@ layernorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, const fl
 #pragma unroll
     for (int j = 0; j < KEEP; j++) {
         const int i = threadIdx.x + j * NT;
-        if (i < n4) layernorm_store(yr + 4 * i, keep[j], mean, s, wr[i], br[i]);
+        if (i < n4) layernorm_store(yr + 4 * i, keep[j], mean, s, gain[j], shift[j]);
     }
     for (int i = threadIdx.x + KEEP * NT; i < n4; i += NT) layernorm_store(yr + 4 * i, xr[i], mean, s, wr[i], br[i]);
 }

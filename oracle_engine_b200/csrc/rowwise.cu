@@ -38,20 +38,27 @@ rmsnorm_add_kernel(float* dst, const float* y, const float* __restrict__ w, int 
                    int accumulate, bf16* cast_out) {
     __shared__ float red[32];
     constexpr int KEEP = 4;
-    pdl_launch_dependents();
-    pdl_wait();
     const float* yr = y + (size_t)blockIdx.x * D;
     float* dr = dst + (size_t)blockIdx.x * D;
     bf16* cr = cast_out ? cast_out + (size_t)blockIdx.x * D : nullptr;
     const bool vec = (D % 4 == 0) && D <= KEEP * 4 * 256 && !(((uintptr_t)y | (uintptr_t)dst | (uintptr_t)w) & 15);
+    // the gains, which no kernel writes, are asked for before the wait, and the stream with the row: a decode step's norm is a
+    // chain of round trips
+    pdl_launch_dependents();
+    float4 gain[KEEP];
+#pragma unroll
+    for (int j = 0; j < KEEP; j++)
+        gain[j] = vec && (int)threadIdx.x + j * 256 < D / 4 ? reinterpret_cast<const float4*>(w)[threadIdx.x + j * 256] : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
     if (vec) {
         const int n4 = D / 4;
-        float4 keep[KEEP];
+        float4 keep[KEEP], old[KEEP];
         float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < KEEP; j++) {
             const int i = threadIdx.x + j * 256;
             keep[j] = i < n4 ? reinterpret_cast<const float4*>(yr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            old[j] = i < n4 && accumulate ? reinterpret_cast<const float4*>(dr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
             ss += keep[j].x * keep[j].x + keep[j].y * keep[j].y + keep[j].z * keep[j].z + keep[j].w * keep[j].w;
         }
         ss = block_sum(ss, red);
@@ -60,8 +67,8 @@ rmsnorm_add_kernel(float* dst, const float* y, const float* __restrict__ w, int 
         for (int j = 0; j < KEEP; j++) {
             const int i = threadIdx.x + j * 256;
             if (i < n4) {
-                const float4 g = reinterpret_cast<const float4*>(w)[i];
-                float4 d = accumulate ? reinterpret_cast<float4*>(dr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 g = gain[j];
+                float4 d = old[j];
                 d.x += coef * ((keep[j].x * s) * g.x); d.y += coef * ((keep[j].y * s) * g.y);
                 d.z += coef * ((keep[j].z * s) * g.z); d.w += coef * ((keep[j].w * s) * g.w);
                 reinterpret_cast<float4*>(dr)[i] = d;
@@ -101,8 +108,6 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
                    float coef, float alpha, const float* __restrict__ w, int D, float eps, bf16* cast_out) {
     __shared__ float red[64], red2[32];
     constexpr int KEEP = 4;
-    pdl_launch_dependents();
-    pdl_wait();
     float* xr = x + (size_t)blockIdx.x * D;
     const float* ar = y0 + (size_t)blockIdx.x * D;
     const float* br = w0 ? y1 + (size_t)blockIdx.x * D : ar;
@@ -110,6 +115,18 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
     const bool vec = (D % 4 == 0) && D <= KEEP * 4 * 256 &&
                      !(((uintptr_t)x | (uintptr_t)y0 | (uintptr_t)y1 | (uintptr_t)w | (uintptr_t)w0 | (uintptr_t)w1) & 15) &&
                      !((uintptr_t)cast_out & 7);
+    // the gains before the wait, as in rmsnorm_add_kernel
+    pdl_launch_dependents();
+    float4 gain[KEEP], gain0[KEEP], gain1[KEEP];
+#pragma unroll
+    for (int j = 0; j < KEEP; j++) {
+        const int i = threadIdx.x + j * 256;
+        gain[j] = gain0[j] = gain1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!vec || i >= D / 4) continue;
+        gain[j] = reinterpret_cast<const float4*>(w)[i];
+        if (w0) { gain0[j] = reinterpret_cast<const float4*>(w0)[i]; gain1[j] = reinterpret_cast<const float4*>(w1)[i]; }
+    }
+    pdl_wait();
     if (vec) {
         const int n4 = D / 4;
         float4 v[KEEP], a[KEEP], b[KEEP];
@@ -134,7 +151,7 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
             for (int j = 0; j < KEEP; j++) {
                 const int i = threadIdx.x + j * 256;
                 if (i >= n4) continue;
-                const float4 p = reinterpret_cast<const float4*>(w0)[i], q = reinterpret_cast<const float4*>(w1)[i];
+                const float4 p = gain0[j], q = gain1[j];
                 a[j].x = coef * (a[j].x * na * p.x + b[j].x * nb * q.x); a[j].y = coef * (a[j].y * na * p.y + b[j].y * nb * q.y);
                 a[j].z = coef * (a[j].z * na * p.z + b[j].z * nb * q.z); a[j].w = coef * (a[j].w * na * p.w + b[j].w * nb * q.w);
             }
@@ -151,7 +168,7 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
         for (int j = 0; j < KEEP; j++) {
             const int i = threadIdx.x + j * 256;
             if (i >= n4) continue;
-            const float4 g = reinterpret_cast<const float4*>(w)[i];
+            const float4 g = gain[j];
             const float4 d = make_float4(v[j].x * s * g.x, v[j].y * s * g.y, v[j].z * s * g.z, v[j].w * s * g.w);
             reinterpret_cast<float4*>(xr)[i] = d;
             if (cr) {
@@ -218,19 +235,45 @@ __device__ __forceinline__ float act_gate(float g, int act) {
 }
 
 // One warp per (token, head).  wmode 0: no weight, 1: w[dv] shared by the heads, 2: w[H * dv].
+constexpr int KEPT = 8;             // values of a head that a lane keeps
 template <typename TI, typename T>
 __global__ void __launch_bounds__(128)
 head_gate_kernel(T* out, const TI* o, long long o_stride, const TI* gate, long long g_stride,
                  const float* __restrict__ w, int n_tokens, int H, int dv, int norm, int wmode, int act, float eps) {
     pdl_launch_dependents();
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= (long long)n_tokens * H) return;
+    if (item >= (long long)n_tokens * H) { pdl_wait(); return; }
     const int t = (int)(item / H), h = (int)(item % H);
     const TI* orow = o + (size_t)t * o_stride + (size_t)h * dv;
     const TI* grow = gate + (size_t)t * g_stride + (size_t)h * dv;
     T* dst = out + ((size_t)t * H + h) * dv;
+    if (dv <= 32 * KEPT) {
+        // heads of up to 256: all loads at once, the weights' before the wait
+        float wv[KEPT], ov[KEPT], gv[KEPT];
+#pragma unroll
+        for (int i = 0; i < KEPT; i++) {
+            const int d = lane + 32 * i;
+            wv[i] = d >= dv || wmode == 0 ? 1.f : w[wmode == 1 ? (size_t)d : (size_t)h * dv + d];
+        }
+        pdl_wait();
+        float s = 1.f, ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < KEPT; i++) {
+            const int d = lane + 32 * i;
+            ov[i] = d < dv ? to_f32(orow[d]) : 0.f;
+            gv[i] = d < dv ? to_f32(grow[d]) : 0.f;
+            ss = fmaf(ov[i], ov[i], ss);
+        }
+        if (norm) s = 1.f / sqrtf(warp_sum(ss) / (float)dv + eps);
+#pragma unroll
+        for (int i = 0; i < KEPT; i++) {
+            const int d = lane + 32 * i;
+            if (d < dv) dst[d] = from_f32<T>(ov[i] * s * wv[i] * act_gate(gv[i], act));
+        }
+        return;
+    }
+    pdl_wait();
     float s = 1.f;
     if (norm) {
         float ss = 0.f;
@@ -355,10 +398,14 @@ scaled_add_norm_kernel(bf16* out, float* dst, const float* y0, const float* y1, 
                        float c1, const float* __restrict__ w, int D, float eps) {
     __shared__ float red[32];
     constexpr int KEEP = 4;
-    pdl_launch_dependents();
-    pdl_wait();
     const size_t row = (size_t)blockIdx.x * D;
     const int n4 = D / 4;
+    pdl_launch_dependents();
+    float4 gain[KEEP];                                // before the wait, as in rmsnorm_add_kernel
+#pragma unroll
+    for (int j = 0; j < KEEP; j++)
+        gain[j] = (int)threadIdx.x + j * 256 < n4 ? reinterpret_cast<const float4*>(w)[threadIdx.x + j * 256] : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
     float4 x[KEEP];
     float ss = 0.f;
 #pragma unroll
@@ -387,7 +434,7 @@ scaled_add_norm_kernel(bf16* out, float* dst, const float* y0, const float* y1, 
     for (int j = 0; j < KEEP; j++) {
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
-        const float4 g = reinterpret_cast<const float4*>(w)[i];
+        const float4 g = gain[j];
         const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[j].x * s * g.x, x[j].y * s * g.y), __floats2bfloat162_rn(x[j].z * s * g.z, x[j].w * s * g.w)};
         reinterpret_cast<uint2*>(out + row)[i] = *reinterpret_cast<const uint2*>(h);
     }
