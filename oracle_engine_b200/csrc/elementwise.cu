@@ -62,19 +62,21 @@ template <> struct Out4<bf16> {
     }
 };
 
-template <typename T, int NT>
+constexpr int FEW_ROWS = 256;         // up to here (a decode step) a row's round trips are the time, beyond it the registers count
+template <typename T, int NT, bool FEW>
 __global__ void __launch_bounds__(NT)
 rmsnorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, int D, float eps) {
     __shared__ float red[32];
     constexpr int KEEP = 4;
     const float4* wr = (const float4*)w;
     const int n4 = D / 4;
-    // A decode step's norm is a chain of round trips: the gains, which no kernel writes and which have left the L2 since the step
+    // A decode step's norm (FEW rows) is a chain of round trips: the gains, which no kernel writes and which have left the L2 since the step
     // before, are asked for before the wait and not behind the sum (8 sequences of 512 tokens, 57 norms a step: 1.623 -> 1.612 ms).
     pdl_launch_dependents();
-    float4 gain[KEEP];
+    float4 gain[FEW ? KEEP : 1];
+    if (FEW)
 #pragma unroll
-    for (int j = 0; j < KEEP; j++) gain[j] = (int)threadIdx.x + j * NT < n4 ? wr[threadIdx.x + j * NT] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < KEEP; j++) gain[FEW ? j : 0] = (int)threadIdx.x + j * NT < n4 ? wr[threadIdx.x + j * NT] : make_float4(0.f, 0.f, 0.f, 0.f);
     pdl_wait();
     const float4* xr = (const float4*)(x + (size_t)blockIdx.x * D);
     T* yr = y + (size_t)blockIdx.x * D;
@@ -96,7 +98,7 @@ rmsnorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, int D, flo
     for (int j = 0; j < KEEP; j++) {
         const int i = threadIdx.x + j * NT;
         if (i < n4) {
-            const float4 g = gain[j];
+            const float4 g = FEW ? gain[FEW ? j : 0] : wr[i];
             Out4<T>::store(yr + 4 * i, (keep[j].x * s) * g.x, (keep[j].y * s) * g.y, (keep[j].z * s) * g.z, (keep[j].w * s) * g.w);
         }
     }
@@ -185,7 +187,7 @@ __device__ __forceinline__ void layernorm_store(T* p, const float4& v, float mea
 }
 
 // A block per row, 16-byte pieces, up to 16 NT columns of the row in registers: both passes read them there.
-template <typename T, int NT>
+template <typename T, int NT, bool FEW>
 __global__ void __launch_bounds__(NT)
 layernorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, const float* __restrict__ b, int D, float eps) {
     __shared__ float red[32];
@@ -193,9 +195,11 @@ layernorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, const fl
     const float4 *wr = (const float4*)w, *br = (const float4*)b;
     const int n4 = D / 4;
     pdl_launch_dependents();
-    float4 gain[KEEP], shift[KEEP];                    // as in rmsnorm_vec_kernel
+    constexpr int HELD = FEW ? KEEP : 1;
+    float4 gain[HELD], shift[HELD];                    // as in rmsnorm_vec_kernel
+    if (FEW)
 #pragma unroll
-    for (int j = 0; j < KEEP; j++) {
+    for (int j = 0; j < HELD; j++) {
         const int i = threadIdx.x + j * NT;
         gain[j] = shift[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < n4) { gain[j] = wr[i]; shift[j] = br[i]; }
@@ -221,7 +225,7 @@ layernorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, const fl
 #pragma unroll
     for (int j = 0; j < KEEP; j++) {
         const int i = threadIdx.x + j * NT;
-        if (i < n4) layernorm_store(yr + 4 * i, keep[j], mean, s, gain[j], shift[j]);
+        if (i < n4) layernorm_store(yr + 4 * i, keep[j], mean, s, FEW ? gain[FEW ? j : 0] : wr[i], FEW ? shift[FEW ? j : 0] : br[i]);
     }
     for (int i = threadIdx.x + KEEP * NT; i < n4; i += NT) layernorm_store(yr + 4 * i, xr[i], mean, s, wr[i], br[i]);
 }
@@ -567,7 +571,7 @@ int oe_embed_gather_bf16(float* x, const bf16* table, const int* ids, int n_toke
 int oe_rmsnorm_f32(float* y, const float* x, const float* w, int rows, int D, float eps, cudaStream_t st) {
     if (rows <= 0) return 0;
     if (D % 4 == 0 && !(((uintptr_t)y | (uintptr_t)x | (uintptr_t)w) & 15))
-        return oe_launch(rmsnorm_vec_kernel<float, 256>, dim3(rows), dim3(256), 0, st, y, x, w, D, eps);
+        return oe_launch(rows <= FEW_ROWS ? rmsnorm_vec_kernel<float, 256, true> : rmsnorm_vec_kernel<float, 256, false>, dim3(rows), dim3(256), 0, st, y, x, w, D, eps);
     const int launch_rc = oe_launch(rmsnorm_kernel<float>, dim3(rows), dim3(256), 0, st, y, x, w, D, eps);
     return launch_rc;
 }
@@ -582,7 +586,7 @@ int oe_rmsnorm_bf16(bf16* y, const float* x, const float* w, int rows, int D, fl
             return oe_launch(rmsnorm_rows_kernel<bf16, 32>, grid, dim3(256), 0, st, y, x, w, rows, D, eps);
         }
         // 512 threads a row: inside the 28-layer decode step 1.4 % faster than 256 at 8 sequences (128: 4 % slower)
-        return oe_launch(rmsnorm_vec_kernel<bf16, 512>, dim3(rows), dim3(512), 0, st, y, x, w, D, eps);
+        return oe_launch(rows <= FEW_ROWS ? rmsnorm_vec_kernel<bf16, 512, true> : rmsnorm_vec_kernel<bf16, 512, false>, dim3(rows), dim3(512), 0, st, y, x, w, D, eps);
     }
     const int launch_rc = oe_launch(rmsnorm_kernel<bf16>, dim3(rows), dim3(256), 0, st, y, x, w, D, eps);
     return launch_rc;
@@ -591,7 +595,7 @@ int oe_rmsnorm_bf16(bf16* y, const float* x, const float* w, int rows, int D, fl
 int oe_layernorm_f32(float* y, const float* x, const float* w, const float* b, int rows, int D, float eps, cudaStream_t st) {
     if (rows <= 0) return 0;
     if (D % 4 == 0 && !(((uintptr_t)y | (uintptr_t)x | (uintptr_t)w | (uintptr_t)b) & 15))
-        return oe_launch(layernorm_vec_kernel<float, 256>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
+        return oe_launch(rows <= FEW_ROWS ? layernorm_vec_kernel<float, 256, true> : layernorm_vec_kernel<float, 256, false>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
     return oe_launch(layernorm_kernel<float>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
 }
 int oe_layernorm_bf16(bf16* y, const float* x, const float* w, const float* b, int rows, int D, float eps, cudaStream_t st) {
@@ -604,7 +608,7 @@ int oe_layernorm_bf16(bf16* y, const float* x, const float* w, const float* b, i
             if (D <= 3072) return oe_launch(layernorm_rows_kernel<bf16, 24>, grid, dim3(256), 0, st, y, x, w, b, rows, D, eps);
             return oe_launch(layernorm_rows_kernel<bf16, 32>, grid, dim3(256), 0, st, y, x, w, b, rows, D, eps);
         }
-        return oe_launch(layernorm_vec_kernel<bf16, 512>, dim3(rows), dim3(512), 0, st, y, x, w, b, D, eps);
+        return oe_launch(rows <= FEW_ROWS ? layernorm_vec_kernel<bf16, 512, true> : layernorm_vec_kernel<bf16, 512, false>, dim3(rows), dim3(512), 0, st, y, x, w, b, D, eps);
     }
     return oe_launch(layernorm_kernel<bf16>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
 }

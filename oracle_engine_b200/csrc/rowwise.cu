@@ -23,6 +23,8 @@
 
 namespace {
 
+constexpr int FEW_ROWS = 256;       // up to here (a decode step) a row's round trips are the time, beyond it the registers count
+
 template <typename T>
 __global__ void cast_rows_kernel(T* y, const float* x, size_t total) {
     pdl_launch_dependents();
@@ -33,6 +35,7 @@ __global__ void cast_rows_kernel(T* y, const float* x, size_t total) {
 
 // One block per row; up to 4,096 columns a thread keeps its part of the row in registers (float4 pieces).
 // accumulate == 0: dst is written, not read.  cast_out: null, or [rows, D] bfloat16 that receives the new dst.
+template <bool FEW>
 __global__ void __launch_bounds__(256)
 rmsnorm_add_kernel(float* dst, const float* y, const float* __restrict__ w, int D, float eps, float coef,
                    int accumulate, bf16* cast_out) {
@@ -42,23 +45,25 @@ rmsnorm_add_kernel(float* dst, const float* y, const float* __restrict__ w, int 
     float* dr = dst + (size_t)blockIdx.x * D;
     bf16* cr = cast_out ? cast_out + (size_t)blockIdx.x * D : nullptr;
     const bool vec = (D % 4 == 0) && D <= KEEP * 4 * 256 && !(((uintptr_t)y | (uintptr_t)dst | (uintptr_t)w) & 15);
-    // the gains, which no kernel writes, are asked for before the wait, and the stream with the row: a decode step's norm is a
-    // chain of round trips
+    // FEW rows (a decode step): the gains, which no kernel writes, are asked for before the wait, and the stream with the row,
+    // since the norm is a chain of round trips.  Many rows hide those behind one another and want the registers (3,925 rows of
+    // 2,048 by rmsnorm_sum_kernel: 22.0 us, 32.8 with all gains in registers).
     pdl_launch_dependents();
-    float4 gain[KEEP];
+    float4 gain[FEW ? KEEP : 1];
+    if (FEW)
 #pragma unroll
     for (int j = 0; j < KEEP; j++)
-        gain[j] = vec && (int)threadIdx.x + j * 256 < D / 4 ? reinterpret_cast<const float4*>(w)[threadIdx.x + j * 256] : make_float4(0.f, 0.f, 0.f, 0.f);
+        gain[FEW ? j : 0] = vec && (int)threadIdx.x + j * 256 < D / 4 ? reinterpret_cast<const float4*>(w)[threadIdx.x + j * 256] : make_float4(0.f, 0.f, 0.f, 0.f);
     pdl_wait();
     if (vec) {
         const int n4 = D / 4;
-        float4 keep[KEEP], old[KEEP];
+        float4 keep[KEEP], old[FEW ? KEEP : 1];
         float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < KEEP; j++) {
             const int i = threadIdx.x + j * 256;
             keep[j] = i < n4 ? reinterpret_cast<const float4*>(yr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-            old[j] = i < n4 && accumulate ? reinterpret_cast<const float4*>(dr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (FEW) old[FEW ? j : 0] = i < n4 && accumulate ? reinterpret_cast<const float4*>(dr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
             ss += keep[j].x * keep[j].x + keep[j].y * keep[j].y + keep[j].z * keep[j].z + keep[j].w * keep[j].w;
         }
         ss = block_sum(ss, red);
@@ -67,8 +72,8 @@ rmsnorm_add_kernel(float* dst, const float* y, const float* __restrict__ w, int 
         for (int j = 0; j < KEEP; j++) {
             const int i = threadIdx.x + j * 256;
             if (i < n4) {
-                const float4 g = gain[j];
-                float4 d = old[j];
+                const float4 g = FEW ? gain[FEW ? j : 0] : reinterpret_cast<const float4*>(w)[i];
+                float4 d = FEW ? old[FEW ? j : 0] : accumulate ? reinterpret_cast<float4*>(dr)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
                 d.x += coef * ((keep[j].x * s) * g.x); d.y += coef * ((keep[j].y * s) * g.y);
                 d.z += coef * ((keep[j].z * s) * g.z); d.w += coef * ((keep[j].w * s) * g.w);
                 reinterpret_cast<float4*>(dr)[i] = d;
@@ -103,6 +108,7 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
 }
 
 // One block per row, in registers up to 4,096 columns.  w0 null: v = alpha x + y0 (y1 and w1 are not read).
+template <bool FEW>
 __global__ void __launch_bounds__(256)
 rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, const float* y1, const float* __restrict__ w1,
                    float coef, float alpha, const float* __restrict__ w, int D, float eps, bf16* cast_out) {
@@ -115,11 +121,13 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
     const bool vec = (D % 4 == 0) && D <= KEEP * 4 * 256 &&
                      !(((uintptr_t)x | (uintptr_t)y0 | (uintptr_t)y1 | (uintptr_t)w | (uintptr_t)w0 | (uintptr_t)w1) & 15) &&
                      !((uintptr_t)cast_out & 7);
-    // the gains before the wait, as in rmsnorm_add_kernel
+    // FEW: the gains before the wait, as in rmsnorm_add_kernel
     pdl_launch_dependents();
-    float4 gain[KEEP], gain0[KEEP], gain1[KEEP];
+    constexpr int HELD = FEW ? KEEP : 1;
+    float4 gain[HELD], gain0[HELD], gain1[HELD];
+    if (FEW)
 #pragma unroll
-    for (int j = 0; j < KEEP; j++) {
+    for (int j = 0; j < HELD; j++) {
         const int i = threadIdx.x + j * 256;
         gain[j] = gain0[j] = gain1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (!vec || i >= D / 4) continue;
@@ -151,7 +159,7 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
             for (int j = 0; j < KEEP; j++) {
                 const int i = threadIdx.x + j * 256;
                 if (i >= n4) continue;
-                const float4 p = gain0[j], q = gain1[j];
+                const float4 p = FEW ? gain0[FEW ? j : 0] : reinterpret_cast<const float4*>(w0)[i], q = FEW ? gain1[FEW ? j : 0] : reinterpret_cast<const float4*>(w1)[i];
                 a[j].x = coef * (a[j].x * na * p.x + b[j].x * nb * q.x); a[j].y = coef * (a[j].y * na * p.y + b[j].y * nb * q.y);
                 a[j].z = coef * (a[j].z * na * p.z + b[j].z * nb * q.z); a[j].w = coef * (a[j].w * na * p.w + b[j].w * nb * q.w);
             }
@@ -168,7 +176,7 @@ rmsnorm_sum_kernel(float* x, const float* y0, const float* __restrict__ w0, cons
         for (int j = 0; j < KEEP; j++) {
             const int i = threadIdx.x + j * 256;
             if (i >= n4) continue;
-            const float4 g = gain[j];
+            const float4 g = FEW ? gain[FEW ? j : 0] : reinterpret_cast<const float4*>(w)[i];
             const float4 d = make_float4(v[j].x * s * g.x, v[j].y * s * g.y, v[j].z * s * g.z, v[j].w * s * g.w);
             reinterpret_cast<float4*>(xr)[i] = d;
             if (cr) {
@@ -393,6 +401,7 @@ int rot_norm_launch(T* qk, long long row_stride, const float* inv_freq, int rot_
 // dst += mult * vec * (c0 y0 + c1 y1) and y = norm(dst) * w in one pass over the stream, a block a row (D a multiple of 4 up
 // to 4,096, kept in registers): the norm that reads what a sublayer's output was just added to.  Bound by the bytes: 1,500
 // rows of 2,048, two outputs, 15 us as two launches of which the second reads the stream again.
+template <bool FEW>
 __global__ void __launch_bounds__(256)
 scaled_add_norm_kernel(bf16* out, float* dst, const float* y0, const float* y1, const float* __restrict__ vec, float mult, float c0,
                        float c1, const float* __restrict__ w, int D, float eps) {
@@ -401,10 +410,11 @@ scaled_add_norm_kernel(bf16* out, float* dst, const float* y0, const float* y1, 
     const size_t row = (size_t)blockIdx.x * D;
     const int n4 = D / 4;
     pdl_launch_dependents();
-    float4 gain[KEEP];                                // before the wait, as in rmsnorm_add_kernel
+    float4 gain[FEW ? KEEP : 1];                      // before the wait, as in rmsnorm_add_kernel
+    if (FEW)
 #pragma unroll
     for (int j = 0; j < KEEP; j++)
-        gain[j] = (int)threadIdx.x + j * 256 < n4 ? reinterpret_cast<const float4*>(w)[threadIdx.x + j * 256] : make_float4(0.f, 0.f, 0.f, 0.f);
+        gain[FEW ? j : 0] = (int)threadIdx.x + j * 256 < n4 ? reinterpret_cast<const float4*>(w)[threadIdx.x + j * 256] : make_float4(0.f, 0.f, 0.f, 0.f);
     pdl_wait();
     float4 x[KEEP];
     float ss = 0.f;
@@ -434,7 +444,7 @@ scaled_add_norm_kernel(bf16* out, float* dst, const float* y0, const float* y1, 
     for (int j = 0; j < KEEP; j++) {
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
-        const float4 g = gain[j];
+        const float4 g = FEW ? gain[FEW ? j : 0] : reinterpret_cast<const float4*>(w)[i];
         const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[j].x * s * g.x, x[j].y * s * g.y), __floats2bfloat162_rn(x[j].z * s * g.z, x[j].w * s * g.w)};
         reinterpret_cast<uint2*>(out + row)[i] = *reinterpret_cast<const uint2*>(h);
     }
@@ -496,7 +506,7 @@ int oe_scaled_add_norm(bf16* out, float* dst, const float* y0, const float* y1, 
     if (rows <= 0) return 0;
     if (D < 4 || D % 4 || D > 4096) return OE_ERR_UNSUPPORTED;
     if ((((uintptr_t)dst | (uintptr_t)y0 | (uintptr_t)y1 | (uintptr_t)vec | (uintptr_t)w) & 15) || ((uintptr_t)out & 7)) return OE_ERR_UNSUPPORTED;
-    return oe_launch(scaled_add_norm_kernel, dim3(rows), dim3(256), 0, st, out, dst, y0, y1, vec, mult, c0, c1, w, D, eps);
+    return oe_launch(rows <= FEW_ROWS ? scaled_add_norm_kernel<true> : scaled_add_norm_kernel<false>, dim3(rows), dim3(256), 0, st, out, dst, y0, y1, vec, mult, c0, c1, w, D, eps);
 }
 
 int oe_cast_rows_bf16(bf16* y, const float* x, long long total, cudaStream_t st) {
@@ -507,14 +517,14 @@ int oe_cast_rows_bf16(bf16* y, const float* x, long long total, cudaStream_t st)
 int oe_rmsnorm_add(float* dst, const float* y, const float* w, int rows, int D, float eps, float coef, int accumulate,
                    bf16* cast_out, cudaStream_t st) {
     if (rows <= 0) return 0;
-    return oe_launch(rmsnorm_add_kernel, dim3(rows), dim3(256), 0, st, dst, y, w, D, eps, coef, accumulate, cast_out);
+    return oe_launch(rows <= FEW_ROWS ? rmsnorm_add_kernel<true> : rmsnorm_add_kernel<false>, dim3(rows), dim3(256), 0, st, dst, y, w, D, eps, coef, accumulate, cast_out);
 }
 
 int oe_rmsnorm_sum(float* x, const float* y0, const float* w0, const float* y1, const float* w1, float coef, float alpha,
                    const float* w, int rows, int D, float eps, bf16* cast_out, cudaStream_t st) {
     if (rows <= 0) return 0;
     if (D < 1 || (w0 != nullptr && (y1 == nullptr || w1 == nullptr))) return OE_ERR_UNSUPPORTED;
-    return oe_launch(rmsnorm_sum_kernel, dim3(rows), dim3(256), 0, st, x, y0, w0, y1, w1, coef, alpha, w, D, eps, cast_out);
+    return oe_launch(rows <= FEW_ROWS ? rmsnorm_sum_kernel<true> : rmsnorm_sum_kernel<false>, dim3(rows), dim3(256), 0, st, x, y0, w0, y1, w1, coef, alpha, w, D, eps, cast_out);
 }
 
 int oe_relu2_f32(float* a, long long total, cudaStream_t st) {
