@@ -4,7 +4,7 @@
 //   o_t = (r_t P_0t)^T S0 + sum_(s<t) (r_t P_st . k_s) v_s + (r_t u . k_t) v_t,   S = P_0(n+1) S0 + sum_s (P_s(n+1) k_s) v_s^T,
 // all decays as products, never as quotients: a channel may forget everything within a chunk.
 //
-// Token by token the chain of dependent steps is the time: 1,111 tokens, 32 heads of 64 x 64, 379 us there, 227 us here (6 us a
+// Token by token the chain of dependent steps is the time: 1,111 tokens, 32 heads of 64 x 64, 379 us there, 150 us here (3 us a
 // chunk, still a chain); 8 heads of 128 x 128 553 and 157 us.  Errors against 64 bits as the walk's (5.2e-7 both).  Here
 // decay_chunk_prepare_kernel makes a chunk's decayed vectors and its 32 x 32 scores for all chunks and heads side by side, and
 // decay_chunk_scan_kernel carries 16 columns of a head's state, in registers, from chunk to chunk.
@@ -118,22 +118,30 @@ decay_chunk_scan_kernel(float* o, float* state, const float* blocks, const int* 
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         const float *Kd = st, *Qd = Kd + CH * D, *V = Qd + CH * D, *M = V + CH * COLS, *Wd = M + CH * CH;
-        // Qd S0: this thread's rows, then the warp's two row groups, then the warps
-#pragma unroll 4
-        for (int t = 0; t < CH; t++) {
-            float q = 0.f;
+        // Qd S0: this thread's rows, then the warp's two row groups, then the warps (eight rows' loads before the first store into
+        // `part`: the compiler moves none across one)
+        constexpr int AT_ONCE = 8;
+#pragma unroll 1
+        for (int t0 = 0; t0 < CH; t0 += AT_ONCE) {
+            float q[AT_ONCE];
 #pragma unroll
-            for (int r = 0; r < ROWS; r += 4) {
-                const float4 c = *(const float4*)(Qd + t * D + rg * ROWS + r);
-                q = fmaf(c.w, s[r + 3], fmaf(c.z, s[r + 2], fmaf(c.y, s[r + 1], fmaf(c.x, s[r], q))));
+            for (int t = 0; t < AT_ONCE; t++) {
+                q[t] = 0.f;
+#pragma unroll
+                for (int r = 0; r < ROWS; r += 4) {
+                    const float4 c = *(const float4*)(Qd + (t0 + t) * D + rg * ROWS + r);
+                    q[t] = fmaf(c.w, s[r + 3], fmaf(c.z, s[r + 2], fmaf(c.y, s[r + 1], fmaf(c.x, s[r], q[t]))));
+                }
             }
-            q += __shfl_xor_sync(0xffffffffu, q, 16);
-            if (lane < 16) part[(warp * CH + t) * COLS + lane] = q;
+#pragma unroll
+            for (int t = 0; t < AT_ONCE; t++) q[t] += __shfl_xor_sync(0xffffffffu, q[t], 16);
+#pragma unroll
+            for (int t = 0; t < AT_ONCE; t++) if (lane < 16) part[(warp * CH + t0 + t) * COLS + lane] = q[t];
         }
         // the state at the chunk's end does not wait for the outputs
 #pragma unroll
         for (int r = 0; r < ROWS; r++) s[r] *= Wd[rg * ROWS + r];
-#pragma unroll 4
+#pragma unroll 8
         for (int t = 0; t < CH; t++) {
             const float v = V[t * COLS + j];
 #pragma unroll

@@ -127,18 +127,22 @@ delta_chunk_solve_kernel(float* blocks, const float* qkv, const float* gb, const
     if (tid == 0) oM[CH * CH] = Gs[n - 1];
 }
 
-// grid (H * dv / 16, sequences).  Thread (rg, j): rows rg ROWS .. of column j.  What a chunk's block holds comes by
-// asynchronous copies while the chunk before it is worked on.
-template <int ROWS>
-__global__ void __launch_bounds__(COLS * GROUPS)
+// grid (H * dv / 16, sequences), DK threads.  A thread has four rows of four columns of the state: a row of W, Qg or Kd is read
+// from shared memory once for four columns, and eight rows are asked for before the first sum is stored (with eight rows of one
+// column a thread, and every row's loads behind the store before it, a chunk took 5.4 us; now 4.1).  What a chunk's block holds
+// comes by asynchronous copies while the chunk before it is worked on.
+template <int DK>
+__global__ void __launch_bounds__(DK)
 delta_chunk_scan_kernel(float* o, float* state, const float* blocks, const int* __restrict__ seq_slot, const int* __restrict__ cu_q, int H, int dv) {
-    constexpr int DK = ROWS * GROUPS, WARPS = COLS * GROUPS / 32;
-    constexpr int STAGE = CH * 3 * DK + CH * COLS + CH * CH + 4;
+    constexpr int WARPS = DK / 32;
+    constexpr int MROW = CH + 4;                       // rows of M in a stage: eight lanes of eight rows meet in no bank
+    constexpr int STAGE = CH * 3 * DK + CH * COLS + CH * MROW + 4;
     extern __shared__ __align__(16) float smem[];
-    float* part = smem + 2 * STAGE;                    // [WARPS][2 CH][COLS]
+    float* part = smem + 2 * STAGE;                    // [WARPS][CH][2][COLS]
     float* U = part + WARPS * 2 * CH * COLS;           // [CH][COLS]
     const int tiles = dv / COLS, h = blockIdx.x / tiles, col0 = blockIdx.x % tiles * COLS, b = blockIdx.y;
-    const int tid = threadIdx.x, j = tid % COLS, rg = tid / COLS, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cg = lane & 3, rg = warp * 8 + (lane >> 2);        // columns 4 cg .., rows 4 rg ..
     int first = 0;
     for (int q = 0; q < b; q++) first += chunks_of(cu_q, seq_slot, q);
     const int chunks = chunks_of(cu_q, seq_slot, b), slot = seq_slot[b];
@@ -146,19 +150,22 @@ delta_chunk_scan_kernel(float* o, float* state, const float* blocks, const int* 
     pdl_launch_dependents();
     if (chunks == 0) return;
     const int row0 = cu_q[b], n_all = cu_q[b + 1] - row0;
-    float* S = state + ((size_t)slot * H + h) * DK * dv + col0 + j;
-    float s[ROWS];
+    float* S = state + ((size_t)slot * H + h) * DK * dv + (size_t)4 * rg * dv + col0 + 4 * cg;
+    float s[4][4];                                     // [row][column]
 #pragma unroll
-    for (int r = 0; r < ROWS; r++) s[r] = S[(size_t)(rg * ROWS + r) * dv];
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) s[r][c] = S[(size_t)r * dv + c];
     auto load = [&](int chunk, float* st) {
         const float* src = blocks + ((size_t)(first + chunk) * H + h) * block_floats(DK, dv);
-        for (int e = tid; e < CH * 3 * DK / 4; e += COLS * GROUPS) cp_async16(st + 4 * e, src + 4 * e);
+#pragma unroll 8
+        for (int e = tid; e < CH * 3 * DK / 4; e += DK) cp_async16(st + 4 * e, src + 4 * e);
         float* d = st + CH * 3 * DK;
         const float* uv = src + CH * 3 * DK + col0;
-        for (int e = tid; e < CH * COLS / 4; e += COLS * GROUPS) cp_async16(d + 4 * e, uv + (size_t)(e / (COLS / 4)) * dv + e % (COLS / 4) * 4);
+        for (int e = tid; e < CH * COLS / 4; e += DK) cp_async16(d + 4 * e, uv + (size_t)(e / (COLS / 4)) * dv + e % (COLS / 4) * 4);
         d += CH * COLS;
         const float* m = src + CH * (3 * DK + dv);
-        for (int e = tid; e < CH * CH / 4 + 1; e += COLS * GROUPS) cp_async16(d + 4 * e, m + 4 * e);
+        for (int e = tid; e < CH * CH / 4 + 1; e += DK) cp_async16(d + e / (CH / 4) * MROW + e % (CH / 4) * 4, m + 4 * e);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     load(0, smem);
@@ -168,69 +175,105 @@ delta_chunk_scan_kernel(float* o, float* state, const float* blocks, const int* 
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         const float *W = st, *Kd = W + CH * DK, *Qg = Kd + CH * DK, *Uv = Qg + CH * DK, *M = Uv + CH * COLS;
-        // W S0 and Qg S0: this thread's rows, then the warp's two row groups, then the warps
-#pragma unroll 4
-        for (int i = 0; i < CH; i++) {
-            float w = 0.f, q = 0.f;
+        // W S0 and Qg S0: this thread's rows, then the warp's eight row groups (each exchange halves what a lane carries on: at the
+        // end it has one value, of W for the lower half of the warp, of Qg for the upper), then the warps
+        // (eight rows' loads before the first store into `part`: the compiler moves none across one)
+        const bool up = lane & 16, high = lane & 8, odd = lane & 4;
+        float* own = part + (warp * CH * 2 + (up ? 1 : 0)) * COLS + 4 * cg + (high ? 2 : 0) + (odd ? 1 : 0);
+        constexpr int AT_ONCE = 8;
+#pragma unroll 1
+        for (int i0 = 0; i0 < CH; i0 += AT_ONCE) {
+            float4 a[AT_ONCE], q[AT_ONCE];
+            float y[AT_ONCE][4], sum[AT_ONCE];
 #pragma unroll
-            for (int r = 0; r < ROWS; r += 4) {
-                const float4 a = *(const float4*)(W + i * DK + rg * ROWS + r), c = *(const float4*)(Qg + i * DK + rg * ROWS + r);
-                w = fmaf(a.w, s[r + 3], fmaf(a.z, s[r + 2], fmaf(a.y, s[r + 1], fmaf(a.x, s[r], w))));
-                q = fmaf(c.w, s[r + 3], fmaf(c.z, s[r + 2], fmaf(c.y, s[r + 1], fmaf(c.x, s[r], q))));
+            for (int i = 0; i < AT_ONCE; i++) {
+                a[i] = *(const float4*)(W + (i0 + i) * DK + 4 * rg);
+                q[i] = *(const float4*)(Qg + (i0 + i) * DK + 4 * rg);
             }
-            w += __shfl_xor_sync(0xffffffffu, w, 16);
-            q += __shfl_xor_sync(0xffffffffu, q, 16);
-            if (lane < 16) part[(warp * 2 * CH + i) * COLS + lane] = w;
-            else part[(warp * 2 * CH + CH + i) * COLS + lane - 16] = q;
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; i++) {
+                float x[8];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    x[c] = fmaf(a[i].w, s[3][c], fmaf(a[i].z, s[2][c], fmaf(a[i].y, s[1][c], a[i].x * s[0][c])));
+                    x[4 + c] = fmaf(q[i].w, s[3][c], fmaf(q[i].z, s[2][c], fmaf(q[i].y, s[1][c], q[i].x * s[0][c])));
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) y[i][c] = (up ? x[4 + c] : x[c]) + __shfl_xor_sync(0xffffffffu, up ? x[c] : x[4 + c], 16);
+            }
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; i++) {
+                float z[2];
+#pragma unroll
+                for (int c = 0; c < 2; c++) z[c] = (high ? y[i][2 + c] : y[i][c]) + __shfl_xor_sync(0xffffffffu, high ? y[i][c] : y[i][2 + c], 8);
+                sum[i] = (odd ? z[1] : z[0]) + __shfl_xor_sync(0xffffffffu, odd ? z[0] : z[1], 4);
+            }
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; i++) own[(i0 + i) * 2 * COLS] = sum[i];
         }
         __syncthreads();
-        float qs[CH * COLS / (COLS * GROUPS)];
+        float4 qs[CH * 4 / DK];
 #pragma unroll
-        for (int e = 0; e < CH / GROUPS; e++) {        // (i, j) = (rg + 16 e, j)
-            const int i = rg + GROUPS * e;
-            float w = 0.f, q = 0.f;
+        for (int e = 0; e < CH * 4 / DK; e++) {        // four columns of row i
+            const int at = e * DK + tid, i = at / 4, c = at % 4 * 4;
+            float4 w = make_float4(0.f, 0.f, 0.f, 0.f), q = w;
 #pragma unroll
-            for (int p = 0; p < WARPS; p++) { w += part[(p * 2 * CH + i) * COLS + j]; q += part[(p * 2 * CH + CH + i) * COLS + j]; }
-            U[i * COLS + j] = Uv[i * COLS + j] - w;
+            for (int p = 0; p < WARPS; p++) {
+                const float4 a = *(const float4*)(part + (p * CH + i) * 2 * COLS + c), d = *(const float4*)(part + ((p * CH + i) * 2 + 1) * COLS + c);
+                w.x += a.x; w.y += a.y; w.z += a.z; w.w += a.w;
+                q.x += d.x; q.y += d.y; q.z += d.z; q.w += d.w;
+            }
+            const float4 v = *(const float4*)(Uv + i * COLS + c);
+            *(float4*)(U + i * COLS + c) = make_float4(v.x - w.x, v.y - w.y, v.z - w.z, v.w - w.w);
             qs[e] = q;
         }
         __syncthreads();
-        const float decay = M[CH * CH];
+        const float decay = M[CH * MROW];
 #pragma unroll
-        for (int r = 0; r < ROWS; r++) s[r] *= decay;
-#pragma unroll 4
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) s[r][c] *= decay;
+#pragma unroll 8
         for (int i = 0; i < CH; i++) {
-            const float u = U[i * COLS + j];
+            const float4 u = *(const float4*)(U + i * COLS + 4 * cg), k = *(const float4*)(Kd + i * DK + 4 * rg);
+            const float kr[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
-            for (int r = 0; r < ROWS; r += 4) {
-                const float4 k = *(const float4*)(Kd + i * DK + rg * ROWS + r);
-                s[r] = fmaf(k.x, u, s[r]); s[r + 1] = fmaf(k.y, u, s[r + 1]); s[r + 2] = fmaf(k.z, u, s[r + 2]); s[r + 3] = fmaf(k.w, u, s[r + 3]);
+            for (int r = 0; r < 4; r++) {
+                s[r][0] = fmaf(kr[r], u.x, s[r][0]); s[r][1] = fmaf(kr[r], u.y, s[r][1]);
+                s[r][2] = fmaf(kr[r], u.z, s[r][2]); s[r][3] = fmaf(kr[r], u.w, s[r][3]);
             }
         }
 #pragma unroll
-        for (int e = 0; e < CH / GROUPS; e++) {
-            const int i = rg + GROUPS * e;
-            float a = qs[e];
+        for (int e = 0; e < CH * 4 / DK; e++) {
+            const int at = e * DK + tid, i = at / 4, c = at % 4 * 4, most = (e * DK + (tid | 31)) / 4;       // the warp's last row
+            float4 a = qs[e];
 #pragma unroll 8
-            for (int l = 0; l < CH; l++) {
-                const float m = fmaf(M[i * CH + l], U[l * COLS + j], a);
-                a = l <= i ? m : a;
+            for (int l = 0; l <= most; l++) {          // a later token's value must not touch this one, were it infinite
+                const float m = M[i * MROW + l];
+                const float4 u = *(const float4*)(U + l * COLS + c);
+                const float4 n = make_float4(fmaf(m, u.x, a.x), fmaf(m, u.y, a.y), fmaf(m, u.z, a.z), fmaf(m, u.w, a.w));
+                a = l <= i ? n : a;
             }
             const int t = chunk * CH + i;
-            if (t < n_all) o[(size_t)(row0 + t) * H * dv + (size_t)h * dv + col0 + j] = a;
+            if (t < n_all) {
+                float* to = o + (size_t)(row0 + t) * H * dv + (size_t)h * dv + col0 + c;
+                to[0] = a.x; to[1] = a.y; to[2] = a.z; to[3] = a.w;
+            }
         }
         __syncthreads();                               // the stage, part and U are free
     }
 #pragma unroll
-    for (int r = 0; r < ROWS; r++) S[(size_t)(rg * ROWS + r) * dv] = s[r];
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) S[(size_t)r * dv + c] = s[r][c];
 }
 
-template <int ROWS>
+template <int DK>
 int launch_scan(float* o, float* state, const float* blocks, const int* seq_slot, const int* cu_q, int n_seqs, int H, int dv, cudaStream_t st) {
-    const size_t bytes = (size_t)(2 * (CH * 3 * ROWS * GROUPS + CH * COLS + CH * CH + 4) + COLS * GROUPS / 32 * 2 * CH * COLS + CH * COLS) * 4;
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const size_t bytes = (size_t)(2 * (CH * 3 * DK + CH * COLS + CH * (CH + 4) + 4) + DK / 32 * 2 * CH * COLS + CH * COLS) * 4;
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
-    return oe_launch(delta_chunk_scan_kernel<ROWS>, dim3(H * (dv / COLS), n_seqs), dim3(COLS * GROUPS), bytes, st, o, state, blocks, seq_slot, cu_q, H, dv);
+    return oe_launch(delta_chunk_scan_kernel<DK>, dim3(H * (dv / COLS), n_seqs), dim3(DK), bytes, st, o, state, blocks, seq_slot, cu_q, H, dv);
 }
 
 }  // namespace
@@ -251,8 +294,8 @@ int oe_delta_chunks(float* o, float* state, float* blocks, const float* qkv, con
     if (e != cudaSuccess) return (int)e;
     int rc = oe_launch(delta_chunk_solve_kernel, dim3(n_tokens / CH + n_seqs, H), dim3(256), bytes, st, blocks, qkv, gb, seq_slot, cu_q, n_seqs, G, H, dk, dv);
     if (rc) return rc;
-    if (dk == 64) return launch_scan<4>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, st);
-    return launch_scan<8>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, st);
+    if (dk == 64) return launch_scan<64>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, st);
+    return launch_scan<128>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, st);
 }
 
 }  // extern "C"
