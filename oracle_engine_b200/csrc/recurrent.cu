@@ -39,9 +39,24 @@ __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log
 // block y == 0 also writes the token's decays and step sizes.
 // out_qkv row [q | k | v] (C = 2 G dk + H dv), out_gb row [g: H | beta: H].
 constexpr int VCHUNK = 256;
+// TAPS 0: any number of them.
+template <int TAPS>
 __device__ __forceinline__ float conv_silu(const float* proj, int P, const float* __restrict__ conv_w, int taps,
                                            const float* st, int C, int t, int rel, int c) {
     float acc = 0.f;
+    if (TAPS > 0) {                             // all loads at once: one after another they were the kernel's time
+        float x[TAPS > 0 ? TAPS : 1], w[TAPS > 0 ? TAPS : 1];
+#pragma unroll
+        for (int j = 0; j < TAPS; j++) {
+            const int r = rel - (TAPS - 1) + j;
+            const float* at = r >= 0 ? proj + (size_t)(t - rel + r) * P + c : st + (size_t)(rel + j) * C + c;
+            x[j] = *at;
+            w[j] = conv_w[(size_t)c * TAPS + j];
+        }
+#pragma unroll
+        for (int j = 0; j < TAPS; j++) acc = fmaf(w[j], x[j], acc);
+        return silu_f(acc);
+    }
     for (int j = 0; j < taps; j++) {
         const int r = rel - (taps - 1) + j;
         const float x = r >= 0 ? proj[(size_t)(t - rel + r) * P + c] : st[(size_t)(rel + j) * C + c];
@@ -50,6 +65,7 @@ __device__ __forceinline__ float conv_silu(const float* proj, int P, const float
     return silu_f(acc);
 }
 
+template <int TAPS>
 __global__ void __launch_bounds__(128)
 short_conv_prepare_kernel(float* out_qkv, float* out_gb, const float* proj, int P,
                           const float* __restrict__ conv_w, int taps, const float* conv_state,
@@ -74,7 +90,7 @@ short_conv_prepare_kernel(float* out_qkv, float* out_gb, const float* proj, int 
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int d = threadIdx.x + e * 128;
-            if (d < dk) { y[e] = conv_silu(proj, P, conv_w, taps, st, C, t, rel, c0 + d); ss = fmaf(y[e], y[e], ss); }
+            if (d < dk) { y[e] = conv_silu<TAPS>(proj, P, conv_w, taps, st, C, t, rel, c0 + d); ss = fmaf(y[e], y[e], ss); }
         }
         ss = block_sum(ss, red);
         const float s = (1.f / sqrtf(ss + 1e-6f)) * (part < G ? q_scale : 1.f);
@@ -86,7 +102,7 @@ short_conv_prepare_kernel(float* out_qkv, float* out_gb, const float* proj, int 
     } else {
         const int c0 = nqk + (part - 2 * G) * VCHUNK;
         for (int c = c0 + threadIdx.x; c < min(c0 + VCHUNK, C); c += 128)
-            out_qkv[(size_t)t * C + c] = conv_silu(proj, P, conv_w, taps, st, C, t, rel, c);
+            out_qkv[(size_t)t * C + c] = conv_silu<TAPS>(proj, P, conv_w, taps, st, C, t, rel, c);
     }
     if (part == 0) {
         const float* row = proj + (size_t)t * P;
@@ -539,7 +555,7 @@ int oe_short_conv_prepare(float* out_qkv, float* out_gb, const float* proj, int 
     if (dk > 256) return OE_ERR_UNSUPPORTED;
     const int parts = 2 * G + (H * dv + VCHUNK - 1) / VCHUNK;
     if (parts > 65535) return OE_ERR_UNSUPPORTED;
-    return oe_launch(short_conv_prepare_kernel, dim3(n_tokens, parts), dim3(128), 0, st, out_qkv, out_gb, proj, P, conv_w, taps,
+    return oe_launch(taps == 4 ? short_conv_prepare_kernel<4> : short_conv_prepare_kernel<0>, dim3(n_tokens, parts), dim3(128), 0, st, out_qkv, out_gb, proj, P, conv_w, taps,
                      conv_state, A_log, dt_bias, tok_seq, seq_slot, cu_q, G, H, dk, dv, q_scale);
 }
 
