@@ -471,11 +471,12 @@ def attention(out, qkv, cache, tables, ctx, n_heads: int, n_kv_heads: int, head_
     if (KNOBS.prompt_kernel == "tcgen05" and head_dim in TCGEN05_ATTENTION_HEAD_DIMS and ctx.max_qlen * group > 64
             and group <= 128 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0):
         # prompts: S and O_blk in tensor memory (csrc/attention_tcgen05.cu)
+        cls = getattr(ctx, "context_class", 0)
         code = _attn_tc5_lib(head_dim).oe_attn_tc_bf16(
             out.data_ptr(), qkv.data_ptr(), qkv.stride(0), cache.data_ptr(), cache.shape[0], tables.data_ptr(),
             tables.shape[1], ctx.cu_q.data_ptr(), ctx.seq_start.data_ptr(), ctx.seq_qlen.data_ptr(), ctx.n_seqs, T,
             ctx.max_qlen, n_heads, n_kv_heads, int(window), float(scale), int(bool(sink)),
-            prompt_cluster(T, ctx.n_seqs, group, n_kv_heads, getattr(ctx, "context_class", 0)), ops._stream())
+            prompt_cluster(T, ctx.n_seqs, group, n_kv_heads, cls) if cls or KNOBS.prompt_cluster else 1, ops._stream())
         ops._check(code, "attention_tcgen05")
         return
     lib = _attn_lib(head_dim)
