@@ -668,8 +668,8 @@ int oe_attn_tc_bf16(bf16* out, const bf16* q, long long q_stride, const bf16* ca
         if (e != cudaSuccess) return (int)e;
         attr_set = true;
     }
-    // A captured step's max_qlen is its padded size and most of a sequence-by-tile grid is empty: where half of it
-    // or more is and all CTAs are resident at once, so that their order matters little, the tiles are listed (4 decoding sequences and 192 tokens at 192 keys, padded to 8
+    // A captured step's max_qlen is its padded size and most of a sequence-by-tile grid is empty: while all CTAs are resident at
+    // once, their order matters little and the tiles are listed (4 decoding sequences and 192 tokens at 192 keys, padded to 8
     // and 256: 12.0 -> 9.8 us; at 1,344 keys 25.6 -> 21.9; 2,048 tokens of one prompt, which do not start at once, 35 against 45)
     static int sms = 0;                                    // (asked once: a step launches this a layer)
     if (sms == 0) {
@@ -679,7 +679,7 @@ int oe_attn_tc_bf16(bf16* out, const bf16* q, long long q_stride, const bf16* ca
         sms = n;
     }
     const long long most = n_tokens / a.tokens_per_tile + n_seqs;
-    a.listed = n_seqs <= 32 && (long long)n_seqs * tiles >= 2 * most && most * KVH * cluster <= 2 * sms ? n_seqs : 0;
+    a.listed = n_seqs <= 32 && most * KVH * cluster <= 2 * sms ? n_seqs : 0;
     const dim3 grid = a.listed ? dim3(KVH * cluster, (unsigned)most, 1) : dim3(KVH * cluster, n_seqs, tiles);
     if (cluster > 1) return oe_launch_cluster(attn_tc_kernel, (unsigned)cluster, grid, dim3(THREADS), smem, st, map_q, map_kv, a);
     return oe_launch(attn_tc_kernel, grid, dim3(THREADS), smem, st, map_q, map_kv, a);
