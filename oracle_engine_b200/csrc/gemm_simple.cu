@@ -40,8 +40,12 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // rl + 8 of one class (A's values, four fifths of what was read from shared memory when a lane had one row, are read once for
 // two); two warps load the weights and one the rows of A, so that the ring runs on from tile to tile.  Rows four words apart
 // from a multiple of 32: no eight lanes meet in a bank.  In the decode step of the 1B shape (3 rows), against a kernel whose
-// warps loaded 128 bytes of every other segment for themselves: 8,192 -> 2,048 43.5 -> 21.5 us (67 MB), 2,048 -> 2,048
-// 9.5 -> 5.2, 2,048 -> 3,072 12.4 -> 10, 2,048 -> 16,384 34.7 -> 32.8 (134 MB).
+// warps loaded 128 bytes of every other segment for themselves: 8,192 -> 2,048 43.5 -> 19.4 us (67 MB), 2,048 -> 2,048
+// 9.5 -> 5.2, 2,048 -> 3,072 12.4 -> 10, 2,048 -> 16,384 34.7 -> 32.8 (134 MB).  Up to 512 k eight lanes of one warp have all there is
+// to add up, and it is still faster than the kernel before, whose sixteen did (K = 64 / 128 / 192 / 512 to 2,048 rows: 1 row 2.5 / 3.8 /
+// 5.0 / 10.8 -> 2.0 / 2.1 / 2.5 / 4.2, 3 rows 2.9 / 4.8 / 6.7 / 16.1 -> 2.5 / 3.3 / 4.1 / 8.1, 16 rows 5.0 / 8.5 / 12.1 / 29.3 -> 3.6 / 4.8 /
+// 7.3 / 14).  Where the ring leaves room for one or two CTAs an SM anyway the registers are theirs: left to itself the compiler
+// took 64 and loaded no value ahead of its use (2 rows of 64 x 2,048 6.7 -> 5.0 us, of 2,048 x 8,192 22 -> 16.3; 8 rows 39 -> 28).
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int RT = 16, RK = 512, RPITCH = RK + 4;    // weight rows of a tile, k of a stage, words between a stage's rows
 
@@ -54,7 +58,7 @@ __device__ __forceinline__ void rows_sync(int id) { asm volatile("barrier.cta.sy
 __device__ __forceinline__ void rows_arrive(int id) { asm volatile("barrier.cta.arrive %0, 160;" ::"r"(id) : "memory"); }
 
 template <int MT, int S, int MODE>
-__global__ void __launch_bounds__(160)
+__global__ void __launch_bounds__(160, MT == 8 && S == 2 ? 0 : 1)
 gemm_rows_kernel(float* C, const float* A, const float* __restrict__ W, int M, int N, int K, long long lda, long long ldc,
                  int tiles_m, int tiles) {
     constexpr int STAGE = RowsShape<MT, S>::STAGE;
@@ -295,6 +299,7 @@ constexpr int WT = 128, WLD = WT;
 struct WideShape {
     static constexpr int STAGE = 2 * TK * WLD;
     static constexpr size_t BYTES = ((size_t)2 * STAGE + 2 * WT * TK + WT * WT) * 4;      // 112 KB: two CTAs an SM, no more
+    static constexpr size_t ALONE = 120 * 1024;                                           // one
 };
 
 __device__ __forceinline__ unsigned long long two(float lo, float hi) {
@@ -597,13 +602,16 @@ int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, l
 }
 
 template <int KG, int MODE>
-int launch_wide(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, cudaStream_t st) {
+int launch_wide(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int sms, cudaStream_t st) {
     if ((KG == 1) != (K <= ONE_CHAIN)) return OE_ERR_UNSUPPORTED;
-    constexpr size_t bytes = WideShape::BYTES;
-    cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<KG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return (int)e;
     const int tiles_m = (M + WT - 1) / WT;
     const long long ctas = (long long)tiles_m * ((N + WT - 1) / WT) * KG;
+    // An SM for each CTA where there are enough: a kernel that starts while the one before it still holds the SMs otherwise gets two
+    // places each on those that are free first, and two CTAs take turns there while other SMs idle (in a row of such products, 1,111 x
+    // 2,048 x 512, 144 CTAs: 97 us, so 58; 130 x 8,192 x 512, 128: 97 and 58).  Clusters of four and eight would not all fit so.
+    const size_t bytes = KG == 1 && ctas <= sms ? WideShape::ALONE : WideShape::BYTES;
+    cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<KG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideShape::ALONE);
+    if (e != cudaSuccess) return (int)e;
     if (tiles_m > 65535 || ctas > 0x7fffffffll) return OE_ERR_UNSUPPORTED;
     if (KG == 1) return oe_launch(gemm_wide_kernel<KG, MODE>, dim3((unsigned)ctas), dim3(256), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m);
     return oe_launch_cluster(gemm_wide_kernel<KG, MODE>, KG, dim3((unsigned)ctas), dim3(256), bytes, st, C, A, W, M, N, K, lda, ldc, tiles_m);
@@ -611,8 +619,31 @@ int launch_wide(float* C, const float* A, const float* W, int M, int N, int K, l
 
 constexpr int ROWS_MAX_M = 32;
 
-// kind: 0 by size, else 1 few rows, 2 tiles of 64, 3 tiles of 128, 4 the general kernel, 5, 6 tiles of 128 whose classes
-// four, eight CTAs share (tests).
+// The kernel for a product (1 few rows, 2 tiles of 64, 3 tiles of 128, 5, 6 tiles of 128 whose classes four, eight CTAs share).
+int f32_kind(int M, int N, int K, int sms) {
+    const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128), t64 = (long long)((M + 63) / 64) * ((N + 63) / 64);
+    // Up to 64 rows a tile of 128 is half empty.  A weight of few rows is streamed (64 x 2,048 x 8,192: 174 us, 191 by tiles of
+    // 128, 297 by tiles of 64; 40 x 3,072 x 3,072: 70, 79, 113; 48 x 2,048 x 2,048: 41, 56, 80); beyond that, while there are two
+    // CTAs an SM for eight shares of every tile, tiles of 128 (64 x 3,072 x 3,072: 137 us streamed by the kernel before, 80, 119); a
+    // weight of more rows has tiles of 64 enough for all SMs (64 x 16,384 x 2,048: 156 us, 197 by tiles of 128; 32 rows 154
+    // streamed, 150).
+    if (M <= ROWS_MAX_M || (M <= 64 && M * t128 <= 1024)) return 1;
+    // A single chain cannot be shared out, and a tile of 128 takes as long for a few columns as for all: small products stream, up to
+    // two tiles of 8 x 16 for each of two CTAs an SM (1,111 x 64 x 64: 6.1 us, 9.9 by tiles of 128; 468 x 64 x 512 16 and 55; 130 x 512 x
+    // 64 6.0 and 9.4; beyond, 1,111 x 128 x 64 10.3 and 9.6, 130 x 2,048 x 64 18 and 9.7)
+    if (K <= ONE_CHAIN) return M > 64 && (long long)((M + 7) / 8) * ((N + 15) / 16) <= 4 * sms ? 1 : 3;
+    if (M <= 64) return 8 * t128 <= 2 * sms ? 6 : 2;
+    // From 65 rows on tiles of 64 are faster only where they are one round of CTAs and eight shares of every tile of 128 are more
+    // (clusters of eight leave a few SMs of each group of them out: up to 8/9 of two CTAs an SM), or two rounds and four shares are
+    // more (192 x 3,072 x 3,072: 113 us, 148 by tiles of 128; 1,111 x 512 x 1,024 40 and 45; 160 x 6,144 x 2,048 149 and 155; else 256 x
+    // 2,048 x 2,048 76 and 57, 300 x 3,072 x 2,048 149 and 127).
+    if ((t64 <= sms && 9 * t128 > 2 * sms) || (t64 <= 2 * sms && 4 * t128 > 2 * sms)) return 2;
+    // eight shares of a tile while four would not fill the SMs (192 x 4,096 x 4,096, 64 tiles: 211 us, 240 with four; 300 rows, 96
+    // tiles: 301 and 301; 468 x 16,384 x 2,048: 769 and 734: a share's adding up costs what it costs)
+    return 4 * t128 <= 2 * sms ? 6 : 5;
+}
+
+// kind: 0 by size, 4 the general kernel, else as f32_kind says (tests).
 template <int MODE>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc, int kind, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
@@ -622,23 +653,13 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, lo
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128);
-    if (kind == 0) {
-        // Up to 64 rows a tile of 128 is half empty.  A weight of few rows is streamed (64 x 2,048 x 8,192: 174 us, 191 by tiles of
-        // 128, 297 by tiles of 64; 40 x 3,072 x 3,072: 70, 79, 113; 48 x 2,048 x 2,048: 41, 56, 80); beyond that, while there are two
-        // CTAs an SM for eight shares of every tile, tiles of 128 (64 x 3,072 x 3,072: 137 us streamed by the kernel before, 80, 119); a
-        // weight of more rows has tiles of 64 enough for all SMs (64 x 16,384 x 2,048: 156 us, 197 by tiles of 128; 32 rows 154
-        // streamed, 150).  From 65 rows on tiles of 128 are faster at every size tried.
-        kind = M <= ROWS_MAX_M || (M <= 64 && M * t128 <= 1024) ? 1 : M > 64 || K <= ONE_CHAIN || 8 * t128 <= 2 * sms ? 3 : 2;
-    }
+    if (kind == 0) kind = f32_kind(M, N, K, sms);
     if (kind == 3) {
-        // eight shares of a tile while four would not fill the SMs (192 x 4,096 x 4,096, 64 tiles: 211 us, 240 with four; 300 rows, 96
-        // tiles: 301 and 301; 468 x 16,384 x 2,048: 769 and 734: a share's adding up costs what it costs)
-        if (K <= ONE_CHAIN) return launch_wide<1, MODE>(C, A, W, M, N, K, lda, ldc, st);
-        kind = 4 * t128 <= 2 * sms ? 6 : 5;
+        if (K <= ONE_CHAIN) return launch_wide<1, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+        kind = 4ll * ((M + 127) / 128) * ((N + 127) / 128) <= 2 * sms ? 6 : 5;
     }
-    if (kind == 5) return launch_wide<4, MODE>(C, A, W, M, N, K, lda, ldc, st);
-    if (kind == 6) return launch_wide<8, MODE>(C, A, W, M, N, K, lda, ldc, st);
+    if (kind == 5) return launch_wide<4, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
+    if (kind == 6) return launch_wide<8, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
     if (kind == 2) return launch_tile<64, 64, 4, MODE>(C, A, W, M, N, K, lda, ldc, st);
     if (M == 1) return launch_rows_for<1, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
     if (M == 2) return launch_rows_for<2, MODE>(C, A, W, M, N, K, lda, ldc, sms, st);
@@ -655,6 +676,8 @@ int oe_gemm_simple_f32(void* C, const float* A, const float* W, int M, int N, in
     if (out_kind == 2) return launch_f32<1>((float*)C, A, W, M, N, K, lda, ldc, 0, st);
     return launch_f32<0>((float*)C, A, W, M, N, K, lda, ldc, 0, st);
 }
+// Which kernel takes a product of aligned operands on a device of `sms` SMs.
+int oe_gemm_simple_f32_kind(int M, int N, int K, int sms) { return f32_kind(M, N, K, sms); }
 // The same through one kernel, whatever the size: they give the same bits.
 int oe_gemm_simple_kind_f32(float* C, const float* A, const float* W, int M, int N, int K, long long lda, long long ldc,
                             int accumulate, int kind, cudaStream_t st) {
