@@ -294,7 +294,7 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
 // The same chain for wide rows (a temperature above zero): a cluster of eight CTAs per row, the row's values in registers
 // (up to 32 a thread) from the first pass to the draw.  What bounds it is the number of exchanges between the CTAs (a cluster
 // barrier and what stands on both sides of it, 1.2 us each), not the row's bytes.
-//   * The usual case, a top-k of at most as many tokens as the cluster has warps (128): the k-th largest of the warps' maxima
+//   * The usual case (BOUND), a top-k of fewer tokens than the cluster has warps (128): the k-th largest of the warps' maxima
 //     is a lower bound of the k-th largest value, and few values are at or above it (about 50 for k = 40 where the order of the
 //     tokens is unrelated to their values).  Those go to the first CTA with the exchange of the softmax's sums, which ends the
 //     row alone by comparing them all with one another: two exchanges in all.  8 rows of 128,256: 34 -> 15 us a launch (12 without the repeat penalty).
@@ -305,7 +305,7 @@ sample_rows_kernel(float* __restrict__ logits, int* __restrict__ out, const int*
 // tokens whatever the number of rows.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int CL = 8, CT = 512, CW = CT / 32;        // CTAs of a cluster, threads and warps of a CTA
-constexpr int SEG = 16, FEW = 1024;                  // values at or above the bound: room for a warp's and for all of them
+constexpr int SEG = 16, FEW = 512;                   // values at or above the bound: room for a warp's and for all of them
 constexpr int KEPT = 1 << 30;                        // marks a kept token's index
 
 struct __align__(16) Sums { float a[4]; unsigned n[4]; };
@@ -382,14 +382,14 @@ __device__ __forceinline__ void record_token(int token, int row, int slot, int d
     }
 }
 
-template <int EPT>
+template <int EPT, bool BOUND>
 __global__ void __launch_bounds__(CT)
 sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float temperature, int top_k, float top_p, float repeat_pen,
                       int repeat_last, SampleState st, int record) {
     __shared__ Sums box[2][CL * CW];
-    __shared__ float2 s_seg[CL * CW][SEG];            // of the first CTA: per warp of the cluster its (value, index) at or above the bound
-    __shared__ float2 s_few[FEW];                     // the same side by side
-    __shared__ int2 s_place[CL * CW];                 // of a warp's values in s_few: the first, how many
+    __shared__ float2 s_seg[BOUND ? CL * CW : 1][SEG];       // of the first CTA: per warp of the cluster its (value, index) at or above the bound
+    __shared__ float2 s_few[BOUND ? FEW : 1];         // the same side by side
+    __shared__ int2 s_place[BOUND ? CL * CW : 1];     // of a warp's values in s_few: the first, how many
     __shared__ unsigned s_hit[CT];
     __shared__ int s_ids[PENALTY_CAP];
     __shared__ float s_part[EPT * CW], s_excl[EPT * CW], s_total[CL];
@@ -462,9 +462,8 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     sums.a[0] = mx;
     mx = cluster_sums<true>(sums, box, turn).a[0];
     // the bound: the top_k-th largest of the warps' maxima.  At least top_k values are at or above it.
-    const bool by_bound = top_k > 0 && top_k < V && top_k <= CL * CW;
     float least = INFINITY;                           // exponentials from here on are marked: a little below the bound's, so
-    if (by_bound) {                                   // that whatever rounds to the bound's probability is among them
+    if (BOUND) {                                      // that whatever rounds to the bound's probability is among them
         const Sums* maxima = box[turn ^ 1];
         if (tid < CL * CW) {
             const float own = maxima[tid].a[0];
@@ -481,10 +480,10 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
 #pragma unroll
     for (int j = 0; j < EPT; j++) {
         v[j] = base + j * CT + tid < V ? expf(v[j] - mx) : 0.f;
-        marked |= v[j] >= least ? 1u << j : 0u;
+        if (BOUND) marked |= v[j] >= least ? 1u << j : 0u;
         sums.a[0] += v[j];
     }
-    if (by_bound) {
+    if (BOUND) {
         const int mine = __popc(marked), all = __reduce_add_sync(0xffffffffu, mine);
         if (all > 0 && all <= SEG) {
             int at = mine;
@@ -509,7 +508,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     const float inv = 1.f / softmax.a[0];
 
     // (a sum that is no number takes the passes, which choose no token)
-    if (by_bound && softmax.n[1] == 0u && softmax.n[0] <= FEW && softmax.a[0] >= 1.f) {
+    if (BOUND && softmax.n[1] == 0u && softmax.n[0] <= FEW && softmax.a[0] >= 1.f) {
         if (rank != 0) return;                        // nothing is written to another CTA any more
         const int n = (int)softmax.n[0];
         // side by side, in the warps' order
@@ -703,11 +702,27 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     if (rank == 0 && tid == 0) record_token(__float_as_int(box[turn][0].a[0]), row, slot, drawn, recorded, out, st, record);
 }
 
+// Whether a row's top-k goes by the bound.  Of W warps that hold values, as many as k have their maximum at or above it where it
+// has W / (W - k + 1) + .. + W / W values at or above it on average, wherever they lie in the row.  Comparing n values with one
+// another takes n^2 / 32 steps, so that beyond some 320 the passes are as fast (8 rows of 128,256: top-k 40 14 us, 104 19, 110 22, by
+// passes 32 to 35; 128, of which 700 values are at or above the bound, 91; 64 of 65,536, 300 values, 30 and 31, 64 rows 67 and 135).  The
+// attempt costs a row that it does not settle 2.6 us (one whose values are all the same, 25 -> 28 us), and the kernel without it is
+// 1 us faster than one that has both.
+bool by_bound(int top_k, int V, int slice) {
+    if (top_k <= 0 || top_k >= V) return false;
+    const int rest = V % slice, warps = V / slice * CW + (rest < CT ? (rest + 31) / 32 : CW);
+    if (top_k > warps) return false;
+    float values = 0.f;
+    for (int i = warps - top_k + 1; i <= warps; i++) values += (float)warps / (float)i;
+    return values <= 320.f;
+}
+
 template <int EPT>
 int launch_cluster(float* logits, int* out, const int* row_slot, int rows, int V, float temperature, int top_k, float top_p,
                    float repeat_pen, int repeat_last, const SampleState& state, int record, cudaStream_t st) {
-    return oe_launch_cluster(sample_cluster_kernel<EPT>, CL, dim3(CL, rows), dim3(CT), 0, st, logits, out, row_slot, V, temperature, top_k, top_p,
-                             repeat_pen, repeat_last, state, record);
+    const auto kernel = by_bound(top_k, V, EPT * CT) ? sample_cluster_kernel<EPT, true> : sample_cluster_kernel<EPT, false>;
+    return oe_launch_cluster(kernel, CL, dim3(CL, rows), dim3(CT), 0, st, logits, out, row_slot, V, temperature, top_k, top_p, repeat_pen,
+                             repeat_last, state, record);
 }
 
 // Row `row` of every tensor of a table of (address, bytes of a row), four bytes at a time.  grid (pieces, tensors)
@@ -770,6 +785,9 @@ int oe_argmax_rows(const float* logits, int* out, int rows, int V, cudaStream_t 
     const int launch_rc = oe_launch(argmax_rows_kernel, dim3(rows), dim3(SAMPLE_THREADS), 0, st, logits, out, V);
     return launch_rc;
 }
+
+// Whether a draw of wide rows looks for a small top-k's values by a bound.
+int oe_sample_by_bound(int top_k, int V) { return by_bound(top_k, V, (V <= CL * CT * 8 ? 8 : 32) * CT) ? 1 : 0; }
 
 int oe_sample_rows(float* logits, int* out, const int* row_slot, int rows, int V, float temperature,
                    int top_k, float top_p, float repeat_pen, int repeat_last, const long long* rng_seed,
