@@ -63,6 +63,9 @@ template <> struct Out4<bf16> {
 };
 
 constexpr int FEW_ROWS = 256;         // up to here (a decode step) a row's round trips are the time, beyond it the registers count
+// The layer norm of 512 threads with gains and shifts in registers (124) has an SM for itself: up to a block an SM, one more and a
+// second round begins (192 and 256 rows of 2,048: 3.1 and 3.3 us so, 2.4 and 2.5 without).
+constexpr int FEW_ROWS_LAYERNORM = 148;
 template <typename T, int NT, bool FEW>
 __global__ void __launch_bounds__(NT)
 rmsnorm_vec_kernel(T* y, const float* x, const float* __restrict__ w, int D, float eps) {
@@ -598,6 +601,8 @@ int oe_layernorm_f32(float* y, const float* x, const float* w, const float* b, i
         return oe_launch(rows <= FEW_ROWS ? layernorm_vec_kernel<float, 256, true> : layernorm_vec_kernel<float, 256, false>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
     return oe_launch(layernorm_kernel<float>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
 }
+// Whether a layer norm of 512 threads keeps gains and shifts in registers.
+int oe_layernorm_bf16_few(int rows) { return rows <= FEW_ROWS_LAYERNORM ? 1 : 0; }
 int oe_layernorm_bf16(bf16* y, const float* x, const float* w, const float* b, int rows, int D, float eps, cudaStream_t st) {
     if (rows <= 0) return 0;
     if (D % 4 == 0 && !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)b) & 15) && !((uintptr_t)y & 7)) {
@@ -608,7 +613,7 @@ int oe_layernorm_bf16(bf16* y, const float* x, const float* w, const float* b, i
             if (D <= 3072) return oe_launch(layernorm_rows_kernel<bf16, 24>, grid, dim3(256), 0, st, y, x, w, b, rows, D, eps);
             return oe_launch(layernorm_rows_kernel<bf16, 32>, grid, dim3(256), 0, st, y, x, w, b, rows, D, eps);
         }
-        return oe_launch(rows <= FEW_ROWS ? layernorm_vec_kernel<bf16, 512, true> : layernorm_vec_kernel<bf16, 512, false>, dim3(rows), dim3(512), 0, st, y, x, w, b, D, eps);
+        return oe_launch(oe_layernorm_bf16_few(rows) ? layernorm_vec_kernel<bf16, 512, true> : layernorm_vec_kernel<bf16, 512, false>, dim3(rows), dim3(512), 0, st, y, x, w, b, D, eps);
     }
     return oe_launch(layernorm_kernel<bf16>, dim3(rows), dim3(256), 0, st, y, x, w, b, D, eps);
 }
