@@ -242,22 +242,22 @@ __device__ __forceinline__ float act_gate(float g, int act) {
     return act == 0 ? sg : g * sg;                 // 0: sigmoid, 1: silu
 }
 
-// One warp per (token, head).  wmode 0: no weight, 1: w[dv] shared by the heads, 2: w[H * dv].
-constexpr int KEPT = 8;             // values of a head that a lane keeps
-template <typename TI, typename T>
+// One warp per (token, head).  wmode 0: no weight, 1: w[dv] shared by the heads, 2: w[H * dv].  KEPT: values of a head that a
+// lane keeps (heads of up to 32 KEPT), all asked for at once, the weights' before the wait; 0: heads of any size.
+template <typename TI, typename T, int KEPT>
 __global__ void __launch_bounds__(128)
 head_gate_kernel(T* out, const TI* o, long long o_stride, const TI* gate, long long g_stride,
                  const float* __restrict__ w, int n_tokens, int H, int dv, int norm, int wmode, int act, float eps) {
     pdl_launch_dependents();
+    if (KEPT == 0) pdl_wait();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= (long long)n_tokens * H) { pdl_wait(); return; }
+    if (item >= (long long)n_tokens * H) { if (KEPT > 0) pdl_wait(); return; }
     const int t = (int)(item / H), h = (int)(item % H);
     const TI* orow = o + (size_t)t * o_stride + (size_t)h * dv;
     const TI* grow = gate + (size_t)t * g_stride + (size_t)h * dv;
     T* dst = out + ((size_t)t * H + h) * dv;
-    if (dv <= 32 * KEPT) {
-        // heads of up to 256: all loads at once, the weights' before the wait
+    if constexpr (KEPT > 0) {
         float wv[KEPT], ov[KEPT], gv[KEPT];
 #pragma unroll
         for (int i = 0; i < KEPT; i++) {
@@ -279,21 +279,20 @@ head_gate_kernel(T* out, const TI* o, long long o_stride, const TI* gate, long l
             const int d = lane + 32 * i;
             if (d < dv) dst[d] = from_f32<T>(ov[i] * s * wv[i] * act_gate(gv[i], act));
         }
-        return;
-    }
-    pdl_wait();
-    float s = 1.f;
-    if (norm) {
-        float ss = 0.f;
-        for (int d = lane; d < dv; d += 32) { const float v = to_f32(orow[d]); ss = fmaf(v, v, ss); }
-        ss = warp_sum(ss);
-        s = 1.f / sqrtf(ss / (float)dv + eps);
-    }
-    for (int d = lane; d < dv; d += 32) {
-        float v = to_f32(orow[d]) * s;
-        if (wmode == 1) v *= w[d];
-        else if (wmode == 2) v *= w[(size_t)h * dv + d];
-        dst[d] = from_f32<T>(v * act_gate(to_f32(grow[d]), act));
+    } else {
+        float s = 1.f;
+        if (norm) {
+            float ss = 0.f;
+            for (int d = lane; d < dv; d += 32) { const float v = to_f32(orow[d]); ss = fmaf(v, v, ss); }
+            ss = warp_sum(ss);
+            s = 1.f / sqrtf(ss / (float)dv + eps);
+        }
+        for (int d = lane; d < dv; d += 32) {
+            float v = to_f32(orow[d]) * s;
+            if (wmode == 1) v *= w[d];
+            else if (wmode == 2) v *= w[(size_t)h * dv + d];
+            dst[d] = from_f32<T>(v * act_gate(to_f32(grow[d]), act));
+        }
     }
 }
 
@@ -380,7 +379,8 @@ int head_gate_launch(T* out, const TI* o, long long o_stride, const TI* gate, lo
     const long long items = (long long)n_tokens * H;
     const long long blocks = (items + 3) / 4;
     if (blocks > 2147483647LL) return OE_ERR_UNSUPPORTED;
-    return oe_launch(head_gate_kernel<TI, T>, dim3((unsigned)blocks), dim3(128), 0, st, out, o, o_stride, gate, g_stride, w,
+    const auto kernel = dv <= 64 ? head_gate_kernel<TI, T, 2> : dv <= 128 ? head_gate_kernel<TI, T, 4> : dv <= 256 ? head_gate_kernel<TI, T, 8> : head_gate_kernel<TI, T, 0>;
+    return oe_launch(kernel, dim3((unsigned)blocks), dim3(128), 0, st, out, o, o_stride, gate, g_stride, w,
                      n_tokens, H, dv, norm, wmode, act, eps);
 }
 
