@@ -39,23 +39,25 @@ __device__ __forceinline__ int group_of(int c, int E, int ff) { const int g = c 
 
 // h [M, D] (rows of lda), w [2 F, D]: F gate rows, then F up rows.  a [M, F] = the unit; columns of experts that no token
 // chose are not written.  F = E ff + shared columns, ff and F multiples of 8.
-template <int NT, int WARPS, int UNROLL>
-__global__ void __launch_bounds__(WARPS * 32)
+// AHEAD: a lane has a round's weights in registers before it uses the first, so that 5 CTAs fill an SM, and the shared expert's
+// columns, which every token uses, come first and are asked for while the kernel before this one still routes.  Otherwise 10 CTAs an
+// SM (8 for 16 tokens), for more columns than that holds at once (ops.moe_up_ahead has both sides' times; as many registers for all
+// sizes cost 8 experts of 1,024 and a shared one of 2,048 for 4 tokens 3 us of 14).  16 tokens, 8 experts of 512: 12.7 us with 56
+// registers, 10.1 with 64 (of 1,024 and 2,048, which 56 hold in one round: 17.9 and 20.2).
+template <int NT, int WARPS, int UNROLL, bool AHEAD>
+__global__ void __launch_bounds__(WARPS * 32, AHEAD ? 5 : NT == 1 ? 10 : 8)
 moe_up_stream_kernel(bf16* a, const bf16* h, const bf16* __restrict__ w, const float* dense, int M, int D, int F, int E, int ff, int W,
                      long long lda, int unit, float limit) {
     __shared__ float red[WARPS][ROWS][8 * NT + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    // The shared expert's columns come first: every token uses them, so that their first weights are asked for while the kernel
-    // before this one still routes.
-    const int col0 = (gridDim.x - 1 - blockIdx.x) * 8, grp = group_of(col0, E, ff);
+    const int col0 = (AHEAD ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * 8, grp = group_of(col0, E, ff);
     const bf16* w0 = w + (size_t)(col0 + g) * D;
     const bf16* w1 = w0 + (size_t)F * D;
     const int n_chunks = (D + CHUNK - 1) / CHUNK, per = (n_chunks + WARPS - 1) / WARPS;
     const int c_begin = warp * per, c_end = min(n_chunks, c_begin + per);
-    uint4 wa[UNROLL][2], wb[UNROLL][2];
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    auto weights = [&](int c) {
+    auto weights = [&](uint4 (&wa)[UNROLL][2], uint4 (&wb)[UNROLL][2], int c) {
 #pragma unroll
         for (int u = 0; u < UNROLL; u++)
 #pragma unroll
@@ -66,8 +68,9 @@ moe_up_stream_kernel(bf16* a, const bf16* h, const bf16* __restrict__ w, const f
                 wb[u][hh] = kv ? ld_weight(w1 + k8) : zero;
             }
     };
-    const bool shared = grp >= E;
-    if (shared) weights(c_begin);
+    const bool shared = AHEAD && grp >= E;
+    uint4 wa0[UNROLL][2], wb0[UNROLL][2];
+    if (shared) weights(wa0, wb0, c_begin);
     pdl_wait();                                   // the routing comes from the kernel before
     float mine = 0.f;
     if (lane < M && grp < W) mine = dense[(size_t)lane * W + grp];
@@ -75,9 +78,7 @@ moe_up_stream_kernel(bf16* a, const bf16* h, const bf16* __restrict__ w, const f
     float acc[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    for (int c = c_begin; c < c_end; c += UNROLL) {
-        if (!shared || c > c_begin) weights(c);
-        __syncwarp();                             // all loads are asked for before the first is used
+    auto products = [&](const uint4 (&wa)[UNROLL][2], const uint4 (&wb)[UNROLL][2], int c) {
 #pragma unroll
         for (int u = 0; u < UNROLL; u++)
 #pragma unroll
@@ -93,6 +94,18 @@ moe_up_stream_kernel(bf16* a, const bf16* h, const bf16* __restrict__ w, const f
                     mma_bf16(acc[n], wa[u][hh].z, wb[u][hh].z, wa[u][hh].w, wb[u][hh].w, x.z, x.w);
                 }
             }
+    };
+    for (int c = c_begin; c < c_end; c += UNROLL) {
+        if constexpr (AHEAD) {
+            if (!shared || c > c_begin) weights(wa0, wb0, c);
+            __syncwarp();                         // all loads are asked for before the first is used
+            products(wa0, wb0, c);
+        } else {
+            uint4 wa[UNROLL][2], wb[UNROLL][2];
+            weights(wa, wb, c);
+            __syncwarp();
+            products(wa, wb, c);
+        }
     }
     pdl_launch_dependents();
 #pragma unroll
@@ -317,13 +330,14 @@ bool unit_ok(int unit, float limit) { return unit >= 0 && unit <= 2 && (unit != 
 
 extern "C" {
 
+// ahead: which of the two kernels (moe_up_stream_kernel says what for); the same bits.
 int oe_moe_up_stream(bf16* a, const bf16* h, const bf16* w, const float* dense, int M, int D, int F, int E, int ff, int W, long long lda,
-                     int unit, float limit, cudaStream_t st) {
+                     int unit, float limit, int ahead, cudaStream_t st) {
     if (M <= 0) return 0;
     if (M > 16 || D % 8 || lda % 8 || ff < 8 || ff % 8 || F % 8 || F < E * ff || E < 1 || E > MAX_GROUPS || W < E || !unit_ok(unit, limit)) return OE_ERR_UNSUPPORTED;
     if (((uintptr_t)h | (uintptr_t)w) & 15) return OE_ERR_UNSUPPORTED;
-    if (M > 8) return oe_launch(moe_up_stream_kernel<2, 4, 4>, dim3(F / 8), dim3(128), 0, st, a, h, w, dense, M, D, F, E, ff, W, lda, unit, limit);
-    return oe_launch(moe_up_stream_kernel<1, 4, 4>, dim3(F / 8), dim3(128), 0, st, a, h, w, dense, M, D, F, E, ff, W, lda, unit, limit);
+    if (M > 8) return oe_launch(moe_up_stream_kernel<2, 4, 4, false>, dim3(F / 8), dim3(128), 0, st, a, h, w, dense, M, D, F, E, ff, W, lda, unit, limit);
+    return oe_launch(ahead ? moe_up_stream_kernel<1, 4, 4, true> : moe_up_stream_kernel<1, 4, 4, false>, dim3(F / 8), dim3(128), 0, st, a, h, w, dense, M, D, F, E, ff, W, lda, unit, limit);
 }
 
 int oe_moe_down_stream(float* out, const bf16* a, const bf16* w, const float* dense, int M, int N, int F, int E, int ff, int W, long long ldc,

@@ -101,7 +101,7 @@ _SIGNATURES = {
         "oe_moe_dense_act": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P],
     },
     "moe_sparse": {
-        "oe_moe_up_stream": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _I, _F, _P],
+        "oe_moe_up_stream": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _I, _F, _I, _P],
         "oe_moe_down_stream": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _I, _P],
         "oe_moe_place": [_P, _I, _I, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P, _P, _P, _I, _P],
         "oe_moe_combine": [_P, _L, _P, _P, _I, _I, _I, _I, _P],
@@ -181,6 +181,18 @@ def _stream() -> int:
     if _raw_stream is not None:
         return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+_sms: dict = {}
+
+
+def sm_count() -> int:
+    """SMs of the current device."""
+    dev = torch.cuda.current_device()
+    n = _sms.get(dev)
+    if n is None:
+        n = _sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+    return n
 
 
 LAUNCHES = [0]          # kernels launched through this module (or captured into a graph)
@@ -1133,16 +1145,28 @@ def _moe_operands(what, h, w, dense, out, n_experts, ff, columns):
         raise KernelError(f"{what}: shapes or types do not agree")
 
 
+def moe_up_ahead(T: int, F: int, n_experts: int, ff: int, top: int, sms: int | None = None) -> bool:
+    """Whether moe_up_stream takes the kernel that keeps a round of weights in registers (5 CTAs of 8 columns an SM; the other
+    has 10): while the columns of as many experts as T tokens with `top` each may choose, and the shared expert's, are all there at
+    once, and the CTAs that only find out that nobody chose their columns are not many rounds.  us in a row of such products,
+    width 2,048, in registers / not: 8 experts of 512 and a shared one, 1 token 6.1 / 9.9, 4 9.9 / 10.6; 8 of 1,024 and 2,048, 1 9.7 / 10.7, 4
+    17.2 / 13.8; 8 of 1,408, 2 10.6 / 10.8, 4 18.9 / 14.1; 32 of 1,024, 1 10.8 / 8.7, 4 16.1 / 14.3.  Above 8 tokens it is never faster."""
+    held = 8 * 5 * (sms or sm_count())
+    return T <= 8 and min(n_experts, T * top) * ff + F - n_experts * ff <= held and F <= 4 * held
+
+
 def moe_up_stream(a: torch.Tensor, h: torch.Tensor, w: torch.Tensor, dense: torch.Tensor, n_experts: int, ff: int,
-                  unit: str = "silu", limit: float = 0.0) -> None:
+                  unit: str = "silu", limit: float = 0.0, top: int = 2) -> None:
     """a [T, F] bfloat16 = the experts' gated units of h [T, D] (T <= 16) times the tokens' weights, of the experts that some
-    token chose (the others' columns are left as they are); w [2 F, D] as moe_dense_act has it: F gate rows, F up rows."""
+    token chose (the others' columns are left as they are); w [2 F, D] as moe_dense_act has it: F gate rows, F up rows.
+    top: how many experts a token has, as far as the choice of the kernel goes (`moe_up_ahead`)."""
     T, F = a.shape
     _moe_operands("moe_up_stream", h, w, dense, a, n_experts, ff, F)
     if tuple(w.shape) != (2 * F, h.shape[1]) or h.shape[0] != T or a.dtype != torch.bfloat16 or not a.is_contiguous():
         raise KernelError("moe_up_stream: a [T, F] contiguous and w [2 F, D] expected")
     _check(_fn("moe_sparse", "oe_moe_up_stream")(_ptr(a), _ptr(h), _ptr(w), _ptr(dense), T, h.shape[1], F, n_experts, ff, dense.shape[1],
-                                                 h.stride(0), _UNITS[unit], float(limit), _stream()), "moe_up_stream", (T, F, h.shape[1]))
+                                                 h.stride(0), _UNITS[unit], float(limit), int(moe_up_ahead(T, F, n_experts, ff, min(top, n_experts))),
+                                                 _stream()), "moe_up_stream", (T, F, h.shape[1]))
 
 
 def moe_down_stream(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, dense: torch.Tensor, n_experts: int, ff: int,

@@ -190,7 +190,7 @@ class MoESwiGLU(Part):
         aligned = h.stride(1) == 1 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
         if self.sparse and aligned and _stream_pays(T, self.top, self.E):
             a = self.rt.buffer("moe.a", T, self.F)
-            ops.moe_up_stream(a, h, self.w_gu, dense, self.E, self.ff, self.unit, self.limit)
+            ops.moe_up_stream(a, h, self.w_gu, dense, self.E, self.ff, self.unit, self.limit, self.top)
             ops.moe_down_stream(residual, a, self.w_down, dense, self.E, self.ff, accumulate=not overwrite)
             return
         if self.sparse and aligned and _sorted_pays(T, self.top, self.E, self.D, self.ff):
