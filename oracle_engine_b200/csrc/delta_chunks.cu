@@ -18,9 +18,12 @@ namespace {
 // What the scan reads of a chunk and head, one block of floats: [W: CH dk | Kd: CH dk | Qg: CH dk | Uv: CH dv | M: CH CH | G: 4].
 __host__ __device__ __forceinline__ size_t block_floats(int dk, int dv) { return (size_t)CH * (3 * dk + dv + CH) + 4; }
 
-// (two blocks an SM: with the 246 registers that the compiler would take, 560 blocks are four rounds: 62 us for 1,111
-// tokens, 48 now)
-__global__ void __launch_bounds__(256, 2)
+// Two blocks an SM where there are more blocks than SMs: with the 246 registers that the compiler would take, 560 blocks are four
+// rounds: 62 us for 1,111 tokens, 48 so, although 240 bytes a thread are then stored to memory and loaded again.  Up to a
+// block an SM that is only lost time (16 heads of 128 x 128, both kernels: 33 tokens 30.5 us, 24.0 with all registers, 200 51.4 and 44.5;
+// 240 blocks 88 and 93).
+template <int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM)
 delta_chunk_solve_kernel(float* blocks, const float* qkv, const float* gb, const int* __restrict__ seq_slot, const int* __restrict__ cu_q,
                          int n_seqs, int G, int H, int dk, int dv) {
     extern __shared__ __align__(16) float smem[];
@@ -270,9 +273,16 @@ delta_chunk_scan_kernel(float* o, float* state, const float* blocks, const int* 
         for (int c = 0; c < 4; c++) S[(size_t)r * dv + c] = s[r][c];
 }
 
+constexpr size_t SM_SHARED = 227 * 1024;              // what the blocks resident on an SM share, each with 1 KB of the system's on top
+
 template <int DK>
-int launch_scan(float* o, float* state, const float* blocks, const int* seq_slot, const int* cu_q, int n_seqs, int H, int dv, cudaStream_t st) {
-    const size_t bytes = (size_t)(2 * (CH * 3 * DK + CH * COLS + CH * (CH + 4) + 4) + DK / 32 * 2 * CH * COLS + CH * COLS) * 4;
+int launch_scan(float* o, float* state, const float* blocks, const int* seq_slot, const int* cu_q, int n_seqs, int H, int dv, int sms, cudaStream_t st) {
+    size_t bytes = (size_t)(2 * (CH * 3 * DK + CH * COLS + CH * (CH + 4) + 4) + DK / 32 * 2 * CH * COLS + CH * COLS) * 4;
+    // No more blocks an SM than one round of them needs: this kernel starts while the one before it drains, and otherwise gets three
+    // places each on the SMs that are free first while others stay empty (heads of 64: 32 of 64 x 64, 1,111 tokens, both kernels 297 -> 241
+    // us, 4,000 1,091 -> 883; 16 of 64 x 128 249 -> 189).
+    const size_t ctas = (size_t)H * (dv / COLS) * n_seqs, share = SM_SHARED / ((ctas + sms - 1) / sms);
+    if (share > bytes + 1024) bytes = (share - 1024) / 16 * 16;
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
     return oe_launch(delta_chunk_scan_kernel<DK>, dim3(H * (dv / COLS), n_seqs), dim3(DK), bytes, st, o, state, blocks, seq_slot, cu_q, H, dv);
@@ -291,13 +301,18 @@ int oe_delta_chunks(float* o, float* state, float* blocks, const float* qkv, con
                     int n_seqs, int G, int H, int dk, int dv, cudaStream_t st) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (!oe_delta_chunks_supported(G, H, dk, dv) || n_seqs > 65535 || H > 65535 || (((uintptr_t)qkv | (uintptr_t)blocks) & 15)) return OE_ERR_UNSUPPORTED;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const dim3 grid(n_tokens / CH + n_seqs, H);
+    const auto solve = (long long)(n_tokens / CH) * H <= sms ? delta_chunk_solve_kernel<1> : delta_chunk_solve_kernel<2>;
     const size_t bytes = (size_t)2 * CH * (dk + 4) * 4;
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = cudaFuncSetAttribute(solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
-    int rc = oe_launch(delta_chunk_solve_kernel, dim3(n_tokens / CH + n_seqs, H), dim3(256), bytes, st, blocks, qkv, gb, seq_slot, cu_q, n_seqs, G, H, dk, dv);
+    int rc = oe_launch(solve, grid, dim3(256), bytes, st, blocks, qkv, gb, seq_slot, cu_q, n_seqs, G, H, dk, dv);
     if (rc) return rc;
-    if (dk == 64) return launch_scan<64>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, st);
-    return launch_scan<128>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, st);
+    if (dk == 64) return launch_scan<64>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, sms, st);
+    return launch_scan<128>(o, state, blocks, seq_slot, cu_q, n_seqs, H, dv, sms, st);
 }
 
 }  // extern "C"
