@@ -436,16 +436,28 @@ def _decode_ctas_per_sm(head_dim: int) -> int:
     return _state[key]
 
 
-def prompt_cluster(n_tokens: int, n_seqs: int, group: int, n_kv_heads: int, context_class: int, sm_count: int | None = None) -> int:
+CLUSTER_PAGES = 12             # the most pages that a tile may see for one CTA to walk them alone
+
+
+def prompt_cluster(n_tokens: int, n_seqs: int, group: int, n_kv_heads: int, context_class: int, sm_count: int | None = None, window: int = 0) -> int:
     """How many CTAs (a thread-block cluster) share the pages of a tile of the tcgen05 prompt attention: more than one
     where a sequence is longer than 768 tokens and the tiles (at most one more a sequence than the tokens fill) leave SMs idle.
     Adding up costs about 6 us, a page 0.6.  Measured (us; 24 heads over 8 KV heads of 128; 1 / 2 / 4 / 8 CTAs): 64 tokens
-    behind 1,900 26.0 / 20.0 / 17.4 / 14.9; 192 behind 768 beside 4 decoding sequences 15.8 / 15.3 / 21.5 / 34.3, behind 1,344
-    21.9 / 18.0 / 23.2 / 36.0; 500 behind 3,000 49.2 / 37.2 / 45.8 / 57.2; without a long cache 192 behind 192 9.8 / 12.0, a prompt
-    of 500 11.6 / 14.5, of 1,000 18.7 / 28.2."""
+    behind 1,900 26.2 / 20.5 / 16.6 / 15.6; 192 behind 768 beside 4 decoding sequences 15.8 / 15.3 / 21.5 / 34.3, behind 1,344 alone
+    22.5 / 20.1 / 17.8 / 27.7; 500 behind 3,000 48.6 / 37.1 / 46.6 / 56.9; without a long cache 192 behind 192 9.8 / 12.0, a prompt
+    of 500 11.6 / 14.5, of 1,000 18.7 / 28.2.
+
+    window: as attention()'s.  A tile sees the pages of its window and of its own tokens, and of a chunk half on average; up to
+    CLUSTER_PAGES of them one CTA is no slower.  1 / 2 CTAs, 192 tokens behind 1,344: a window of 128 9.1 / 11.8, 256 10.4 / 12.5, 600 14.0 /
+    14.2, 1,024 18.6 / 17.1, chunks of 1,024 11.1 / 13.7 (behind 6,000, further into one, 21.8 / 18.2); 500 behind 3,000: 256 11.9 / 14.7, 600
+    16.2 / 17.2, 1,024 21.7 / 20.9; 32 heads over 8, 192 behind 1,344: 256 10.2 / 12.8, 1,024 19.6 / 18.1; 32 of 64 over 8: 256 7.7 / 10.0,
+    1,024 17.3 / 14.7; 16 over 2: 256 8.6 / 12.1."""
     if KNOBS.prompt_cluster > 0:
         return KNOBS.prompt_cluster
     if context_class < MID_CONTEXT:
+        return 1
+    span = window if window > 0 else -window // 2
+    if span and (span + 128 // group) // ops.PAGE + 1 <= CLUSTER_PAGES:
         return 1
     sms = sm_count or _sm_count()
     tiles = (n_tokens // (128 // group) + n_seqs) * n_kv_heads
@@ -476,7 +488,7 @@ def attention(out, qkv, cache, tables, ctx, n_heads: int, n_kv_heads: int, head_
             out.data_ptr(), qkv.data_ptr(), qkv.stride(0), cache.data_ptr(), cache.shape[0], tables.data_ptr(),
             tables.shape[1], ctx.cu_q.data_ptr(), ctx.seq_start.data_ptr(), ctx.seq_qlen.data_ptr(), ctx.n_seqs, T,
             ctx.max_qlen, n_heads, n_kv_heads, int(window), float(scale), int(bool(sink)),
-            prompt_cluster(T, ctx.n_seqs, group, n_kv_heads, cls) if cls or KNOBS.prompt_cluster else 1, ops._stream())
+            prompt_cluster(T, ctx.n_seqs, group, n_kv_heads, cls, window=int(window)) if cls or KNOBS.prompt_cluster else 1, ops._stream())
         ops._check(code, "attention_tcgen05")
         return
     lib = _attn_lib(head_dim)
