@@ -1026,6 +1026,12 @@ int oe_attn_decode_warps_bf16(bf16* out, const bf16* qkv, long long qkv_stride, 
     return oe_launch(f.kernel, dim3(1, KVH, n_seqs), dim3(f.threads), f.smem, st, a);
 }
 
+// How many CTAs of a form an SM holds, or -1.
+int oe_attn_decode_warps_per_sm(int shape) {
+    const WarpsForm f = warps_form(shape);
+    int n = 0;
+    return f.rc == 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f.kernel, f.threads, f.smem) == cudaSuccess ? n : -1;
+}
 // Registers a thread of a form takes, or -1.  (A CTA of 6 x 2 has 46,080 of an SM's 65,536 at head size 128: the products beside it
 // get what is left.  The places in a page are taken from unsigned numbers: from signed ones the form took 250 registers, not 236, and a
 // walk over 8,000 keys at head size 64 50.4 us, not 43.6.)

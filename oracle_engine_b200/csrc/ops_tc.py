@@ -539,9 +539,20 @@ def decode_uses_warps(n_seqs: int, context_class: int, head_dim: int, n_heads: i
 
 
 def decode_warps_per_sm(shape: tuple, head_dim: int) -> int:
-    """How many CTAs of a form of the warps kernel an SM holds (0: the form does not fit)."""
+    """How many CTAs of a form of the warps kernel an SM holds (0: the form does not fit): by its shared memory, and, where there
+    is a device to ask, by its registers (heads of 32: 2 x 3 has shared memory for 7 CTAs and registers for 5, 1 x 3 14 and 10)."""
     smem = shape[0] * shape[1] * 2 * 32 * (head_dim * 2 + 16)      # K and V tiles of 32 padded rows
-    return 0 if smem > 220 * 1024 else SM_SHARED_BYTES // (smem + 1024)
+    if smem > 220 * 1024:
+        return 0
+    if not torch.cuda.is_available():
+        return SM_SHARED_BYTES // (smem + 1024)
+    key = ("decode_warps_per_sm", head_dim, shape)
+    if key not in _state:
+        n = int(_attn_lib(head_dim).oe_attn_decode_warps_per_sm(shape[0] * 16 + shape[1]))
+        if n < 0:
+            raise KernelError(f"attention_decode_warps: no count of CTAs for the form {shape} at head size {head_dim}")
+        _state[key] = n
+    return _state[key]
 
 
 def decode_warps_shape(n_seqs: int, context_class: int, head_dim: int, n_kv_heads: int,

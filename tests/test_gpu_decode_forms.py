@@ -14,3 +14,16 @@ def test_the_form_of_six_warps_leaves_the_products_their_share():
     regs = _registers(128, (6, 2))
     assert 0 < regs <= 240, regs
     assert _registers(128, (5, 2)) == -1
+
+
+@pytest.mark.parametrize("head_dim", [32, 64, 128])
+def test_the_rule_counts_ctas_that_an_sm_can_hold(head_dim):
+    from oracle_engine_b200.csrc import ops_tc
+    warps = {(6, 2): 6, (2, 3): 4, (1, 3): 2}              # the last two: a pair of warps for each
+    for shape in ops_tc.DECODE_WARPS_FORMS:
+        held = ops_tc.decode_warps_per_sm(shape, head_dim)
+        if held:
+            granules = (_registers(head_dim, shape) + 7) // 8 * 8
+            assert held * warps[shape] * 32 * granules <= 65536, (shape, held, granules)
+    if head_dim == 128:
+        assert [ops_tc.decode_warps_per_sm(f, 128) for f in ops_tc.DECODE_WARPS_FORMS] == [1, 2, 4]
