@@ -619,10 +619,11 @@ int oe_attn_tc_head_dim() { return HD; }
 
 // Prompt attention.  q: rows of q_stride bf16 with head h at h*HD (the fused qkv buffer after
 // rotation); cache: one entry [pages][2][KVH][64][HD]; out [T, H*HD].  Needs 16-byte aligned
-// rows (q_stride a multiple of 8) and G = H/KVH <= 128.  cluster: how many CTAs (1 to 8) share the pages of a tile.
+// rows (q_stride a multiple of 8) and G = H/KVH <= 128.  cluster: how many CTAs (1 to 8) share the pages of a tile;
+// sms: the device's SMs.
 int oe_attn_tc_bf16(bf16* out, const bf16* q, long long q_stride, const bf16* cache, long long n_pages, const int* tables,
                     int max_pages, const int* cu_q, const int* seq_start, const int* seq_qlen, int n_seqs, int n_tokens,
-                    int max_qlen, int H, int KVH, int window, float scale, int sink, int cluster, cudaStream_t st) {
+                    int max_qlen, int H, int KVH, int window, float scale, int sink, int cluster, int sms, cudaStream_t st) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (cluster < 1 || cluster > MAX_CLUSTER) return OE_ERR_UNSUPPORTED;
     if (H % KVH || (q_stride % 8) || ((uintptr_t)q & 15) || ((uintptr_t)cache & 15) || ((uintptr_t)out & 15)) return OE_ERR_UNSUPPORTED;
@@ -671,13 +672,6 @@ int oe_attn_tc_bf16(bf16* out, const bf16* q, long long q_stride, const bf16* ca
     // A captured step's max_qlen is its padded size and most of a sequence-by-tile grid is empty: while all CTAs are resident at
     // once, their order matters little and the tiles are listed (4 decoding sequences and 192 tokens at 192 keys, padded to 8
     // and 256: 12.0 -> 9.8 us; at 1,344 keys 25.6 -> 21.9; 2,048 tokens of one prompt, which do not start at once, 35 against 45)
-    static int sms = 0;                                    // (asked once: a step launches this a layer)
-    if (sms == 0) {
-        int dev = 0, n = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        sms = n;
-    }
     const long long most = n_tokens / a.tokens_per_tile + n_seqs;
     a.listed = n_seqs <= 32 && most * KVH * cluster <= 2 * sms ? n_seqs : 0;
     const dim3 grid = a.listed ? dim3(KVH * cluster, (unsigned)most, 1) : dim3(KVH * cluster, n_seqs, tiles);

@@ -149,7 +149,7 @@ def uses_pair(M: int, N: int, K: int, sm_count: int | None = None) -> bool:
         return False
     if M <= 384 and N >= 256 and K >= 2048:
         tiles = -(-M // 128) * -(-N // 256)              # tiles of 128 x 256 of the one-SM kernel
-        if tiles * 4 <= (sm_count or _sm_count()):       # it splits K over a cluster of 4 to 8 CTAs per tile
+        if tiles * 4 <= (sm_count or ops.sm_count()):       # it splits K over a cluster of 4 to 8 CTAs per tile
             return False
     return True
 
@@ -381,7 +381,7 @@ def _attn_tc5_lib(head_dim: int):
         lib = _build.load("attention_tc5", {"OE_HD": head_dim})
         lib.oe_attn_tc_bf16.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_void_p,
                                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
-                                        c_int, c_void_p]
+                                        c_int, c_int, c_void_p]
         lib.oe_attn_tc_bf16.restype = c_int
         lib.oe_attn_tc_error.argtypes = []
         lib.oe_attn_tc_error.restype = c_int
@@ -459,7 +459,7 @@ def prompt_cluster(n_tokens: int, n_seqs: int, group: int, n_kv_heads: int, cont
     span = window if window > 0 else -window // 2
     if span and (span + 128 // group) // ops.PAGE + 1 <= CLUSTER_PAGES:
         return 1
-    sms = sm_count or _sm_count()
+    sms = sm_count or ops.sm_count()
     tiles = (n_tokens // (128 // group) + n_seqs) * n_kv_heads
     if tiles * 4 <= sms:
         return 8 if tiles * 8 <= sms else 4
@@ -488,7 +488,8 @@ def attention(out, qkv, cache, tables, ctx, n_heads: int, n_kv_heads: int, head_
             out.data_ptr(), qkv.data_ptr(), qkv.stride(0), cache.data_ptr(), cache.shape[0], tables.data_ptr(),
             tables.shape[1], ctx.cu_q.data_ptr(), ctx.seq_start.data_ptr(), ctx.seq_qlen.data_ptr(), ctx.n_seqs, T,
             ctx.max_qlen, n_heads, n_kv_heads, int(window), float(scale), int(bool(sink)),
-            prompt_cluster(T, ctx.n_seqs, group, n_kv_heads, cls, window=int(window)) if cls or KNOBS.prompt_cluster else 1, ops._stream())
+            prompt_cluster(T, ctx.n_seqs, group, n_kv_heads, cls, window=int(window)) if cls or KNOBS.prompt_cluster else 1, ops.sm_count(),
+            ops._stream())
         ops._check(code, "attention_tcgen05")
         return
     lib = _attn_lib(head_dim)
@@ -572,7 +573,7 @@ def decode_warps_shape(n_seqs: int, context_class: int, head_dim: int, n_kv_head
                 96: 139 / 132 / 155,  128: 182 / 174 / 169;   8,000 keys, 64: 314 / 309 / 349."""
     if KNOBS.decode_warps_shape is not None:
         return tuple(KNOBS.decode_warps_shape)
-    sms = sm_count or _sm_count()
+    sms = sm_count or ops.sm_count()
     pairs = max(1, n_seqs * n_kv_heads)
     forms, seen = [], set()
     for shape in DECODE_WARPS_FORMS:                # most warps first; one form for each number of CTAs an SM holds
@@ -618,18 +619,12 @@ def decode_warps_cluster(n_seqs: int, context_class: int, n_kv_heads: int, sm_co
     # about 64 of them on 148 SMs the step loses more than the attention gains (ms a step of the 28-layer
     # model, 1 / 2 / 4 CTAs per pair; 2,048-token contexts: 1 sequence 1.93 / 1.76 / 1.69, 4: 1.98 / 1.85 /
     # 2.62, 8: 2.05 / 2.93 / 3.13; 6,000 tokens: 2: 2.77 / 2.20 / 1.95, 4: 2.82 / 2.27 / 2.93, 8: 2.88 / 3.49 / 3.68).
-    budget = (sm_count or _sm_count()) * 7 // 16
+    budget = (sm_count or ops.sm_count()) * 7 // 16
     pairs = max(1, n_seqs * n_kv_heads)
     for cr in ((8, 4, 2) if context_class >= VERY_LONG_CONTEXT else (4, 2)):
         if pairs * cr <= budget:
             return cr
     return 1
-
-
-def _sm_count() -> int:
-    if "sms" not in _state:
-        _state["sms"] = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-    return _state["sms"]
 
 
 def attention_decode_warps(out, qkv, cos, sin, cache, tables, ctx, n_heads: int, n_kv_heads: int, head_dim: int,
@@ -768,7 +763,7 @@ def attention_split(out, q, kcache, vcache, tables, ctx, n_heads: int, n_kv_head
     n_splits, partial = 1, None
     if ctx.all_decode and ctx.n_tokens == ctx.n_seqs:
         keys = min(abs(window), ctx.max_kvlen) if window else ctx.max_kvlen
-        n_splits = max(1, min(keys // PAGE + 1, (2 * _sm_count()) // max(1, ctx.n_seqs * n_kv_heads), 32))
+        n_splits = max(1, min(keys // PAGE + 1, (2 * ops.sm_count()) // max(1, ctx.n_seqs * n_kv_heads), 32))
         if n_splits > 1:
             partial = torch.empty(ctx.n_seqs * n_heads * n_splits * (dv + 2), dtype=torch.float32, device=out.device)
     code = _attn_split_lib(dk, dv, shared)(out.data_ptr(), q.data_ptr(), q.stride(0), kcache.data_ptr(), vcache.data_ptr(),
