@@ -60,7 +60,7 @@ latent_write_kernel(const TD* d, long long ldd, const float* __restrict__ w, flo
     __shared__ float red[32];
     pdl_launch_dependents();
     const int t = blockIdx.x, parts = gridDim.y, part = blockIdx.y;
-    const int b = tok_seq[t], pos = tok_pos[t];                          // (the step's integers)
+    const int b = tok_seq[t], pos = tok_pos[t];                          // (written before the step's first kernel, as the gains are)
     const int R = r + rd;
     float gain[2] = {0.f, 0.f};                                          // of latents up to 256, before the wait
     if (write_cache && part == 0) {

@@ -637,7 +637,7 @@ attn_decode_warps_kernel(const AttnArgs a) {
             __syncwarp();
         }
 
-        // S = Q K^T for the 16 rows and the tile's 32 keys
+        // S = Q K^T for the 16 rows and the tile's keys
         float sacc[TB / 8][4];
 #pragma unroll
         for (int n = 0; n < TB / 8; n++) { sacc[n][0] = sacc[n][1] = sacc[n][2] = sacc[n][3] = 0.f; }

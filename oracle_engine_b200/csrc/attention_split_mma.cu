@@ -419,7 +419,9 @@ extern "C" {
 
 int oe_attn_split_mma_dims(int* dk, int* dv) { *dk = DK; *dv = DV; return 0; }
 
-// max_qlen: the most tokens any sequence of the step brings (sizes the grid).
+// max_qlen: the most tokens any sequence of the step brings (sizes the grid).  tables, cu_q, seq_start, seq_qlen and the pages wholly
+// before seq_start are read before the kernel waits for the one before it: no kernel that may still run may write them (the engine
+// copies a step's integers to the device before the step's first kernel, and a copy waits for all kernels before it).
 int oe_attn_split_mma(bf16* out, const bf16* q, long long q_stride, const bf16* kcache, const bf16* vcache,
                       const int* tables, int max_pages, const int* cu_q, const int* seq_start, const int* seq_qlen,
                       int n_seqs, int max_qlen, int H, int KVH, int window, float scale, float cap, int n_splits,

@@ -302,7 +302,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const uint32_t tmem_base = *(volatile uint32_t*)&ctl->tmem_base;
 
     pdl_launch_dependents();
-    pdl_wait();                                            // q, the cache and the step's integers come from earlier kernels
+    pdl_wait();                                            // q and the new tokens' rows of the cache come from earlier kernels
 
     const int G = a.H / a.KVH;
     const int start = a.seq_start[b], t0 = q_tile * tpt, nt = min(tpt, qlen - t0);
@@ -620,7 +620,8 @@ int oe_attn_tc_head_dim() { return HD; }
 // Prompt attention.  q: rows of q_stride bf16 with head h at h*HD (the fused qkv buffer after
 // rotation); cache: one entry [pages][2][KVH][64][HD]; out [T, H*HD].  Needs 16-byte aligned
 // rows (q_stride a multiple of 8) and G = H/KVH <= 128.  cluster: how many CTAs (1 to 8) share the pages of a tile;
-// sms: the device's SMs.
+// sms: the device's SMs.  seq_qlen is read before the kernel waits for the one before it: no kernel that may still run may write it
+// (the engine copies a step's integers to the device before the step's first kernel, and a copy waits for all kernels before it).
 int oe_attn_tc_bf16(bf16* out, const bf16* q, long long q_stride, const bf16* cache, long long n_pages, const int* tables,
                     int max_pages, const int* cu_q, const int* seq_start, const int* seq_qlen, int n_seqs, int n_tokens,
                     int max_qlen, int H, int KVH, int window, float scale, int sink, int cluster, int sms, cudaStream_t st) {

@@ -27,7 +27,9 @@ typedef __nv_bfloat16 bf16;
 // A kernel that starts early must read what earlier kernels wrote through the coherent path:
 // pointers to such data are NOT `const __restrict__` (which lets the compiler use the read-only
 // cache, valid only for data that does not change while the kernel is resident); weights and
-// the step's integer tables, written before the step's first kernel, may be.
+// the step's integer tables, written before the step's first kernel, may be.  Those two a kernel may also read before it waits:
+// whoever calls an entry point with weights (gains, taps, router rows) or tables that one of these kernels makes puts something
+// between them that waits, a copy or a kernel of another library.
 // Set OE_PDL=0 in the environment to launch without the attribute.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

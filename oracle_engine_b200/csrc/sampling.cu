@@ -134,7 +134,7 @@ struct SampleState {
     int hist_cap;
 };
 
-constexpr int PENALTY_CAP = 256;                    // the longest history whose tokens fit the shared array of penalise()
+constexpr int PENALTY_CAP = 256;                    // the longest history whose tokens fit the kernels' shared arrays
 
 // The repeat penalty over the last `repeat_last` recorded tokens, for those in [lo, hi), by the whole block: the first of
 // equal tokens is penalised once for each of them.  (One thread going through the history took 1.2 us a token.)
