@@ -1613,7 +1613,8 @@ def sample_rows(logits: torch.Tensor, out: torch.Tensor, row_slot: torch.Tensor,
     i32 = torch.int32
     if not (out.dtype is i32 and row_slot.dtype is i32 and rng_counter.dtype is i32 and out.is_contiguous() and row_slot.is_contiguous()
             and rng_counter.is_contiguous()):
-        raise KernelError("out, row_slot and rng_counter must be contiguous int32 tensors")
+        for t, n in ((out, "out"), (row_slot, "row_slot"), (rng_counter, "rng_counter")):
+            _i32(t, n)
     if rng_seed.dtype is not torch.int64:
         raise KernelError("sample_rows: rng_seed must be int64")
     if logits.dtype is not torch.float32 or not logits.is_contiguous():
@@ -1624,9 +1625,8 @@ def sample_rows(logits: torch.Tensor, out: torch.Tensor, row_slot: torch.Tensor,
         _i32(hist, "hist")
         _i32(hist_count, "hist_count")
         cap, ring, recorded = hist.shape[1], hist.data_ptr(), hist_count.data_ptr()
-    rows, width = logits.shape
     _check(_fn("sampling", "oe_sample_rows")(
-        logits.data_ptr(), out.data_ptr(), row_slot.data_ptr(), rows, width, float(temperature), int(top_k), float(top_p),
+        logits.data_ptr(), out.data_ptr(), row_slot.data_ptr(), logits.shape[0], logits.shape[1], float(temperature), int(top_k), float(top_p),
         float(repeat_penalty), int(repeat_last_n),
         rng_seed.data_ptr(), rng_counter.data_ptr(), ring, recorded, cap, int(record), _stream()), "sample_rows")
 
