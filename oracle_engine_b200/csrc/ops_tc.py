@@ -514,7 +514,7 @@ def decode_fused_supported(head_dim: int, n_heads: int, n_kv_heads: int) -> bool
     return attention_supported(head_dim, n_heads, n_kv_heads) and head_dim % 32 == 0
 
 
-DECODE_WARPS_FORMS = ((6, 2), (2, 3), (1, 3))    # (warps, tiles in a warp's ring) the rule picks from (csrc/attention_mma.cu)
+DECODE_WARPS_FORMS = ((6, 2), (2, 3), (1, 3))    # (warps, or pairs of warps in the last two, tiles in a ring) the rule picks from (csrc/attention_mma.cu)
 SM_SHARED_BYTES = 227 * 1024   # what the CTAs resident on an SM share, each with 1 KB of the system's on top
 
 
@@ -564,13 +564,20 @@ def decode_warps_shape(n_seqs: int, context_class: int, head_dim: int, n_kv_head
     merge hide only behind another CTA of the same SM.  So: the form with the most warps whose
     CTAs are all resident at once (at head size 128 one CTA an SM for up to 148 pairs, then two,
     then four); with more pairs than that, short contexts take the smallest CTAs.  Long contexts
-    leave the one-warp form out (a lone warp's arithmetic shows there) and, past one round, take
-    the form whose last round of CTAs is fullest.  Measured before a pair of warps shared each tile of the last two (us; 24
-    heads over 8 KV heads of 128; 6x2 / 2x3 / 1x3 / the one-warp kernel with one staged page):
-    600 keys:   16 sequences 10.5 / 14.0 / 20.6 / -,  24: 19.2 / 15.0 / 22.8 / -,  32: 21.2 / 16.1 / 24.2 / -,
-                48: 31.5 / 31.4 / 24.9 / 35.2,  64: 41.9 / 33.1 / 31.3 / 37.8,  128: 74.1 / 64.1 / 55.3 / 74.2
-    2,100 keys: 24: 46.0 / 40.0 / 67.3,  32: 48.3 / 49.0 / 70.5,  48: 71.9 / 83.8 / 73.9,  64: 95.1 / 87.2 / 96.4,
-                96: 139 / 132 / 155,  128: 182 / 174 / 169;   8,000 keys, 64: 314 / 309 / 349."""
+    leave those out (the smallest are never much faster there and often slower, below) and, past one
+    round, take the form whose last round of CTAs is fullest.  In 2x3 and 1x3 each of the warps is a pair that shares its tiles.
+    Measured (us in a row of launches; 24 heads over 8 KV heads of 128; 6x2 / 2x3 / 1x3):
+    130 keys:   16 sequences 5.2 / 5.1 / 5.9,  32: 10.8 / 7.2 / 7.5,  48: 15.5 / 12.6 / 8.6,  64: 20.1 / 13.9 / 9.8,  128: 36.8 / 26.8 / 18.9
+    530 keys:   16: 9.5 / 10.7 / 12.9,  24: 16.5 / 12.1 / 16.0,  32: 18.3 / 14.0 / 17.5,  48: 27.2 / 25.9 / 21.9,  64: 35.2 / 27.6 / 25.9,
+                96: 52.9 / 41.1 / 44.2,  128: 66.2 / 54.6 / 48.8
+    1,400 keys: 16: 17.9 / 22.3 / 30.3,  24: 33.2 / 27.0 / 36.1,  32: 34.6 / 32.2 / 39.6,  48: 52.2 / 53.9 / 52.3,  64: 69.6 / 59.6 / 63.6,
+                96: 104 / 87 / 101,  128: 127 / 116 / 114
+    2,100 keys: 24: 45.0 / 39.4 / 52.1,  32: 47.0 / 47.3 / 57.2,  48: 70.6 / 77.4 / 76.1,  64: 93.9 / 86.3 / 93.8,  96: 138 / 126 / 147,
+                128: 176 / 170 / 167
+    8,000 keys: 19: 138 / 116 / 151,  24: 147 / 141 / 186,  32: 157 / 172 / 203,  48: 236 / 275 / 277,  64: 315 / 309 / 343
+    33 to 480 keys: 24: 12.1 / 9.0 / 11.3,  48: 18.5 / 15.9 / 13.8,  64: 25.1 / 17.0 / 14.5;  300 to 1,400: 24: 22.3 / 20.1 / 26.8,  64: 47.8 / 40.8
+                / 44.3;  33 to 4,000: 32: 52.7 / 54.9 / 71.2,  64: 93.3 / 93.3 / 102.7.
+    (One warp a tile of 32 keys in 2x3: 24 equal sequences of 8,000 133, of 1,400 26.7, and 24 of 300 to 1,400 24.5.)"""
     if KNOBS.decode_warps_shape is not None:
         return tuple(KNOBS.decode_warps_shape)
     sms = sm_count or ops.sm_count()

@@ -165,8 +165,8 @@ def test_one_sequence_across_both_context_class_boundaries(real_heads, tmp_path)
 
 def test_sixty_four_sequences_across_the_first_boundary(real_heads, tmp_path):
     """64 sequences of 1,460 to 1,523 tokens decode 90 tokens each, across 1,536: 512 (sequence, KV
-    head) pairs go to one-warp CTAs with rings of three tiles up to 1,536 tokens (four CTAs an SM) and to
-    two-warp CTAs beyond.  CUDA
+    head) pairs go to CTAs of a pair of warps with rings of three tiles up to 1,536 tokens (four CTAs an SM) and to
+    CTAs of two pairs beyond.  CUDA
     graphs on, as in serving; every decoded position against the plain model."""
     from oracle_engine_b200.csrc import ops_tc
     from oracle_engine_b200.engine.engine import Engine
