@@ -712,6 +712,7 @@ bool by_bound(int top_k, int V, int slice) {
     if (top_k <= 0 || top_k >= V) return false;
     const int rest = V % slice, warps = V / slice * CW + (rest < CT ? (rest + 31) / 32 : CW);
     if (top_k > warps) return false;
+    if (16 * top_k <= 13 * warps) return true;        // 1.7 W at most
     float values = 0.f;
     for (int i = warps - top_k + 1; i <= warps; i++) values += (float)warps / (float)i;
     return values <= 320.f;
