@@ -564,19 +564,21 @@ def decode_warps_shape(n_seqs: int, context_class: int, head_dim: int, n_kv_head
     merge hide only behind another CTA of the same SM.  So: the form with the most warps whose
     CTAs are all resident at once (at head size 128 one CTA an SM for up to 148 pairs, then two,
     then four); with more pairs than that, short contexts take the smallest CTAs.  Long contexts
-    leave those out (the smallest are never much faster there and often slower, below) and, past one
+    leave those out (they are never the fastest there, below) and, past one
     round, take the form whose last round of CTAs is fullest.  In 2x3 and 1x3 each of the warps is a pair that shares its tiles.
-    Measured (us in a row of launches; 24 heads over 8 KV heads of 128; 6x2 / 2x3 / 1x3):
-    130 keys:   16 sequences 5.2 / 5.1 / 5.9,  32: 10.8 / 7.2 / 7.5,  48: 15.5 / 12.6 / 8.6,  64: 20.1 / 13.9 / 9.8,  128: 36.8 / 26.8 / 18.9
-    530 keys:   16: 9.5 / 10.7 / 12.9,  24: 16.5 / 12.1 / 16.0,  32: 18.3 / 14.0 / 17.5,  48: 27.2 / 25.9 / 21.9,  64: 35.2 / 27.6 / 25.9,
-                96: 52.9 / 41.1 / 44.2,  128: 66.2 / 54.6 / 48.8
-    1,400 keys: 16: 17.9 / 22.3 / 30.3,  24: 33.2 / 27.0 / 36.1,  32: 34.6 / 32.2 / 39.6,  48: 52.2 / 53.9 / 52.3,  64: 69.6 / 59.6 / 63.6,
-                96: 104 / 87 / 101,  128: 127 / 116 / 114
-    2,100 keys: 24: 45.0 / 39.4 / 52.1,  32: 47.0 / 47.3 / 57.2,  48: 70.6 / 77.4 / 76.1,  64: 93.9 / 86.3 / 93.8,  96: 138 / 126 / 147,
-                128: 176 / 170 / 167
-    8,000 keys: 19: 138 / 116 / 151,  24: 147 / 141 / 186,  32: 157 / 172 / 203,  48: 236 / 275 / 277,  64: 315 / 309 / 343
-    33 to 480 keys: 24: 12.1 / 9.0 / 11.3,  48: 18.5 / 15.9 / 13.8,  64: 25.1 / 17.0 / 14.5;  300 to 1,400: 24: 22.3 / 20.1 / 26.8,  64: 47.8 / 40.8
-                / 44.3;  33 to 4,000: 32: 52.7 / 54.9 / 71.2,  64: 93.3 / 93.3 / 102.7.
+    Measured inside the decode step (ms a step of the 28-layer model, 24 heads over 8 KV heads of 128; 6x2 / 2x3 / 1x3; all sequences
+    equal, then evenly spread from a few tokens to that length):
+    130 keys:   16 sequences 1.80 / 1.82 / 1.88,  24 2.28 / 2.21 / 2.26,  32 2.36 / 2.25 / 2.30,  48 2.45 / 2.34 / 2.28,  64 2.60 / 2.43 / 2.35,
+                128 3.44 / 3.14 / 2.93;  spread, 48 2.37 / 2.27 / 2.25
+    500 keys:   16 1.92 / 1.97 / 2.16,  24 2.52 / 2.38 / 2.55,  32 2.62 / 2.47 / 2.61,  48 2.79 / 2.69 / 2.65,  64 3.08 / 2.80 / 2.83,  128 4.22 /
+                3.83 / 3.74;  spread, 48 2.58 / 2.48 / 2.52, 64 2.81 / 2.60 / 2.60
+    1,400 keys: 16 2.19 / 2.32 / 2.83,  24 3.02 / 2.81 / 3.23,  32 3.10 / 3.01 / 3.27,  48 3.51 / 3.55 / 3.53,  64 4.02 / 3.75 / 3.93;  spread, 48
+                3.02 / 2.96 / 3.17, 64 3.36 / 3.15 / 3.29
+    2,100 keys: 16 2.41 / 2.58 / 3.34,  24 3.36 / 3.13 / 3.73,  32 3.45 / 3.43 / 3.79,  48 4.06 / 4.19 / 4.20,  64 4.77 / 4.49 / 4.77,  96 6.32 /
+                5.93 / 6.45;  spread, 24 2.91 / 2.94 / 3.62, 64 3.68 / 3.60 / 3.80
+    6,000 keys: 16 3.60 / 4.05 / 6.16,  24 5.24 / 4.95 / 6.58,  32 5.50 / 5.77 / 6.66,  48 7.28 / 7.94 / 7.97;  spread, 24 4.00 / 4.36 / 6.26.
+    Alone (us in a row of launches): 530 keys, 16 sequences 9.5 / 10.7 / 12.9, 32 18.3 / 14.0 / 17.5, 64 35.2 / 27.6 / 25.9;  8,000 keys, 24
+    147 / 141 / 186, 64 315 / 309 / 343.
     (One warp a tile of 32 keys in 2x3: 24 equal sequences of 8,000 133, of 1,400 26.7, and 24 of 300 to 1,400 24.5.)"""
     if KNOBS.decode_warps_shape is not None:
         return tuple(KNOBS.decode_warps_shape)
