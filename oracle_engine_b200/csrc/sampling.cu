@@ -370,6 +370,20 @@ __device__ __forceinline__ Sums cluster_sums(Sums v, Sums (*box)[CL * CW], int& 
     return t;
 }
 
+// A sum of probabilities, RUN of them at a time: pairs of pairs, then with what rounding left of the sum so far.  No further from the
+// sum in 64 bits than the passes' trees (50 values 1e-8 on average, 7e-8 at most; 320 4e-9 and 7e-8), where one value after another in 32
+// bits was up to six times further off.
+constexpr int RUN = 8;
+struct Sum {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void add(const float (&q)[RUN]) {
+        const float y = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7])) - c, t = s + y;
+        c = (t - s) - y;
+        s = t;
+    }
+    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
+};
+
 // drawn, recorded: what the slot's counters hold.
 __device__ __forceinline__ void record_token(int token, int row, int slot, int drawn, int recorded, int* out, const SampleState& st, int record) {
     out[row] = token;
@@ -388,7 +402,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
                       int repeat_last, SampleState st, int record) {
     __shared__ Sums box[2][CL * CW];
     __shared__ float2 s_seg[BOUND ? CL * CW : 1][SEG];       // of the first CTA: per warp of the cluster its (value, index) at or above the bound
-    __shared__ float2 s_few[BOUND ? FEW : 1];         // the same side by side
+    __shared__ __align__(16) float2 s_few[BOUND ? FEW : 1];  // the same side by side
     __shared__ int2 s_place[BOUND ? CL * CW : 1];     // of a warp's values in s_few: the first, how many
     __shared__ unsigned s_hit[CT];
     __shared__ int s_ids[PENALTY_CAP];
@@ -510,7 +524,7 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
     // (a sum that is no number takes the passes, which choose no token)
     if (BOUND && softmax.n[1] == 0u && softmax.n[0] <= FEW && softmax.a[0] >= 1.f) {
         if (rank != 0) return;                        // nothing is written to another CTA any more
-        const int n = (int)softmax.n[0];
+        const int n = (int)softmax.n[0], whole = (n + RUN - 1) / RUN * RUN;
         // side by side, in the warps' order
         if (warp == 0) {
             const Sums* of = box[turn ^ 1];
@@ -530,16 +544,22 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
             static_assert(CT == 4 * CL * CW, "four threads a warp's values");
             const int2 place = s_place[tid >> 2];
             for (int i = tid & 3; i < place.y; i += 4) { const float2 c = s_seg[tid >> 2][i]; s_few[place.x + i] = make_float2(c.x * inv, c.y); }
+            if (tid < RUN && n + tid < whole) s_few[n + tid] = make_float2(-1.f, 0.f);      // kept by nothing
         }
         __syncthreads();
         // kept by top-k: fewer than top_k are above it; the cut of top-p: the largest value with which the mass reaches top_p
         for (int i = tid; i < n; i += CT) {
             const float p = s_few[i].x;
             int above = 0;
-            float mass = 0.f;
-            for (int j = 0; j < n; j++) { const float q = s_few[j].x; above += q > p ? 1 : 0; mass += q >= p ? q : 0.f; }
+            Sum mass;
+            for (int j = 0; j < whole; j += RUN) {
+                float q[RUN];
+#pragma unroll
+                for (int e = 0; e < RUN; e++) { const float o = s_few[j + e].x; above += o > p ? 1 : 0; q[e] = o >= p ? o : 0.f; }
+                mass.add(q);
+            }
             if (above < top_k) {
-                if (top_p < 1.f && mass >= top_p) atomicMax(&s_cut, __float_as_uint(p));
+                if (top_p < 1.f && (float)mass.value() >= top_p) atomicMax(&s_cut, __float_as_uint(p));
                 s_few[i].y = __int_as_float(__float_as_int(s_few[i].y) | KEPT);
             }
         }
@@ -552,15 +572,20 @@ sample_cluster_kernel(float* logits, int* out, const int* row_slot, int V, float
             const float2 c = s_few[i];
             const int id = __float_as_int(c.y);
             if (!(id & KEPT) || __float_as_uint(c.x) < cut) continue;
-            float run = 0.f, total = 0.f;
-            for (int j = 0; j < n; j++) {
-                const float2 o = s_few[j];
-                const int other = __float_as_int(o.y);
-                const float q = (other & KEPT) && __float_as_uint(o.x) >= cut ? o.x : 0.f;
-                total += q;
-                run += other <= id ? q : 0.f;
+            Sum run, total;
+            for (int j = 0; j < whole; j += RUN) {
+                float q[RUN], r[RUN];
+#pragma unroll
+                for (int e = 0; e < RUN; e++) {
+                    const float2 o = s_few[j + e];
+                    const int other = __float_as_int(o.y);
+                    q[e] = (other & KEPT) && __float_as_uint(o.x) >= cut ? o.x : 0.f;
+                    r[e] = other <= id ? q[e] : 0.f;
+                }
+                total.add(q);
+                run.add(r);
             }
-            if (run > u * total) atomicMin(&s_entry, id & ~KEPT);
+            if (run.value() > (double)u * total.value()) atomicMin(&s_entry, id & ~KEPT);
             last_kept = max(last_kept, id & ~KEPT);
         }
         __syncthreads();
